@@ -380,22 +380,36 @@ PT_API int pt_qk_norm_rope_bwd(const void* dq, const void* dk, const void* qkv, 
 // QK-norm scales) and accumulates into the gradient buffer in one launch.
 // ----------------------------------------------------------------------------------------------
 namespace pt {
+// A latency problem, not a bandwidth one (G = 592 partial rows of 128..2048 columns, 0.3..5 MB, all in L2): with one thread
+// per column every thread walked a serial chain of G / 4 loads and only H / 128 blocks ran. Here a block owns 32 columns
+// and its 32 warps split the rows, eight loads in flight each, so the chain is ceil(G / 256) long.
+constexpr int COLSUM_WARPS = 32;
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(32 * COLSUM_WARPS)
 colsum_accumulate_kernel(const float* __restrict__ part, int G, int ld, int H, T* __restrict__ dst) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= H) return;
-  float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f, acc3 = 0.f;
-  int g = 0;
-  for (; g + 3 < G; g += 4) {
-    acc0 += part[(size_t)g * ld + c];
-    acc1 += part[(size_t)(g + 1) * ld + c];
-    acc2 += part[(size_t)(g + 2) * ld + c];
-    acc3 += part[(size_t)(g + 3) * ld + c];
+  __shared__ float red[COLSUM_WARPS][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
+  float acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+  if (c < H) {
+    for (int g = warp; g < G; g += 8 * COLSUM_WARPS) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = g + i * COLSUM_WARPS;
+        if (r < G) acc[i] += part[(size_t)r * ld + c];
+      }
+    }
   }
-  for (; g < G; ++g) acc0 += part[(size_t)g * ld + c];
-  const float s = (acc0 + acc1) + (acc2 + acc3);
-  dst[c] = (T)((float)dst[c] + s);
+  red[warp][lane] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+  __syncthreads();
+  // warp w finishes column w of the block: lane l brings the sum of row group l
+  float v = red[lane][warp];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int cc = blockIdx.x * 32 + warp;
+  if (lane == 0 && cc < H) dst[cc] = (T)((float)dst[cc] + v);
 }
 }  // namespace pt
 
@@ -403,8 +417,8 @@ colsum_accumulate_kernel(const float* __restrict__ part, int G, int ld, int H, T
 PT_API int pt_colsum_accumulate(const float* part, int G, int ld, int H, void* dst, int dst_fp32, void* stream_) {
   cudaStream_t st = (cudaStream_t)stream_;
   if (G <= 0 || H <= 0) return 0;
-  int grid = (H + 127) / 128;
-  if (dst_fp32) pt::colsum_accumulate_kernel<float><<<grid, 128, 0, st>>>(part, G, ld, H, (float*)dst);
-  else pt::colsum_accumulate_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(part, G, ld, H, (__nv_bfloat16*)dst);
+  const int grid = (H + 31) / 32, threads = 32 * pt::COLSUM_WARPS;
+  if (dst_fp32) pt::colsum_accumulate_kernel<float><<<grid, threads, 0, st>>>(part, G, ld, H, (float*)dst);
+  else pt::colsum_accumulate_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(part, G, ld, H, (__nv_bfloat16*)dst);
   return (int)cudaGetLastError();
 }
