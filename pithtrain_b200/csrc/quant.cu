@@ -98,12 +98,16 @@ quant_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const int*
   }
 }
 
-// One CTA (256 threads) per 128x128 tile of W[g]; writes the tile in both orientations.
+// One CTA (256 threads) per 128x128 tile of W[g]; writes the tile in both orientations. Bound by memory: 2 bytes in, 2
+// out per weight. The transposed copy goes through shared memory as 32-bit words of four k: a thread collects the words
+// of 16 rows for one k quad, turns them into four 16-byte pieces of W^T with byte permutes and stores those, eight
+// neighbouring threads to a full 128-byte line. Word c of row r lies at column (c + 4 * (r / 16)) mod 32, so that the 8 row
+// groups x 4 quads a warp reads at once fall into 32 different banks.
 __global__ void __launch_bounds__(256)
 quant_block_kernel(const __nv_bfloat16* __restrict__ w, int N, int K, uint8_t* __restrict__ q,
                    uint8_t* __restrict__ qt, float* __restrict__ s, float* __restrict__ st) {
   __shared__ float red[8];
-  __shared__ __align__(16) uint8_t tile[128][128 + 16];
+  __shared__ __align__(16) uint32_t tile[128][32];
   const int g = blockIdx.z, nb = blockIdx.y, kb = blockIdx.x;
   const int nblocks = gridDim.y, kblocks = gridDim.x;
   const __nv_bfloat16* wg = w + (long long)g * N * K;
@@ -151,7 +155,7 @@ quant_block_kernel(const __nv_bfloat16* __restrict__ w, int N, int K, uint8_t* _
     out.x = cvt_e4m3x4(v[p][0] * rcp, v[p][1] * rcp, v[p][2] * rcp, v[p][3] * rcp);
     out.y = cvt_e4m3x4(v[p][4] * rcp, v[p][5] * rcp, v[p][6] * rcp, v[p][7] * rcp);
     const int r = p * 16 + tr;
-    *reinterpret_cast<uint2*>(&tile[r][tc]) = out;
+    *reinterpret_cast<uint2*>(&tile[r][((tc >> 2) + 4 * p) & 31]) = out;
     const int n = nb * 128 + r, k = kb * 128 + tc;
     if (n < N && k < K) {
       uint8_t* dst = q + ((long long)g * N + n) * K + k;
@@ -165,20 +169,33 @@ quant_block_kernel(const __nv_bfloat16* __restrict__ w, int N, int K, uint8_t* _
   }
   if (!qt) return;
   __syncthreads();
-  // transposed orientation: thread (tr, tc) writes 8 consecutive n for one k
+  // transposed orientation: rows 16 ng .. 16 ng + 15 (n) of k quad kq
+  const int ng = threadIdx.x & 7, kq = threadIdx.x >> 3;
+  uint32_t o[4][4];
 #pragma unroll
-  for (int p = 0; p < 8; ++p) {
-    const int kk = p * 16 + tr;  // k within the tile
-    const int k = kb * 128 + kk, n = nb * 128 + tc;
+  for (int q4 = 0; q4 < 4; ++q4) {
+    uint32_t a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = tile[16 * ng + 4 * q4 + i][(kq + 4 * ng) & 31];
+    const uint32_t lo01 = __byte_perm(a[0], a[1], 0x5140), hi01 = __byte_perm(a[0], a[1], 0x7362);
+    const uint32_t lo23 = __byte_perm(a[2], a[3], 0x5140), hi23 = __byte_perm(a[2], a[3], 0x7362);
+    o[0][q4] = __byte_perm(lo01, lo23, 0x5410);
+    o[1][q4] = __byte_perm(lo01, lo23, 0x7632);
+    o[2][q4] = __byte_perm(hi01, hi23, 0x5410);
+    o[3][q4] = __byte_perm(hi01, hi23, 0x7632);
+  }
+  const int n = nb * 128 + 16 * ng;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int k = kb * 128 + 4 * kq + j;
     if (k < K && n < N) {
-      __align__(8) uint8_t b[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) b[i] = tile[tc + i][kk];
       uint8_t* dst = qt + ((long long)g * K + k) * N + n;
-      if (n + 8 <= N && ((reinterpret_cast<uintptr_t>(dst) & 7) == 0)) {
-        *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(b);
+      if (n + 16 <= N && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(o[j][0], o[j][1], o[j][2], o[j][3]);
       } else {
-        for (int i = 0; i < 8 && n + i < N; ++i) dst[i] = b[i];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (n + i < N) dst[i] = (uint8_t)(o[j][i >> 2] >> (8 * (i & 3)));
       }
     }
   }

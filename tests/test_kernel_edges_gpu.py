@@ -22,3 +22,17 @@ def test_colsum_accumulate(G, ld, H, dtype):
     # the bf16 result is rounded once more
     bound = G * 5 * 2.0 ** -24 * 24 + (want.abs() * 2.0 ** -8 if dtype == torch.bfloat16 else 0)
     assert ((dst.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("G,R,K", [(1, 8, 16), (2, 128, 128), (1, 130, 264), (3, 24, 136), (2, 272, 40), (1, 2880, 144)])
+def test_quant_blocks_both_orientations(G, R, K):
+    """Bytes and scales equal the plain tensor-op recipe, ragged edge tiles and unaligned pitches of W^T included."""
+    from pithtrain_b200.ops.quant import quant_blocks, quant_blocks_ref
+
+    torch.manual_seed(R)
+    w = (torch.randn(G, R, K, device="cuda") * 0.02).bfloat16()
+    q, s, qt, st = quant_blocks(w)
+    q0, s0 = quant_blocks_ref(w)
+    assert torch.equal(q.view(torch.uint8), q0.view(torch.uint8)) and torch.equal(s, s0)
+    assert torch.equal(qt.view(torch.uint8), q0.transpose(1, 2).contiguous().view(torch.uint8))
+    assert torch.equal(st, s0.transpose(1, 2).contiguous())
