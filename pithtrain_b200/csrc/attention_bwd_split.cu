@@ -1,0 +1,553 @@
+// Attention backward that keeps P and dS at fp32 accuracy, for sm_100a (tcgen05 / TMEM / TMA): head dims 64, 128, 192/128
+// (MLA) and 256, any sequence length, with the masks of the forward kernel. It covers what csrc/attention_bwd.cu does
+// not (wider heads, lengths that are no multiple of 4), where gradients come from unrounded probabilities:
+//   P = hi + lo and dS = hi + lo as two bf16 numbers each (16 mantissa bits and more; error 2^-17 of the value), so every
+//   product with them is two MMAs into the same fp32 accumulator. S and dP need no split: their operands are bf16.
+//
+// What bounds the shapes is on-chip memory: at head dim 256 a 128-row dK and dV tile alone fill the 512 TMEM columns, and
+// two stationary plus two streamed 128-row tiles do not fit in shared memory. Hence one accumulator per launch and
+// 64-row streamed tiles, one kernel with three uses (X stationary, 128 rows; Y streamed, 64 rows):
+//   DV : X1 = K           Y1 = Q, Y2 = dO    dV += P^T dO
+//   DK : X1 = K, X2 = V   Y1 = Q, Y2 = dO    dK += dS^T Q
+//   DQ : X1 = Q, X2 = dO  Y1 = K, Y2 = V     dQ += dS K
+//     S = X1 Y1^T, dP = X2 Y2^T -> TMEM (two buffers of 64 columns each); P = exp2(S c - lse2), dS = P o (dP - delta);
+//     hi / lo go back over S's own columns in TMEM and are the A operand of the accumulating MMA (B = Y1 or Y2 read
+//     MN-major). S and dP of step n+1 are issued before the accumulation of step n, so they run under its exponentials.
+// Recomputing S twice and dP once costs 11 products of the tile instead of 5, all on the tensor core; the tensor-op
+// backward it replaces ran fp32 SIMT products over [heads, S, S] matrices in memory. Measured, causal, DQ + DK + DV:
+//   1 x 2048, 16 heads x 192/128    :  80 +  74 +  53 us  (tensor ops: about 3 ms)
+//   1 x 3072, 16/2 heads x 256      : 200 + 202 + 156 us  (tensor ops: about 9 ms)
+//   1 x 4093 in 9 documents, 32/4 heads x 128, with forward and the passes around it: 0.64 ms (tensor ops: 21 ms)
+//
+// No atomics: dQ rows belong to one CTA; dK / dV of a query head are written once, directly when there is no GQA group,
+// else to per-head fp32 partials that attn_split_group_sum_kernel adds in head order. Results are reproducible.
+// Every wait is bounded; on a timeout the roles leave their loops and the status word carries the code.
+#include "host_common.h"
+#include "ptx.cuh"
+
+namespace pt {
+
+enum : int { ASP_DV = 0, ASP_DK = 1, ASP_DQ = 2 };
+constexpr int ASP_XSLAB = 128 * 64 * 2;  // [128 x 64] bf16 swizzle slab
+constexpr int ASP_YSLAB = 64 * 64 * 2;   // [64 x 64]
+
+struct AttnSplitArgs {
+  int B, Sq, Sk, Hq, Hkv;
+  int Sp;                // row pitch of lse2 / delta: Sq rounded up to 4 (their tiles move in 16-byte pieces)
+  int causal, q_off;
+  float scale_log2, out_scale;
+  const int* row_lo;     // optional [B*Sq]
+  const float* lse2;     // [B, Hq, Sp] log2-domain log-sum-exp (+inf for rows that saw no key)
+  const float* delta;    // [B, Hq, Sp]
+  __nv_bfloat16* out;    // bf16 result (DQ: [B*Sq, Hq*D1]; DK / DV without a group: [B*Sk, Hkv*DA]), or
+  float* part;           // fp32 partials [B*Sk, Hq, DA] (DK / DV with a group)
+  int* err;
+};
+
+template <int D1, int D2, int MODE>
+struct AttnSplitCfg {
+  static constexpr bool HAS_DP = MODE != ASP_DV;
+  static constexpr int DA = MODE == ASP_DV ? D2 : D1;     // columns of the accumulator
+  static constexpr int X1_BYTES = (D1 / 64) * ASP_XSLAB, X2_BYTES = HAS_DP ? (D2 / 64) * ASP_XSLAB : 0;
+  static constexpr int Y1_BYTES = (D1 / 64) * ASP_YSLAB, Y2_BYTES = (D2 / 64) * ASP_YSLAB;
+  // stages of the streamed tiles: at head dim 256 with dP (128 KB stationary) only one of Y2 fits, which is enough: its
+  // only reader is the dP product, issued a step ahead
+  static constexpr int NST1 = 2, NST2 = (HAS_DP && D1 + D2 > 320) ? 1 : 2;
+  static constexpr int STAT_BYTES = NST1 * 512;           // lse2[64] | delta[64] per Y1 stage (DV, DK)
+  static constexpr int BAR_BYTES = 256;
+  static constexpr int SMEM = X1_BYTES + X2_BYTES + NST1 * Y1_BYTES + NST2 * Y2_BYTES + STAT_BYTES + BAR_BYTES;
+  static_assert(SMEM <= 227 * 1024, "shared memory");
+  static_assert(256 + DA <= 512, "TMEM columns");
+  static constexpr int THREADS = 12 * 32;
+};
+
+template <int D1, int D2, int MODE>
+__global__ void __launch_bounds__(384, 1)
+attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
+                      const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2, const AttnSplitArgs args) {
+  using Cfg = AttnSplitCfg<D1, D2, MODE>;
+  constexpr bool HAS_DP = Cfg::HAS_DP;
+  constexpr int DA = Cfg::DA, NST1 = Cfg::NST1, NST2 = Cfg::NST2;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  if ((smem_u32(smem) & 1023u) != 0) {  // uniform over the CTA
+    if (threadIdx.x == 0 && args.err) atomicCAS(args.err, 0, PT_ERR_SMEM_ALIGN);
+    return;
+  }
+  uint8_t* sX1 = smem;
+  uint8_t* sX2 = sX1 + Cfg::X1_BYTES;
+  uint8_t* sY1 = sX2 + Cfg::X2_BYTES;
+  uint8_t* sY2 = sY1 + NST1 * Cfg::Y1_BYTES;
+  uint8_t* sStat = sY2 + NST2 * Cfg::Y2_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + Cfg::STAT_BYTES);
+  uint64_t* x_full = bars;          // 1
+  uint64_t* y1_full = bars + 1;     // NST1
+  uint64_t* y1_empty = bars + 3;    // NST1
+  uint64_t* y2_full = bars + 5;     // NST2
+  uint64_t* y2_empty = bars + 7;    // NST2
+  uint64_t* s_full = bars + 9;      // 2: S (and dP) of a step are in TMEM
+  uint64_t* a_ready = bars + 11;    // 2: compute (8 warps) -> MMA: hi / lo are in TMEM, dP has been read
+  uint64_t* acc_done = bars + 13;   // 1
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 14);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int hq = blockIdx.x % args.Hq, b = blockIdx.x / args.Hq;
+  const int hk = hq / (args.Hq / args.Hkv);
+  // the tiles with the most work under a causal mask start first: the first key tiles, the last query tiles
+  const int tile = MODE == ASP_DQ ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
+  const int row_base = b * args.Sq, kv_base = b * args.Sk;
+  const int x0 = tile * 128;                                   // first row of the stationary tile within the batch entry
+  const int x_len = MODE == ASP_DQ ? args.Sq : args.Sk, x_base = MODE == ASP_DQ ? row_base : kv_base;
+  const int hx = MODE == ASP_DQ ? hq : hk, hy = MODE == ASP_DQ ? hk : hq;
+
+  // streamed tiles [t_lo, t_lo + N) that share a visible (query, key) pair with the stationary tile
+  int t_lo = 0, t_hi;
+  if (MODE == ASP_DQ) {
+    const int lo = args.row_lo ? max(args.row_lo[row_base + x0], 0) : 0;  // non-decreasing in the row
+    const int hi = args.causal ? min(args.Sk - 1, args.q_off + min(x0 + 127, args.Sq - 1)) : args.Sk - 1;
+    t_lo = lo / 64;
+    t_hi = hi >= lo ? hi / 64 : t_lo - 1;
+  } else {
+    const int k_last = min(x0 + 127, args.Sk - 1);
+    t_hi = (args.Sq + 63) / 64 - 1;
+    if (args.causal) {
+      const int need = x0 - args.q_off - 63;  // last row of tile i: q_off + 64 i + 63 >= x0
+      t_lo = need > 0 ? (need + 63) / 64 : 0;
+    }
+    if (args.row_lo && t_lo <= t_hi) {
+      // largest i with row_lo[first row of tile i] <= k_last
+      int a = t_lo, z = t_hi;
+      if (args.row_lo[row_base + a * 64] > k_last) {
+        t_hi = t_lo - 1;
+      } else {
+        while (a < z) {
+          const int mid = (a + z + 1) >> 1;
+          if (args.row_lo[row_base + mid * 64] <= k_last) a = mid; else z = mid - 1;
+        }
+        t_hi = a;
+      }
+    }
+  }
+  const int N = t_hi - t_lo + 1;
+
+  // where a row of the result goes: bf16, or the fp32 partial of this query head
+  const bool grouped = MODE != ASP_DQ && args.Hq != args.Hkv;
+  const long long out_row0 = (long long)(x_base + x0);
+  if (N <= 0) {  // uniform over the CTA: nothing visible, the gradient is zero
+    for (int i = threadIdx.x; i < 128 * (DA / 8); i += Cfg::THREADS) {
+      const int r = i / (DA / 8), c = (i % (DA / 8)) * 8;
+      if (x0 + r < x_len) {
+        if (grouped) {
+          float4* p = reinterpret_cast<float4*>(args.part + ((out_row0 + r) * args.Hq + hq) * DA + c);
+          p[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+          p[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+          const int H = MODE == ASP_DQ ? args.Hq : args.Hkv;
+          *reinterpret_cast<uint4*>(args.out + ((out_row0 + r) * H + hx) * DA + c) = make_uint4(0u, 0u, 0u, 0u);
+        }
+      }
+    }
+    return;
+  }
+
+  if (threadIdx.x == 0) {
+    mbar_init(x_full, 1);
+    for (int s = 0; s < NST1; ++s) { mbar_init(&y1_full[s], 1); mbar_init(&y1_empty[s], 1); }
+    for (int s = 0; s < NST2; ++s) { mbar_init(&y2_full[s], 1); mbar_init(&y2_empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&a_ready[s], 8); }
+    mbar_init(acc_done, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmX1); tma_prefetch_desc(&tmY1); tma_prefetch_desc(&tmY2);
+    if (HAS_DP) tma_prefetch_desc(&tmX2);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_ptr, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tACC = tmem_base + 256;  // S: columns 0..127 (two buffers), dP: 128..255
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- producer
+    if (lane == 0) {
+      mbar_expect_tx(x_full, Cfg::X1_BYTES + Cfg::X2_BYTES);
+#pragma unroll
+      for (int db = 0; db < D1 / 64; ++db) tma_load_3d(sX1 + db * ASP_XSLAB, &tmX1, x_full, hx * D1 + 64 * db, x0, b);
+      if (HAS_DP) {
+#pragma unroll
+        for (int db = 0; db < D2 / 64; ++db) tma_load_3d(sX2 + db * ASP_XSLAB, &tmX2, x_full, hx * D2 + 64 * db, x0, b);
+      }
+      bool ok = true;
+      int n1 = 0, n2 = 0;
+      for (int n = 0; n < N && ok; ++n) {
+        const int s1 = n % NST1, s2 = n % NST2;
+        const int y0 = (t_lo + n) * 64;
+        ok = mbar_wait_bounded(&y1_empty[s1], ((n / NST1) & 1) ^ 1, abort_flag, args.err, PT_ERR_TIMEOUT_PRODUCER);
+        if (!ok) break;
+        mbar_expect_tx(&y1_full[s1], Cfg::Y1_BYTES + (MODE == ASP_DQ ? 0 : (MODE == ASP_DK ? 512 : 256)));
+#pragma unroll
+        for (int db = 0; db < D1 / 64; ++db)
+          tma_load_3d(sY1 + s1 * Cfg::Y1_BYTES + db * ASP_YSLAB, &tmY1, &y1_full[s1], hy * D1 + 64 * db, y0, b);
+        if (MODE != ASP_DQ) {
+          const long long so = ((long long)b * args.Hq + hq) * args.Sp + y0;
+          bulk_load_1d(sStat + s1 * 512, args.lse2 + so, 256, &y1_full[s1]);
+          if (MODE == ASP_DK) bulk_load_1d(sStat + s1 * 512 + 256, args.delta + so, 256, &y1_full[s1]);
+        }
+        ++n1;
+        ok = mbar_wait_bounded(&y2_empty[s2], ((n / NST2) & 1) ^ 1, abort_flag, args.err, PT_ERR_TIMEOUT_PRODUCER);
+        if (!ok) break;
+        mbar_expect_tx(&y2_full[s2], Cfg::Y2_BYTES);
+#pragma unroll
+        for (int db = 0; db < D2 / 64; ++db)
+          tma_load_3d(sY2 + s2 * Cfg::Y2_BYTES + db * ASP_YSLAB, &tmY2, &y2_full[s2], hy * D2 + 64 * db, y0, b);
+        ++n2;
+      }
+      if (*abort_flag) {
+        // let copies in flight land before the CTA retires (bounded)
+        const uint64_t t0 = globaltimer_ns();
+        bool drained = false;
+        while (!drained && globaltimer_ns() - t0 < 20000000ull) {
+          drained = mbar_try_wait(x_full, 0);
+          for (int i = 0; i < 2 && drained; ++i) {
+            const int c1 = n1 - 1 - i, c2 = n2 - 1 - i;
+            if (c1 >= 0 && i < NST1) drained = drained && mbar_try_wait(&y1_full[c1 % NST1], (c1 / NST1) & 1);
+            if (c2 >= 0 && i < NST2) drained = drained && mbar_try_wait(&y2_full[c2 % NST2], (c2 / NST2) & 1);
+          }
+        }
+        if (!drained && args.err) atomicCAS(args.err, 0, PT_ERR_TIMEOUT_DRAIN);
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- MMA issuer (its MMAs execute in order)
+    if (lane == 0) {
+      constexpr uint32_t IDESC_S = make_idesc(1, 1, 128, 64, false, false);   // both operands K-major
+      constexpr uint32_t IDESC_A = make_idesc(1, 1, 128, DA, false, true);    // A in TMEM, B MN-major
+      constexpr uint32_t HI = smem_desc_hi_sw128(1024);
+      const uint32_t x1 = smem_desc_lo(smem_u32(sX1), 16), x2 = smem_desc_lo(smem_u32(sX2), 16);
+      const uint32_t y1k = smem_desc_lo(smem_u32(sY1), 16), y2k = smem_desc_lo(smem_u32(sY2), 16);
+      const uint32_t ym = MODE == ASP_DV ? smem_desc_lo(smem_u32(sY2), ASP_YSLAB) : smem_desc_lo(smem_u32(sY1), ASP_YSLAB);
+      // S(n) and dP(n). Buffer n & 1 was last read by the accumulation of step n-2 (issued earlier by this thread) and its dP
+      // half by the compute warps of step n-2 (their arrival was awaited before that accumulation).
+      auto scores = [&](int n) -> bool {
+        const int s1 = n % NST1, s2 = n % NST2;
+        if (!mbar_wait_bounded(&y1_full[s1], (n / NST1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_MMA)) return false;
+        tc_fence_after();
+        const uint32_t d = tmem_base + (n & 1) * 64, yb = y1k + s1 * (Cfg::Y1_BYTES >> 4);
+#pragma unroll
+        for (int db = 0; db < D1 / 64; ++db)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            umma_f16_lh(d, x1 + ((db * ASP_XSLAB + k * 32) >> 4), HI, yb + ((db * ASP_YSLAB + k * 32) >> 4), HI, IDESC_S,
+                        (db | k) != 0 ? 1u : 0u);
+        if (HAS_DP) {
+          if (!mbar_wait_bounded(&y2_full[s2], (n / NST2) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_MMA)) return false;
+          tc_fence_after();
+          const uint32_t yc = y2k + s2 * (Cfg::Y2_BYTES >> 4);
+#pragma unroll
+          for (int db = 0; db < D2 / 64; ++db)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              umma_f16_lh(d + 128, x2 + ((db * ASP_XSLAB + k * 32) >> 4), HI, yc + ((db * ASP_YSLAB + k * 32) >> 4), HI, IDESC_S,
+                          (db | k) != 0 ? 1u : 0u);
+          umma_commit(&y2_empty[s2]);
+        }
+        umma_commit(&s_full[n & 1]);
+        return true;
+      };
+      bool ok = mbar_wait_bounded(x_full, 0, abort_flag, args.err, PT_ERR_TIMEOUT_MMA);
+      if (ok) ok = scores(0);
+      for (int n = 0; n < N && ok; ++n) {
+        if (n + 1 < N) ok = scores(n + 1);
+        if (!ok) break;
+        const int s1 = n % NST1, s2 = n % NST2;
+        if (MODE == ASP_DV) ok = mbar_wait_bounded(&y2_full[s2], (n / NST2) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_MMA);
+        if (ok) ok = mbar_wait_bounded(&a_ready[n & 1], (n >> 1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_MMA);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t yb = ym + (MODE == ASP_DV ? s2 * (Cfg::Y2_BYTES >> 4) : s1 * (Cfg::Y1_BYTES >> 4));
+        // columns of the buffer, per half h of 32 streamed rows: hi 16 columns at 32 h, lo 16 columns at 32 h + 16
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t a = tmem_base + (n & 1) * 64 + (k >> 1) * 32 + (k & 1) * 8;
+          umma_f16_ts_lh(tACC, a, yb + ((k * 2048) >> 4), HI, IDESC_A, (k != 0 || n != 0) ? 1u : 0u);
+          umma_f16_ts_lh(tACC, a + 16, yb + ((k * 2048) >> 4), HI, IDESC_A, 1u);
+        }
+        umma_commit(&y1_empty[s1]);
+        if (MODE == ASP_DV) umma_commit(&y2_empty[s2]);
+      }
+      if (ok) umma_commit(acc_done);
+    }
+  } else if (warp >= 4) {
+    // ---------------------------------------------------------------- compute: thread = stationary row, 32 streamed rows
+    const int g = (warp - 4) >> 2;            // half of the streamed rows
+    const int qd = warp & 3;                  // TMEM lane quarter
+    const int r = qd * 32 + lane;
+    const int xr = x0 + r;                    // my row within the batch entry: a query (DQ) or a key (DK, DV)
+    const bool x_valid = xr < x_len;
+    const uint32_t lane_off = static_cast<uint32_t>(qd * 32) << 16;
+    float my_lse = INFINITY, my_delta = 0.f;
+    // The streamed rows that form visible pairs with my row are a range [my_lo, my_hi]: keys of a query (DQ); queries of a
+    // key (DK, DV), because the lower key bounds do not decrease with the query row.
+    int my_lo = 0, my_hi = -1;
+    if (MODE == ASP_DQ && x_valid) {
+      const long long so = ((long long)b * args.Hq + hq) * args.Sp + xr;
+      my_lse = args.lse2[so];
+      my_delta = args.delta[so];
+      my_lo = args.row_lo ? args.row_lo[row_base + xr] : 0;
+      my_hi = args.causal ? min(args.Sk - 1, args.q_off + xr) : args.Sk - 1;
+    }
+    if (MODE != ASP_DQ && x_valid) {
+      my_lo = args.causal ? xr - args.q_off : 0;
+      my_hi = args.Sq - 1;
+      if (args.row_lo) {
+        int c = -1, z = my_hi;  // largest c with row_lo[c] <= xr
+        while (c < z) {
+          const int mid = (c + z + 1) >> 1;
+          if (args.row_lo[row_base + mid] <= xr) c = mid; else z = mid - 1;
+        }
+        my_hi = c;
+      }
+    }
+    bool ok = true;
+    for (int n = 0; n < N; ++n) {
+      const int y0 = (t_lo + n) * 64 + g * 32;
+      int good = 1;
+      if (lane == 0) {
+        good = mbar_wait_bounded(&s_full[n & 1], (n >> 1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE) ? 1 : 0;
+        // the statistics came with Y1, which the S product has already read: complete, but this thread has to observe it
+        if (MODE != ASP_DQ && good)
+          good = mbar_wait_bounded(&y1_full[n % NST1], (n / NST1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE) ? 1 : 0;
+      }
+      good = __shfl_sync(0xffffffffu, good, 0);
+      if (!good) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t tS = tmem_base + lane_off + (n & 1) * 64 + g * 32;
+      uint32_t sv[32], dp[32];
+      tmem_ld_32x32(tS, sv);
+      if (HAS_DP) tmem_ld_32x32(tS + 128, dp);
+      tmem_ld_wait();
+      // element masks only where a lane needs them (warp-uniform: the stores below are collective)
+      const bool masked = __any_sync(0xffffffffu, y0 < my_lo || y0 + 31 > my_hi);
+      const float* st = reinterpret_cast<const float*>(sStat + (n % NST1) * 512) + g * 32;
+      uint32_t hi[16], lo[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        float v[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int c = 2 * i + e;
+          const float l2 = MODE == ASP_DQ ? my_lse : st[c];
+          float p = ex2_approx(fmaf(__uint_as_float(sv[c]), args.scale_log2, -l2));
+          if (HAS_DP) p *= __uint_as_float(dp[c]) - (MODE == ASP_DQ ? my_delta : st[64 + c]);
+          if (masked) p = (y0 + c >= my_lo && y0 + c <= my_hi) ? p : 0.f;
+          v[e] = p;
+        }
+        hi[i] = pack_bf16x2(v[0], v[1]);
+        const float2 h = unpack_bf16x2(hi[i]);
+        lo[i] = pack_bf16x2(v[0] - h.x, v[1] - h.y);
+      }
+      tmem_st_32x16(tS, hi);
+      tmem_st_32x16(tS + 16, lo);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&a_ready[n & 1]);
+    }
+    if (ok) {
+      int good = 1;
+      if (lane == 0) good = mbar_wait_bounded(acc_done, 0, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE) ? 1 : 0;
+      good = __shfl_sync(0xffffffffu, good, 0);
+      if (good) {
+        tc_fence_after();
+        const int H = MODE == ASP_DQ ? args.Hq : args.Hkv;
+        __nv_bfloat16* orow = args.out + ((out_row0 + r) * H + hx) * DA;
+        float* prow = args.part + ((out_row0 + r) * args.Hq + hq) * DA;
+#pragma unroll 1
+        for (int c = g * 32; c < DA; c += 64) {
+          uint32_t v[32];
+          tmem_ld_32x32(tACC + lane_off + c, v);
+          tmem_ld_wait();
+          if (x_valid) {
+            if (grouped) {
+#pragma unroll
+              for (int u = 0; u < 8; ++u)
+                *reinterpret_cast<uint4*>(prow + c + 4 * u) = make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+            } else {
+              const float sc = args.out_scale;
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                uint4 w;
+                w.x = pack_bf16x2(__uint_as_float(v[8 * u + 0]) * sc, __uint_as_float(v[8 * u + 1]) * sc);
+                w.y = pack_bf16x2(__uint_as_float(v[8 * u + 2]) * sc, __uint_as_float(v[8 * u + 3]) * sc);
+                w.z = pack_bf16x2(__uint_as_float(v[8 * u + 4]) * sc, __uint_as_float(v[8 * u + 5]) * sc);
+                w.w = pack_bf16x2(__uint_as_float(v[8 * u + 6]) * sc, __uint_as_float(v[8 * u + 7]) * sc);
+                *reinterpret_cast<uint4*>(orow + c + 8 * u) = w;
+              }
+            }
+          }
+        }
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// delta = rowsum(dO * O), lse2 = lse * log2(e) (+inf where lse is -inf), both with row pitch Sp; the pad rows get zeros.
+// One thread per 8 elements of a (row, head); D is the value head dim.
+template <int D>
+__global__ void attn_split_pre_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
+                                      const float* __restrict__ lse, float* __restrict__ delta, float* __restrict__ lse2,
+                                      int B, int Sq, int Sp, int Hq, long long ldo, long long lddo) {
+  constexpr int TPR = D / 8;  // threads per (row, head): 8, 16 or 32
+  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long pair = gid / TPR;
+  const int part = static_cast<int>(gid % TPR);
+  const long long total = (long long)B * Sp * Hq;
+  const long long row = pair / Hq;
+  const int h = static_cast<int>(pair % Hq);
+  const long long bb = row / Sp, r = row % Sp;
+  const bool live = pair < total && r < Sq;
+  float acc = 0.f;
+  if (live) {
+    const long long t = bb * Sq + r;
+    const uint4 a = *reinterpret_cast<const uint4*>(out + t * ldo + h * D + part * 8);
+    const uint4 c = *reinterpret_cast<const uint4*>(dout + t * lddo + h * D + part * 8);
+    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, cw[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = unpack_bf16x2(aw[i]), y = unpack_bf16x2(cw[i]);
+      acc = fmaf(x.x, y.x, acc);
+      acc = fmaf(x.y, y.y, acc);
+    }
+  }
+#pragma unroll
+  for (int o = TPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (pair < total && part == 0) {
+    const long long idx = (bb * Hq + h) * Sp + r;
+    delta[idx] = acc;
+    const float l = live ? lse[(bb * Hq + h) * Sq + r] : 0.f;
+    lse2[idx] = (l == -INFINITY) ? INFINITY : l * 1.4426950408889634f;
+  }
+}
+
+// out[row, hk, c] = bf16(scale * sum over the group's query heads, in head order, of part[row, hk * group + i, c]).
+__global__ void attn_split_group_sum_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, long long n8,
+                                            int group, int D, float scale) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // 8 columns of one (row, kv head)
+  if (i >= n8) return;
+  const int d8 = D / 8;
+  const long long rh = i / d8;
+  const int c = static_cast<int>(i % d8) * 8;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int x = 0; x < group; ++x) {
+    const float4* p = reinterpret_cast<const float4*>(part + (rh * group + x) * D + c);
+    const float4 a = p[0], e = p[1];
+    acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+    acc[4] += e.x; acc[5] += e.y; acc[6] += e.z; acc[7] += e.w;
+  }
+  uint4 w;
+  w.x = pack_bf16x2(acc[0] * scale, acc[1] * scale);
+  w.y = pack_bf16x2(acc[2] * scale, acc[3] * scale);
+  w.z = pack_bf16x2(acc[4] * scale, acc[5] * scale);
+  w.w = pack_bf16x2(acc[6] * scale, acc[7] * scale);
+  *reinterpret_cast<uint4*>(out + i * 8) = w;
+}
+
+}  // namespace pt
+
+namespace {
+using namespace pt;
+
+struct SplitTensors {
+  const void *q, *k, *v, *dout;
+  long long ldq, ldk, ldv, lddo;
+};
+
+template <int D1, int D2, int MODE>
+int attn_split_launch(const SplitTensors& t, const AttnSplitArgs& a, cudaStream_t stream) {
+  using Cfg = AttnSplitCfg<D1, D2, MODE>;
+  constexpr bool DQ = MODE == ASP_DQ;
+  // [B, S, cols] maps: rows past the end of a batch entry read zeros, never the next entry's rows (0 x inf is not 0)
+  const uint64_t B = a.B, Sq = a.Sq, Sk = a.Sk;
+  CUtensorMap q, k, v, g;  // queries, keys, values, output gradients: 128 stationary or 64 streamed rows
+  if (encode_tmap_3d(&q, t.q, TM_BF16, B, Sq, (uint64_t)a.Hq * D1, t.ldq, Sq * t.ldq, 1, DQ ? 128 : 64, 64, TM_SW_128)) return -3;
+  if (encode_tmap_3d(&g, t.dout, TM_BF16, B, Sq, (uint64_t)a.Hq * D2, t.lddo, Sq * t.lddo, 1, DQ ? 128 : 64, 64, TM_SW_128)) return -3;
+  if (encode_tmap_3d(&k, t.k, TM_BF16, B, Sk, (uint64_t)a.Hkv * D1, t.ldk, Sk * t.ldk, 1, DQ ? 64 : 128, 64, TM_SW_128)) return -3;
+  if (encode_tmap_3d(&v, t.v, TM_BF16, B, Sk, (uint64_t)a.Hkv * D2, t.ldv, Sk * t.ldv, 1, DQ ? 64 : 128, 64, TM_SW_128)) return -3;
+  if (cudaFuncSetAttribute(attn_bwd_split_kernel<D1, D2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
+    return -4;
+  dim3 grid(a.Hq * a.B, ((DQ ? a.Sq : a.Sk) + 127) / 128);
+  if (DQ) attn_bwd_split_kernel<D1, D2, MODE><<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(q, g, k, v, a);
+  else attn_bwd_split_kernel<D1, D2, MODE><<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(k, v, q, g, a);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+template <int D1, int D2>
+int attn_split_all(const SplitTensors& t, AttnSplitArgs a, const void* out, const void* lse, float* delta, float* lse2, float* part,
+                   void* dq, void* dk, void* dv, long long ldo, float scale, cudaStream_t stream) {
+  const long long threads = (long long)a.B * a.Sp * a.Hq * (D2 / 8);
+  attn_split_pre_kernel<D2><<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(
+      static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(t.dout), static_cast<const float*>(lse), delta, lse2,
+      a.B, a.Sq, a.Sp, a.Hq, ldo, t.lddo);
+  a.lse2 = lse2;
+  a.delta = delta;
+  a.part = nullptr;
+  a.out = static_cast<__nv_bfloat16*>(dq);
+  a.out_scale = scale;
+  int rc = attn_split_launch<D1, D2, ASP_DQ>(t, a, stream);
+  if (rc) return rc;
+  const int group = a.Hq / a.Hkv;
+  for (int w = 0; w < 2; ++w) {  // the partials of dK are summed before dV's overwrite them
+    void* dst = w == 0 ? dk : dv;
+    const int D = w == 0 ? D1 : D2;
+    a.out = static_cast<__nv_bfloat16*>(dst);
+    a.part = part;
+    a.out_scale = w == 0 ? scale : 1.f;
+    rc = w == 0 ? attn_split_launch<D1, D2, ASP_DK>(t, a, stream) : attn_split_launch<D1, D2, ASP_DV>(t, a, stream);
+    if (rc) return rc;
+    if (group > 1) {
+      const long long n8 = (long long)a.B * a.Sk * a.Hkv * (D / 8);
+      attn_split_group_sum_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(part, static_cast<__nv_bfloat16*>(dst), n8, group, D,
+                                                                                   a.out_scale);
+    }
+  }
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+}  // namespace
+
+// Gradients of pt_attn_fwd for (dqk, dv) in {(64,64), (128,128), (192,128), (256,256)} and any Sq, Sk. q, k, v, out, dout: bf16
+// token-major with row pitches (elements, multiples of 8, 16-byte aligned bases); lse [B,Hq,Sq] fp32 from the forward.
+// delta, lse2: fp32 scratch of B*Hq*Sp + 128 elements each, Sp = Sq rounded up to 4, 16-byte aligned (delta holds the row sums
+// of dO*O afterwards, row pitch Sp). part: fp32 scratch [B*Sk, Hq, max(dqk, dv)] when Hq > Hkv, else null. dq / dk / dv
+// receive contiguous bf16 results.
+PT_API int pt_attn_bwd_split(const void* q, const void* k, const void* v, const void* out, const void* dout, const void* lse,
+                             const void* row_lo, void* dq, void* dk, void* dv, void* delta, void* lse2, void* part, int B, int Sq,
+                             int Sk, int Hq, int Hkv, int dqk, int dvd, long long ldq, long long ldk, long long ldv, long long ldo,
+                             long long lddo, float scale, int causal, int q_off, void* stream_) {
+  if (B <= 0 || Sq <= 0 || Sk <= 0 || Hkv <= 0 || Hq % Hkv != 0 || scale <= 0.f) return -2;
+  AttnSplitArgs a{};
+  a.B = B; a.Sq = Sq; a.Sk = Sk; a.Hq = Hq; a.Hkv = Hkv; a.causal = causal; a.q_off = q_off;
+  a.Sp = (Sq + 3) & ~3;
+  a.scale_log2 = scale * 1.4426950408889634f;
+  a.row_lo = static_cast<const int*>(row_lo);
+  a.err = device_status_word();
+  const SplitTensors t{q, k, v, dout, ldq, ldk, ldv, lddo};
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  float *de = static_cast<float*>(delta), *l2 = static_cast<float*>(lse2), *pa = static_cast<float*>(part);
+  if (dqk == 64 && dvd == 64) return attn_split_all<64, 64>(t, a, out, lse, de, l2, pa, dq, dk, dv, ldo, scale, stream);
+  if (dqk == 128 && dvd == 128) return attn_split_all<128, 128>(t, a, out, lse, de, l2, pa, dq, dk, dv, ldo, scale, stream);
+  if (dqk == 192 && dvd == 128) return attn_split_all<192, 128>(t, a, out, lse, de, l2, pa, dq, dk, dv, ldo, scale, stream);
+  if (dqk == 256 && dvd == 256) return attn_split_all<256, 256>(t, a, out, lse, de, l2, pa, dq, dk, dv, ldo, scale, stream);
+  return -2;
+}

@@ -1,4 +1,5 @@
-"""The framework's own attention kernels (``csrc/attention.cu`` forward, ``csrc/attention_bwd.cu`` backward).
+"""The framework's own attention kernels (``csrc/attention.cu`` forward, ``csrc/attention_bwd.cu`` and
+``csrc/attention_bwd_split.cu`` backward).
 
 tcgen05 / TMEM / TMA kernels for bf16 attention in the token-major ``[B, S, H, D]`` layout the projections write:
 causal or unmasked, GQA, sliding windows, packed documents (``cu_seqlens``), learned per-head sinks, and the head
@@ -20,7 +21,8 @@ import torch
 
 ENABLED = True
 _DIMS = {(64, 64), (128, 128), (192, 128), (256, 256)}
-# head-dim pairs the backward kernel covers; the others differentiate through the fp32 math
+# head-dim pairs of csrc/attention_bwd.cu, for lengths that are a multiple of 4 (its row statistics move in 16-byte
+# pieces); every other gradient comes from csrc/attention_bwd_split.cu
 _BWD_DIMS = {(64, 64), (128, 128)}
 _ROW_LO_CACHE: dict = {}
 
@@ -105,22 +107,46 @@ def backward(do, q, k, v, out, lse, scale: float, causal: bool, q_off: int, row_
     lse = lse.contiguous()  # ring attention hands in halves of a longer sequence's statistics
     B, Sq, Hq, D = q.shape
     Sk, Hkv, Dv = k.shape[1], k.shape[2], v.shape[-1]
-    # fp32 accumulators (dq over key tiles; dk / dv over the heads of a GQA group), zeroed in one memset
-    nq, nk = B * Sq * Hq * D, B * Sk * Hkv * D
-    acc = torch.zeros(nq + 2 * nk, dtype=torch.float32, device=q.device)
+    # one zeroed buffer: the fp32 accumulators (dq over key tiles; dk / dv over the heads of a GQA group), then the row
+    # statistics, padded by one tile because the kernel reads them in whole 128-row tiles
+    nq, nk, ns = B * Sq * Hq * D, B * Sk * Hkv * D, B * Hq * Sq
+    buf = torch.zeros(nq + 2 * nk + 2 * (ns + 128), dtype=torch.float32, device=q.device)
+    delta, lse2 = buf[nq + 2 * nk:nq + 2 * nk + ns + 128], buf[nq + 2 * nk + ns + 128:]
     dq = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device)
     dk = torch.empty((B, Sk, Hkv, D), dtype=k.dtype, device=q.device)
     dv = torch.empty((B, Sk, Hkv, Dv), dtype=v.dtype, device=q.device)
-    # the kernel reads statistics in whole 128-row tiles: pad the flat arrays by one tile
-    stats = torch.zeros(2 * (B * Hq * Sq + 128), dtype=torch.float32, device=q.device)
-    delta, lse2 = stats[:B * Hq * Sq + 128], stats[B * Hq * Sq + 128:]
     rc = _native.lib().pt_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), do.data_ptr(), lse.data_ptr(),
-                                   _native.ptr(row_lo), acc.data_ptr(), acc[nq:].data_ptr(), acc[nq + nk:].data_ptr(),
+                                   _native.ptr(row_lo), buf.data_ptr(), buf[nq:].data_ptr(), buf[nq + nk:].data_ptr(),
                                    dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr(), lse2.data_ptr(),
                                    B, Sq, Sk, Hq, Hkv, D, q.stride(1), k.stride(1), v.stride(1), out.stride(1), do.stride(1),
                                    float(scale), int(bool(causal)), int(q_off), _native.stream_ptr())
     _native.check(rc, "pt_attn_bwd")
-    return dq, dk, dv, delta[:B * Hq * Sq].view(B, Hq, Sq)
+    return dq, dk, dv, delta[:ns].view(B, Hq, Sq)
+
+
+def backward_split(do, q, k, v, out, lse, scale: float, causal: bool, q_off: int, row_lo: Optional[torch.Tensor]
+                   ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
+    """:func:`backward` on the kernels that keep P and dS at fp32 accuracy (two bf16 terms each), for every head-dim pair
+    of the forward kernel and any length. Same results; ``delta`` is a strided view."""
+    from .. import _native
+
+    q, k, v, do, out = (_as_token_major(t) for t in (q, k, v, do, out))
+    lse = lse.contiguous()
+    B, Sq, Hq, D = q.shape
+    Sk, Hkv, Dv = k.shape[1], k.shape[2], v.shape[-1]
+    dev, Sp = q.device, (Sq + 3) // 4 * 4
+    ns = B * Hq * Sp
+    stats = torch.empty(2 * (ns + 128), dtype=torch.float32, device=dev)  # read in whole 64-row tiles: padded
+    delta, lse2 = stats[:ns + 128], stats[ns + 128:]
+    dq, dk, dv = (torch.empty(t.shape, dtype=t.dtype, device=dev) for t in (q, k, v))
+    part = torch.empty(B * Sk * Hq * max(D, Dv), dtype=torch.float32, device=dev) if Hq != Hkv else None
+    rc = _native.lib().pt_attn_bwd_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), do.data_ptr(), lse.data_ptr(),
+                                         _native.ptr(row_lo), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr(),
+                                         lse2.data_ptr(), _native.ptr(part), B, Sq, Sk, Hq, Hkv, D, Dv, q.stride(1), k.stride(1),
+                                         v.stride(1), out.stride(1), do.stride(1), float(scale), int(bool(causal)), int(q_off),
+                                         _native.stream_ptr())
+    _native.check(rc, "pt_attn_bwd_split")
+    return dq, dk, dv, delta[:ns].view(B, Hq, Sp)[..., :Sq]
 
 
 class _Attention(torch.autograd.Function):
@@ -139,44 +165,13 @@ class _Attention(torch.autograd.Function):
         q, k, v, out, lse, sinks, row_lo = ctx.saved_tensors
         sinks = sinks if ctx.has_sinks else None
         row_lo = row_lo if ctx.has_lo else None
-        if (q.shape[-1], v.shape[-1]) in _BWD_DIMS and q.shape[1] % 4 == 0:  # row statistics move in 16-byte pieces
-            dq, dk, dv, delta = backward(do, q, k, v, out, lse, ctx.scale, ctx.causal, ctx.q_off, row_lo)
-        else:
-            dq, dk, dv, delta = _math_backward(do, q, k, v, out, lse, ctx.scale, ctx.causal, ctx.q_off, row_lo)
+        fast = (q.shape[-1], v.shape[-1]) in _BWD_DIMS and q.shape[1] % 4 == 0
+        dq, dk, dv, delta = (backward if fast else backward_split)(do, q, k, v, out, lse, ctx.scale, ctx.causal, ctx.q_off, row_lo)
         d_sinks = None
         if sinks is not None:
             # d lse-normalised weight of the sink column: -exp(sink - lse) * delta, summed over batch and rows
             d_sinks = -(torch.exp(sinks.float().view(1, -1, 1) - lse) * delta).sum((0, 2)).to(sinks.dtype)
         return dq, dk, dv, d_sinks, None, None, None, None
-
-
-def _math_backward(do, q, k, v, out, lse, scale, causal, q_off, row_lo):
-    """fp32 tensor-op backward against the kernel's ``out`` and ``lse`` for the head dims the backward kernel does not
-    cover (MLA 192/128 and 256): same formulas as the kernel, O(S^2) memory."""
-    B, Sq, Hq, D = q.shape
-    Sk, Hkv = k.shape[1], k.shape[2]
-    g = Hq // Hkv
-    qf = q.float().permute(0, 2, 1, 3)
-    kf = k.float().permute(0, 2, 1, 3).repeat_interleave(g, dim=1)
-    vf = v.float().permute(0, 2, 1, 3).repeat_interleave(g, dim=1)
-    dof = do.float().permute(0, 2, 1, 3)
-    s = torch.matmul(qf, kf.transpose(-1, -2)) * scale
-    kp = torch.arange(Sk, device=q.device).view(1, 1, 1, Sk)
-    qp = (torch.arange(Sq, device=q.device) + q_off).view(1, 1, Sq, 1)
-    vis = torch.ones(1, 1, Sq, Sk, dtype=torch.bool, device=q.device)
-    if causal:
-        vis = vis & (kp <= qp)
-    if row_lo is not None:
-        vis = vis & (kp >= row_lo.view(B, 1, Sq, 1))
-    lse_safe = torch.where(torch.isinf(lse), torch.zeros_like(lse), lse)
-    p = torch.exp(s - lse_safe.unsqueeze(-1)).masked_fill(~vis, 0.0)
-    delta = (dof * out.float().permute(0, 2, 1, 3)).sum(-1)
-    dp = torch.matmul(dof, vf.transpose(-1, -2))
-    ds = p * (dp - delta.unsqueeze(-1)) * scale
-    dq = torch.matmul(ds, kf).permute(0, 2, 1, 3)
-    dk = torch.matmul(ds.transpose(-1, -2), qf).view(B, Hkv, g, Sk, D).sum(2).permute(0, 2, 1, 3)
-    dv = torch.matmul(p.transpose(-1, -2), dof).view(B, Hkv, g, Sk, v.shape[-1]).sum(2).permute(0, 2, 1, 3)
-    return dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), delta
 
 
 def attention(q, k, v, causal, scale, window_left, sinks, cu_seqlens, return_lse=False, q_off: Optional[int] = None):

@@ -4,8 +4,100 @@ import pytest
 import torch
 
 from pithtrain_b200 import _native
+from pithtrain_b200.ops import attention as A
+from pithtrain_b200.ops import attention_native as N
 
 pytestmark = pytest.mark.gpu
+
+
+def _backward64(do, q, k, v, out, lse, scale, causal, q_off, row_lo):
+    """The flash-attention backward formulas in 64 bits, from the same bf16 ``out`` and fp32 ``lse``."""
+    B, Sq, Hq, D = q.shape
+    Sk, Hkv = k.shape[1], k.shape[2]
+    g = Hq // Hkv
+    qf, dof = q.double().permute(0, 2, 1, 3), do.double().permute(0, 2, 1, 3)
+    kf, vf = (t.double().permute(0, 2, 1, 3).repeat_interleave(g, dim=1) for t in (k, v))
+    kp = torch.arange(Sk, device=q.device).view(1, 1, 1, Sk)
+    qp = (torch.arange(Sq, device=q.device) + q_off).view(1, 1, Sq, 1)
+    vis = torch.ones(1, 1, Sq, Sk, dtype=torch.bool, device=q.device)
+    if causal:
+        vis = vis & (kp <= qp)
+    if row_lo is not None:
+        vis = vis & (kp >= row_lo.view(B, 1, Sq, 1))
+    safe = torch.where(torch.isinf(lse), torch.zeros_like(lse), lse).double()
+    p = torch.exp(qf @ kf.mT * scale - safe[..., None]).masked_fill(~vis, 0.0)
+    delta = (dof * out.double().permute(0, 2, 1, 3)).sum(-1)
+    ds = p * (dof @ vf.mT - delta[..., None]) * scale
+    dq = (ds @ kf).permute(0, 2, 1, 3)
+    dk = (ds.mT @ qf).view(B, Hkv, g, Sk, D).sum(2).permute(0, 2, 1, 3)
+    dv = (p.mT @ dof).view(B, Hkv, g, Sk, -1).sum(2).permute(0, 2, 1, 3)
+    return dq, dk, dv, delta
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
+
+
+@pytest.mark.parametrize("Dqk,Dv,Hq,Hkv", [(64, 64, 4, 2), (128, 128, 2, 2), (192, 128, 2, 2), (256, 256, 4, 1)])
+@pytest.mark.parametrize("B,Sq,Sk,causal,window,docs", [
+    (1, 1, 1, True, None, None), (2, 3, 3, True, None, None), (1, 63, 63, True, None, None), (2, 65, 65, True, None, None),
+    (1, 127, 127, True, None, None), (2, 130, 130, True, None, None), (1, 257, 257, False, None, None),
+    (1, 64, 320, True, None, None), (2, 96, 200, False, None, None), (1, 515, 515, True, 100, None),
+    (1, 517, 517, True, None, [0, 1, 130, 131, 400, 517]), (1, 640, 640, True, 64, [0, 128, 129, 512, 640]),
+])
+def test_attention_backward_split(Dqk, Dv, Hq, Hkv, B, Sq, Sk, causal, window, docs):
+    """dq, dk, dv are the 64-bit gradients rounded to bf16 (2^-9 at most): P and dS lose nothing on the way."""
+    torch.manual_seed(Sq)
+    q = torch.randn(B, Sq, Hq, Dqk, device="cuda").bfloat16()
+    k, v = torch.randn(B, Sk, Hkv, Dqk, device="cuda").bfloat16(), torch.randn(B, Sk, Hkv, Dv, device="cuda").bfloat16()
+    do = torch.randn(B, Sq, Hq, Dv, device="cuda").bfloat16()
+    cu = None if docs is None else torch.tensor(docs, dtype=torch.int32, device="cuda")
+    scale, q_off = Dqk ** -0.5, Sk - Sq
+    row_lo = N.row_lower_bounds(B, Sq, q_off, window, cu, q.device)
+    out, lse = N.forward(q, k, v, scale, causal, q_off, row_lo, None)
+    got = N.backward_split(do, q, k, v, out, lse, scale, causal, q_off, row_lo)
+    _native.check_status()
+    want = _backward64(do, q, k, v, out, lse, scale, causal, q_off, row_lo)
+    if Sq == 1 and Sk == 1:
+        # one key: P = 1 and dS = dP - delta, which cancels up to the rounding of out (2^-9 of terms of size D^0.5 * 3)
+        assert _rel(got[2], want[2]) < 2.0 ** -9
+        assert (got[0].double() - want[0]).abs().max() < 2.0 ** -9 * 3 * Dv ** 0.5 * scale * 4
+        return
+    for name, a, b in zip(("dq", "dk", "dv"), got, want):
+        # fp32 accumulation and lse add less than 2^-12 to the rounding of the result
+        assert _rel(a, b) < 2.0 ** -9 + 2.0 ** -12, name
+    assert _rel(got[3], want[3]) < 1e-5
+
+
+def test_attention_backward_split_keeps_batch_entries_apart():
+    """Rows past the end of a batch entry read as zero: an infinity in the next entry stays there."""
+    q, k, v, do = (torch.randn(2, 70, 2, 256, device="cuda").bfloat16() for _ in range(4))
+    for t in (q, k, v, do):
+        t[1] = float("inf")
+    out, lse = N.forward(q[:1], k[:1], v[:1], 0.0625, True, 0, None, None)
+    out, lse = torch.cat([out, out]), torch.cat([lse, lse])
+    got = N.backward_split(do, q, k, v, out, lse, 0.0625, True, 0, None)
+    want = _backward64(do[:1], q[:1], k[:1], v[:1], out[:1], lse[:1], 0.0625, True, 0, None)
+    for a, b in zip(got[:3], want):
+        assert _rel(a[:1], b) < 2.0 ** -9 + 2.0 ** -12
+
+
+@pytest.mark.parametrize("S", [126, 1021])
+def test_attention_with_odd_lengths_and_sinks(S):
+    torch.manual_seed(S)
+    q = torch.randn(1, S, 4, 128, device="cuda").bfloat16()
+    k, v = (torch.randn(1, S, 2, 128, device="cuda").bfloat16() for _ in range(2))
+    sinks, do = torch.randn(4, device="cuda").bfloat16(), torch.randn(1, S, 4, 128, device="cuda").bfloat16()
+
+    def grads(fn):
+        leaves = [t.detach().clone().requires_grad_() for t in (q, k, v, sinks)]
+        return torch.autograd.grad(fn(*leaves), leaves, do)
+
+    got = grads(lambda a, b, c, s: N.attention(a, b, c, True, None, 200, s, None))
+    want = grads(lambda a, b, c, s: A.attention_ref(a, b, c, True, None, 200, s, None))
+    _native.check_status()
+    for a, b in zip(got, want):
+        assert _rel(a, b.double()) < 1e-2  # the oracle differentiates an fp32 output, the kernels its bf16 rounding
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
