@@ -119,6 +119,8 @@ SIGS = {
     "pt_attn_bwd_split": "PPPPPPPPPPPPP" + "IIIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_attn_bwd": "PPPPPPPPPPPPPPP" + "IIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_gemm2cta_nt": "PPPIIILLLP",
+    "pt_gdr_fwd": "PPPPPPPPPPPPPP" + "III" + "F" + "P",
+    "pt_gdr_bwd": "PPPPPPPPPPPPPPPPPPPP" + "III" + "F" + "P",
     "pt_gdr_state_fwd": "PPPPPPPPIIIIP",
     "pt_gdr_state_bwd": "PPPPPPPPPPPPPIIIIP",
 }
@@ -144,7 +146,7 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 # Number of kernel launches issued through this module since it was last reset (bench bookkeeping).
 LAUNCHES = 0
-_LAUNCHES_PER_CALL = {"pt_route_sort": 4, "pt_attn_bwd": 3, "pt_attn_bwd_split": 6, "pt_merge_partial": 2}
+_LAUNCHES_PER_CALL = {"pt_route_sort": 4, "pt_attn_bwd": 3, "pt_attn_bwd_split": 6, "pt_gdr_fwd": 3, "pt_gdr_bwd": 3, "pt_merge_partial": 2}
 
 
 def check(rc: int, what: str) -> None:

@@ -1,12 +1,12 @@
-"""Gated delta rule linear attention (Gated DeltaNet), chunked, in plain PyTorch autograd.
+"""Gated delta rule linear attention (Gated DeltaNet), chunked.
 
 Per head the recurrence over a ``[dk, dv]`` state is
 ``S <- exp(g_t) * S``, ``S <- S + k_t (beta_t (v_t - S^T k_t))^T``, ``o_t = S^T q_t / sqrt(dk)``.
-``gated_delta_rule`` evaluates it chunk by chunk (chunk 64): inside a chunk the sequential
-dependence is resolved with a triangular solve (batched tensor ops over all chunks at once), across
-chunks the state is carried by the recurrence kernels of ``csrc/gdr.cu`` (forward and backward, state
-resident in shared memory) — the same blocking as the library kernel the reference wraps
-(pithtrain/operators/gated_delta_rule.py:21-56).
+``gated_delta_rule`` evaluates it chunk by chunk (chunk 64), the blocking of the library kernel the
+reference wraps (pithtrain/operators/gated_delta_rule.py:21-56). bf16 q, k, v with head dims 128 on a
+GPU run on the kernels of ``csrc/gdr_fused.cu``, forward and backward, in fp32 arithmetic. Other dtypes
+and head dims resolve a chunk with a triangular solve (batched tensor ops over all chunks at once) and
+carry the state across chunks with the recurrence kernels of ``csrc/gdr.cu``.
 ``gated_delta_rule_recurrent`` is the token-by-token oracle.
 """
 
@@ -94,8 +94,72 @@ def chunk_state(w, u, qg, kd, a):
     return _chunk_state_math(w, u, qg, kd, a)
 
 
+def _rows_of_8(t: torch.Tensor) -> torch.Tensor:
+    """``t [B,S,H,128]`` with rows the kernels can read in 16-byte pieces (a slice of a wider projection qualifies)."""
+    ok = t.stride(-1) == 1 and all(s % 8 == 0 for s in t.stride()[:3]) and t.data_ptr() % 16 == 0
+    return t if ok else t.contiguous()
+
+
+class _GatedDeltaRule(torch.autograd.Function):
+    """The whole rule on ``csrc/gdr_fused.cu``."""
+
+    @staticmethod
+    def _strides(*ts):
+        import ctypes
+
+        return (ctypes.c_longlong * 9)(*(x for t in ts for x in t.stride()[:3]))
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, beta):
+        from .. import _native
+
+        q, k, v = _rows_of_8(q), _rows_of_8(k), _rows_of_8(v)
+        B, S, H, D = q.shape
+        N, dev = (S + 63) // 64, q.device
+        gf, bf = g.float().contiguous(), beta.float().contiguous()
+        f32 = lambda *s: torch.empty(s, dtype=torch.float32, device=dev)  # noqa: E731
+        gc, P, T = f32(B * H, N, 64), f32(B * H, N, 64, 64), f32(B * H, N, 64, 64)
+        u, w, vn, st = f32(B * H, N, 64, D), f32(B * H, N, 64, D), f32(B * H, N, 64, D), f32(B * H, N, D, D)
+        o = torch.empty((B, S, H, D), dtype=v.dtype, device=dev)
+        rc = _native.lib().pt_gdr_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), _GatedDeltaRule._strides(q, k, v), gf.data_ptr(),
+                                      bf.data_ptr(), gc.data_ptr(), P.data_ptr(), T.data_ptr(), u.data_ptr(), w.data_ptr(),
+                                      vn.data_ptr(), st.data_ptr(), o.data_ptr(), B, S, H, D ** -0.5, _native.stream_ptr())
+        _native.check(rc, "pt_gdr_fwd")
+        ctx.save_for_backward(q, k, v, bf, gc, P, T, u, w, vn, st)
+        ctx.dtypes = (g.dtype, beta.dtype)
+        return o
+
+    @staticmethod
+    def backward(ctx, d_o):
+        from .. import _native
+
+        q, k, v, bf, gc, P, T, u, w, vn, st = ctx.saved_tensors
+        B, S, H, D = q.shape
+        d_o = d_o.contiguous()
+        if d_o.data_ptr() % 16:
+            d_o = d_o.clone()
+        dvn, dst = torch.empty_like(vn), torch.empty_like(st)
+        dq, dk, dv = (torch.empty((B, S, H, D), dtype=q.dtype, device=q.device) for _ in range(3))
+        dg, dbeta = torch.empty_like(bf), torch.empty_like(bf)
+        rc = _native.lib().pt_gdr_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), _GatedDeltaRule._strides(q, k, v), bf.data_ptr(),
+                                      gc.data_ptr(), P.data_ptr(), T.data_ptr(), u.data_ptr(), w.data_ptr(), vn.data_ptr(),
+                                      st.data_ptr(), d_o.data_ptr(), dvn.data_ptr(), dst.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+                                      dv.data_ptr(), dg.data_ptr(), dbeta.data_ptr(), B, S, H, D ** -0.5, _native.stream_ptr())
+        _native.check(rc, "pt_gdr_bwd")
+        return dq, dk, dv, dg.to(ctx.dtypes[0]), dbeta.to(ctx.dtypes[1])
+
+
+def _fused_ok(q, k, v, g, beta, chunk_size: int) -> bool:
+    """The fused kernels hold 64 x 128 tiles of bf16 inputs; everything else takes the general path below."""
+    return (q.is_cuda and chunk_size == 64 and all(t.dtype == torch.bfloat16 for t in (q, k, v)) and q.shape[1] > 0
+            and q.shape[0] > 0 and q.shape == k.shape == v.shape and q.shape[-1] == 128 and g.shape == beta.shape == q.shape[:3]
+            and q.shape[0] * q.shape[2] <= 65535)
+
+
 def gated_delta_rule(q, k, v, g, beta, chunk_size: int = 64):
     """Chunked evaluation; same signature and result as :func:`gated_delta_rule_recurrent`."""
+    if _fused_ok(q, k, v, g, beta, chunk_size):
+        return _GatedDeltaRule.apply(q, k, v, g, beta)
     B, S, H, dk = q.shape
     dv = v.shape[-1]
     C = chunk_size

@@ -128,3 +128,47 @@ def test_quant_blocks_both_orientations(G, R, K):
     assert torch.equal(q.view(torch.uint8), q0.view(torch.uint8)) and torch.equal(s, s0)
     assert torch.equal(qt.view(torch.uint8), q0.transpose(1, 2).contiguous().view(torch.uint8))
     assert torch.equal(st, s0.transpose(1, 2).contiguous())
+
+
+def _delta_rule64(q, k, v, g, beta):
+    """Token-by-token recurrence in 64 bits."""
+    B, S, H, dk = q.shape
+    state = torch.zeros(B, H, dk, v.shape[-1], dtype=torch.float64, device=q.device)
+    outs = []
+    for t in range(S):
+        state = state * g[:, t].exp()[..., None, None]
+        new = (v[:, t] - torch.einsum("bhkv,bhk->bhv", state, k[:, t])) * beta[:, t][..., None]
+        state = state + k[:, t][..., None] * new[..., None, :]
+        outs.append(torch.einsum("bhkv,bhk->bhv", state, q[:, t]) * dk ** -0.5)
+    return torch.stack(outs, 1)
+
+
+@pytest.mark.parametrize("B,S,H,strong", [(1, 1, 1, False), (2, 63, 2, False), (1, 64, 3, True), (1, 65, 2, False), (2, 130, 2, True),
+                                          (1, 321, 4, False)])
+def test_gated_delta_rule_fused(B, S, H, strong):
+    """Outputs and all gradients of the fused kernels against the recurrence in 64 bits, q / k / v as slices of one projection;
+    bf16 results carry one rounding (2^-9), the fp32 gate gradients the error of fp32 sums."""
+    from pithtrain_b200.ops.gated_delta_rule import gated_delta_rule
+
+    torch.manual_seed(S)
+    x = torch.randn(B, S, 3 * H * 128 + 8, device="cuda").bfloat16()
+    q, k, v = (x[..., i * H * 128:(i + 1) * H * 128].view(B, S, H, 128) for i in range(3))
+    q, k = (torch.nn.functional.normalize(t.float(), dim=-1).bfloat16() for t in (q, k))
+    g = -torch.rand(B, S, H, device="cuda") * (6.0 if strong else 0.3)
+    beta = torch.rand(B, S, H, device="cuda").bfloat16()
+    do = torch.randn(B, S, H, 128, device="cuda").bfloat16()
+    leaves = [t.detach().requires_grad_() for t in (q, k, v, g, beta)]
+    assert S == 1 or leaves[2].stride(1) == x.stride(1)  # read in place
+    o = gated_delta_rule(*leaves)
+    got = torch.autograd.grad(o, leaves, do)
+    wide = [t.detach().double().requires_grad_() for t in (q, k, v, g, beta)]
+    ref = _delta_rule64(*wide)
+    want = torch.autograd.grad(ref, wide, do.double())
+    assert o.dtype == torch.bfloat16 and got[3].dtype == torch.float32 and got[4].dtype == torch.bfloat16
+    assert _rel(o, ref.detach()) < 2.0 ** -9
+    for name, a, b in zip(("dq", "dk", "dv", "dg", "dbeta"), got, want):
+        if name == "dg":
+            # a gate's gradient sums D^2 products that partly cancel: bounded against the size of its terms
+            assert (a.double() - b).abs().max() < 1e-4 * b.abs().max().clamp_min(1.0), name
+        else:
+            assert _rel(a, b) < 2.0 ** -8.9, name
