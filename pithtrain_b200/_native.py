@@ -137,7 +137,9 @@ def _declare(L: ctypes.CDLL) -> None:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device, without building a ``torch.cuda.Stream`` object: that took 17 us a
+    call, a fifth of the host time of a launch-bound step."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
