@@ -119,6 +119,12 @@ SIGS = {
     "pt_attn_bwd_split": "PPPPPPPPPPPPP" + "IIIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_attn_bwd": "PPPPPPPPPPPPPPP" + "IIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_gemm2cta_nt": "PPPIIILLLP",
+    "pt_gdn_conv_fwd": "PPPPPIIIIP",
+    "pt_gdn_conv_parts": "II",
+    "pt_gdn_conv_bwd": "PPPPPPPIIIIP",
+    "pt_gdn_gnorm_fwd": "PPPPLFP",
+    "pt_gdn_gnorm_parts": "L",
+    "pt_gdn_gnorm_bwd": "PPPPPPPLFP",
     "pt_gdr_fwd": "PPPPPPPPPPPPPP" + "III" + "F" + "P",
     "pt_gdr_bwd": "PPPPPPPPPPPPPPPPPPPP" + "III" + "F" + "P",
     "pt_gdr_state_fwd": "PPPPPPPPIIIIP",

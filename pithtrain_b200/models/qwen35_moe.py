@@ -16,6 +16,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..contexts import distributed
+from ..ops import gdn_mix
 from ..ops.attention import attention, attention_ref
 from ..ops.common import grad_buffer
 from ..ops.gated_delta_rule import gated_delta_rule, gated_delta_rule_recurrent
@@ -33,7 +34,9 @@ class Qwen35MoeRMSNormGated(nn.Module):
         self.weight._init_fill = 1.0
         self.eps = eps
 
-    def forward(self, x: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, gate: torch.Tensor, reference: bool = False) -> torch.Tensor:
+        if not reference and gdn_mix.gated_norm_supported(x, gate, self.weight):
+            return gdn_mix.gated_norm(x, gate, self.weight, self.eps)
         xf = x.float()
         out = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps)
         return (out * self.weight.float() * F.silu(gate.float())).type_as(x)
@@ -67,22 +70,26 @@ class Qwen35MoeGatedDeltaNet(nn.Module):
     def forward(self, x: torch.Tensor, reference: bool = False) -> torch.Tensor:
         B, S, _ = x.shape
         lin = (lambda m, t: F.linear(t, m.weight)) if reference else (lambda m, t: m(t))
-        mixed = lin(self.in_proj_qkv, x).transpose(1, 2)
+        mixed = lin(self.in_proj_qkv, x)
         z = lin(self.in_proj_z, x).reshape(B, S, -1, self.head_v_dim)
         b, a = lin(self.in_proj_b, x), lin(self.in_proj_a, x)
-        mixed = F.silu(self.conv1d(mixed)[..., :S]).transpose(1, 2)
-        q, k, v = torch.split(mixed, [self.key_dim, self.key_dim, self.value_dim], dim=-1)
-        q = F.normalize(q.reshape(B, S, -1, self.head_k_dim), dim=-1)
-        k = F.normalize(k.reshape(B, S, -1, self.head_k_dim), dim=-1)
-        v = v.reshape(B, S, -1, self.head_v_dim)
+        if not reference and gdn_mix.conv_supported(mixed, self.conv1d.weight, self.num_k_heads, self.num_v_heads, self.head_k_dim,
+                                                    self.head_v_dim):
+            q, k, v = gdn_mix.conv_qkv(mixed, self.conv1d.weight, self.num_k_heads, self.num_v_heads)
+        else:
+            mixed = F.silu(self.conv1d(mixed.transpose(1, 2))[..., :S]).transpose(1, 2)
+            q, k, v = torch.split(mixed, [self.key_dim, self.key_dim, self.value_dim], dim=-1)
+            q = F.normalize(q.reshape(B, S, -1, self.head_k_dim), dim=-1)
+            k = F.normalize(k.reshape(B, S, -1, self.head_k_dim), dim=-1)
+            v = v.reshape(B, S, -1, self.head_v_dim)
+            rep = self.num_v_heads // self.num_k_heads
+            if rep > 1:
+                q, k = q.repeat_interleave(rep, dim=2), k.repeat_interleave(rep, dim=2)
         beta = b.sigmoid()
         g = -self.A_log.float().exp() * F.softplus(a.float() + self.dt_bias.float())
-        rep = self.num_v_heads // self.num_k_heads
-        if rep > 1:
-            q, k = q.repeat_interleave(rep, dim=2), k.repeat_interleave(rep, dim=2)
         fn = gated_delta_rule_recurrent if reference else gated_delta_rule
         o = fn(q, k, v, g, beta).reshape(-1, self.head_v_dim)
-        o = self.norm(o, z.reshape(-1, self.head_v_dim)).reshape(B, S, -1)
+        o = self.norm(o, z.reshape(-1, self.head_v_dim), reference).reshape(B, S, -1)
         return lin(self.out_proj, o)
 
 

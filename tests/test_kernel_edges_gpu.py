@@ -34,6 +34,11 @@ def _backward64(do, q, k, v, out, lse, scale, causal, q_off, row_lo):
     return dq, dk, dv, delta
 
 
+# Rounding to bf16 is off by at most 2^-8 of a value (half a unit in the last of 8 bits); over many values the 2-norm of
+# errors uniform over that half unit is at most 2^-8 / sqrt(3).
+BF16_MAX, BF16_NORM = 2.0 ** -8, 2.0 ** -8 / 3 ** 0.5
+
+
 def _rel(a, b):
     return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
 
@@ -46,7 +51,8 @@ def _rel(a, b):
     (1, 517, 517, True, None, [0, 1, 130, 131, 400, 517]), (1, 640, 640, True, 64, [0, 128, 129, 512, 640]),
 ])
 def test_attention_backward_split(Dqk, Dv, Hq, Hkv, B, Sq, Sk, causal, window, docs):
-    """dq, dk, dv are the 64-bit gradients rounded to bf16 (2^-9 at most): P and dS lose nothing on the way."""
+    """dq, dk, dv are the 64-bit gradients rounded to bf16: P and dS lose nothing on the way (rounding them too would show as
+    3e-3)."""
     torch.manual_seed(Sq)
     q = torch.randn(B, Sq, Hq, Dqk, device="cuda").bfloat16()
     k, v = torch.randn(B, Sk, Hkv, Dqk, device="cuda").bfloat16(), torch.randn(B, Sk, Hkv, Dv, device="cuda").bfloat16()
@@ -59,13 +65,13 @@ def test_attention_backward_split(Dqk, Dv, Hq, Hkv, B, Sq, Sk, causal, window, d
     _native.check_status()
     want = _backward64(do, q, k, v, out, lse, scale, causal, q_off, row_lo)
     if Sq == 1 and Sk == 1:
-        # one key: P = 1 and dS = dP - delta, which cancels up to the rounding of out (2^-9 of terms of size D^0.5 * 3)
-        assert _rel(got[2], want[2]) < 2.0 ** -9
-        assert (got[0].double() - want[0]).abs().max() < 2.0 ** -9 * 3 * Dv ** 0.5 * scale * 4
+        # one key: P = 1 and dS = dP - delta, which cancels up to the rounding of out (2^-8 of terms of size D^0.5 * 3)
+        assert _rel(got[2], want[2]) < BF16_MAX
+        assert (got[0].double() - want[0]).abs().max() < BF16_MAX * 3 * Dv ** 0.5 * scale * 4
         return
     for name, a, b in zip(("dq", "dk", "dv"), got, want):
         # fp32 accumulation and lse add less than 2^-12 to the rounding of the result
-        assert _rel(a, b) < 2.0 ** -9 + 2.0 ** -12, name
+        assert _rel(a, b) < BF16_NORM + 2.0 ** -12, name
     assert _rel(got[3], want[3]) < 1e-5
 
 
@@ -79,7 +85,7 @@ def test_attention_backward_split_keeps_batch_entries_apart():
     got = N.backward_split(do, q, k, v, out, lse, 0.0625, True, 0, None)
     want = _backward64(do[:1], q[:1], k[:1], v[:1], out[:1], lse[:1], 0.0625, True, 0, None)
     for a, b in zip(got[:3], want):
-        assert _rel(a[:1], b) < 2.0 ** -9 + 2.0 ** -12
+        assert _rel(a[:1], b) < BF16_NORM + 2.0 ** -12
 
 
 @pytest.mark.parametrize("S", [126, 1021])
@@ -147,7 +153,7 @@ def _delta_rule64(q, k, v, g, beta):
                                           (1, 321, 4, False)])
 def test_gated_delta_rule_fused(B, S, H, strong):
     """Outputs and all gradients of the fused kernels against the recurrence in 64 bits, q / k / v as slices of one projection;
-    bf16 results carry one rounding (2^-9), the fp32 gate gradients the error of fp32 sums."""
+    bf16 results carry one rounding, the fp32 gate gradients the error of fp32 sums."""
     from pithtrain_b200.ops.gated_delta_rule import gated_delta_rule
 
     torch.manual_seed(S)
@@ -165,10 +171,56 @@ def test_gated_delta_rule_fused(B, S, H, strong):
     ref = _delta_rule64(*wide)
     want = torch.autograd.grad(ref, wide, do.double())
     assert o.dtype == torch.bfloat16 and got[3].dtype == torch.float32 and got[4].dtype == torch.bfloat16
-    assert _rel(o, ref.detach()) < 2.0 ** -9
+    assert _rel(o, ref.detach()) < BF16_NORM + 2.0 ** -12
     for name, a, b in zip(("dq", "dk", "dv", "dg", "dbeta"), got, want):
         if name == "dg":
             # a gate's gradient sums D^2 products that partly cancel: bounded against the size of its terms
             assert (a.double() - b).abs().max() < 1e-4 * b.abs().max().clamp_min(1.0), name
         else:
-            assert _rel(a, b) < 2.0 ** -8.9, name
+            assert _rel(a, b) < BF16_MAX, name
+
+
+@pytest.mark.parametrize("B,S,nk,nv", [(1, 1, 1, 1), (2, 3, 1, 2), (1, 31, 2, 2), (2, 33, 2, 4), (1, 97, 3, 9)])
+def test_gdn_conv(B, S, nk, nv):
+    """Convolution + SiLU + l2 norm + repetition and its gradients against tensor ops in 64 bits: one bf16 rounding each."""
+    from pithtrain_b200.ops import gdn_mix
+
+    F = torch.nn.functional
+    torch.manual_seed(S)
+    C = (2 * nk + nv) * 128
+    x, w = torch.randn(B, S, C, device="cuda").bfloat16(), (torch.randn(C, 1, 4, device="cuda") * 0.4).bfloat16()
+    go = [torch.randn(B, S, nv, 128, device="cuda").bfloat16() for _ in range(3)]
+    xg, wp = x.clone().requires_grad_(), torch.nn.Parameter(w.clone())
+    wp.main_grad = torch.zeros(w.shape, device="cuda")
+    assert gdn_mix.conv_supported(xg, wp, nk, nv, 128, 128)
+    got = gdn_mix.conv_qkv(xg, wp, nk, nv)
+    torch.autograd.backward(got, go)
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    m = F.silu(F.conv1d(F.pad(xd.mT, (3, 0)), wd, groups=C)).mT
+    q, k, v = m.split([nk * 128, nk * 128, nv * 128], -1)
+    q, k = (F.normalize(t.reshape(B, S, nk, 128), dim=-1).repeat_interleave(nv // nk, 2) for t in (q, k))
+    want = (q, k, v.reshape(B, S, nv, 128))
+    torch.autograd.backward(want, [g.double() for g in go])
+    for a, b in zip(got, want):
+        assert _rel(a.detach(), b.detach()) < BF16_MAX
+    assert _rel(xg.grad, xd.grad) < BF16_MAX
+    assert _rel(wp.main_grad, wd.grad) < 1e-5
+
+
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 20000])
+def test_gdn_gated_norm(rows):
+    from pithtrain_b200.ops import gdn_mix
+
+    torch.manual_seed(rows)
+    x, z, d = (torch.randn(rows, 128, device="cuda").bfloat16() for _ in range(3))
+    w = (1 + 0.1 * torch.randn(128, device="cuda")).bfloat16()
+    xg, zg, wp = x.clone().requires_grad_(), z.clone().requires_grad_(), torch.nn.Parameter(w.clone())
+    wp.main_grad = torch.zeros(128, device="cuda")
+    got = gdn_mix.gated_norm(xg, zg, wp, 1e-6)
+    got.backward(d)
+    xd, zd, wd = (t.double().requires_grad_() for t in (x, z, w))
+    want = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * wd * torch.nn.functional.silu(zd)
+    want.backward(d.double())
+    for a, b in ((got.detach(), want.detach()), (xg.grad, xd.grad), (zg.grad, zd.grad)):
+        assert _rel(a, b) < BF16_MAX
+    assert _rel(wp.main_grad, wd.grad) < 1e-5
