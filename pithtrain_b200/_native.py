@@ -71,6 +71,7 @@ SIGS = {
     "pt_qk_norm_rope_bwd_grid": "",
     "pt_qk_norm_rope_bwd": "PPPPPPPPPPPPIIIIILIP",
     "pt_router_topk_fwd": "PIPPPIIIIIFP",
+    "pt_router_given_fwd": "PIPPPIIIIFP",
     "pt_router_topk_bwd": "PPPPPPIIIIIIFP",
     "pt_route_sort": "PPIIIPLPPPIP",
     "pt_route_sort_noalloc": "PIIIPPPIP",

@@ -29,6 +29,16 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   *reinterpret_cast<uint4*>(p) = raw;
 }
 
+// e^x with the rounding of x * log2(e) compensated (the build's fast expf loses |x| ulp); 0 where e^x < 2^-126.
+__device__ __forceinline__ float exp_compensated(float x) {
+  x = fminf(fmaxf(x, -138.f), 138.f);
+  const float t = x * 1.4426950408889634f;
+  const float r = fmaf(x, 1.4426950408889634f, -t) + x * 1.92596299e-8f;
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(t));
+  return fmaf(y, r * 0.6931471805599453f, y);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -32,7 +32,9 @@ __device__ __forceinline__ float ld_as_float<float>(const float* p) { return *p;
 template <>
 __device__ __forceinline__ float ld_as_float<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 
-template <typename T>
+// GIVEN: the experts are handed in through topk_idx (a router replay) and only their weights are computed; mode 0. A pick
+// outside [0, E) has no weight: it reads as NaN.
+template <typename T, bool GIVEN>
 __global__ void __launch_bounds__(256)
 router_topk_fwd_kernel(const T* __restrict__ logits, float* __restrict__ probs,
                        int* __restrict__ topk_idx, float* __restrict__ topk_w, int n, int E, int k,
@@ -54,7 +56,8 @@ router_topk_fwd_kernel(const T* __restrict__ logits, float* __restrict__ probs,
     float s = 0.f;
 #pragma unroll
     for (int j = 0; j < MAX_EPL; ++j) {
-      v[j] = (v[j] == -INFINITY) ? 0.f : __expf(v[j] - mx);
+      // a replay takes the place of a library softmax, whose exponential is right to the last bits
+      v[j] = (v[j] == -INFINITY) ? 0.f : GIVEN ? exp_compensated(v[j] - mx) : __expf(v[j] - mx);
       s += v[j];
     }
     s = warp_sum(s);
@@ -67,30 +70,43 @@ router_topk_fwd_kernel(const T* __restrict__ logits, float* __restrict__ probs,
       if (!(j < epl && e < E)) v[j] = -1.f;  // never selected
     }
   }
-  // iterative arg-max; ties resolve to the lowest expert index
   float picked_w[16];
   int picked_i[16];
   float wsum = 0.f;
-  for (int t = 0; t < k; ++t) {
-    float best = -INFINITY;
-    int bi = 0x7fffffff;
+  if constexpr (GIVEN) {
+    for (int t = 0; t < k; ++t) {
+      const int e = topk_idx[(size_t)tok * k + t];
+      float mine = 0.f;
 #pragma unroll
-    for (int j = 0; j < MAX_EPL; ++j) {
-      int e = lane + 32 * j;
-      if (j < epl && e < E && (v[j] > best)) { best = v[j]; bi = e; }
+      for (int j = 0; j < MAX_EPL; ++j) if (j == (e >> 5)) mine = v[j];
+      const float p = __shfl_sync(0xffffffffu, mine, e & 31);
+      picked_w[t] = (e >= 0 && e < E) ? p : NAN;
+      picked_i[t] = e;
+      wsum += picked_w[t];
     }
+  } else {
+    // iterative arg-max; ties resolve to the lowest expert index
+    for (int t = 0; t < k; ++t) {
+      float best = -INFINITY;
+      int bi = 0x7fffffff;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
-    picked_w[t] = best;
-    picked_i[t] = bi;
-    wsum += best;
-    if ((bi & 31) == lane) {
+      for (int j = 0; j < MAX_EPL; ++j) {
+        int e = lane + 32 * j;
+        if (j < epl && e < E && (v[j] > best)) { best = v[j]; bi = e; }
+      }
 #pragma unroll
-      for (int j = 0; j < MAX_EPL; ++j) if (j == (bi >> 5)) v[j] = -INFINITY;
+      for (int o = 16; o > 0; o >>= 1) {
+        float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+      }
+      picked_w[t] = best;
+      picked_i[t] = bi;
+      wsum += best;
+      if ((bi & 31) == lane) {
+#pragma unroll
+        for (int j = 0; j < MAX_EPL; ++j) if (j == (bi >> 5)) v[j] = -INFINITY;
+      }
     }
   }
   if (mode == 1) {
@@ -105,7 +121,7 @@ router_topk_fwd_kernel(const T* __restrict__ logits, float* __restrict__ probs,
   }
   if (lane == 0) {
     for (int t = 0; t < k; ++t) {
-      topk_idx[(size_t)tok * k + t] = picked_i[t];
+      if (!GIVEN) topk_idx[(size_t)tok * k + t] = picked_i[t];
       topk_w[(size_t)tok * k + t] = picked_w[t];
     }
   }
@@ -134,7 +150,7 @@ router_topk_bwd_kernel(const float* __restrict__ probs, const int* __restrict__ 
     for (int t = 0; t < k; ++t) {
       float w = topk_w[(size_t)tok * k + t], dw = d_topk_w[(size_t)tok * k + t];
       int e = topk_idx[(size_t)tok * k + t];
-      s += probs[(size_t)tok * E + e];
+      if (e >= 0 && e < E) s += probs[(size_t)tok * E + e];  // a replayed pick may be out of range
       dot += dw * w;
     }
     for (int t = 0; t < k; ++t) {
@@ -527,9 +543,25 @@ PT_API int pt_router_topk_fwd(const void* logits, int logits_fp32, float* probs,
   if (E > 32 * MAX_EPL || k > 16 || k > E) return -1;
   int grid = (n + 7) / 8;
   if (logits_fp32)
-    router_topk_fwd_kernel<float><<<grid, 256, 0, st>>>((const float*)logits, probs, topk_idx, topk_w, n, E, k, mode, renorm, scale);
+    router_topk_fwd_kernel<float, false><<<grid, 256, 0, st>>>((const float*)logits, probs, topk_idx, topk_w, n, E, k, mode, renorm, scale);
   else
-    router_topk_fwd_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)logits, probs, topk_idx, topk_w, n, E, k, mode, renorm, scale);
+    router_topk_fwd_kernel<__nv_bfloat16, false><<<grid, 256, 0, st>>>((const __nv_bfloat16*)logits, probs, topk_idx, topk_w, n, E, k, mode, renorm, scale);
+  return (int)cudaGetLastError();
+}
+
+// Weights of given picks (int32 [n, k]): w = softmax(logits)[idx] (/ their sum if renorm) * scale; probs [n, E] is written.
+// pt_router_topk_bwd with mode 0 differentiates it.
+PT_API int pt_router_given_fwd(const void* logits, int logits_fp32, float* probs, const int* idx, float* w, int n, int E, int k, int renorm,
+                               float scale, void* stream_) {
+  cudaStream_t st = (cudaStream_t)stream_;
+  if (n <= 0) return 0;
+  if (E > 32 * MAX_EPL || k > 16 || k <= 0) return -1;
+  const int grid = (n + 7) / 8;
+  int* picks = const_cast<int*>(idx);  // read only
+  if (logits_fp32)
+    router_topk_fwd_kernel<float, true><<<grid, 256, 0, st>>>((const float*)logits, probs, picks, w, n, E, k, 0, renorm, scale);
+  else
+    router_topk_fwd_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>((const __nv_bfloat16*)logits, probs, picks, w, n, E, k, 0, renorm, scale);
   return (int)cudaGetLastError();
 }
 

@@ -20,7 +20,7 @@ from ..ops.embedding import Embedding
 from ..ops.linear import FusedWeights, Linear, fused_linear, linear
 from ..ops.moe import ExpertWeights, moe_experts, moe_experts_ref
 from ..ops.norm import RMSNorm, rmsnorm_ref
-from ..ops.router import router_topk, router_topk_ref
+from ..ops.router import router_replayed, router_topk, router_topk_ref
 from ..parallel import ep as ep_mod
 from .interface import RoutingInfo
 
@@ -184,12 +184,7 @@ class Gate(nn.Module):
         logits = self.logits(tokens)
         fn = router_topk_ref if reference else router_topk
         if self.router_replay is not None and self.mode == "softmax_topk":
-            scores = logits.float().softmax(-1)
-            idx = self.router_replay(torch.topk(scores, self.num_experts_per_tok, dim=-1).indices)
-            w = scores.gather(-1, idx.long())
-            if self.norm_topk_prob:
-                w = w / w.sum(-1, keepdim=True)
-            w, idx = w * self.scale, idx.int()
+            w, idx, scores = router_replayed(logits, self.num_experts_per_tok, self.router_replay, self.norm_topk_prob, self.scale)
         else:
             w, idx, scores = fn(logits, self.num_experts_per_tok, self.mode, self.norm_topk_prob, self.scale)
         lb_loss = None

@@ -150,8 +150,10 @@ def force_balance(num_experts: int) -> Callable[[torch.Tensor], torch.Tensor]:
     def replay(topk_idx: torch.Tensor) -> torch.Tensor:
         n, k = topk_idx.shape
         stride = num_experts // k
-        t = torch.arange(n, device=topk_idx.device).unsqueeze(1)
-        j = torch.arange(k, device=topk_idx.device).unsqueeze(0)
-        return ((t + j * stride) % num_experts).to(topk_idx.dtype)
+        t = torch.arange(n, device=topk_idx.device, dtype=topk_idx.dtype).unsqueeze(1)
+        if stride == 0:  # more slots than experts: every slot of a token goes to the same one
+            return (t % num_experts).expand(n, k).clone()
+        j = torch.arange(0, k * stride, stride, device=topk_idx.device, dtype=topk_idx.dtype).unsqueeze(0)
+        return (t + j) % num_experts
 
     return replay

@@ -86,6 +86,51 @@ def router_topk(logits: torch.Tensor, k: int, mode: str = "softmax_topk", renorm
     return router_topk_ref(logits, k, mode, renorm, scale)
 
 
+class _RouterGivenFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, logits, idx, renorm, scale):
+        n, E = logits.shape
+        k = idx.shape[1]
+        lg = logits.contiguous()
+        probs = torch.empty((n, E), dtype=torch.float32, device=lg.device)
+        w = torch.empty((n, k), dtype=torch.float32, device=lg.device)
+        rc = _native.lib().pt_router_given_fwd(lg.data_ptr(), int(lg.dtype == torch.float32), probs.data_ptr(), idx.data_ptr(), w.data_ptr(),
+                                               n, E, k, int(renorm), float(scale), sp())
+        _native.check(rc, "pt_router_given_fwd")
+        ctx.save_for_backward(probs, idx, w)
+        ctx.cfg = (k, 0, renorm, scale, lg.dtype)
+        return w, probs
+
+    @staticmethod
+    def backward(ctx, dw, dprobs=None):
+        return _RouterFn.backward(ctx, dw, None, dprobs)[0], None, None, None
+
+
+def router_replayed(logits: torch.Tensor, k: int, replay, renorm: bool = False, scale: float = 1.0
+                    ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """:func:`router_topk` (``softmax_topk``) with the picks exchanged by ``replay(top-k indices) -> indices``: the weights are the
+    softmax scores of the replayed experts."""
+    n, E = logits.shape
+    if logits.is_cuda and logits.dtype in (torch.float32, torch.bfloat16) and E <= 512 and k <= 16 and n > 0:
+        lg = logits.detach().contiguous()
+        picks = torch.empty((n, k), dtype=torch.int32, device=lg.device)
+        w = torch.empty((n, k), dtype=torch.float32, device=lg.device)
+        rc = _native.lib().pt_router_topk_fwd(lg.data_ptr(), int(lg.dtype == torch.float32), None, picks.data_ptr(), w.data_ptr(), n, E, k, 0, 0,
+                                              1.0, sp())
+        _native.check(rc, "pt_router_topk_fwd")
+        idx = replay(picks.long()).int().contiguous()
+        if idx.dim() == 2 and idx.shape[0] == n and 0 < idx.shape[1] <= 16:
+            w, probs = _RouterGivenFn.apply(logits, idx, renorm, scale)
+            return w, idx, probs
+    else:
+        idx = replay(torch.topk(logits.float().softmax(-1), k, dim=-1).indices)
+    scores = logits.float().softmax(-1)
+    w = scores.gather(-1, idx.long())
+    if renorm:
+        w = w / w.sum(-1, keepdim=True)
+    return w * scale, idx.int(), scores
+
+
 class _RouterTopkSoftmax(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, k, renorm, scale):

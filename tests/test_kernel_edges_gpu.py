@@ -224,3 +224,35 @@ def test_gdn_gated_norm(rows):
     for a, b in ((got.detach(), want.detach()), (xg.grad, xd.grad), (zg.grad, zd.grad)):
         assert _rel(a, b) < BF16_MAX
     assert _rel(wp.main_grad, wd.grad) < 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,E,k,renorm", [(1, 4, 1, True), (9, 16, 4, False), (257, 130, 6, True), (64, 512, 16, True)])
+def test_router_replayed(n, E, k, renorm, dtype):
+    """Weights, scores and logit gradients of replayed picks against the tensor-op form in 64 bits, repeated picks included."""
+    from pithtrain_b200.ops.router import router_replayed
+
+    torch.manual_seed(n)
+    logits = (torch.randn(n, E, device="cuda") * 4).to(dtype)
+    picks = torch.randint(0, E, (n, k), device="cuda")
+    seen = []
+
+    def replay(idx):
+        seen.append(idx)
+        return picks
+
+    lg = logits.clone().requires_grad_()
+    w, idx, probs = router_replayed(lg, k, replay, renorm, 2.5)
+    dw, dp = torch.randn(n, k, device="cuda"), torch.randn(n, E, device="cuda")
+    torch.autograd.backward((w, probs), (dw, dp))
+    ld = logits.double().requires_grad_()
+    p = ld.softmax(-1)
+    want = p.gather(1, picks)
+    want = (want / want.sum(-1, keepdim=True) if renorm else want) * 2.5
+    torch.autograd.backward((want, p), (dw.double(), dp.double()))
+    assert seen[0].dtype == torch.int64 and torch.equal(seen[0], p.topk(k).indices) or dtype == torch.bfloat16  # bf16 logits tie
+    assert torch.equal(idx.long(), picks)
+    assert _rel(w.detach(), want.detach()) < 1e-6 and _rel(probs.detach(), p.detach()) < 1e-6
+    # a logit's gradient is p times a difference that may cancel: fp32 error of its terms, then the rounding of the result
+    size = 2.5 * float(dw.abs().max()) * k + float(dp.abs().max())
+    assert ((lg.grad.double() - ld.grad).abs() <= 1e-6 * size + (BF16_MAX * ld.grad.abs() if dtype == torch.bfloat16 else 0)).all()
