@@ -256,3 +256,19 @@ def test_router_replayed(n, E, k, renorm, dtype):
     # a logit's gradient is p times a difference that may cancel: fp32 error of its terms, then the rounding of the result
     size = 2.5 * float(dw.abs().max()) * k + float(dp.abs().max())
     assert ((lg.grad.double() - ld.grad).abs() <= 1e-6 * size + (BF16_MAX * ld.grad.abs() if dtype == torch.bfloat16 else 0)).all()
+
+
+@pytest.mark.parametrize("k", [1, 3, 4, 6, 8])
+@pytest.mark.parametrize("n,H", [(1, 8), (3, 264), (64, 2048), (5000, 512)])
+def test_combine_rows(n, H, k):
+    from pithtrain_b200.ops.moe import combine_rows
+
+    torch.manual_seed(n)
+    y = torch.randn(2 * n + 1, H, device="cuda").bfloat16()
+    rows = torch.randint(-1, 2 * n + 1, (n * k,), device="cuda", dtype=torch.int32)  # -1: a slot whose expert is elsewhere
+    w, res = torch.rand(n, k, device="cuda"), torch.randn(n, H, device="cuda").bfloat16()
+    r = rows.view(n, k).long()
+    picked = y.double()[r.clamp(min=0)] * (r >= 0)[..., None]
+    for got, want in ((combine_rows(y, rows, k), picked.sum(1)), (combine_rows(y, rows, k, w, res), (picked * w.double()[..., None]).sum(1) + res.double())):
+        # fp32 sums of k + 1 terms, one bf16 rounding
+        assert ((got.double() - want).abs() <= BF16_MAX * want.abs() + 2.0 ** -20 * (k + 1) * 5).all()
