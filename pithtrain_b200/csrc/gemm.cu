@@ -42,7 +42,8 @@ struct GemmArgs {
   int out_fp32;
   int accumulate;
   int use_tma_store;
-  int epi;  // 0 staged coalesced rows, 1 direct per-thread rows, 2 TMA reduce-add when accumulating (else direct)
+  int epi;  // 0 staged coalesced rows, 1 direct per-thread rows, 2 TMA reduce-add when accumulating (else direct),
+            // 3 (kgroup into fp32, DEEP_EPI) prefetched read-modify-write
   int* err;
   // A-operand row gather (K-major A only): tile row r reads source row a_idx[r] / a_idx_div, a negative
   // index (or r >= a_idx_len) reads zeros. Replaces a separate gather pass over the activations.
@@ -130,9 +131,14 @@ struct Scheduler {
   }
 };
 
-// DEEP_EPI trades operand ring depth for epilogue staging: the TMA reduce-add (a read-modify-write in L2) has a
-// long latency, and with two 4 KB slabs per warp only 32 KB per SM are in flight; six slabs per warp keep the
-// gradient accumulation of the short-K expert weight-gradient tiles fed.
+// DEEP_EPI trades operand ring depth for epilogue staging: accumulating into the gradient buffer has a long latency, and
+// with two 4 KB slabs per warp only 32 KB per SM are in flight; five or six slabs per warp keep the accumulation of the
+// short-K expert weight-gradient tiles fed. bf16 accumulators go out as TMA reduce-adds (read-modify-write in L2, 5.8 TB/s).
+// For fp32 that unit is the bound (4.7 TB/s of reads and writes where plain copies reach 6.9), so the epilogue warps
+// read-modify-write themselves (epi 3): TMA loads bring the old slabs in ahead of the accumulators, across tiles, the sum is
+// made in shared memory and stored by TMA. Every element belongs to one tile of the launch, so no load overtakes a store.
+// Measured, 256 rows an expert, reduce-add / epi 3: 128 x [1536, 2048] 681 / 584 us, 32 x [5760, 2880] 926 / 796,
+// 256 x [1024, 2048] 883 / 760, 64 x [2816, 2048] (192 rows) 618 / 524.
 template <int BN, bool A_MN, bool B_MN, bool A_GATHER, bool DEEP_EPI>
 __global__ void __launch_bounds__(192, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -153,19 +159,22 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* empty = full + STAGES;
   uint64_t* tmem_full = empty + STAGES;
   uint64_t* tmem_empty = tmem_full + 2;
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  uint64_t* d_full = tmem_empty + 2;  // DEEP_EPI: an old slab has arrived, per warp and slab
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(d_full + (DEEP_EPI ? EPI_WARPS * NSTG : 0));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    if (DEEP_EPI)
+      for (int s = 0; s < EPI_WARPS * NSTG; ++s) mbar_init(&d_full[s], 1);
     for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], EPI_WARPS); }
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
-    if (args.use_tma_store || args.epi == 2) tma_prefetch_desc(&tmD);
+    if (args.use_tma_store || args.epi >= 2) tma_prefetch_desc(&tmD);
   }
   if (warp == 1) {
     tmem_alloc(tmem_ptr, TMEM_COLS);
@@ -341,7 +350,31 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     TileInfo ti;
     uint32_t tc = 0;
     bool used_tma = false;
-    uint32_t slab = 0;  // rotation through the staging slabs of this warp (TMA reduce epilogue)
+    uint32_t slab = 0;  // rotation through the staging slabs of this warp (TMA reduce and epi 3)
+    // epi 3: a second walk over the tiles, NSTG slabs ahead, that fetches the old values (state uniform over the warp)
+    Scheduler<BN> ahead(args);
+    TileInfo ta;
+    uint32_t fetched = 0;
+    int ta_c = 0;
+    bool ta_ok = false;
+    auto fetch = [&]() {
+      if (!ta_ok) return;
+      if (lane == 0) {
+        const int slot = q * NSTG + (int)(fetched % NSTG);
+        mbar_expect_tx(&d_full[slot], 4096);
+        tma_load_3d(staging + slot * 4096, &tmD, &d_full[slot], ta.col0 + ta_c * 32, ta.row0 + q * 32, (int)ta.d_off);
+      }
+      ++fetched;
+      ++ta_c;
+      if (ta_c * 32 >= BN || ta.col0 + ta_c * 32 >= args.N) {
+        ta_c = 0;
+        ta_ok = ahead.next(ta);
+      }
+    };
+    if (DEEP_EPI && args.epi == 3) {
+      ta_ok = ahead.next(ta);
+      for (int i = 0; i < NSTG; ++i) fetch();
+    }
     while (sch.next(ti)) {
       int acc = tc & 1;
       uint32_t aph = (tc >> 1) & 1;
@@ -391,6 +424,39 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tma_store_commit();
           }
         }
+      } else if (DEEP_EPI && args.epi == 3) {
+        used_tma = true;
+        bool good = true;
+#pragma unroll 1
+        for (int cc = 0; cc * 32 < BN; ++cc) {
+          if (ti.col0 + cc * 32 >= args.N) break;
+          const int slot = q * NSTG + (int)(slab % NSTG);
+          good = mbar_wait_bounded_warp(&d_full[slot], (slab / NSTG) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE);
+          if (!good) break;
+          ++slab;
+          uint8_t* st = staging + slot * 4096;
+          uint8_t* rowp = st + lane * 128;
+          uint32_t r0[32];
+          tmem_ld_32x32(taddr + cc * 32, r0);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            float4* p = reinterpret_cast<float4*>(rowp + ((j ^ (lane & 7)) << 4));
+            float4 o = *p;
+            o.x += __uint_as_float(r0[4 * j]); o.y += __uint_as_float(r0[4 * j + 1]);
+            o.z += __uint_as_float(r0[4 * j + 2]); o.w += __uint_as_float(r0[4 * j + 3]);
+            *p = o;
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&tmD, st, ti.col0 + cc * 32, ti.row0 + q * 32, (int)ti.d_off);
+            tma_store_commit();
+            tma_store_wait_read<1>();  // the slab before this one has been read: it takes the next old values
+          }
+          if (slab > 1) fetch();
+        }
+        if (!good) break;
       } else if (args.epi == 2 && args.accumulate && (args.mode != GEMM_MGROUP || full_tile)) {
         // ---- TMA reduce-add: stage a 32x(128 B) slab per warp, let the copy engine do D += slab
         used_tma = true;
@@ -562,6 +628,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (lane == 0) mbar_arrive(&tmem_empty[acc]);
       ++tc;
     }
+    if (DEEP_EPI && args.epi == 3 && lane == 0 && *abort_flag) {
+      // let fetches in flight land before the CTA retires (bounded)
+      const uint64_t t0 = globaltimer_ns();
+      for (uint32_t f = slab; f < fetched; ++f) {
+        const int slot = q * NSTG + (int)(f % NSTG);
+        while (!mbar_try_wait(&d_full[slot], (f / NSTG) & 1)) {
+          if (globaltimer_ns() - t0 > 20000000ull) {
+            if (args.err) atomicCAS(args.err, 0, PT_ERR_TIMEOUT_DRAIN);
+            break;
+          }
+        }
+      }
+    }
     if (used_tma && lane == 0) tma_store_wait_all<0>();
   }
 
@@ -576,7 +655,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 template <int BN, bool DEEP_EPI>
 constexpr int gemm_smem_bytes() {
   return (DEEP_EPI ? 3 : ((BN == 256) ? 4 : 6)) * (A_TILE_BYTES + BN * BK * 2) +
-         EPI_WARPS * (DEEP_EPI ? ((BN == 256) ? 5 : 6) : 2) * 4096 + 256 + 1024;
+         EPI_WARPS * (DEEP_EPI ? ((BN == 256) ? 5 : 6) : 2) * 4096 + 512 + 1024;
 }
 
 template <int BN, bool A_MN, bool B_MN, bool A_GATHER = false, bool DEEP_EPI = false>
@@ -654,7 +733,7 @@ PT_API int pt_gemm_bf16(const void* A, const void* B, void* D, int mode, int M, 
   args.offs = offs; args.offs2 = nullptr; args.b_group_rows = b_group_rows; args.D = D; args.ldd = ldd;
   args.d_group_stride = d_group_stride; args.out_fp32 = out_fp32; args.accumulate = accumulate;
   args.use_tma_store = tma_store_ok ? 1 : 0;
-  args.epi = epi;
+  args.epi = (tma_reduce && out_fp32 && mode == GEMM_KGROUP && a_mn && b_mn && !gather) ? 3 : epi;
   args.err = device_status_word();
   args.a_idx = a_idx; args.a_idx_div = a_idx_div > 0 ? a_idx_div : 1; args.a_idx_len = a_idx_len;
 
@@ -718,7 +797,7 @@ PT_API int pt_gemm_bf16_kgroup2(const void* A1, const void* B1, const int* offs1
   args.offs = offs1; args.offs2 = offs2; args.b_group_rows = 0; args.D = D; args.ldd = ldd;
   args.d_group_stride = d_group_stride; args.out_fp32 = out_fp32; args.accumulate = 1;
   args.use_tma_store = 0;
-  args.epi = 2;
+  args.epi = out_fp32 ? 3 : 2;
   args.err = device_status_word();
   args.a_idx = nullptr; args.a_idx_div = 1; args.a_idx_len = 0;
   const int grid = sm_count();

@@ -272,3 +272,35 @@ def test_combine_rows(n, H, k):
     for got, want in ((combine_rows(y, rows, k), picked.sum(1)), (combine_rows(y, rows, k, w, res), (picked * w.double()[..., None]).sum(1) + res.double())):
         # fp32 sums of k + 1 terms, one bf16 rounding
         assert ((got.double() - want).abs() <= BF16_MAX * want.abs() + 2.0 ** -20 * (k + 1) * 5).all()
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("sizes,N,K", [([16], 8, 8), ([0, 16, 80], 136, 40), ([48, 0, 0, 64], 264, 296), ([32] * 40, 392, 776)])
+def test_grouped_weight_gradient_into_fp32(sizes, N, K, pair):
+    """The prefetched read-modify-write epilogue: ragged tiles, empty groups (left alone), more tiles than CTAs, reproducible."""
+    from pithtrain_b200.ops import gemm as G
+
+    torch.manual_seed(N)
+    o = [0]
+    for s in sizes:
+        o.append(o[-1] + s)
+    offs = torch.tensor(o, dtype=torch.int32, device="cuda")
+    mk = lambda c: torch.randn(o[-1] + 16, c, device="cuda").bfloat16()  # noqa: E731
+    ops = [(mk(N), mk(K)) for _ in range(1 + pair)]
+    start = torch.randn(len(sizes), N, K, device="cuda")
+    want = start.double()
+    for dy, x in ops:
+        for g in range(len(sizes)):
+            want[g] += dy[o[g]:o[g + 1]].double().T @ x[o[g]:o[g + 1]].double()
+    outs = []
+    for _ in range(2):
+        out = start.clone()
+        if pair:
+            G.grouped_gemm_tn_pair(*ops[0], offs, *ops[1], offs, out)
+        else:
+            G.grouped_gemm_tn(*ops[0], offs, out, accumulate=True)
+        _native.check_status()
+        outs.append(out)
+    # fp32 accumulation of at most 2 x 80 products of size < 25
+    assert (outs[0].double() - want).abs().max() < 2.0 ** -24 * 160 * 25 * 2
+    assert torch.equal(outs[0], outs[1])
