@@ -247,6 +247,20 @@ def indexed_bias_add_rows(x: torch.Tensor, bias: torch.Tensor, offs: torch.Tenso
     return x + bias[gid].to(x.dtype)
 
 
+def row_bias_dot(x: torch.Tensor, bias: torch.Tensor, offs: torch.Tensor, slot_of_row: torch.Tensor, dw: torch.Tensor,
+                 n_rows: Optional[torch.Tensor] = None) -> None:
+    """``dw[slot_of_row[r]] += <x[r], bias[group(r)]>`` for expert-sorted rows (pad rows, slot -1, are skipped)."""
+    E, H = bias.shape
+    if use_native(x) and bias.dtype == torch.bfloat16 and H % 8 == 0 and x.is_contiguous() and bias.is_contiguous():
+        rc = _native.lib().pt_row_bias_dot(x.data_ptr(), bias.data_ptr(), offs.data_ptr(), E, slot_of_row.data_ptr(), dw.data_ptr(),
+                                           _native.ptr(n_rows), x.shape[0], H, sp())
+        _native.check(rc, "pt_row_bias_dot")
+        return
+    gid = rows_group_id(offs, x.shape[0]).clamp(max=E - 1)
+    live = slot_of_row >= 0
+    dw[slot_of_row[live].long()] += (x[live].float() * bias[gid[live]].float()).sum(-1)
+
+
 def rows_group_id(offs: torch.Tensor, R: int) -> torch.Tensor:
     row = torch.arange(R, device=offs.device)
     return torch.bucketize(row, offs[1:].long(), right=True)
@@ -366,30 +380,18 @@ class _MoEExpertsFn(torch.autograd.Function):
             del dq, dsc
         else:
             da = G.grouped_gemm_nn(dyg, ew.w2, offs)
-        plain = ew.b1 is None and ew.b2 is None
-        if plain:
-            # routing weights and their gradients are looked up / scattered through the slot index in the kernel
-            dgu, act_s, d_w_flat = swiglu_bwd(gu, da, w.reshape(-1), n_rows, ew.interleaved, ew.alpha, ew.limit,
-                                              want_act=True, want_dw=True, slot_of_row=slot_of_row)
-            d_row_w = row_w = None
-        else:
-            w_ext = torch.cat([w.reshape(-1).float(), w.new_zeros(1, dtype=torch.float32)])
-            row_w = w_ext[slot_of_row.long()]  # -1 (pad) picks the appended zero
-            dgu, act_s, d_row_w = swiglu_bwd(gu, da, row_w, n_rows, ew.interleaved, ew.alpha, ew.limit,
-                                             want_act=True, want_dw=True)
+        # routing weights and their gradients are looked up / scattered through the slot index in the kernel
+        dgu, act_s, d_w_flat = swiglu_bwd(gu, da, w.reshape(-1), n_rows, ew.interleaved, ew.alpha, ew.limit,
+                                          want_act=True, want_dw=True, slot_of_row=slot_of_row)
         del da
         if ew.b2 is not None:
             # y = act @ W2.T + b2 ; the routing-weight gradient also sees the bias term
-            gid = rows_group_id(offs, gu.shape[0]).clamp(max=E - 1)
-            d_row_w = d_row_w + (dyg.float() * ew.b2.detach()[gid].float()).sum(-1)
+            row_bias_dot(dyg, ew.b2.detach(), offs, slot_of_row, d_w_flat, n_rows)
+            row_w = w.reshape(-1).float()[slot_of_row.clamp(min=0)]  # pad rows of dyg are zero, whatever their weight
             accumulate_grad(ew.b2, segment_sum(dyg, offs, E, row_w=row_w))
         if ew.b1 is not None:
             accumulate_grad(ew.b1, segment_sum(dgu, offs, E))
-        if plain:
-            d_w = d_w_flat.view(w.shape).to(w.dtype)
-        else:
-            dw_ext = torch.cat([d_row_w, d_row_w.new_zeros(1)])
-            d_w = dw_ext[row_of_slot.long()].view(w.shape).to(w.dtype)
+        d_w = d_w_flat.view(w.shape).to(w.dtype)
         if ctx.fp8:
             _, _, q1t, s1t = F8.quantized_weight(ew.w1)
             gq, gsc = quant_rows(dgu, n_rows=n_rows)

@@ -304,3 +304,33 @@ def test_grouped_weight_gradient_into_fp32(sizes, N, K, pair):
     # fp32 accumulation of at most 2 x 80 products of size < 25
     assert (outs[0].double() - want).abs().max() < 2.0 ** -24 * 160 * 25 * 2
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("sizes", [[16], [0, 48, 16], [272, 0, 16, 528]])
+@pytest.mark.parametrize("H", [8, 264, 2880])
+def test_segment_sum_and_row_bias_dot(sizes, H):
+    from pithtrain_b200.ops.moe import row_bias_dot, segment_sum
+
+    torch.manual_seed(H)
+    o = [0]
+    for s in sizes:
+        o.append(o[-1] + s)
+    R, E = o[-1] + 32, len(sizes)
+    offs = torch.tensor(o, dtype=torch.int32, device="cuda")
+    x, bias, w = torch.randn(R, H, device="cuda").bfloat16(), torch.randn(E, H, device="cuda").bfloat16(), torch.rand(R, device="cuda")
+    slots = torch.full((R,), -1, dtype=torch.int32, device="cuda")
+    slots[: o[-1]] = torch.randperm(o[-1], device="cuda").int()
+    slots[: o[-1] : 7] = -1
+    group = torch.cat([torch.full((s,), g, device="cuda") for g, s in enumerate(sizes)])
+    for t in (x, x.float()):
+        for rw in (None, w):
+            want = torch.zeros(E, H, dtype=torch.float64, device="cuda")
+            want.index_add_(0, group, t[: o[-1]].double() * (1.0 if rw is None else rw[: o[-1], None].double()))
+            got = segment_sum(t, offs, E, rw)
+            assert (got.double() - want).abs().max() < 2.0 ** -24 * max(sizes) * 5 * 24
+    dw = torch.randn(o[-1], device="cuda")
+    want = dw.double()
+    live = slots[: o[-1]] >= 0
+    want[slots[: o[-1]][live].long()] += (x[: o[-1]][live].double() * bias[group[live]].double()).sum(-1)
+    row_bias_dot(x, bias, offs, slots, dw, offs[E:E + 1])
+    assert (dw.double() - want).abs().max() < 2.0 ** -24 * H * 25 * 16
