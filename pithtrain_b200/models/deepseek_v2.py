@@ -19,6 +19,7 @@ import torch.nn.functional as F
 
 from ..contexts import distributed
 from ..modules.load_balance import MoELoadBalanceLossInjector
+from ..ops import mla
 from ..ops.attention import attention, attention_ref
 from ..ops.linear import FusedWeights, Linear, fused_linear
 from ..ops.norm import RMSNorm, rmsnorm_ref
@@ -156,8 +157,26 @@ class DeepSeekV2Attention(nn.Module):
         cos, sin = cos.view(B, S, -1).to(q_pe.dtype), sin.view(B, S, -1).to(q_pe.dtype)
         return apply_rope_ref(interleaved_to_half(q_pe), cos, sin), apply_rope_ref(interleaved_to_half(k_pe), cos, sin)
 
+    def _assembled(self, x, rotary: RotaryPos):
+        """q, k ``[B,S,nh,192]`` and v ``[B,S,nh,128]`` through the assembly kernel (one rank's own sequence)."""
+        B, S, H = x.shape
+        n, nh, dn, dr, dv = B * S, self.num_heads, self.qk_nope_head_dim, self.qk_rope_head_dim, self.v_head_dim
+        both = fused_linear(x.view(n, H), self.fused_in)
+        n_first = self.fused_in.params[0].shape[0]
+        q, compressed, k_pe = mla.split_columns(both, (n_first, self.kv_lora_rank, dr))
+        if self.q_lora_rank is not None:
+            q = self.q_b_proj(self.q_a_layernorm(q))
+        kvb = self.kv_b_proj(self.kv_a_layernorm(compressed))
+        q, k, v = mla.mla_assemble(q, k_pe, kvb, rotary.cos, rotary.sin, rotary.token_positions(n), rotary.S, nh, dn, dr, dv)
+        return q.view(B, S, nh, dn + dr), k.view(B, S, nh, dn + dr), v.view(B, S, nh, dv)
+
     def forward(self, x, rotary: RotaryPos, cu_seqlens=None, reference: bool = False):
         B, S, _ = x.shape
+        if not reference and distributed.cp_size == 1 and mla.supported(x, rotary.cos, self.num_heads, self.qk_nope_head_dim,
+                                                                        self.qk_rope_head_dim, self.v_head_dim):
+            q, k, v = self._assembled(x, rotary)
+            o = attention(q, k, v, causal=True, scale=self.softmax_scale, cu_seqlens=cu_seqlens)
+            return self.o_proj(o.reshape(B, S, self.num_heads * self.v_head_dim))
         q_nope, q_pe, normed_kv, k_pe = self._project(x, reference)
         q_pe, k_pe = self._rope(q_pe, k_pe, rotary)
         if distributed.cp_size > 1 and not reference:

@@ -306,6 +306,45 @@ def test_grouped_weight_gradient_into_fp32(sizes, N, K, pair):
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("positions", [False, True])
+@pytest.mark.parametrize("n,S,H,dn,dr,dv", [(1, 1, 1, 8, 16, 8), (6, 3, 2, 128, 64, 128), (67, 67, 16, 128, 64, 128), (10, 5, 3, 24, 32, 40)])
+def test_mla_assembly(n, S, H, dn, dr, dv, positions):
+    from pithtrain_b200.ops import mla
+
+    torch.manual_seed(n)
+    wide = torch.randn(n, H * (dn + dr) + 40 + dr, device="cuda").bfloat16()  # q | latent | k_pe, as the fused projection writes them
+    kv = torch.randn(n, H * (dn + dv), device="cuda").bfloat16()
+    ang = torch.rand(S + 3, dr // 2, device="cuda") * 6
+    cos, sin = (torch.cat([f(ang)] * 2, -1).bfloat16() for f in (torch.cos, torch.sin))
+    pos = torch.randint(0, S + 3, (n,), device="cuda") if positions else None
+    go = [torch.randn(n, H, d, device="cuda").bfloat16() for d in (dn + dr, dn + dr, dv)]
+    assert mla.supported(wide, cos, H, dn, dr, dv)
+
+    def leaves(dtype):
+        return [t.to(dtype).requires_grad_() for t in (wide.clone(), kv.clone())]
+
+    wl, kl = leaves(torch.bfloat16)
+    q, lat, kp = mla.split_columns(wl, (H * (dn + dr), 40, dr))
+    got = mla.mla_assemble(q, kp, kl, cos, sin, pos, S, H, dn, dr, dv)
+    torch.autograd.backward((*got, lat), (*go, torch.ones_like(lat)))
+    wd, kd = leaves(torch.float64)
+    p = pos if positions else torch.arange(n, device="cuda") % S
+    c, s = cos[p].double()[:, None], sin[p].double()[:, None]
+
+    def rope(t):
+        t = t.unflatten(-1, (dr // 2, 2)).transpose(-1, -2).flatten(-2)
+        return t * c + torch.cat([-t[..., dr // 2:], t[..., : dr // 2]], -1) * s
+
+    qd, ld, pd = wd.split((H * (dn + dr), 40, dr), -1)
+    qd, kvd = qd.view(n, H, -1), kd.view(n, H, -1)
+    want = (torch.cat([qd[..., :dn], rope(qd[..., dn:])], -1), torch.cat([kvd[..., :dn], rope(pd[:, None]).expand(-1, H, -1)], -1), kvd[..., dn:])
+    torch.autograd.backward((*want, ld), (*(g.double() for g in go), torch.ones_like(ld)))
+    for a, b in ((*zip(got, want), (wl.grad, wd.grad), (kl.grad, kd.grad))):
+        # a rotation of two terms in fp32 (a sum of H of them for the shared key), rounded once
+        a, b = a.detach().double(), b.detach()
+        assert ((a - b).abs() <= BF16_MAX * b.abs() + 1e-6 * H * 5).all()
+
+
 @pytest.mark.parametrize("sizes", [[16], [0, 48, 16], [272, 0, 16, 528]])
 @pytest.mark.parametrize("H", [8, 264, 2880])
 def test_segment_sum_and_row_bias_dot(sizes, H):
