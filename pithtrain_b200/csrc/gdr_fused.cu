@@ -21,14 +21,19 @@
 // operands from shared memory in 16-byte pieces, 8 to 11 FMA per piece, tiles padded to 132 or 68 columns so that the eight
 // threads of a phase hit different banks. The sequential kernels prefetch the next chunk with cp.async.
 //
-// Measured, 1 x 3072, 32 heads (48 chunks): chunk_fwd 224, scan_fwd 279, out 242, dvp 50, scan_bwd 393, chunk_bwd 1122 us; the
-// tensor-op form with the recurrence kernels of csrc/gdr.cu took about 8 ms for the two directions.
+// A product phase of a chunk kernel has eight warps and nothing beside it, so what it needs is fetched before it: tiles by
+// cp.async under the phase in front, rows of q, k and v into registers.
+// Measured, 1 x 3072, 32 heads (48 chunks): chunk_fwd 202, scan_fwd 280, out 129, dvp 50, scan_bwd 383, chunk_bwd 802 us; with
+// plain loads between the phases out took 242 and chunk_bwd 1122. The tensor-op form with the recurrence kernels of csrc/gdr.cu
+// took about 8 ms for the two directions. Counters of chunk_bwd before: issue slots 28 %, waits for global memory 2.7 per issue.
 // The sums of a row or column are made in a fixed order: results are reproducible.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "elementwise.cuh"
 #include "host_common.h"
+#include "ptx.cuh"
 
 namespace pt {
 namespace gdr {
@@ -56,15 +61,20 @@ struct Args {
   float scale;
 };
 
-// e^x with the rounding of x * log2(e) compensated (the build's fast expf loses |x| ulp)
-__device__ __forceinline__ float exp_c(float x) {
-  const float t = x * 1.4426950408889634f;
-  const float r = fmaf(x, 1.4426950408889634f, -t) + x * 1.92596299e-8f;
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(t));
-  return fmaf(y, r * 0.6931471805599453f, y);
-}
+__device__ __forceinline__ float exp_c(float x) { return exp_compensated(x); }
 
+// Two fp32 FMAs in one instruction (fma.rn.f32x2, same rounding as two fmaf): half the issue slots beside the loads.
+typedef uint64_t f2;
+struct Pair2 { f2 lo, hi; };  // a 16-byte piece as two packed pairs
+__device__ __forceinline__ Pair2 ld2(const float* p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return Pair2{v.x, v.y};
+}
+__device__ __forceinline__ float sum2(f2 v) {
+  float a, b;
+  f2_unpack(v, a, b);
+  return a + b;
+}
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) { *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d); }
 __device__ __forceinline__ float4 bf4(uint2 r) {
@@ -85,35 +95,63 @@ __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0
 // Thread layout of every 64-row product: ti = tid / 16, tj = tid % 16; rows ti + 16 r (r < 4). Columns of a 64-column result:
 // tj + 16 c (c < 4); of a 128-column result: 4 tj + 64 h + e, index x = 4 h + e (h < 2, e < 4).
 
-// acc[r][c] += sum_d A[ti + 16 r][d] * B[tj + 16 c][d]
+// acc[r][c] += sum_d A[ti + 16 r][d] * B[tj + 16 c][d] (even and odd d in the two halves of a packed sum)
 __device__ __forceinline__ void mm_nt64(const float* A, const float* B, float (&acc)[4][4]) {
   const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
+  f2 s[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) s[r][c] = 0ull;
 #pragma unroll 2
   for (int d = 0; d < D; d += 4) {
-    float4 a[4], b[4];
+    Pair2 a[4], b[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) a[r] = ld4(A + (ti + 16 * r) * LD + d);
+    for (int r = 0; r < 4; ++r) a[r] = ld2(A + (ti + 16 * r) * LD + d);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) b[c] = ld4(B + (tj + 16 * c) * LD + d);
+    for (int c = 0; c < 4; ++c) b[c] = ld2(B + (tj + 16 * c) * LD + d);
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        acc[r][c] = fmaf(a[r].x, b[c].x, acc[r][c]);
-        acc[r][c] = fmaf(a[r].y, b[c].y, acc[r][c]);
-        acc[r][c] = fmaf(a[r].z, b[c].z, acc[r][c]);
-        acc[r][c] = fmaf(a[r].w, b[c].w, acc[r][c]);
-      }
+      for (int c = 0; c < 4; ++c) s[r][c] = f2_fma(a[r].hi, b[c].hi, f2_fma(a[r].lo, b[c].lo, s[r][c]));
   }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[r][c] += sum2(s[r][c]);
 }
-__device__ __forceinline__ void fma8(float a, float4 p, float4 q, float (&acc)[8]) {
-  acc[0] = fmaf(a, p.x, acc[0]); acc[1] = fmaf(a, p.y, acc[1]); acc[2] = fmaf(a, p.z, acc[2]); acc[3] = fmaf(a, p.w, acc[3]);
-  acc[4] = fmaf(a, q.x, acc[4]); acc[5] = fmaf(a, q.y, acc[5]); acc[6] = fmaf(a, q.z, acc[6]); acc[7] = fmaf(a, q.w, acc[7]);
+// acc[0..8) += a * (p, q): four packed FMAs
+__device__ __forceinline__ void fma8(float a, const Pair2& p, const Pair2& q, f2 (&acc)[4]) {
+  const f2 aa = f2_pack(a, a);
+  acc[0] = f2_fma(aa, p.lo, acc[0]);
+  acc[1] = f2_fma(aa, p.hi, acc[1]);
+  acc[2] = f2_fma(aa, q.lo, acc[2]);
+  acc[3] = f2_fma(aa, q.hi, acc[3]);
+}
+// m += x * p, n += y * p for a piece p of four
+__device__ __forceinline__ void fma4x2(float x, float y, const Pair2& p, f2 (&m)[2], f2 (&n)[2]) {
+  const f2 xx = f2_pack(x, x), yy = f2_pack(y, y);
+  m[0] = f2_fma(xx, p.lo, m[0]); m[1] = f2_fma(xx, p.hi, m[1]);
+  n[0] = f2_fma(yy, p.lo, n[0]); n[1] = f2_fma(yy, p.hi, n[1]);
+}
+__device__ __forceinline__ void pack8(const float (&a)[4][8], f2 (&s)[4][4]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) s[r][x] = f2_pack(a[r][2 * x], a[r][2 * x + 1]);
+}
+__device__ __forceinline__ void unpack8(const f2 (&s)[4][4], float (&a)[4][8]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) f2_unpack(s[r][x], a[r][2 * x], a[r][2 * x + 1]);
 }
 // acc[r][x] += sum_{j < K} A[ti + 16 r][j] * B[j][col x]; pitches LA and LB
 template <int K, int LA, int LB>
 __device__ __forceinline__ void mm_nn(const float* A, const float* B, float (&acc)[4][8]) {
   const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
+  f2 s[4][4];
+  pack8(acc, s);
 #pragma unroll 2
   for (int j = 0; j < K; j += 4) {
     float4 a[4];
@@ -121,21 +159,25 @@ __device__ __forceinline__ void mm_nn(const float* A, const float* B, float (&ac
     for (int r = 0; r < 4; ++r) a[r] = ld4(A + (ti + 16 * r) * LA + j);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const float4 p = ld4(B + (j + e) * LB + 4 * tj), q = ld4(B + (j + e) * LB + 4 * tj + 64);
+      const Pair2 p = ld2(B + (j + e) * LB + 4 * tj), q = ld2(B + (j + e) * LB + 4 * tj + 64);
 #pragma unroll
-      for (int r = 0; r < 4; ++r) fma8(e == 0 ? a[r].x : e == 1 ? a[r].y : e == 2 ? a[r].z : a[r].w, p, q, acc[r]);
+      for (int r = 0; r < 4; ++r) fma8(e == 0 ? a[r].x : e == 1 ? a[r].y : e == 2 ? a[r].z : a[r].w, p, q, s[r]);
     }
   }
+  unpack8(s, acc);
 }
 // acc[r][x] += sum_{j < 64} A[j][ti + 16 r] * B[j][col x]; A pitch LS, B pitch LD
 __device__ __forceinline__ void mm_tn(const float* A, const float* B, float (&acc)[4][8]) {
   const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
+  f2 s[4][4];
+  pack8(acc, s);
 #pragma unroll 4
   for (int j = 0; j < C; ++j) {
-    const float4 p = ld4(B + j * LD + 4 * tj), q = ld4(B + j * LD + 4 * tj + 64);
+    const Pair2 p = ld2(B + j * LD + 4 * tj), q = ld2(B + j * LD + 4 * tj + 64);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) fma8(A[j * LS + ti + 16 * r], p, q, acc[r]);
+    for (int r = 0; r < 4; ++r) fma8(A[j * LS + ti + 16 * r], p, q, s[r]);
   }
+  unpack8(s, acc);
 }
 // A [128 x 128] tile whose rows are read as columns of a 128-column result: row d lies at physical row state_row(d), so that
 // the threads tj of a phase read neighbouring physical rows (tj + 16 x).
@@ -143,23 +185,27 @@ __device__ __forceinline__ int state_row(int d) { return ((d & 63) >> 2) + 16 * 
 // acc[r][x] += sum_v A[ti + 16 r][v] * St[col x][v]
 __device__ __forceinline__ void mm_nt128(const float* A, const float* St, float (&acc)[4][8]) {
   const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
+  f2 s[4][8];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int x = 0; x < 8; ++x) s[r][x] = 0ull;
 #pragma unroll 1
   for (int v = 0; v < D; v += 4) {
-    float4 a[4];
+    Pair2 a[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) a[r] = ld4(A + (ti + 16 * r) * LD + v);
+    for (int r = 0; r < 4; ++r) a[r] = ld2(A + (ti + 16 * r) * LD + v);
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
-      const float4 s = ld4(St + (tj + 16 * x) * LD + v);
+      const Pair2 b = ld2(St + (tj + 16 * x) * LD + v);
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        acc[r][x] = fmaf(a[r].x, s.x, acc[r][x]);
-        acc[r][x] = fmaf(a[r].y, s.y, acc[r][x]);
-        acc[r][x] = fmaf(a[r].z, s.z, acc[r][x]);
-        acc[r][x] = fmaf(a[r].w, s.w, acc[r][x]);
-      }
+      for (int r = 0; r < 4; ++r) s[r][x] = f2_fma(a[r].hi, b.hi, f2_fma(a[r].lo, b.lo, s[r][x]));
     }
   }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int x = 0; x < 8; ++x) acc[r][x] += sum2(s[r][x]);
 }
 template <int R, int X>
 __device__ __forceinline__ void zero(float (&a)[R][X]) {
@@ -175,26 +221,40 @@ __device__ __forceinline__ float row_sum(float v) {
   return v;
 }
 
-// [64 x 128] bf16 rows of one head -> fp32 tile, each row times rs[i] (null: 1); rows past the sequence are zero.
+// [64 x 128] bf16 rows of one head -> fp32 tile, each row times rs[i] (null: 1); rows past the sequence are zero. All loads are
+// in flight before the first is used: between two products nothing else hides their latency.
 __device__ __forceinline__ void load_bf16(float* dst, const __nv_bfloat16* src, long long pitch, int rows, const float* rs) {
-  for (int i = threadIdx.x; i < C * (D / 8); i += NT) {
-    const int r = i >> 4, c = (i & 15) * 8;
-    uint4 x = make_uint4(0u, 0u, 0u, 0u);
-    if (r < rows) x = *reinterpret_cast<const uint4*>(src + r * pitch + c);
+  constexpr int IT = C * (D / 8) / NT;
+  uint4 x[IT];
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int i = threadIdx.x + it * NT, r = i >> 4;
+    x[it] = make_uint4(0u, 0u, 0u, 0u);
+    if (r < rows) x[it] = *reinterpret_cast<const uint4*>(src + r * pitch + (i & 15) * 8);
+  }
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int i = threadIdx.x + it * NT, r = i >> 4, c = (i & 15) * 8;
     const float f = rs ? rs[r] : 1.f;
-    const float4 a = bf4(make_uint2(x.x, x.y)), b = bf4(make_uint2(x.z, x.w));
+    const float4 a = bf4(make_uint2(x[it].x, x[it].y)), b = bf4(make_uint2(x[it].z, x[it].w));
     st4(dst + r * LD + c, a.x * f, a.y * f, a.z * f, a.w * f);
     st4(dst + r * LD + c + 4, b.x * f, b.y * f, b.z * f, b.w * f);
   }
 }
-// fp32 [64 x 128] -> padded tile, and [64 x 64] -> padded tile
+// fp32 [64 x 128] and [64 x 64] -> padded tiles, asynchronously (cp_commit / cp_wait by the caller)
 __device__ __forceinline__ void load_f32(float* dst, const float* src) {
-  for (int i = threadIdx.x; i < C * (D / 4); i += NT)
-    *reinterpret_cast<float4*>(dst + (i >> 5) * LD + (i & 31) * 4) = reinterpret_cast<const float4*>(src)[i];
+#pragma unroll
+  for (int it = 0; it < C * (D / 4) / NT; ++it) {
+    const int i = threadIdx.x + it * NT;
+    cp16(dst + (i >> 5) * LD + (i & 31) * 4, src + i * 4, 16);
+  }
 }
 __device__ __forceinline__ void load_sq(float* dst, const float* src) {
-  for (int i = threadIdx.x; i < C * (C / 4); i += NT)
-    *reinterpret_cast<float4*>(dst + (i >> 4) * LS + (i & 15) * 4) = reinterpret_cast<const float4*>(src)[i];
+#pragma unroll
+  for (int it = 0; it < C * (C / 4) / NT; ++it) {
+    const int i = threadIdx.x + it * NT;
+    cp16(dst + (i >> 4) * LS + (i & 15) * 4, src + i * 4, 16);
+  }
 }
 // result rows ti + 16 r, 8 columns -> fp32 [64 x 128]
 __device__ __forceinline__ void store_f32(float* dst, const float (&a)[4][8]) {
@@ -399,18 +459,17 @@ __global__ void __launch_bounds__(NT) gdr_scan_fwd_kernel(const Args p) {
     for (int i = tid; i < D * (VS / 4); i += NT)
       *reinterpret_cast<float4*>(so + (i >> 3) * D + (i & 7) * 4) = ld4(S + (i >> 3) * LV + (i & 7) * 4);
     const float* Ws = W + s * T64;
-    float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f};
+    f2 m0[2] = {0ull, 0ull}, m1[2] = {0ull, 0ull};
 #pragma unroll 4
     for (int d = 0; d < D; d += 4) {
       const float4 x = ld4(Ws + r8 * LD + d), y = ld4(Ws + (r8 + 32) * LD + d);
       const float xa[4] = {x.x, x.y, x.z, x.w}, ya[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float4 t = ld4(S + (d + e) * LV + c4);
-        a0[0] = fmaf(xa[e], t.x, a0[0]); a0[1] = fmaf(xa[e], t.y, a0[1]); a0[2] = fmaf(xa[e], t.z, a0[2]); a0[3] = fmaf(xa[e], t.w, a0[3]);
-        a1[0] = fmaf(ya[e], t.x, a1[0]); a1[1] = fmaf(ya[e], t.y, a1[1]); a1[2] = fmaf(ya[e], t.z, a1[2]); a1[3] = fmaf(ya[e], t.w, a1[3]);
-      }
+      for (int e = 0; e < 4; ++e) fma4x2(xa[e], ya[e], ld2(S + (d + e) * LV + c4), m0, m1);
     }
+    float a0[4], a1[4];
+    f2_unpack(m0[0], a0[0], a0[1]); f2_unpack(m0[1], a0[2], a0[3]);
+    f2_unpack(m1[0], a1[0], a1[1]); f2_unpack(m1[1], a1[2], a1[3]);
     const float* Gs = G + s * C;
     const float gl = Gs[C - 1], a = exp_c(gl);
     float* vo = p.vn + ((long long)bh * p.N + n) * C * D + vs + c4;
@@ -425,25 +484,23 @@ __global__ void __launch_bounds__(NT) gdr_scan_fwd_kernel(const Args p) {
       st4(V + r * LV + c4, v.x * f, v.y * f, v.z * f, v.w * f);
     }
     __syncthreads();
-    float acc[4][4];
+    f2 acc[4][2];
     const __nv_bfloat16* Ks = Kb + s * C * LK + 4 * r8;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float4 t = ld4(S + (4 * r8 + e) * LV + c4);
-      acc[e][0] = a * t.x; acc[e][1] = a * t.y; acc[e][2] = a * t.z; acc[e][3] = a * t.w;
+      acc[e][0] = f2_pack(a * t.x, a * t.y);
+      acc[e][1] = f2_pack(a * t.z, a * t.w);
     }
 #pragma unroll 8
     for (int j = 0; j < C; ++j) {
-      const float4 k = bf4(*reinterpret_cast<const uint2*>(Ks + j * LK)), v = ld4(V + j * LV + c4);
-      const float ka[4] = {k.x, k.y, k.z, k.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        acc[e][0] = fmaf(ka[e], v.x, acc[e][0]); acc[e][1] = fmaf(ka[e], v.y, acc[e][1]);
-        acc[e][2] = fmaf(ka[e], v.z, acc[e][2]); acc[e][3] = fmaf(ka[e], v.w, acc[e][3]);
-      }
+      const float4 k = bf4(*reinterpret_cast<const uint2*>(Ks + j * LK));
+      const Pair2 v = ld2(V + j * LV + c4);
+      fma4x2(k.x, k.y, v, acc[0], acc[1]);
+      fma4x2(k.z, k.w, v, acc[2], acc[3]);
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) st4(S + (4 * r8 + e) * LV + c4, acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
+    for (int e = 0; e < 4; ++e) *reinterpret_cast<ulonglong2*>(S + (4 * r8 + e) * LV + c4) = make_ulonglong2(acc[e][0], acc[e][1]);
     __syncthreads();
   }
 }
@@ -459,15 +516,26 @@ __global__ void __launch_bounds__(NT) gdr_out_kernel(const Args p) {
   const Where x = where(p, blockIdx.x, blockIdx.y);
   const int tid = threadIdx.x, ti = tid >> 4, tj = tid & 15, v0 = blockIdx.z * 64;
   const long long id = (long long)x.bh * p.N + x.n;
+#pragma unroll
+  for (int it = 0; it < D * 16 / NT; ++it) {
+    const int i = tid + it * NT;
+    cp16(S + (i >> 4) * LH + (i & 15) * 4, p.st + id * D * D + (i >> 4) * D + v0 + (i & 15) * 4, 16);
+  }
+#pragma unroll
+  for (int it = 0; it < C * 16 / NT; ++it) {
+    const int i = tid + it * NT;
+    cp16(V + (i >> 4) * LH + (i & 15) * 4, p.vn + id * C * D + (i >> 4) * D + v0 + (i & 15) * 4, 16);
+  }
+  load_sq(P, p.P + id * C * C);
+  cp_commit();
   if (tid < C) f[tid] = p.scale * exp_c(p.gc[id * C + tid]);
   __syncthreads();
   load_bf16(Q, p.q + x.b * p.q_b + x.s0 * p.q_s + x.h * p.q_h, p.q_s, x.rows, f);
-  load_sq(P, p.P + id * C * C);
-  for (int i = tid; i < D * 16; i += NT) *reinterpret_cast<float4*>(S + (i >> 4) * LH + (i & 15) * 4) = ld4(p.st + id * D * D + (i >> 4) * D + v0 + (i & 15) * 4);
-  for (int i = tid; i < C * 16; i += NT) *reinterpret_cast<float4*>(V + (i >> 4) * LH + (i & 15) * 4) = ld4(p.vn + id * C * D + (i >> 4) * D + v0 + (i & 15) * 4);
+  cp_wait<0>();
   __syncthreads();
-  float acc[4][4];
-  zero(acc);
+  f2 s2[4][2];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) s2[r][0] = s2[r][1] = 0ull;
   auto product = [&](const float* A, int la, const float* B, int K) {
 #pragma unroll 2
     for (int j = 0; j < K; j += 4) {
@@ -476,12 +544,12 @@ __global__ void __launch_bounds__(NT) gdr_out_kernel(const Args p) {
       for (int r = 0; r < 4; ++r) a[r] = ld4(A + (ti + 16 * r) * la + j);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float4 b = ld4(B + (j + e) * LH + 4 * tj);
+        const Pair2 b = ld2(B + (j + e) * LH + 4 * tj);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+        for (int r = 0; r < 4; r += 2) {
           const float y = e == 0 ? a[r].x : e == 1 ? a[r].y : e == 2 ? a[r].z : a[r].w;
-          acc[r][0] = fmaf(y, b.x, acc[r][0]); acc[r][1] = fmaf(y, b.y, acc[r][1]);
-          acc[r][2] = fmaf(y, b.z, acc[r][2]); acc[r][3] = fmaf(y, b.w, acc[r][3]);
+          const float z = e == 0 ? a[r + 1].x : e == 1 ? a[r + 1].y : e == 2 ? a[r + 1].z : a[r + 1].w;
+          fma4x2(y, z, b, s2[r], s2[r + 1]);
         }
       }
     }
@@ -491,9 +559,11 @@ __global__ void __launch_bounds__(NT) gdr_out_kernel(const Args p) {
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int i = ti + 16 * r;
+    float o[4];
+    f2_unpack(s2[r][0], o[0], o[1]);
+    f2_unpack(s2[r][1], o[2], o[3]);
     if (i < x.rows)
-      *reinterpret_cast<uint2*>(p.o + (((long long)x.b * p.S + x.s0 + i) * p.H + x.h) * D + v0 + 4 * tj) =
-          pack4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+      *reinterpret_cast<uint2*>(p.o + (((long long)x.b * p.S + x.s0 + i) * p.H + x.h) * D + v0 + 4 * tj) = pack4(o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -505,8 +575,10 @@ __global__ void __launch_bounds__(NT) gdr_dvp_kernel(const Args p) {
   float *X = sm, *P = X + T64;
   const Where x = where(p, blockIdx.x, blockIdx.y);
   const long long id = (long long)x.bh * p.N + x.n;
-  load_bf16(X, p.d_o + (((long long)x.b * p.S + x.s0) * p.H + x.h) * D, (long long)p.H * D, x.rows, nullptr);
   load_sq(P, p.P + id * C * C);
+  cp_commit();
+  load_bf16(X, p.d_o + (((long long)x.b * p.S + x.s0) * p.H + x.h) * D, (long long)p.H * D, x.rows, nullptr);
+  cp_wait<0>();
   __syncthreads();
   float acc[4][8];
   zero(acc);
@@ -555,19 +627,18 @@ __global__ void __launch_bounds__(NT) gdr_scan_bwd_kernel(const Args p) {
       *reinterpret_cast<float4*>(so + (i >> 3) * D + (i & 7) * 4) = ld4(S + (i >> 3) * LV + (i & 7) * 4);
     const float* Gs = G + s * C;
     const float gl = Gs[C - 1], a = exp_c(gl);
-    float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f};
+    f2 m0[2] = {0ull, 0ull}, m1[2] = {0ull, 0ull};
     const __nv_bfloat16* Ks = Kb + s * C * LK;
 #pragma unroll 4
     for (int d = 0; d < D; d += 4) {
       const float4 x = bf4(*reinterpret_cast<const uint2*>(Ks + r8 * LK + d)), y = bf4(*reinterpret_cast<const uint2*>(Ks + (r8 + 32) * LK + d));
       const float xa[4] = {x.x, x.y, x.z, x.w}, ya[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float4 t = ld4(S + (d + e) * LV + c4);
-        a0[0] = fmaf(xa[e], t.x, a0[0]); a0[1] = fmaf(xa[e], t.y, a0[1]); a0[2] = fmaf(xa[e], t.z, a0[2]); a0[3] = fmaf(xa[e], t.w, a0[3]);
-        a1[0] = fmaf(ya[e], t.x, a1[0]); a1[1] = fmaf(ya[e], t.y, a1[1]); a1[2] = fmaf(ya[e], t.z, a1[2]); a1[3] = fmaf(ya[e], t.w, a1[3]);
-      }
+      for (int e = 0; e < 4; ++e) fma4x2(xa[e], ya[e], ld2(S + (d + e) * LV + c4), m0, m1);
     }
+    float a0[4], a1[4];
+    f2_unpack(m0[0], a0[0], a0[1]); f2_unpack(m0[1], a0[2], a0[3]);
+    f2_unpack(m1[0], a1[0], a1[1]); f2_unpack(m1[1], a1[2], a1[3]);
     float* vo = p.dvn + ((long long)bh * p.N + n) * C * D + vs + c4;
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
@@ -583,29 +654,26 @@ __global__ void __launch_bounds__(NT) gdr_scan_bwd_kernel(const Args p) {
       st4(O + r * LV + c4, o.x * q, o.y * q, o.z * q, o.w * q);
     }
     __syncthreads();
-    float acc[4][4];
+    f2 acc[4][2];
     const __nv_bfloat16* Qs = Qb + s * C * LK + 4 * r8;
     const float* Ws = W + s * T64 + 4 * r8;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float4 t = ld4(S + (4 * r8 + e) * LV + c4);
-      acc[e][0] = a * t.x; acc[e][1] = a * t.y; acc[e][2] = a * t.z; acc[e][3] = a * t.w;
+      acc[e][0] = f2_pack(a * t.x, a * t.y);
+      acc[e][1] = f2_pack(a * t.z, a * t.w);
     }
 #pragma unroll 4
     for (int j = 0; j < C; ++j) {
-      const float4 k = bf4(*reinterpret_cast<const uint2*>(Qs + j * LK)), o = ld4(O + j * LV + c4);
-      const float4 w = ld4(Ws + j * LD), v = ld4(V + j * LV + c4);
-      const float ka[4] = {k.x, k.y, k.z, k.w}, wa[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        acc[e][0] = fmaf(ka[e], o.x, acc[e][0]); acc[e][1] = fmaf(ka[e], o.y, acc[e][1]);
-        acc[e][2] = fmaf(ka[e], o.z, acc[e][2]); acc[e][3] = fmaf(ka[e], o.w, acc[e][3]);
-        acc[e][0] = fmaf(wa[e], v.x, acc[e][0]); acc[e][1] = fmaf(wa[e], v.y, acc[e][1]);
-        acc[e][2] = fmaf(wa[e], v.z, acc[e][2]); acc[e][3] = fmaf(wa[e], v.w, acc[e][3]);
-      }
+      const float4 k = bf4(*reinterpret_cast<const uint2*>(Qs + j * LK)), w = ld4(Ws + j * LD);
+      const Pair2 o = ld2(O + j * LV + c4), v = ld2(V + j * LV + c4);
+      fma4x2(k.x, k.y, o, acc[0], acc[1]);
+      fma4x2(k.z, k.w, o, acc[2], acc[3]);
+      fma4x2(w.x, w.y, v, acc[0], acc[1]);
+      fma4x2(w.z, w.w, v, acc[2], acc[3]);
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) st4(S + (4 * r8 + e) * LV + c4, acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
+    for (int e = 0; e < 4; ++e) *reinterpret_cast<ulonglong2*>(S + (4 * r8 + e) * LV + c4) = make_ulonglong2(acc[e][0], acc[e][1]);
     __syncthreads();
   }
 }
@@ -623,40 +691,54 @@ __global__ void __launch_bounds__(NT, 1) gdr_chunk_bwd_kernel(const Args p) {
   const __nv_bfloat16 *kp = p.k + x.b * p.k_b + x.s0 * p.k_s + x.h * p.k_h, *qp = p.q + x.b * p.q_b + x.s0 * p.q_s + x.h * p.q_h;
   const __nv_bfloat16* vp = p.v + x.b * p.v_b + x.s0 * p.v_s + x.h * p.v_h;
   const long long row0 = ((long long)x.b * p.S + x.s0) * p.H + x.h;  // (position, head) index of row 0; rows are H apart
+#pragma unroll
+  for (int it = 0; it < D * (D / 4) / NT; ++it) {
+    const int i = tid + it * NT;
+    cp16(St + state_row(i >> 5) * LD + (i & 31) * 4, p.st + id * D * D + i * 4, 16);
+  }
+  load_f32(Y, p.dvn + id * C * D);
+  cp_commit();
+  load_f32(Z, p.vn + id * C * D);  // first read after the next barrier but one
+  cp_commit();
   if (tid < C) {
     gc[tid] = p.gc[id * C + tid];
     be[tid] = tid < x.rows ? p.beta[row0 + (long long)tid * p.H] : 0.f;
     eg[tid] = exp_c(gc[tid]);
   }
   load_bf16(X, p.d_o + row0 * D, (long long)p.H * D, x.rows, nullptr);
-  load_f32(Y, p.dvn + id * C * D);
-  load_f32(Z, p.vn + id * C * D);
-  for (int i = tid; i < D * (D / 4); i += NT)
-    *reinterpret_cast<float4*>(St + state_row(i >> 5) * LD + (i & 31) * 4) = reinterpret_cast<const float4*>(p.st + id * D * D)[i];
+  cp_wait<1>();
   __syncthreads();
   const float gl = gc[C - 1];
-  // my 8 columns of a bf16 row of q, k or v (zero past the sequence)
-  auto row8 = [&](const __nv_bfloat16* base, long long pitch, int i, float (&o)[8]) {
-    uint2 lo = make_uint2(0u, 0u), hi = lo;
-    if (i < x.rows) {
-      lo = *reinterpret_cast<const uint2*>(base + i * pitch + 4 * tj);
-      hi = *reinterpret_cast<const uint2*>(base + i * pitch + 4 * tj + 64);
+  // my 4 rows x 8 columns of q, k or v in bf16 (zero past the sequence): fetched before a product, read after it
+  auto fetch8 = [&](const __nv_bfloat16* base, long long pitch, uint2 (&o)[4][2]) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = ti + 16 * r;
+      o[r][0] = o[r][1] = make_uint2(0u, 0u);
+      if (i < x.rows) {
+        o[r][0] = *reinterpret_cast<const uint2*>(base + i * pitch + 4 * tj);
+        o[r][1] = *reinterpret_cast<const uint2*>(base + i * pitch + 4 * tj + 64);
+      }
     }
-    const float4 a = bf4(lo), c = bf4(hi);
+  };
+  auto row8 = [&](const uint2 (&raw)[2], float (&o)[8]) {
+    const float4 a = bf4(raw[0]), c = bf4(raw[1]);
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = c.x; o[5] = c.y; o[6] = c.z; o[7] = c.w;
   };
+  uint2 raw[4][2], raw2[4][2];
   float dq[4][8], dk[4][8], acc[4][8];
   float db_row[4] = {0.f, 0.f, 0.f, 0.f}, dbeta_row[4] = {0.f, 0.f, 0.f, 0.f};  // gradients of b_i and beta_i, rows ti + 16 r
   float dlast = 0.f;                                                            // my share of the gradient of b_last
 
   // dq from the state: (do S^T) e^b scale;  dw = -dv' S^T
+  fetch8(qp, p.q_s, raw);
   zero(dq);
   mm_nt128(X, St, dq);
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int i = ti + 16 * r;
     float t[8], s = 0.f;
-    row8(qp, p.q_s, i, t);
+    row8(raw[r], t);
     const float f = p.scale * eg[i];
 #pragma unroll
     for (int c = 0; c < 8; ++c) { dq[r][c] *= f; s = fmaf(dq[r][c], t[c], s); }
@@ -673,14 +755,25 @@ __global__ void __launch_bounds__(NT, 1) gdr_chunk_bwd_kernel(const Args p) {
   // the exit-state gradient takes the state's place; <dS, S> on the way: d e^{b_last}
   {
     float s = 0.f;
-    for (int i = tid; i < D * (D / 4); i += NT) {
-      float* q4 = St + state_row(i >> 5) * LD + (i & 31) * 4;
-      const float4 a = ld4(q4), g = reinterpret_cast<const float4*>(p.dst + id * D * D)[i];
-      s = fmaf(a.x, g.x, s); s = fmaf(a.y, g.y, s); s = fmaf(a.z, g.z, s); s = fmaf(a.w, g.w, s);
-      *reinterpret_cast<float4*>(q4) = g;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      constexpr int IT = D * (D / 4) / NT / 2;
+      float4 g[IT];
+#pragma unroll
+      for (int it = 0; it < IT; ++it) g[it] = reinterpret_cast<const float4*>(p.dst + id * D * D)[tid + (it + h * IT) * NT];
+#pragma unroll
+      for (int it = 0; it < IT; ++it) {
+        const int i = tid + (it + h * IT) * NT;
+        float* q4 = St + state_row(i >> 5) * LD + (i & 31) * 4;
+        const float4 a = ld4(q4);
+        s = fmaf(a.x, g[it].x, s); s = fmaf(a.y, g[it].y, s); s = fmaf(a.z, g[it].z, s); s = fmaf(a.w, g[it].w, s);
+        *reinterpret_cast<float4*>(q4) = g[it];
+      }
     }
     dlast = s * exp_c(gl);
   }
+  fetch8(kp, p.k_s, raw);
+  cp_wait<0>();  // v'
   __syncthreads();
   // dk from the state update: (v' dS^T) e^{b_last - b}
   zero(dk);
@@ -689,7 +782,7 @@ __global__ void __launch_bounds__(NT, 1) gdr_chunk_bwd_kernel(const Args p) {
   for (int r = 0; r < 4; ++r) {
     const int i = ti + 16 * r;
     float t[8], s = 0.f;
-    row8(kp, p.k_s, i, t);
+    row8(raw[r], t);
     const float f = exp_c(gl - gc[i]);
 #pragma unroll
     for (int c = 0; c < 8; ++c) { dk[r][c] *= f; s = fmaf(dk[r][c], t[c], s); }
@@ -700,7 +793,11 @@ __global__ void __launch_bounds__(NT, 1) gdr_chunk_bwd_kernel(const Args p) {
   load_bf16(K, kp, p.k_s, x.rows, nullptr);
   load_bf16(Q, qp, p.q_s, x.rows, nullptr);
   // dP = lower(do v'^T); b_i and b_j through D_ij; E = dP D
-  float e4[4][4], col[4];
+  float e4[4][4], col[4], pij[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) pij[r][c] = p.P[id * C * C + (ti + 16 * r) * C + tj + 16 * c];
   zero(e4);
   mm_nt64(X, Z, e4);
 #pragma unroll
@@ -712,7 +809,7 @@ __global__ void __launch_bounds__(NT, 1) gdr_chunk_bwd_kernel(const Args p) {
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const int j = tj + 16 * c;
-      const float t = j <= i ? e4[r][c] * p.P[id * C * C + i * C + j] : 0.f;
+      const float t = j <= i ? e4[r][c] * pij[r][c] : 0.f;
       s += t;
       col[c] += t;
       e4[r][c] = j <= i ? e4[r][c] * exp_c(gc[i] - gc[j]) * p.scale : 0.f;
@@ -724,7 +821,8 @@ __global__ void __launch_bounds__(NT, 1) gdr_chunk_bwd_kernel(const Args p) {
   for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int c = 0; c < 4; ++c) X[(ti + 16 * r) * LS + tj + 16 * c] = e4[r][c];
-  load_sq(Z, p.T + id * C * C);
+  load_sq(Z, p.T + id * C * C);  // first read after these two products
+  cp_commit();
   __syncthreads();
   mm_nn<C, LS, LD>(X, K, dq);
   mm_tn(X, Q, dk);
@@ -734,6 +832,9 @@ __global__ void __launch_bounds__(NT, 1) gdr_chunk_bwd_kernel(const Args p) {
     if (i < x.rows) store_bf16_row(p.dq + (row0 + (long long)i * p.H) * D, dq[r]);
   }
   // through T: dRv = T^T dv', dRk = T^T dw
+  fetch8(vp, p.v_s, raw2);  // raw still holds my rows of k
+  cp_wait<0>();
+  __syncthreads();
   zero(acc);
   mm_tn(Z, Y, acc);
   zero(dq);
@@ -742,11 +843,11 @@ __global__ void __launch_bounds__(NT, 1) gdr_chunk_bwd_kernel(const Args p) {
   for (int r = 0; r < 4; ++r) {
     const int i = ti + 16 * r;
     float t[8], s = 0.f, o[8];
-    row8(vp, p.v_s, i, t);
+    row8(raw2[r], t);
 #pragma unroll
     for (int c = 0; c < 8; ++c) { s = fmaf(acc[r][c], t[c], s); o[c] = be[i] * acc[r][c]; }
     if (i < x.rows) store_bf16_row(p.dv + (row0 + (long long)i * p.H) * D, o);
-    row8(kp, p.k_s, i, t);
+    row8(raw[r], t);
     float sk = 0.f;
     const float f = be[i] * eg[i];
 #pragma unroll
@@ -756,18 +857,20 @@ __global__ void __launch_bounds__(NT, 1) gdr_chunk_bwd_kernel(const Args p) {
     db_row[r] += f * sk;
   }
   __syncthreads();  // X, Z, Y, W have been read
-  store_tile(X, acc);
-  store_tile(Z, dq);
   load_f32(Y, p.u + id * C * D);
   load_f32(W, p.w + id * C * D);
-  __syncthreads();
+  cp_commit();
+  store_tile(X, acc);
+  store_tile(Z, dq);
   // dA = -strict_lower(dRv u^T + dRk w^T); A = beta_i kk D
+  float kk[4][4];
+  zero(kk);
+  mm_nt64(K, K, kk);  // under the fetch of u and w
+  cp_wait<0>();
+  __syncthreads();
   zero(e4);
   mm_nt64(X, Y, e4);
   mm_nt64(Z, W, e4);
-  float kk[4][4];
-  zero(kk);
-  mm_nt64(K, K, kk);
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int i = ti + 16 * r;
