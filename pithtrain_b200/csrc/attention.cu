@@ -509,6 +509,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
 }
 
+// row_lo[b * Sq + r]: first visible key of query row r from a sliding window and packed documents (document s covers positions
+// [cu[s], cu[s+1]); rows past the last boundary belong to the last one). One launch instead of nine tensor operations a layer.
+__global__ void row_lower_bounds_kernel(const int* __restrict__ cu, int n_cu, int* __restrict__ row_lo, int B, int Sq, int q_off, int window) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (long long)B * Sq) return;
+  const int pos = static_cast<int>(i % Sq);
+  int lo = window >= 0 ? max(pos + q_off - window, 0) : 0;
+  if (cu) {
+    int a = 1, z = n_cu;  // first boundary beyond pos
+    while (a < z) {
+      const int mid = (a + z) >> 1;
+      if (cu[mid] <= pos) a = mid + 1; else z = mid;
+    }
+    lo = max(lo, cu[min(a - 1, n_cu - 2)]);
+  }
+  row_lo[i] = lo;
+}
+
 }  // namespace pt
 
 namespace {
@@ -558,4 +576,12 @@ PT_API int pt_attn_fwd(const void* q, const void* k, const void* v, void* out, v
   if (dqk == 192 && dv == 128) return attn_fwd_launch_t<192, 128, 1, 2>(q, k, v, a, ldq, ldk, ldv, stream);
   if (dqk == 256 && dv == 256) return attn_fwd_launch_t<256, 256, 1, 1>(q, k, v, a, ldq, ldk, ldv, stream);
   return -2;
+}
+
+// row_lo int32 [B*Sq]; cu int32 [n_cu] (document boundaries, n_cu >= 2) or null; window < 0: none.
+PT_API int pt_row_lower_bounds(const int* cu, int n_cu, int* row_lo, int B, int Sq, int q_off, int window, void* stream_) {
+  if (B <= 0 || Sq <= 0 || (cu && n_cu < 2)) return -2;
+  const long long n = (long long)B * Sq;
+  row_lower_bounds_kernel<<<(unsigned)((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream_)>>>(cu, n_cu, row_lo, B, Sq, q_off, window);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -55,6 +55,15 @@ def row_lower_bounds(B: int, Sq: int, q_off: int, window_left: Optional[int], cu
     has_w = window_left is not None and window_left >= 0
     if not has_w and cu_seqlens is None:
         return None
+    if cu_seqlens is not None and cu_seqlens.is_cuda and cu_seqlens.numel() >= 2 and cu_seqlens.device == torch.device(device):
+        from .. import _native
+
+        cu = cu_seqlens.to(torch.int32).contiguous()
+        lo = torch.empty(B * Sq, dtype=torch.int32, device=device)
+        rc = _native.lib().pt_row_lower_bounds(cu.data_ptr(), cu.numel(), lo.data_ptr(), B, Sq, int(q_off), min(int(window_left), 1 << 30) if has_w else -1,
+                                               _native.stream_ptr())
+        _native.check(rc, "pt_row_lower_bounds")
+        return lo
     key = (str(device), B, Sq, q_off, window_left if has_w else None)
     lo = _ROW_LO_CACHE.get(key) if cu_seqlens is None else None
     if lo is None:

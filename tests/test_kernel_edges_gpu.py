@@ -373,3 +373,14 @@ def test_segment_sum_and_row_bias_dot(sizes, H):
     want[slots[: o[-1]][live].long()] += (x[: o[-1]][live].double() * bias[group[live]].double()).sum(-1)
     row_bias_dot(x, bias, offs, slots, dw, offs[E:E + 1])
     assert (dw.double() - want).abs().max() < 2.0 ** -24 * H * 25 * 16
+
+
+@pytest.mark.parametrize("window", [None, 0, 5, 300])
+@pytest.mark.parametrize("docs", [[0, 1], [0, 7, 7, 8, 300], [0, 128, 256, 300], [0, 100, 200]])
+def test_row_lower_bounds(docs, window):
+    """Against the tensor-op form on the CPU: empty documents, rows past the last boundary, int64 boundaries."""
+    for dtype in (torch.int32, torch.int64):
+        cu = torch.tensor(docs, dtype=dtype)
+        for Sq in (docs[-1], 300):
+            got = N.row_lower_bounds(1, Sq, 0, window, cu.cuda(), torch.device("cuda", 0))
+            assert torch.equal(got.cpu(), N.row_lower_bounds(1, Sq, 0, window, cu, torch.device("cpu")))
