@@ -62,6 +62,12 @@ def zeropower_via_newtonschulz5(Gm: torch.Tensor, steps: int = 5) -> torch.Tenso
     assert Gm.ndim >= 2
     if _own_gemm_usable(Gm):
         return newtonschulz5_own_gemm(Gm, steps)
+    return _newton_schulz(Gm, steps, None)
+
+
+def _newton_schulz(Gm: torch.Tensor, steps: int, scales) -> torch.Tensor:
+    """``scales``: None, or bf16 ``(s, s^2)`` of every matrix of a CUDA stack whose smaller side is a multiple of 8; the
+    first step's scalings, copy and diagonal then take two passes over the Gram matrices instead of five."""
     a, b, c = 3.4445, -4.7750, 2.0315
     G = Gm.to(torch.bfloat16)
     squeeze = G.ndim == 2
@@ -75,18 +81,28 @@ def zeropower_via_newtonschulz5(Gm: torch.Tensor, steps: int = 5) -> torch.Tenso
         nrm = torch.linalg.vector_norm(G, dim=(-2, -1), keepdim=True, dtype=torch.float32)
         out = G / (nrm + 1e-7).to(G.dtype)
     else:
-        nrm = torch.linalg.vector_norm(G, dim=(-2, -1), keepdim=True, dtype=torch.float32)
-        s = 1.0 / (nrm + 1e-7)
-        s1, s2 = s.to(G.dtype), (s * s).to(G.dtype)
+        if scales is None:
+            nrm = torch.linalg.vector_norm(G, dim=(-2, -1), keepdim=True, dtype=torch.float32)
+            s = 1.0 / (nrm + 1e-7)
+            s1, s2 = s.to(G.dtype), (s * s).to(G.dtype)
         out = None
         for it in range(steps):
             A = torch.bmm(X, X.mT)
-            if it == 0:
-                A.mul_(s2)
-            B = torch.baddbmm(A, A, A, beta=b, alpha=c)
-            B.diagonal(dim1=-2, dim2=-1).add_(a)
-            if it == 0:
-                B.mul_(s1)
+            if it == 0 and scales is not None:
+                B = torch.empty_like(A)
+                L, E, m = _native.lib(), A.shape[0], A.shape[1]
+                _native.check(L.pt_gram_scale_copy(A.data_ptr(), B.data_ptr(), scales[1].data_ptr(), E, m, _native.stream_ptr()),
+                              "pt_gram_scale_copy")
+                B.baddbmm_(A, A, beta=b, alpha=c)
+                _native.check(L.pt_gram_shift_scale(B.data_ptr(), scales[0].data_ptr(), E, m, a, _native.stream_ptr()),
+                              "pt_gram_shift_scale")
+            else:
+                if it == 0:
+                    A.mul_(s2)
+                B = torch.baddbmm(A, A, A, beta=b, alpha=c)
+                B.diagonal(dim1=-2, dim2=-1).add_(a)
+                if it == 0:
+                    B.mul_(s1)
             last = it == steps - 1
             if last and tall:
                 out = torch.bmm(X.mT, B)  # [n, m]: the input's own orientation
@@ -290,22 +306,35 @@ class Muon(torch.optim.Optimizer):
     def _update_chunk(self, w, g, buf, beta, lr, wd, gscale=None) -> None:
         """``buf`` is on the same device as ``w`` here."""
         n, m = w.shape[-2], w.shape[-1]
+        scales = None
         native = (w.is_cuda and w.dtype == torch.bfloat16 and w.is_contiguous() and g.is_contiguous()
                   and buf.is_contiguous() and w.numel() % 8 == 0 and g.dtype in (torch.float32, torch.bfloat16)
                   and buf.dtype in (torch.float32, torch.bfloat16))
         if native:
             L = _native.lib()
             upd = torch.empty(w.shape, dtype=torch.bfloat16, device=w.device)
-            rc = L.pt_muon_momentum(g.data_ptr(), int(g.dtype == torch.float32), buf.data_ptr(),
-                                    int(buf.dtype == torch.float32), upd.data_ptr(), w.numel(), float(beta),
-                                    None if gscale is None else gscale.data_ptr(), _native.stream_ptr())
-            _native.check(rc, "pt_muon_momentum")
+            # the fused norm and the passes over the Gram matrices work on whole 16-byte vectors of one matrix's rows
+            E, per = w.numel() // (n * m), n * m
+            fused = min(n, m) % 8 == 0 and min(n, m) <= 65536 and not _own_gemm_usable(upd)
+            partial = torch.empty((E, L.pt_muon_slabs(E, per)), dtype=torch.float32, device=w.device) if fused else None
+            if not fused:
+                E, per = 1, w.numel()
+            rc = L.pt_muon_momentum_sumsq(g.data_ptr(), int(g.dtype == torch.float32), buf.data_ptr(),
+                                          int(buf.dtype == torch.float32), upd.data_ptr(), E, per, float(beta),
+                                          None if gscale is None else gscale.data_ptr(),
+                                          None if partial is None else partial.data_ptr(), _native.stream_ptr())
+            _native.check(rc, "pt_muon_momentum_sumsq")
+            if fused:
+                scales = torch.empty((2, E), dtype=torch.bfloat16, device=w.device)
+                rc = L.pt_frobenius_scales(partial.data_ptr(), E, partial.shape[1], scales[0].data_ptr(), scales[1].data_ptr(),
+                                           _native.stream_ptr())
+                _native.check(rc, "pt_frobenius_scales")
         else:
             g32 = g.float() if gscale is None else g.float() * gscale.to(g.device)
             b32 = buf.float().lerp_(g32, 1 - beta)
             buf.copy_(b32)
             upd = g32.lerp(b32, beta)
-        orth = zeropower_via_newtonschulz5(upd, steps=5)
+        orth = zeropower_via_newtonschulz5(upd, steps=5) if scales is None else _newton_schulz(upd, 5, scales)
         scale = muon_scale_factor(n, m)
         if native:
             orth = orth.contiguous()
