@@ -122,6 +122,7 @@ SIGS = {
     "pt_quant_blocks": "PIIIPPPPP",
     "pt_gemm_fp8": "PPPIIIILLLLPLPPIIIIP",
     "pt_attn_fwd": "PPPPPPP" + "IIIIIII" + "LLLL" + "F" + "II" + "P",
+    "pt_balanced_replay": "PIIIIP",
     "pt_row_lower_bounds": "PIPIIIIP",
     "pt_attn_bwd_split": "PPPPPPPPPPPPP" + "IIIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_attn_bwd": "PPPPPPPPPPPPPPP" + "IIIIII" + "LLLLL" + "F" + "II" + "P",

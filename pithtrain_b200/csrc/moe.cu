@@ -606,6 +606,13 @@ segment_sum_kernel(const T* __restrict__ x, const float* __restrict__ row_w, con
   }
 }
 
+// out[t, j] = (t + j * stride) mod E: one launch for the five tensor operations of a balanced replay.
+template <typename T>
+__global__ void __launch_bounds__(256) balanced_replay_kernel(T* __restrict__ out, long long total, int k, int E, int stride) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i < total) out[i] = (T)((i / k + (i % k) * stride) % E);
+}
+
 }  // namespace pt
 
 using namespace pt;
@@ -644,6 +651,17 @@ PT_API int pt_router_given_fwd(const void* logits, int logits_fp32, float* probs
     router_topk_fwd_kernel<float, true><<<grid, 256, 0, st>>>((const float*)logits, probs, picks, w, n, E, k, 0, renorm, scale);
   else
     router_topk_fwd_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>((const __nv_bfloat16*)logits, probs, picks, w, n, E, k, 0, renorm, scale);
+  return (int)cudaGetLastError();
+}
+
+// out: int32 or int64 [n, k]; E / k == 0 (more slots than experts) gives all slots of a token the same expert.
+PT_API int pt_balanced_replay(void* out, int is_int64, int n, int k, int E, void* stream_) {
+  if (n <= 0) return 0;
+  if (k <= 0 || E <= 0) return -2;
+  const long long total = (long long)n * k;
+  const unsigned grid = (unsigned)((total + 255) / 256);
+  if (is_int64) balanced_replay_kernel<long long><<<grid, 256, 0, (cudaStream_t)stream_>>>((long long*)out, total, k, E, E / k);
+  else balanced_replay_kernel<int><<<grid, 256, 0, (cudaStream_t)stream_>>>((int*)out, total, k, E, E / k);
   return (int)cudaGetLastError();
 }
 

@@ -14,6 +14,8 @@ from typing import Callable, List, Optional, Tuple
 import torch
 import torch.distributed as dist
 
+from .. import _native
+
 
 def expert_token_counts(idx_flat: torch.Tensor, n_bins: int) -> torch.Tensor:
     """Histogram without the host sync of ``torch.bincount`` on CUDA (ids must lie in [0, n_bins))."""
@@ -150,10 +152,16 @@ def force_balance(num_experts: int) -> Callable[[torch.Tensor], torch.Tensor]:
     def replay(topk_idx: torch.Tensor) -> torch.Tensor:
         n, k = topk_idx.shape
         stride = num_experts // k
+        if topk_idx.is_cuda and topk_idx.dtype in (torch.int32, torch.int64) and 0 < n * k < 2 ** 31 and 0 < num_experts < 2 ** 31:
+            out = torch.empty((n, k), dtype=topk_idx.dtype, device=topk_idx.device)
+            rc = _native.lib().pt_balanced_replay(out.data_ptr(), int(out.dtype == torch.int64), n, k, num_experts, _native.stream_ptr())
+            _native.check(rc, "pt_balanced_replay")
+            return out
         t = torch.arange(n, device=topk_idx.device, dtype=topk_idx.dtype).unsqueeze(1)
         if stride == 0:  # more slots than experts: every slot of a token goes to the same one
             return (t % num_experts).expand(n, k).clone()
         j = torch.arange(0, k * stride, stride, device=topk_idx.device, dtype=topk_idx.dtype).unsqueeze(0)
         return (t + j) % num_experts
 
+    replay.any_int = True  # takes the picks in the type that the router kernel writes
     return replay

@@ -109,7 +109,7 @@ class _RouterGivenFn(torch.autograd.Function):
 def router_replayed(logits: torch.Tensor, k: int, replay, renorm: bool = False, scale: float = 1.0
                     ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """:func:`router_topk` (``softmax_topk``) with the picks exchanged by ``replay(top-k indices) -> indices``: the weights are the
-    softmax scores of the replayed experts."""
+    softmax scores of the replayed experts. The indices are int64, or int32 for a ``replay`` with a true ``any_int``."""
     n, E = logits.shape
     if logits.is_cuda and logits.dtype in (torch.float32, torch.bfloat16) and E <= 512 and k <= 16 and n > 0:
         lg = logits.detach().contiguous()
@@ -118,7 +118,7 @@ def router_replayed(logits: torch.Tensor, k: int, replay, renorm: bool = False, 
         rc = _native.lib().pt_router_topk_fwd(lg.data_ptr(), int(lg.dtype == torch.float32), None, picks.data_ptr(), w.data_ptr(), n, E, k, 0, 0,
                                               1.0, sp())
         _native.check(rc, "pt_router_topk_fwd")
-        idx = replay(picks.long()).int().contiguous()
+        idx = replay(picks if getattr(replay, "any_int", False) else picks.long()).int().contiguous()
         if idx.dim() == 2 and idx.shape[0] == n and 0 < idx.shape[1] <= 16:
             w, probs = _RouterGivenFn.apply(logits, idx, renorm, scale)
             return w, idx, probs

@@ -411,3 +411,13 @@ def test_muon_update_with_fused_norm(shape, gdt, bdt):
     assert torch.isfinite(got).all()
     bound = 3 * BF16_MAX * float(step.norm()) + BF16_NORM * float(want.norm()) * 2
     assert float((got - want).norm()) <= bound
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("n,E,k", [(1, 1, 1), (3, 4, 8), (257, 130, 6), (5000, 512, 16)])
+def test_balanced_replay(n, E, k, dtype):
+    from pithtrain_b200.modules.load_balance import force_balance
+
+    picks = torch.zeros(n, k, dtype=dtype)
+    got = force_balance(E)(picks.cuda())
+    assert got.dtype == dtype and torch.equal(got.cpu(), force_balance(E)(picks))
