@@ -122,6 +122,11 @@ SIGS = {
     "pt_quant_blocks": "PIIIPPPPP",
     "pt_gemm_fp8": "PPPIIIILLLLPLPPIIIIP",
     "pt_attn_fwd": "PPPPPPP" + "IIIIIII" + "LLLL" + "F" + "II" + "P",
+    "pt_gated_attn_parts": "IIII",
+    "pt_gated_attn_pre_fwd": "PPPPPPPPPIIIIILFP",
+    "pt_gated_attn_pre_bwd": "PPPPPPPPPPPPIIIIILP",
+    "pt_gated_attn_post_fwd": "PPLPIIIP",
+    "pt_gated_attn_post_bwd": "PPPLPPIIIP",
     "pt_balanced_replay": "PIIIIP",
     "pt_row_lower_bounds": "PIPIIIIP",
     "pt_attn_bwd_split": "PPPPPPPPPPPPP" + "IIIIIII" + "LLLLL" + "F" + "II" + "P",

@@ -19,6 +19,7 @@ from ..contexts import distributed
 from ..ops import gdn_mix
 from ..ops.attention import attention, attention_ref
 from ..ops.common import grad_buffer
+from ..ops.gated_attn import gated_attn_post, gated_attn_pre, gated_attn_supported
 from ..ops.gated_delta_rule import gated_delta_rule, gated_delta_rule_recurrent
 from ..ops.linear import FusedWeights, Linear, fused_linear
 from ..ops.moe import ExpertWeights, moe_experts_ref
@@ -121,13 +122,20 @@ class Qwen35MoeAttention(nn.Module):
         B, S, H = x.shape
         nq = self.num_heads * self.head_dim * 2
         nkv = self.num_kv_heads * self.head_dim
+        cos, sin = rotary.gathered(B * S)
         if reference:
             qg = F.linear(x, self.q_proj.weight, self.q_proj.bias)
             kx = F.linear(x, self.k_proj.weight, self.k_proj.bias)
             vx = F.linear(x, self.v_proj.weight, self.v_proj.bias)
         else:
             biases = [self.q_proj.bias, self.k_proj.bias, self.v_proj.bias] if self.q_proj.bias is not None else None
-            qkv = fused_linear(x.view(B * S, H), self.fused_qkv, biases).view(B, S, -1)
+            qkv = fused_linear(x.view(B * S, H), self.fused_qkv, biases)
+            if gated_attn_supported(qkv, self.q_norm.weight, self.k_norm.weight, cos.shape[-1], self.num_heads, self.num_kv_heads, self.head_dim):
+                q, k, v, gate = gated_attn_pre(qkv, self.q_norm.weight, self.k_norm.weight, cos.to(qkv.dtype), sin.to(qkv.dtype), self.num_heads,
+                                               self.num_kv_heads, self.head_dim, self.eps)
+                o = attention(*(t.view(B, S, -1, self.head_dim) for t in (q, k, v)), causal=True, scale=self.scaling)
+                return self.o_proj(gated_attn_post(o.reshape(q.shape), gate).view(B, S, -1))
+            qkv = qkv.view(B, S, -1)
             qg, kx, vx = qkv[..., :nq], qkv[..., nq:nq + nkv], qkv[..., nq + nkv:]
         q, gate = torch.chunk(qg.reshape(B, S, self.num_heads, self.head_dim * 2), 2, dim=-1)
         gate = gate.reshape(B, S, -1)
@@ -138,7 +146,6 @@ class Qwen35MoeAttention(nn.Module):
             k = rmsnorm_ref(k, self.k_norm.weight, self.eps, zero_centered=True)
         else:
             q, k = self.q_norm(q.contiguous()), self.k_norm(k.contiguous())
-        cos, sin = rotary.gathered(B * S)
         cos, sin = cos.view(B, S, -1).to(q.dtype), sin.view(B, S, -1).to(q.dtype)
         q, k = self.partial_rope(q, cos, sin), self.partial_rope(k, cos, sin)
         o = (attention_ref if reference else attention)(q, k, v, causal=True, scale=self.scaling)

@@ -421,3 +421,45 @@ def test_balanced_replay(n, E, k, dtype):
     picks = torch.zeros(n, k, dtype=dtype)
     got = force_balance(E)(picks.cuda())
     assert got.dtype == dtype and torch.equal(got.cpu(), force_balance(E)(picks))
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,R", [(1, 1, 64, 16), (3, 1, 64, 64), (4, 2, 128, 32), (2, 1, 256, 64), (5, 2, 256, 256)])
+@pytest.mark.parametrize("n,view", [(1, False), (37, False), (515, True)])
+def test_gated_attention_passes(n, view, Hq, Hkv, D, R):
+    """Values and gradients against 64 bits: one bf16 rounding on each value; the weight sums are fp32."""
+    from pithtrain_b200.ops import gated_attn as GA
+
+    torch.manual_seed(n + D)
+    C = 2 * (Hq + Hkv) * D
+    lo = 8 if view else 0
+    a = torch.randn(n, C + lo, device="cuda").bfloat16().requires_grad_()
+    qw, kw = (torch.nn.Parameter((torch.randn(D, device="cuda") * 0.2).bfloat16()) for _ in range(2))
+    for w in (qw, kw):
+        w.main_grad = torch.ones(D, device="cuda")
+    ang = torch.rand(n, R, device="cuda") * 6
+    cos, sin = ang.cos().bfloat16(), ang.sin().bfloat16()
+    assert GA.gated_attn_supported(a[:, lo:], qw, kw, R, Hq, Hkv, D)
+    q, k, v, gate = GA.gated_attn_pre(a[:, lo:], qw, kw, cos, sin, Hq, Hkv, D, 1e-6)
+    o = torch.randn(n, Hq, D, device="cuda").bfloat16().requires_grad_()
+    y = GA.gated_attn_post(o, gate)
+
+    a64, o64 = a.detach().double().requires_grad_(), o.detach().double().requires_grad_()
+    w64 = [w.detach().double().requires_grad_() for w in (qw, kw)]
+    x = a64[:, lo:]
+    qg = x[:, :2 * Hq * D].view(n, Hq, 2, D)
+
+    def normed(t, w):
+        t = t * (t.pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt() * (1 + w)
+        r, c, s = t[..., :R], cos.double()[:, None], sin.double()[:, None]
+        return torch.cat([r * c + torch.cat([-r[..., R // 2:], r[..., :R // 2]], -1) * s, t[..., R:]], -1)
+
+    wants = (normed(qg[:, :, 0], w64[0]), normed(x[:, 2 * Hq * D:(2 * Hq + Hkv) * D].view(n, Hkv, D), w64[1]),
+             x[:, (2 * Hq + Hkv) * D:].view(n, Hkv, D), o64 * qg[:, :, 1].sigmoid())
+    ds = [torch.randn_like(t) for t in (q, k, v, y)]
+    torch.autograd.backward((q, k, v, y), ds)
+    torch.autograd.backward(wants, [d.double() for d in ds])
+    # every result is rounded to bf16 once (the gate's gradient by its kernel, then copied)
+    for got, want in list(zip((q, k, v, y), wants)) + [(o.grad, o64.grad), (a.grad, a64.grad)]:
+        assert ((got.detach().double() - want.detach()).abs() <= BF16_MAX * want.detach().abs() + 1e-5 * want.detach().abs().max()).all()
+    for w, d in zip((qw, kw), w64):
+        assert _rel(w.main_grad - 1, d.grad) < 1e-5
