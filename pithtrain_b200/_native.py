@@ -67,9 +67,10 @@ SIGS = {
     "pt_rmsnorm_bwd_grid": "I",
     "pt_rmsnorm_bwd": "PPPPPPPIIIP",
     "pt_colsum_accumulate": "PIIIPIP",
+    "pt_colsum_accumulate_pair": "PIIIPPIP",
     "pt_qk_norm_rope_fwd": "PPPPPPPPPPIIIIILFIP",
-    "pt_qk_norm_rope_bwd_grid": "",
-    "pt_qk_norm_rope_bwd": "PPPPPPPPPPPPIIIIILIP",
+    "pt_qk_norm_rope_bwd_grid": "IIII",
+    "pt_qk_norm_rope_bwd": "PPPPPPPPPPPPPIIIIILLIP",
     "pt_router_topk_fwd": "PIPPPIIIIIFP",
     "pt_router_given_fwd": "PIPPPIIIIFP",
     "pt_router_topk_bwd": "PPPPPPIIIIIIFP",

@@ -38,11 +38,12 @@ __global__ void __launch_bounds__(256) pre_fwd_kernel(Args a, __nv_bfloat16* __r
   const int lane = threadIdx.x & 31, sub = lane % LPH, half = a.R / 16, partner = partner_of(lane, sub, half);
   const int heads = a.Hq + 2 * a.Hk;
   const long long total = (long long)a.n * heads, warps = (long long)gridDim.x * 8;
+  const bool narrow = total <= 0x7fffffffLL;  // a 64-bit division costs more than the head's arithmetic
   for (long long base = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * HPW; base < total; base += warps * HPW) {
     const long long item = base + lane / LPH;
     const bool live = item < total;
     const long long it = live ? item : total - 1;  // a spare group repeats the last head and stores nothing
-    const int tok = (int)(it / heads), hd = (int)(it % heads);
+    const int tok = narrow ? (int)it / heads : (int)(it / heads), hd = (int)(it - (long long)tok * heads);
     const bool is_q = hd < a.Hq, is_v = hd >= a.Hq + a.Hk;
     const __nv_bfloat16* src = a.qkv + tok * a.stride + (long long)(is_q ? 2 * hd : a.Hq + hd) * D + sub * 8;
     float x[8];
@@ -87,12 +88,11 @@ __global__ void __launch_bounds__(256) pre_bwd_kernel(Args a, const __nv_bfloat1
                                                       const __nv_bfloat16* __restrict__ dv, const __nv_bfloat16* __restrict__ dgate,
                                                       __nv_bfloat16* __restrict__ dqkv, float* __restrict__ part) {
   constexpr int LPH = D / 8, HPW = 32 / LPH;
-  __shared__ float acc[2 * D];
+  __shared__ float acc[8][2 * D];  // weight sums of each warp
   const int lane = threadIdx.x & 31, sub = lane % LPH, half = a.R / 16, partner = partner_of(lane, sub, half);
   const int heads = 2 * a.Hq + 2 * a.Hk;  // in the order of the packed row
   const long long total = (long long)a.n * heads, warps = (long long)gridDim.x * 8;
-  for (int i = threadIdx.x; i < 2 * D; i += 256) acc[i] = 0.f;
-  __syncthreads();
+  const bool narrow = total <= 0x7fffffffLL;  // a 64-bit division costs more than the head's arithmetic
   float wq[8], wk[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) wq[e] = wk[e] = 0.f;
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(256) pre_bwd_kernel(Args a, const __nv_bfloat1
     const long long item = base + lane / LPH;
     const bool live = item < total;
     const long long it = live ? item : total - 1;
-    const int tok = (int)(it / heads), hd = (int)(it % heads);
+    const int tok = narrow ? (int)it / heads : (int)(it / heads), hd = (int)(it - (long long)tok * heads);
     const bool q_part = hd < 2 * a.Hq, is_q = q_part && (hd & 1) == 0, is_k = !q_part && hd < 2 * a.Hq + a.Hk;
     const __nv_bfloat16* g = q_part ? (is_q ? dq : dgate) + ((long long)tok * a.Hq + (hd >> 1)) * D
                                     : (is_k ? dk + ((long long)tok * a.Hk + hd - 2 * a.Hq) * D : dv + ((long long)tok * a.Hk + hd - 2 * a.Hq - a.Hk) * D);
@@ -147,13 +147,26 @@ __global__ void __launch_bounds__(256) pre_bwd_kernel(Args a, const __nv_bfloat1
     }
     if (live) store8(dqkv + at, y);
   }
+  // folded over the warp's heads by shuffles, over the warps in shared memory: fp32 atomics there are a compare-and-swap loop
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    atomicAdd(&acc[sub * 8 + e], wq[e]);
-    atomicAdd(&acc[D + sub * 8 + e], wk[e]);
+#pragma unroll
+    for (int o = 16; o >= LPH; o >>= 1) {
+      wq[e] += __shfl_xor_sync(0xffffffffu, wq[e], o);
+      wk[e] += __shfl_xor_sync(0xffffffffu, wk[e], o);
+    }
+    if (lane < LPH) {
+      acc[threadIdx.x >> 5][sub * 8 + e] = wq[e];
+      acc[threadIdx.x >> 5][D + sub * 8 + e] = wk[e];
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 2 * D; i += 256) part[(long long)blockIdx.x * 2 * D + i] = acc[i];
+  for (int i = threadIdx.x; i < 2 * D; i += 256) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += acc[w][i];
+    part[(long long)blockIdx.x * 2 * D + i] = t;
+  }
 }
 
 __device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + __expf(-x)); }

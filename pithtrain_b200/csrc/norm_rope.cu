@@ -203,23 +203,36 @@ qk_norm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __
   }
 }
 
+// Sum of v over the lanes that hold the same channels of a warp's heads.
+template <int LPH>
+__device__ __forceinline__ float across_groups(float v) {
+#pragma unroll
+  for (int o = 16; o >= LPH; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// dqkv from dq, dk, dv; dw_partial [gridDim.x, 2 * D]: sums of the q and k weight gradients of this block.
+// Bound by memory traffic at large sizes and by its tail at small ones. The weight sums are folded over the head groups of a
+// warp by shuffles and over the warps in shared memory: fp32 atomics in shared memory are a compare-and-swap loop, and 32 lane
+// groups on one address held a block for 15 us. dv is copied here rather than by a launch of its own. The head of an item is
+// found by a 32-bit division when it can be. Measured (32 / 4 heads of 128): 4096 tokens 66 -> 52 us, 512 tokens 31 -> 12, the dv copy
+// (8 and 4) included.
 template <int PAIRS>
 __global__ void __launch_bounds__(256)
-qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16* __restrict__ dk,
+qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16* __restrict__ dk, const __nv_bfloat16* __restrict__ dv,
                         const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ dqkv,
                         const __nv_bfloat16* __restrict__ qw, const __nv_bfloat16* __restrict__ kw,
                         const __nv_bfloat16* __restrict__ cosb, const __nv_bfloat16* __restrict__ sinb,
                         const int* __restrict__ pos, const float* __restrict__ rstd_q,
                         const float* __restrict__ rstd_k, float* __restrict__ dw_partial,
-                        int n_tokens, int S, int Hq, int Hkv, long long qkv_stride, int w_plus_one) {
+                        int n_tokens, int S, int Hq, int Hkv, long long qkv_stride, long long dqkv_stride, int w_plus_one) {
   constexpr int D = PAIRS * 64, HALF = D / 2, LPH = D / 16, HPW = 32 / LPH;
-  __shared__ float acc[2 * D];  // weight-gradient sums of this CTA: q scales then k scales
+  __shared__ float acc[8][2 * D];  // weight-gradient sums of each warp: q scales then k scales
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int sub = lane % LPH, i0 = sub * 8;
-  const int heads = Hq + Hkv;
+  const int heads = Hq + 2 * Hkv;
   const long long total = (long long)n_tokens * heads;
-  for (int cidx = threadIdx.x; cidx < 2 * D; cidx += blockDim.x) acc[cidx] = 0.f;
-  __syncthreads();
+  const bool narrow = total <= 0x7fffffffLL;
   float dwq_a[8], dwq_b[8], dwk_a[8], dwk_b[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) dwq_a[e] = dwq_b[e] = dwk_a[e] = dwk_b[e] = 0.f;
@@ -227,30 +240,46 @@ qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat1
     const long long item = base + lane / LPH;
     const bool live = item < total;
     const long long it = live ? item : total - 1;
-    const int tok = (int)(it / heads), hd = (int)(it % heads);
-    const bool is_q = hd < Hq;
-    const __nv_bfloat16* g = is_q ? dq + ((size_t)tok * Hq + hd) * D : dk + ((size_t)tok * Hkv + (hd - Hq)) * D;
+    const int tok = narrow ? (int)it / heads : (int)(it / heads), hd = (int)(it - (long long)tok * heads);
+    __nv_bfloat16* dst = dqkv + (size_t)tok * dqkv_stride + (size_t)hd * D;
+    const bool is_q = hd < Hq, is_v = hd >= Hq + Hkv;
+    const __nv_bfloat16* g = is_q ? dq + ((size_t)tok * Hq + hd) * D
+                                  : is_v ? (dv ? dv + ((size_t)tok * Hkv + (hd - Hq - Hkv)) * D : nullptr) : dk + ((size_t)tok * Hkv + (hd - Hq)) * D;
     const __nv_bfloat16* src = qkv + (size_t)tok * qkv_stride + (size_t)hd * D;
-    __nv_bfloat16* dst = dqkv + (size_t)tok * qkv_stride + (size_t)hd * D;
     const __nv_bfloat16* wn = is_q ? qw : kw;
     const int p = pos ? pos[tok] : (tok % S);
     float ga[8], gb[8], c[8], sn[8], dna[8], dnb[8], xa[8], xb[8];
-    load8(g + i0, ga);
-    load8(g + HALF + i0, gb);
-    load8(cosb + (size_t)p * D + i0, c);
-    load8(sinb + (size_t)p * D + i0, sn);
+    if (g) {
+      load8(g + i0, ga);
+      load8(g + HALF + i0, gb);
+    } else {  // no gradient reached v
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ga[e] = gb[e] = 0.f;
+    }
+    if (!is_v) {
+      load8(cosb + (size_t)p * D + i0, c);
+      load8(sinb + (size_t)p * D + i0, sn);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) c[e] = sn[e] = 0.f;  // not used
+    }
     float rstd = 1.f;
-    if (wn) rstd = is_q ? rstd_q[(size_t)tok * Hq + hd] : rstd_k[(size_t)tok * Hkv + (hd - Hq)];
+    if (wn && !is_v) rstd = is_q ? rstd_q[(size_t)tok * Hq + hd] : rstd_k[(size_t)tok * Hkv + (hd - Hq)];
     float dot = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      dna[e] = ga[e] * c[e] + gb[e] * sn[e];
-      dnb[e] = gb[e] * c[e] - ga[e] * sn[e];
+      dna[e] = is_v ? ga[e] : ga[e] * c[e] + gb[e] * sn[e];
+      dnb[e] = is_v ? gb[e] : gb[e] * c[e] - ga[e] * sn[e];
     }
     if (wn) {
       float wa[8], wb[8];
-      load8(src + i0, xa);
-      load8(src + HALF + i0, xb);
+      if (!is_v) {
+        load8(src + i0, xa);
+        load8(src + HALF + i0, xb);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) xa[e] = xb[e] = 0.f;
+      }
       load8(wn + i0, wa);
       load8(wn + HALF + i0, wb);
 #pragma unroll
@@ -258,18 +287,22 @@ qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat1
         xa[e] *= rstd; xb[e] *= rstd;
         float x = wa[e], y = wb[e];
         if (w_plus_one) { x += 1.f; y += 1.f; }
-        if (live) {
+        if (live && !is_v) {
           if (is_q) { dwq_a[e] += dna[e] * xa[e]; dwq_b[e] += dnb[e] * xb[e]; }
           else { dwk_a[e] += dna[e] * xa[e]; dwk_b[e] += dnb[e] * xb[e]; }
         }
-        dna[e] *= x; dnb[e] *= y;
-        dot += dna[e] * xa[e] + dnb[e] * xb[e];
+        if (!is_v) {
+          dna[e] *= x; dnb[e] *= y;
+          dot += dna[e] * xa[e] + dnb[e] * xb[e];
+        }
       }
       dot = group_sum<LPH>(dot) / D;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        dna[e] = rstd * (dna[e] - xa[e] * dot);
-        dnb[e] = rstd * (dnb[e] - xb[e] * dot);
+        if (!is_v) {
+          dna[e] = rstd * (dna[e] - xa[e] * dot);
+          dnb[e] = rstd * (dnb[e] - xb[e] * dot);
+        }
       }
     }
     if (live) {
@@ -280,13 +313,19 @@ qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat1
   if (qw && dw_partial) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      atomicAdd(&acc[i0 + e], dwq_a[e]);
-      atomicAdd(&acc[HALF + i0 + e], dwq_b[e]);
-      atomicAdd(&acc[D + i0 + e], dwk_a[e]);
-      atomicAdd(&acc[D + HALF + i0 + e], dwk_b[e]);
+      const float s[4] = {across_groups<LPH>(dwq_a[e]), across_groups<LPH>(dwq_b[e]), across_groups<LPH>(dwk_a[e]), across_groups<LPH>(dwk_b[e])};
+      if (lane < LPH) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[wib][j * HALF + i0 + e] = s[j];
+      }
     }
     __syncthreads();
-    for (int cidx = threadIdx.x; cidx < 2 * D; cidx += blockDim.x) dw_partial[(size_t)blockIdx.x * 2 * D + cidx] = acc[cidx];
+    for (int cidx = threadIdx.x; cidx < 2 * D; cidx += blockDim.x) {
+      float t = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) t += acc[w][cidx];
+      dw_partial[(size_t)blockIdx.x * 2 * D + cidx] = t;
+    }
   }
 }
 
@@ -353,25 +392,26 @@ PT_API int pt_qk_norm_rope_fwd(const void* qkv, void* q_out, void* k_out, const 
   return (int)cudaGetLastError();
 }
 
-PT_API int pt_qk_norm_rope_bwd_grid() { return sm_count() * 4; }
-// dw_partial: [grid, 2*D] floats (q weight grads then k weight grads per row); may be null when qw is null.
-PT_API int pt_qk_norm_rope_bwd(const void* dq, const void* dk, const void* qkv, void* dqkv,
+PT_API int pt_qk_norm_rope_bwd_grid(int n_tokens, int Hq, int Hkv, int D) {
+  const long long want = ((long long)n_tokens * (Hq + 2 * Hkv) * (D / 16) + 255) / 256, cap = sm_count() * 4;
+  return (int)(want < 1 ? 1 : want < cap ? want : cap);
+}
+// dw_partial: [grid, 2*D] floats (q weight grads then k weight grads per row); may be null when qw is null. dv may be null (zeros).
+PT_API int pt_qk_norm_rope_bwd(const void* dq, const void* dk, const void* dv, const void* qkv, void* dqkv,
                                const void* qw, const void* kw, const void* cosb, const void* sinb,
                                const int* pos, const float* rstd_q, const float* rstd_k,
                                float* dw_partial, int n_tokens, int S, int Hq, int Hkv, int D,
-                               long long qkv_stride, int w_plus_one, void* stream_) {
+                               long long qkv_stride, long long dqkv_stride, int w_plus_one, void* stream_) {
   cudaStream_t st = (cudaStream_t)stream_;
   if (n_tokens <= 0) return 0;
   if (D != 64 && D != 128) return -1;
-  int grid = pt_qk_norm_rope_bwd_grid();
-  if (D == 128)
-    qk_norm_rope_bwd_kernel<2><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)qkv,
-        (__nv_bfloat16*)dqkv, (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, (const __nv_bfloat16*)cosb,
-        (const __nv_bfloat16*)sinb, pos, rstd_q, rstd_k, dw_partial, n_tokens, S, Hq, Hkv, qkv_stride, w_plus_one);
-  else
-    qk_norm_rope_bwd_kernel<1><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)qkv,
-        (__nv_bfloat16*)dqkv, (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, (const __nv_bfloat16*)cosb,
-        (const __nv_bfloat16*)sinb, pos, rstd_q, rstd_k, dw_partial, n_tokens, S, Hq, Hkv, qkv_stride, w_plus_one);
+  const int grid = pt_qk_norm_rope_bwd_grid(n_tokens, Hq, Hkv, D);
+#define LAUNCH(P) qk_norm_rope_bwd_kernel<P><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, \
+    (const __nv_bfloat16*)qkv, (__nv_bfloat16*)dqkv, (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, (const __nv_bfloat16*)cosb,             \
+    (const __nv_bfloat16*)sinb, pos, rstd_q, rstd_k, dw_partial, n_tokens, S, Hq, Hkv, qkv_stride, dqkv_stride, w_plus_one)
+  if (D == 128) LAUNCH(2);
+  else LAUNCH(1);
+#undef LAUNCH
   return (int)cudaGetLastError();
 }
 
@@ -386,7 +426,7 @@ namespace pt {
 constexpr int COLSUM_WARPS = 32;
 template <typename T>
 __global__ void __launch_bounds__(32 * COLSUM_WARPS)
-colsum_accumulate_kernel(const float* __restrict__ part, int G, int ld, int H, T* __restrict__ dst) {
+colsum_accumulate_kernel(const float* __restrict__ part, int G, int ld, int H, T* __restrict__ dst, T* __restrict__ dst2, int split) {
   __shared__ float red[COLSUM_WARPS][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -409,7 +449,8 @@ colsum_accumulate_kernel(const float* __restrict__ part, int G, int ld, int H, T
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   const int cc = blockIdx.x * 32 + warp;
-  if (lane == 0 && cc < H) dst[cc] = (T)((float)dst[cc] + v);
+  T* d = cc < split ? dst + cc : dst2 + (cc - split);
+  if (lane == 0 && cc < H) *d = (T)((float)*d + v);
 }
 }  // namespace pt
 
@@ -418,7 +459,17 @@ PT_API int pt_colsum_accumulate(const float* part, int G, int ld, int H, void* d
   cudaStream_t st = (cudaStream_t)stream_;
   if (G <= 0 || H <= 0) return 0;
   const int grid = (H + 31) / 32, threads = 32 * pt::COLSUM_WARPS;
-  if (dst_fp32) pt::colsum_accumulate_kernel<float><<<grid, threads, 0, st>>>(part, G, ld, H, (float*)dst);
-  else pt::colsum_accumulate_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(part, G, ld, H, (__nv_bfloat16*)dst);
+  if (dst_fp32) pt::colsum_accumulate_kernel<float><<<grid, threads, 0, st>>>(part, G, ld, H, (float*)dst, nullptr, H);
+  else pt::colsum_accumulate_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(part, G, ld, H, (__nv_bfloat16*)dst, nullptr, H);
+  return (int)cudaGetLastError();
+}
+
+// Columns [0, H) into dst0 and [H, 2 H) into dst1: the q and k norms of a layer in one launch.
+PT_API int pt_colsum_accumulate_pair(const float* part, int G, int ld, int H, void* dst0, void* dst1, int dst_fp32, void* stream_) {
+  cudaStream_t st = (cudaStream_t)stream_;
+  if (G <= 0 || H <= 0) return 0;
+  const int grid = (2 * H + 31) / 32, threads = 32 * pt::COLSUM_WARPS;
+  if (dst_fp32) pt::colsum_accumulate_kernel<float><<<grid, threads, 0, st>>>(part, G, ld, 2 * H, (float*)dst0, (float*)dst1, H);
+  else pt::colsum_accumulate_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(part, G, ld, 2 * H, (__nv_bfloat16*)dst0, (__nv_bfloat16*)dst1, H);
   return (int)cudaGetLastError();
 }

@@ -62,3 +62,18 @@ def accumulate_colsum(p: torch.Tensor, part: torch.Tensor, lo: int = 0, hi: int 
         _native.check(rc, "pt_colsum_accumulate")
         return
     accumulate_grad(p, part[:, lo:hi].sum(0))
+
+
+def accumulate_colsum_pair(p0: torch.Tensor, p1: torch.Tensor, part: torch.Tensor, d: int) -> None:
+    """:func:`accumulate_colsum` of ``part[:, :d]`` into ``p0`` and ``part[:, d:2d]`` into ``p1``, in one launch where both have
+    gradient buffers of one type."""
+    mgs = [getattr(p, "main_grad", None) for p in (p0, p1)]
+    if (p0 is not p1 and part.is_cuda and part.stride(1) == 1 and part.dtype == torch.float32
+            and all(m is not None and m.is_cuda and m.is_contiguous() and m.dtype in (torch.float32, torch.bfloat16) and m.numel() == d for m in mgs)
+            and mgs[0].dtype == mgs[1].dtype):
+        rc = _native.lib().pt_colsum_accumulate_pair(part.data_ptr(), part.shape[0], part.stride(0), d, mgs[0].data_ptr(), mgs[1].data_ptr(),
+                                                     int(mgs[0].dtype == torch.float32), _native.stream_ptr())
+        _native.check(rc, "pt_colsum_accumulate_pair")
+        return
+    accumulate_colsum(p0, part, 0, d)
+    accumulate_colsum(p1, part, d, 2 * d)

@@ -8,7 +8,7 @@ from __future__ import annotations
 import torch
 
 from .. import _native
-from .common import accumulate_colsum, sp, use_native
+from .common import accumulate_colsum, accumulate_colsum_pair, sp, use_native
 
 
 def _dense(t: torch.Tensor) -> torch.Tensor:
@@ -54,9 +54,12 @@ class _Pre(torch.autograd.Function):
                                      cos.data_ptr(), sin.data_ptr(), rstd.data_ptr(), dqkv.data_ptr(), part.data_ptr(), n, Hq, Hkv, D,
                                      cos.shape[1], qkv.stride(0), sp())
         _native.check(rc, "pt_gated_attn_pre_bwd")
-        for i, ref in enumerate(ctx.refs):
-            if ctx.needs_input_grad[1 + i]:
-                accumulate_colsum(ref, part, i * D, (i + 1) * D)
+        if all(ctx.needs_input_grad[1:3]):
+            accumulate_colsum_pair(*ctx.refs, part, D)
+        else:
+            for i, ref in enumerate(ctx.refs):
+                if ctx.needs_input_grad[1 + i]:
+                    accumulate_colsum(ref, part, i * D, (i + 1) * D)
         return (dqkv,) + (None,) * 8
 
 

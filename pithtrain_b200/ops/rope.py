@@ -15,7 +15,7 @@ from typing import Optional
 import torch
 
 from .. import _native
-from .common import accumulate_colsum, sp, use_native
+from .common import accumulate_colsum_pair, sp, use_native
 
 
 def rotate_half(x):
@@ -80,23 +80,21 @@ class _QKNormRopeFn(torch.autograd.Function):
         L = _native.lib()
         dqkv = torch.empty_like(qkv)
         has_norm = q_w is not None
-        grid = L.pt_qk_norm_rope_bwd_grid()
+        grid = L.pt_qk_norm_rope_bwd_grid(n, Hq, Hkv, D)
         part = torch.empty((grid, 2 * D), dtype=torch.float32, device=qkv.device) if has_norm else None
         dq = dq.contiguous() if dq is not None else torch.zeros((n, Hq, D), dtype=qkv.dtype, device=qkv.device)
         dk = dk.contiguous() if dk is not None else torch.zeros((n, Hkv, D), dtype=qkv.dtype, device=qkv.device)
+        if dv is not None:
+            dv = dv.contiguous()
+            dv = dv if dv.data_ptr() % 16 == 0 else dv.clone()
         rc = L.pt_qk_norm_rope_bwd(
-            dq.data_ptr(), dk.data_ptr(), qkv.data_ptr(), dqkv.data_ptr(), None if not has_norm else q_w.data_ptr(),
+            dq.data_ptr(), dk.data_ptr(), None if dv is None else dv.data_ptr(), qkv.data_ptr(), dqkv.data_ptr(), None if not has_norm else q_w.data_ptr(),
             None if not has_norm else k_w.data_ptr(), cos.data_ptr(), sin.data_ptr(), None if pos is None else pos.data_ptr(),
             None if rq is None else rq.data_ptr(), None if rk is None else rk.data_ptr(),
-            None if part is None else part.data_ptr(), n, S, Hq, Hkv, D, qkv.stride(0), int(zc), sp())
+            None if part is None else part.data_ptr(), n, S, Hq, Hkv, D, qkv.stride(0), dqkv.stride(0), int(zc), sp())
         _native.check(rc, "pt_qk_norm_rope_bwd")
-        if dv is not None:
-            dqkv[:, (Hq + Hkv) * D:].copy_(dv.reshape(n, Hkv * D))
-        else:
-            dqkv[:, (Hq + Hkv) * D:].zero_()
         if has_norm:
-            accumulate_colsum(ctx.qw_ref, part, 0, D)
-            accumulate_colsum(ctx.kw_ref, part, D, 2 * D)
+            accumulate_colsum_pair(ctx.qw_ref, ctx.kw_ref, part, D)
         return (dqkv,) + (None,) * 11
 
 

@@ -463,3 +463,40 @@ def test_gated_attention_passes(n, view, Hq, Hkv, D, R):
         assert ((got.detach().double() - want.detach()).abs() <= BF16_MAX * want.detach().abs() + 1e-5 * want.detach().abs().max()).all()
     for w, d in zip((qw, kw), w64):
         assert _rel(w.main_grad - 1, d.grad) < 1e-5
+
+
+@pytest.mark.parametrize("Hq,Hkv,D", [(1, 1, 64), (5, 1, 64), (4, 2, 128), (7, 7, 128)])
+@pytest.mark.parametrize("n,pad,norm,with_dv", [(1, 0, True, True), (33, 8, True, True), (1030, 0, False, True), (600, 0, True, False)])
+def test_qk_norm_rope_backward(n, pad, norm, with_dv, Hq, Hkv, D):
+    """Gradients of the packed projection against 64 bits, rounded once; v's gradient is a copy, or zero if none reached it. The
+    rotated and normalised value is rounded once more inside (before the rotation), which the gradient does not see."""
+    from pithtrain_b200.ops.rope import qk_norm_rope
+
+    torch.manual_seed(n)
+    C = (Hq + 2 * Hkv) * D
+    a = torch.randn(n, C + pad, device="cuda").bfloat16().requires_grad_()  # pad: rows further apart than they are long
+    ws = [torch.nn.Parameter((torch.rand(D, device="cuda") + 0.5).bfloat16()) for _ in range(2)] if norm else [None, None]
+    for w in ws if norm else []:
+        w.main_grad = torch.ones(D, device="cuda")
+    ang = torch.rand(n, D // 2, device="cuda").repeat(1, 2) * 6
+    cos, sin = ang.cos().bfloat16(), ang.sin().bfloat16()
+    q, k, v = qk_norm_rope(a[:, :C], ws[0], ws[1], cos, sin, Hq, Hkv, D, 1e-6)
+    a64 = a.detach().double().requires_grad_()
+    w64 = [w.detach().double().requires_grad_() for w in ws] if norm else ws
+
+    def rotated(t, w):
+        if w is not None:
+            t = t * (t.pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt() * w
+        return t * cos.double()[:, None] + torch.cat([-t[..., D // 2:], t[..., :D // 2]], -1) * sin.double()[:, None]
+
+    wants = [rotated(a64[:, :Hq * D].view(n, Hq, D), w64[0]), rotated(a64[:, Hq * D:(Hq + Hkv) * D].view(n, Hkv, D), w64[1]),
+             a64[:, (Hq + Hkv) * D:C].view(n, Hkv, D)]
+    outs = [q, k, v]
+    if not with_dv:
+        outs, wants = outs[:2], wants[:2]
+    ds = [torch.randn_like(t) for t in outs]
+    torch.autograd.backward(outs, ds)
+    torch.autograd.backward(wants, [d.double() for d in ds])
+    assert ((a.grad.double() - a64.grad).abs() <= BF16_MAX * a64.grad.abs() + 1e-5 * a64.grad.abs().max()).all()
+    for w, d in zip(ws, w64) if norm else []:
+        assert _rel(w.main_grad - 1, d.grad) < 1e-5
