@@ -82,70 +82,81 @@ __global__ void __launch_bounds__(256) pre_fwd_kernel(Args a, __nv_bfloat16* __r
   }
 }
 
-// dqkv from dq, dk, dv [n, heads, D] and the gate's gradient [n, Hq, D]; part [gridDim.x, 2 * D]: sums for the q and k weights.
+// One group of heads of one kind (q or k) on the way back; place: elements from the start of a packed row to the kind's first
+// head, pitch: between its heads, rs0: its first column of rstd. wsum collects the norm weight's gradient for my channels.
 template <int D>
-__global__ void __launch_bounds__(256) pre_bwd_kernel(Args a, const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16* __restrict__ dk,
+__device__ __forceinline__ void bwd_group(const Args& a, long long grp, int H, long long place, int pitch, int rs0, const __nv_bfloat16* __restrict__ grad,
+                                          const __nv_bfloat16* __restrict__ wn, __nv_bfloat16* __restrict__ dqkv, float (&wsum)[8]) {
+  constexpr int LPH = D / 8, HPW = 32 / LPH;
+  const int lane = threadIdx.x & 31, sub = lane % LPH, half = a.R / 16, partner = partner_of(lane, sub, half);
+  const long long total = (long long)a.n * H, item = grp * HPW + lane / LPH;
+  const bool live = item < total, rot = sub < 2 * half;
+  const long long it = live ? item : total - 1;
+  const int tok = total <= 0x7fffffffLL ? (int)it / H : (int)(it / H), hd = (int)(it - (long long)tok * H);
+  const long long at = tok * a.stride + place + (long long)hd * pitch + sub * 8;
+  float y[8], t[8], x[8], w[8];
+  load8(grad + it * D + sub * 8, y);
+  load8(a.qkv + at, x);
+  const float r = a.rstd[(long long)tok * (a.Hq + a.Hk) + rs0 + hd];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) t[e] = 0.f;
+  if (rot) {
+    float c[8], s[8];
+    load8(a.cosb + (long long)tok * a.R + sub * 8, c);
+    load8(a.sinb + (long long)tok * a.R + sub * 8, s);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) { t[e] = y[e] * s[e]; y[e] *= c[e]; }
+  }
+  // transposed rotation: the first half gets + the partner's g sin, the second half - it
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float o = __shfl_sync(0xffffffffu, t[e], partner);
+    if (rot) y[e] += sub < half ? o : -o;
+  }
+  load8(wn + sub * 8, w);
+  float dot = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    x[e] *= r;
+    if (live) wsum[e] += y[e] * x[e];
+    y[e] *= 1.f + w[e];
+    dot += y[e] * x[e];
+  }
+  dot = group_sum<LPH>(dot) / D;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) y[e] = r * (y[e] - x[e] * dot);
+  if (live) store8(dqkv + at, y);
+}
+
+// dqkv from dq, dk, dv [n, heads, D] and the gate's gradient [n, Hq, D]; part [gridDim.x, 2 * D]: sums for the q and k weights.
+// A warp's heads are all of one kind, so the copies of dv and the gate's gradient do none of the arithmetic of the others: 3072 tokens,
+// 16 / 2 heads of 256: 90 us with kinds mixed, 60 with two blocks an SM, 42 with four.
+template <int D>
+__global__ void __launch_bounds__(256, 4) pre_bwd_kernel(Args a, const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16* __restrict__ dk,
                                                       const __nv_bfloat16* __restrict__ dv, const __nv_bfloat16* __restrict__ dgate,
                                                       __nv_bfloat16* __restrict__ dqkv, float* __restrict__ part) {
   constexpr int LPH = D / 8, HPW = 32 / LPH;
   __shared__ float acc[8][2 * D];  // weight sums of each warp
-  const int lane = threadIdx.x & 31, sub = lane % LPH, half = a.R / 16, partner = partner_of(lane, sub, half);
-  const int heads = 2 * a.Hq + 2 * a.Hk;  // in the order of the packed row
-  const long long total = (long long)a.n * heads, warps = (long long)gridDim.x * 8;
-  const bool narrow = total <= 0x7fffffffLL;  // a 64-bit division costs more than the head's arithmetic
+  const int lane = threadIdx.x & 31, sub = lane % LPH;
+  const long long gq = ((long long)a.n * a.Hq + HPW - 1) / HPW, gk = ((long long)a.n * a.Hk + HPW - 1) / HPW;
   float wq[8], wk[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) wq[e] = wk[e] = 0.f;
-  for (long long base = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * HPW; base < total; base += warps * HPW) {
-    const long long item = base + lane / LPH;
-    const bool live = item < total;
-    const long long it = live ? item : total - 1;
-    const int tok = narrow ? (int)it / heads : (int)(it / heads), hd = (int)(it - (long long)tok * heads);
-    const bool q_part = hd < 2 * a.Hq, is_q = q_part && (hd & 1) == 0, is_k = !q_part && hd < 2 * a.Hq + a.Hk;
-    const __nv_bfloat16* g = q_part ? (is_q ? dq : dgate) + ((long long)tok * a.Hq + (hd >> 1)) * D
-                                    : (is_k ? dk + ((long long)tok * a.Hk + hd - 2 * a.Hq) * D : dv + ((long long)tok * a.Hk + hd - 2 * a.Hq - a.Hk) * D);
-    const long long at = tok * a.stride + (long long)hd * D + sub * 8;
-    float y[8], t[8], c[8], x[8];
-    load8(g + sub * 8, y);
-    const bool norm = is_q || is_k, rot = norm && sub < 2 * half;
-    float r = 0.f;
-    if (norm) {
-      load8(a.qkv + at, x);
-      r = a.rstd[(long long)tok * (a.Hq + a.Hk) + (is_q ? hd >> 1 : hd - a.Hq)];
-    }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) { t[e] = 0.f; c[e] = 1.f; }
-    if (rot) {
-      float s[8];
-      load8(a.cosb + (long long)tok * a.R + sub * 8, c);
-      load8(a.sinb + (long long)tok * a.R + sub * 8, s);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) t[e] = y[e] * s[e];
-    }
-    // transposed rotation: the first half gets + the partner's g sin, the second half - it
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float o = __shfl_sync(0xffffffffu, t[e], partner);
-      if (rot) y[e] = y[e] * c[e] + (sub < half ? o : -o);
-    }
-    float dot = 0.f;
-    if (norm) {
-      float w[8];
-      load8((is_q ? a.qw : a.kw) + sub * 8, w);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        x[e] *= r;
-        if (live) (is_q ? wq[e] : wk[e]) += y[e] * x[e];
-        y[e] *= 1.f + w[e];
-        dot += y[e] * x[e];
+  for (long long grp = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); grp < 2 * (gq + gk); grp += (long long)gridDim.x * 8) {
+    if (grp < gq) {
+      bwd_group<D>(a, grp, a.Hq, 0, 2 * D, 0, dq, a.qw, dqkv, wq);
+    } else if (grp < gq + gk) {
+      bwd_group<D>(a, grp - gq, a.Hk, 2LL * a.Hq * D, D, a.Hq, dk, a.kw, dqkv, wk);
+    } else {
+      const bool gate = grp < 2 * gq + gk;
+      const int H = gate ? a.Hq : a.Hk;
+      const long long item = (grp - (gate ? gq + gk : 2 * gq + gk)) * HPW + lane / LPH;
+      if (item < (long long)a.n * H) {
+        const long long tok = item / H, hd = item - tok * H;
+        const long long at = tok * a.stride + (gate ? hd * 2 * D + D : (2LL * a.Hq + a.Hk + hd) * D) + sub * 8;
+        *reinterpret_cast<uint4*>(dqkv + at) = *reinterpret_cast<const uint4*>((gate ? dgate : dv) + item * D + sub * 8);
       }
     }
-    dot = group_sum<LPH>(dot) / D;
-    if (norm) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) y[e] = r * (y[e] - x[e] * dot);
-    }
-    if (live) store8(dqkv + at, y);
   }
   // folded over the warp's heads by shuffles, over the warps in shared memory: fp32 atomics there are a compare-and-swap loop
 #pragma unroll

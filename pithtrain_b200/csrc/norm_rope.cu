@@ -211,103 +211,101 @@ __device__ __forceinline__ float across_groups(float v) {
   return v;
 }
 
-// dqkv from dq, dk, dv; dw_partial [gridDim.x, 2 * D]: sums of the q and k weight gradients of this block.
-// Bound by memory traffic at large sizes and by its tail at small ones. The weight sums are folded over the head groups of a
-// warp by shuffles and over the warps in shared memory: fp32 atomics in shared memory are a compare-and-swap loop, and 32 lane
-// groups on one address held a block for 15 us. dv is copied here rather than by a launch of its own. The head of an item is
-// found by a 32-bit division when it can be. Measured (32 / 4 heads of 128): 4096 tokens 66 -> 52 us, 512 tokens 31 -> 12, the dv copy
-// (8 and 4) included.
-template <int PAIRS>
-__global__ void __launch_bounds__(256)
-qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16* __restrict__ dk, const __nv_bfloat16* __restrict__ dv,
-                        const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ dqkv,
-                        const __nv_bfloat16* __restrict__ qw, const __nv_bfloat16* __restrict__ kw,
-                        const __nv_bfloat16* __restrict__ cosb, const __nv_bfloat16* __restrict__ sinb,
-                        const int* __restrict__ pos, const float* __restrict__ rstd_q,
-                        const float* __restrict__ rstd_k, float* __restrict__ dw_partial,
-                        int n_tokens, int S, int Hq, int Hkv, long long qkv_stride, long long dqkv_stride, int w_plus_one) {
-  constexpr int D = PAIRS * 64, HALF = D / 2, LPH = D / 16, HPW = 32 / LPH;
-  __shared__ float acc[8][2 * D];  // weight-gradient sums of each warp: q scales then k scales
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  const int sub = lane % LPH, i0 = sub * 8;
-  const int heads = Hq + 2 * Hkv;
-  const long long total = (long long)n_tokens * heads;
-  const bool narrow = total <= 0x7fffffffLL;
-  float dwq_a[8], dwq_b[8], dwk_a[8], dwk_b[8];
+struct RopeBwdArgs {
+  const __nv_bfloat16 *qkv, *cosb, *sinb;
+  const int* pos;
+  __nv_bfloat16* dqkv;
+  long long qkv_stride, dqkv_stride;
+  int n, S, w_plus_one;
+};
+
+// One group of heads of one kind (q or k): grp counts groups of HPW heads among the n * H of that kind, head0 is the kind's place
+// in the packed row. ka, kb collect the norm weight's gradient for my channels.
+template <int D>
+__device__ __forceinline__ void rope_bwd_group(const RopeBwdArgs& a, long long grp, int H, int head0, const __nv_bfloat16* __restrict__ grad,
+                                               const __nv_bfloat16* __restrict__ wn, const float* __restrict__ rstd_in, float (&ka)[8], float (&kb)[8]) {
+  constexpr int HALF = D / 2, LPH = D / 16, HPW = 32 / LPH;
+  const int lane = threadIdx.x & 31, i0 = lane % LPH * 8;
+  const long long total = (long long)a.n * H, item = grp * HPW + lane / LPH;
+  const bool live = item < total;
+  const long long it = live ? item : total - 1;  // a spare group repeats the last head and stores nothing
+  const int tok = total <= 0x7fffffffLL ? (int)it / H : (int)(it / H), hd = (int)(it - (long long)tok * H);
+  const __nv_bfloat16* src = a.qkv + (size_t)tok * a.qkv_stride + (size_t)(head0 + hd) * D;
+  const int p = a.pos ? a.pos[tok] : tok % a.S;
+  float ga[8], gb[8], c[8], sn[8], da[8], db[8];
+  load8(grad + (size_t)it * D + i0, ga);
+  load8(grad + (size_t)it * D + HALF + i0, gb);
+  load8(a.cosb + (size_t)p * D + i0, c);
+  load8(a.sinb + (size_t)p * D + i0, sn);
 #pragma unroll
-  for (int e = 0; e < 8; ++e) dwq_a[e] = dwq_b[e] = dwk_a[e] = dwk_b[e] = 0.f;
-  for (long long base = ((long long)blockIdx.x * wpb + wib) * HPW; base < total; base += (long long)gridDim.x * wpb * HPW) {
-    const long long item = base + lane / LPH;
-    const bool live = item < total;
-    const long long it = live ? item : total - 1;
-    const int tok = narrow ? (int)it / heads : (int)(it / heads), hd = (int)(it - (long long)tok * heads);
-    __nv_bfloat16* dst = dqkv + (size_t)tok * dqkv_stride + (size_t)hd * D;
-    const bool is_q = hd < Hq, is_v = hd >= Hq + Hkv;
-    const __nv_bfloat16* g = is_q ? dq + ((size_t)tok * Hq + hd) * D
-                                  : is_v ? (dv ? dv + ((size_t)tok * Hkv + (hd - Hq - Hkv)) * D : nullptr) : dk + ((size_t)tok * Hkv + (hd - Hq)) * D;
-    const __nv_bfloat16* src = qkv + (size_t)tok * qkv_stride + (size_t)hd * D;
-    const __nv_bfloat16* wn = is_q ? qw : kw;
-    const int p = pos ? pos[tok] : (tok % S);
-    float ga[8], gb[8], c[8], sn[8], dna[8], dnb[8], xa[8], xb[8];
-    if (g) {
-      load8(g + i0, ga);
-      load8(g + HALF + i0, gb);
-    } else {  // no gradient reached v
-#pragma unroll
-      for (int e = 0; e < 8; ++e) ga[e] = gb[e] = 0.f;
-    }
-    if (!is_v) {
-      load8(cosb + (size_t)p * D + i0, c);
-      load8(sinb + (size_t)p * D + i0, sn);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) c[e] = sn[e] = 0.f;  // not used
-    }
-    float rstd = 1.f;
-    if (wn && !is_v) rstd = is_q ? rstd_q[(size_t)tok * Hq + hd] : rstd_k[(size_t)tok * Hkv + (hd - Hq)];
+  for (int e = 0; e < 8; ++e) {
+    da[e] = ga[e] * c[e] + gb[e] * sn[e];
+    db[e] = gb[e] * c[e] - ga[e] * sn[e];
+  }
+  if (wn) {
+    float xa[8], xb[8], wa[8], wb[8];
+    load8(src + i0, xa);
+    load8(src + HALF + i0, xb);
+    load8(wn + i0, wa);
+    load8(wn + HALF + i0, wb);
+    const float rstd = rstd_in[it], one = a.w_plus_one ? 1.f : 0.f;
     float dot = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      dna[e] = is_v ? ga[e] : ga[e] * c[e] + gb[e] * sn[e];
-      dnb[e] = is_v ? gb[e] : gb[e] * c[e] - ga[e] * sn[e];
+      xa[e] *= rstd; xb[e] *= rstd;
+      const float ta = da[e] * xa[e], tb = db[e] * xb[e];
+      if (live) { ka[e] += ta; kb[e] += tb; }
+      const float sa = wa[e] + one, sb = wb[e] + one;
+      dot += ta * sa + tb * sb;
+      da[e] *= sa; db[e] *= sb;
     }
-    if (wn) {
-      float wa[8], wb[8];
-      if (!is_v) {
-        load8(src + i0, xa);
-        load8(src + HALF + i0, xb);
-      } else {
+    dot = group_sum<LPH>(dot) / D;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) xa[e] = xb[e] = 0.f;
-      }
-      load8(wn + i0, wa);
-      load8(wn + HALF + i0, wb);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        xa[e] *= rstd; xb[e] *= rstd;
-        float x = wa[e], y = wb[e];
-        if (w_plus_one) { x += 1.f; y += 1.f; }
-        if (live && !is_v) {
-          if (is_q) { dwq_a[e] += dna[e] * xa[e]; dwq_b[e] += dnb[e] * xb[e]; }
-          else { dwk_a[e] += dna[e] * xa[e]; dwk_b[e] += dnb[e] * xb[e]; }
-        }
-        if (!is_v) {
-          dna[e] *= x; dnb[e] *= y;
-          dot += dna[e] * xa[e] + dnb[e] * xb[e];
-        }
-      }
-      dot = group_sum<LPH>(dot) / D;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        if (!is_v) {
-          dna[e] = rstd * (dna[e] - xa[e] * dot);
-          dnb[e] = rstd * (dnb[e] - xb[e] * dot);
-        }
-      }
+    for (int e = 0; e < 8; ++e) {
+      da[e] = rstd * (da[e] - xa[e] * dot);
+      db[e] = rstd * (db[e] - xb[e] * dot);
     }
-    if (live) {
-      store8(dst + i0, dna);
-      store8(dst + HALF + i0, dnb);
+  }
+  if (live) {
+    __nv_bfloat16* dst = a.dqkv + (size_t)tok * a.dqkv_stride + (size_t)(head0 + hd) * D;
+    store8(dst + i0, da);
+    store8(dst + HALF + i0, db);
+  }
+}
+
+// dqkv from dq, dk, dv (null: zeros); dw_partial [gridDim.x, 2 * D]: sums of the q and k weight gradients of this block.
+// Bound by instructions first (conversions, two rotations' worth of products on 16 channels a lane), then by memory traffic, and
+// at small sizes by its tail. So a warp's heads are all of one kind (no selects between q and k, v is a plain copy), and heads are
+// counted in 32 bits when they fit. The weight sums are folded over the head groups of a warp by shuffles and over the warps in
+// shared memory: fp32 atomics there are a compare-and-swap loop, and 32 lane groups on one address held a block for 15 us.
+// Measured (32 / 4 heads of 128), with the copy of dv that used to be a launch: 4096 tokens 66 -> 43 us (52 with kinds mixed in a
+// warp), 512 tokens 31 -> 9.6. Two blocks an SM: three (85 registers) measured 52, four 43 and 13.
+template <int PAIRS>
+__global__ void __launch_bounds__(256, 2)
+qk_norm_rope_bwd_kernel(RopeBwdArgs a, const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16* __restrict__ dk, const __nv_bfloat16* __restrict__ dv,
+                        const __nv_bfloat16* __restrict__ qw, const __nv_bfloat16* __restrict__ kw, const float* __restrict__ rstd_q,
+                        const float* __restrict__ rstd_k, float* __restrict__ dw_partial, int Hq, int Hkv) {
+  constexpr int D = PAIRS * 64, HALF = D / 2, LPH = D / 16, HPW = 32 / LPH;
+  __shared__ float acc[8][2 * D];  // weight-gradient sums of each warp: q scales then k scales
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, i0 = lane % LPH * 8;
+  const long long gq = ((long long)a.n * Hq + HPW - 1) / HPW, gk = ((long long)a.n * Hkv + HPW - 1) / HPW;
+  float dwq_a[8], dwq_b[8], dwk_a[8], dwk_b[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) dwq_a[e] = dwq_b[e] = dwk_a[e] = dwk_b[e] = 0.f;
+  for (long long grp = (long long)blockIdx.x * 8 + wib; grp < gq + 2 * gk; grp += (long long)gridDim.x * 8) {
+    if (grp < gq) {
+      rope_bwd_group<D>(a, grp, Hq, 0, dq, qw, rstd_q, dwq_a, dwq_b);
+    } else if (grp < gq + gk) {
+      rope_bwd_group<D>(a, grp - gq, Hkv, Hq, dk, kw, rstd_k, dwk_a, dwk_b);
+    } else {
+      const long long item = (grp - gq - gk) * HPW + lane / LPH;
+      if (item < (long long)a.n * Hkv) {
+        const long long tok = item / Hkv;
+        __nv_bfloat16* dst = a.dqkv + (size_t)tok * a.dqkv_stride + (size_t)(Hq + Hkv + (item - tok * Hkv)) * D;
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4*>(dst + i0) = dv ? *reinterpret_cast<const uint4*>(dv + (size_t)item * D + i0) : zero;
+        *reinterpret_cast<uint4*>(dst + HALF + i0) = dv ? *reinterpret_cast<const uint4*>(dv + (size_t)item * D + HALF + i0) : zero;
+      }
     }
   }
   if (qw && dw_partial) {
@@ -406,9 +404,10 @@ PT_API int pt_qk_norm_rope_bwd(const void* dq, const void* dk, const void* dv, c
   if (n_tokens <= 0) return 0;
   if (D != 64 && D != 128) return -1;
   const int grid = pt_qk_norm_rope_bwd_grid(n_tokens, Hq, Hkv, D);
-#define LAUNCH(P) qk_norm_rope_bwd_kernel<P><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, \
-    (const __nv_bfloat16*)qkv, (__nv_bfloat16*)dqkv, (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, (const __nv_bfloat16*)cosb,             \
-    (const __nv_bfloat16*)sinb, pos, rstd_q, rstd_k, dw_partial, n_tokens, S, Hq, Hkv, qkv_stride, dqkv_stride, w_plus_one)
+  const RopeBwdArgs a{(const __nv_bfloat16*)qkv, (const __nv_bfloat16*)cosb, (const __nv_bfloat16*)sinb, pos, (__nv_bfloat16*)dqkv,
+                      qkv_stride, dqkv_stride, n_tokens, S, w_plus_one};
+#define LAUNCH(P) qk_norm_rope_bwd_kernel<P><<<grid, 256, 0, st>>>(a, (const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, \
+    (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, rstd_q, rstd_k, dw_partial, Hq, Hkv)
   if (D == 128) LAUNCH(2);
   else LAUNCH(1);
 #undef LAUNCH
