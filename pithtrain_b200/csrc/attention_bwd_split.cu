@@ -17,7 +17,7 @@
 // backward it replaces ran fp32 SIMT products over [heads, S, S] matrices in memory. Measured, causal, DQ + DK + DV:
 //   1 x 2048, 16 heads x 192/128    :  80 +  74 +  53 us  (tensor ops: about 3 ms)
 //   1 x 3072, 16/2 heads x 256      : 200 + 202 + 156 us  (tensor ops: about 9 ms)
-//   1 x 4093 in 9 documents, 32/4 heads x 128, with forward and the passes around it: 0.64 ms (tensor ops: 21 ms)
+//   1 x 4093 in 9 documents, 32/4 heads x 128, with forward and the passes around it: 0.61 ms (tensor ops: 21 ms)
 //
 // No atomics: dQ rows belong to one CTA; dK / dV of a query head are written once, directly when there is no GQA group,
 // else to per-head fp32 partials that attn_split_group_sum_kernel adds in head order. Results are reproducible.

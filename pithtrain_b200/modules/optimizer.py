@@ -314,11 +314,9 @@ class Muon(torch.optim.Optimizer):
             L = _native.lib()
             upd = torch.empty(w.shape, dtype=torch.bfloat16, device=w.device)
             # the fused norm and the passes over the Gram matrices work on whole 16-byte vectors of one matrix's rows
-            E, per = w.numel() // (n * m), n * m
-            fused = min(n, m) % 8 == 0 and min(n, m) <= 65536 and not _own_gemm_usable(upd)
+            fused = w.numel() > 0 and min(n, m) % 8 == 0 and min(n, m) <= 65536 and not _own_gemm_usable(upd)
+            E, per = (w.numel() // (n * m), n * m) if fused else (1, w.numel())
             partial = torch.empty((E, L.pt_muon_slabs(E, per)), dtype=torch.float32, device=w.device) if fused else None
-            if not fused:
-                E, per = 1, w.numel()
             rc = L.pt_muon_momentum_sumsq(g.data_ptr(), int(g.dtype == torch.float32), buf.data_ptr(),
                                           int(buf.dtype == torch.float32), upd.data_ptr(), E, per, float(beta),
                                           None if gscale is None else gscale.data_ptr(),

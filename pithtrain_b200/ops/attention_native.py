@@ -55,7 +55,8 @@ def row_lower_bounds(B: int, Sq: int, q_off: int, window_left: Optional[int], cu
     has_w = window_left is not None and window_left >= 0
     if not has_w and cu_seqlens is None:
         return None
-    if cu_seqlens is not None and cu_seqlens.is_cuda and cu_seqlens.numel() >= 2 and cu_seqlens.device == torch.device(device):
+    if (cu_seqlens is not None and cu_seqlens.is_cuda and cu_seqlens.dim() == 1 and cu_seqlens.numel() >= 2 and B * Sq > 0
+            and cu_seqlens.device == torch.device(device)):
         from .. import _native
 
         cu = cu_seqlens.to(torch.int32).contiguous()

@@ -500,3 +500,14 @@ def test_qk_norm_rope_backward(n, pad, norm, with_dv, Hq, Hkv, D):
     assert ((a.grad.double() - a64.grad).abs() <= BF16_MAX * a64.grad.abs() + 1e-5 * a64.grad.abs().max()).all()
     for w, d in zip(ws, w64) if norm else []:
         assert _rel(w.main_grad - 1, d.grad) < 1e-5
+
+
+def test_updates_and_bounds_without_elements():
+    from pithtrain_b200.modules.optimizer import Muon
+
+    w = torch.empty(0, 8, 16, device="cuda", dtype=torch.bfloat16)
+    Muon([torch.nn.Parameter(w)])._update_chunk(w, w.float(), w.float(), 0.95, 0.1, 0.0)
+    cu = torch.zeros(2, dtype=torch.int32, device="cuda")
+    assert N.row_lower_bounds(1, 0, 0, None, cu, cu.device).numel() == 0
+    with pytest.raises(RuntimeError):
+        N.row_lower_bounds(1, 4, 0, None, torch.zeros(2, 2, dtype=torch.int32, device="cuda"), cu.device)
