@@ -129,6 +129,7 @@ SIGS = {
     "pt_gated_attn_post_fwd": "PPLPIIIP",
     "pt_gated_attn_post_bwd": "PPPLPPIIIP",
     "pt_balanced_replay": "PIIIIP",
+    "pt_packed_positions": "PIPLP",
     "pt_row_lower_bounds": "PIPIIIIP",
     "pt_attn_bwd_split": "PPPPPPPPPPPPP" + "IIIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_attn_bwd": "PPPPPPPPPPPPPPP" + "IIIIII" + "LLLLL" + "F" + "II" + "P",

@@ -327,6 +327,20 @@ qk_norm_rope_bwd_kernel(RopeBwdArgs a, const __nv_bfloat16* __restrict__ dq, con
   }
 }
 
+// out[i] = i - start of the document that row i lies in: document s holds cu[s + 1] - cu[s] rows, one after the other from row 0;
+// rows past the last one count on. One launch for the slices, casts, differences, scan and repetition of the tensor-op form.
+__global__ void __launch_bounds__(256) packed_positions_kernel(const int* __restrict__ cu, int n_cu, long long* __restrict__ out, long long S) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= S) return;
+  const long long first = cu[0];
+  int a = 1, z = n_cu;  // first boundary beyond row i
+  while (a < z) {
+    const int mid = (a + z) >> 1;
+    if (cu[mid] - first <= i) a = mid + 1; else z = mid;
+  }
+  out[i] = i - cu[min(a - 1, n_cu - 2)];
+}
+
 }  // namespace pt
 
 using namespace pt;
@@ -470,5 +484,13 @@ PT_API int pt_colsum_accumulate_pair(const float* part, int G, int ld, int H, vo
   const int grid = (2 * H + 31) / 32, threads = 32 * pt::COLSUM_WARPS;
   if (dst_fp32) pt::colsum_accumulate_kernel<float><<<grid, threads, 0, st>>>(part, G, ld, 2 * H, (float*)dst0, (float*)dst1, H);
   else pt::colsum_accumulate_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(part, G, ld, 2 * H, (__nv_bfloat16*)dst0, (__nv_bfloat16*)dst1, H);
+  return (int)cudaGetLastError();
+}
+
+// cu: int32 [n_cu], n_cu >= 2; out: int64 [S].
+PT_API int pt_packed_positions(const int* cu, int n_cu, long long* out, long long S, void* stream_) {
+  if (S <= 0) return 0;
+  if (n_cu < 2 || S > 0x7fffffffLL) return -2;
+  packed_positions_kernel<<<(unsigned)((S + 255) / 256), 256, 0, (cudaStream_t)stream_>>>(cu, n_cu, out, S);
   return (int)cudaGetLastError();
 }

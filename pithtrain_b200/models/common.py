@@ -11,6 +11,7 @@ from typing import Any, Callable, Optional, Tuple
 import torch
 import torch.nn as nn
 
+from .. import _native
 from ..contexts import distributed
 from ..dualpipe.dualpipev import layer_partition
 from ..dualpipe.execution import ChunkRecord, model_forward
@@ -119,6 +120,13 @@ def zigzag_positions(S_local: int, cp_size: int, cp_rank: int, device) -> torch.
 
 
 def packed_positions(S: int, cu_seqlens: torch.Tensor) -> torch.Tensor:
+    """Position of each of ``S`` packed tokens within its document."""
+    if (cu_seqlens.is_cuda and cu_seqlens.dim() == 1 and cu_seqlens.numel() >= 2 and 0 < S < 2 ** 31
+            and cu_seqlens.dtype in (torch.int32, torch.int64)):
+        cu = cu_seqlens.to(torch.int32).contiguous()
+        out = torch.empty(S, dtype=torch.int64, device=cu.device)
+        _native.check(_native.lib().pt_packed_positions(cu.data_ptr(), cu.numel(), out.data_ptr(), S, _native.stream_ptr()), "pt_packed_positions")
+        return out
     starts = cu_seqlens[:-1].long()
     lengths = (cu_seqlens[1:] - cu_seqlens[:-1]).long()
     return torch.arange(S, device=cu_seqlens.device) - torch.repeat_interleave(starts, lengths, output_size=S)

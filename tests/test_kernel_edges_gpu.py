@@ -511,3 +511,15 @@ def test_updates_and_bounds_without_elements():
     assert N.row_lower_bounds(1, 0, 0, None, cu, cu.device).numel() == 0
     with pytest.raises(RuntimeError):
         N.row_lower_bounds(1, 4, 0, None, torch.zeros(2, 2, dtype=torch.int32, device="cuda"), cu.device)
+
+
+@pytest.mark.parametrize("docs", [[0, 1], [0, 7, 7, 8, 300], [0, 128, 256, 257], [0, 0, 5, 5], [3, 10, 700]])
+def test_packed_positions(docs):
+    """Against the tensor-op form on the CPU: empty documents, boundaries that do not start at 0."""
+    from pithtrain_b200.models.common import packed_positions
+
+    for dtype in (torch.int32, torch.int64):
+        cu = torch.tensor(docs, dtype=dtype)
+        S = docs[-1] - docs[0]
+        got = packed_positions(S, cu.cuda())
+        assert got.dtype == torch.int64 and torch.equal(got.cpu(), packed_positions(S, cu))
