@@ -29,14 +29,14 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   *reinterpret_cast<uint4*>(p) = raw;
 }
 
-// e^x with the rounding of x * log2(e) compensated (the build's fast expf loses |x| ulp); 0 where e^x < 2^-126.
+// e^x with the rounding of x * log2(e) compensated (the build's fast expf loses |x| ulp); 0 where e^x < 2^-126. A NaN stays a
+// NaN, and an infinite result (or argument) takes no correction, which would turn it into one.
 __device__ __forceinline__ float exp_compensated(float x) {
-  x = fminf(fmaxf(x, -138.f), 138.f);
   const float t = x * 1.4426950408889634f;
   const float r = fmaf(x, 1.4426950408889634f, -t) + x * 1.92596299e-8f;
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(t));
-  return fmaf(y, r * 0.6931471805599453f, y);
+  return fabsf(t) < 128.f ? fmaf(y, r * 0.6931471805599453f, y) : y;
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

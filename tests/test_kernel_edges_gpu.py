@@ -180,6 +180,43 @@ def test_gated_delta_rule_fused(B, S, H, strong):
             assert _rel(a, b) < BF16_MAX, name
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("-inf")])
+@pytest.mark.parametrize("t", [0, 70, 199])
+def test_gated_delta_rule_keeps_a_broken_gate_visible(t, bad):
+    """A NaN or infinite log gate shows in every output that the tensor-op form (fp32 inputs) loses to it, in gradients of q, k,
+    v, g and beta of that head, and nowhere in the other heads."""
+    from pithtrain_b200.ops.gated_delta_rule import gated_delta_rule
+
+    torch.manual_seed(t)
+    S = 200
+    q, k, v = (torch.nn.functional.normalize(torch.randn(1, S, 2, 128, device="cuda"), dim=-1).bfloat16() for _ in range(3))
+    g, beta = -torch.rand(1, S, 2, device="cuda") * 0.3, torch.rand(1, S, 2, device="cuda")
+    g[0, t, 1] = bad
+    fine = {}
+    for name, dtype in (("fused", torch.bfloat16), ("general", torch.float32)):
+        leaves = [x.detach().to(dtype).requires_grad_() for x in (q, k, v)] + [x.clone().requires_grad_() for x in (g, beta)]
+        o = gated_delta_rule(*leaves)
+        grads = torch.autograd.grad(o, leaves, torch.ones_like(o))
+        fine[name] = [torch.isfinite(x.detach()).view(S, 2, -1).all(-1) for x in (o, *grads)]
+    assert torch.equal(fine["fused"][0], fine["general"][0])
+    for got, want in zip(fine["fused"], fine["general"]):
+        assert got[:, 0].all() and want[:, 0].all()
+        assert not got[:, 1].all() and not want[:, 1].all()
+
+
+def test_gated_delta_rule_with_gates_beyond_the_range_of_exp():
+    """Gates that close a head entirely (e^-200 = 0) or grow its state (e^1 a step): as the tensor-op form."""
+    from pithtrain_b200.ops.gated_delta_rule import gated_delta_rule
+
+    torch.manual_seed(1)
+    q, k, v = (torch.nn.functional.normalize(torch.randn(1, 130, 3, 128, device="cuda"), dim=-1).bfloat16() for _ in range(3))
+    g = torch.tensor([-200.0, -0.1, 0.3], device="cuda").expand(1, 130, 3)
+    beta = torch.rand(1, 130, 3, device="cuda")
+    got, want = gated_delta_rule(q, k, v, g, beta), gated_delta_rule(q.float(), k.float(), v.float(), g, beta)
+    for h in range(3):
+        assert _rel(got[:, :, h], want[:, :, h].double()) < BF16_NORM + 2.0 ** -12, h
+
+
 @pytest.mark.parametrize("B,S,nk,nv", [(1, 1, 1, 1), (2, 3, 1, 2), (1, 31, 2, 2), (2, 33, 2, 4), (1, 97, 3, 9)])
 def test_gdn_conv(B, S, nk, nv):
     """Convolution + SiLU + l2 norm + repetition and its gradients against tensor ops in 64 bits: one bf16 rounding each."""
@@ -256,6 +293,27 @@ def test_router_replayed(n, E, k, renorm, dtype):
     # a logit's gradient is p times a difference that may cancel: fp32 error of its terms, then the rounding of the result
     size = 2.5 * float(dw.abs().max()) * k + float(dp.abs().max())
     assert ((lg.grad.double() - ld.grad).abs() <= 1e-6 * size + (BF16_MAX * ld.grad.abs() if dtype == torch.bfloat16 else 0)).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_router_replayed_keeps_nan(dtype):
+    """A NaN or +inf logit, or a row of -inf, spoils its own row as the library softmax has it, and no other; forward and backward."""
+    from pithtrain_b200.ops.router import router_replayed
+
+    torch.manual_seed(3)
+    logits = torch.randn(6, 40, device="cuda").to(dtype)
+    logits[1, 35], logits[2], logits[3, 0], logits[4, 7] = float("nan"), float("-inf"), float("inf"), float("-inf")
+    picks = torch.tensor([[0, 7, 35]], device="cuda").repeat(6, 1)
+    lg = logits.clone().requires_grad_()
+    w, _, probs = router_replayed(lg, 3, lambda idx: picks, True)
+    w.sum().backward()
+    ld = logits.double().requires_grad_()
+    want = ld.softmax(-1)
+    wd = want.gather(1, picks) / want.gather(1, picks).sum(-1, keepdim=True)
+    wd.sum().backward()
+    assert torch.equal(probs.isnan(), want.isnan()) and torch.equal(w.isnan(), wd.isnan()) and torch.equal(lg.grad.isnan(), ld.grad.isnan())
+    ok = [0, 4, 5]
+    assert _rel(probs[ok].detach(), want[ok].detach()) < 1e-6 and float(probs[4, 7]) == 0.0
 
 
 @pytest.mark.parametrize("k", [1, 3, 4, 6, 8])
