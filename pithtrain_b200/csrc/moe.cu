@@ -100,6 +100,10 @@ router_topk_fwd_kernel(const T* __restrict__ logits, float* __restrict__ probs,
         int oi = __shfl_xor_sync(0xffffffffu, bi, o);
         if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
       }
+      if (mode == 0 && bi == 0x7fffffff) {  // a row of NaN scores has no order: the first k experts, weight NaN
+        bi = t;
+        best = NAN;
+      }
       picked_w[t] = best;
       picked_i[t] = bi;
       wsum += best;

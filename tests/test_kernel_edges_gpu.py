@@ -316,6 +316,20 @@ def test_router_replayed_keeps_nan(dtype):
     assert _rel(probs[ok].detach(), want[ok].detach()) < 1e-6 and float(probs[4, 7]) == 0.0
 
 
+@pytest.mark.parametrize("E,k", [(4, 4), (40, 3), (512, 16)])
+def test_router_picks_of_a_nan_row_are_experts(E, k):
+    """The replay, and the natural router's callers, get k different experts of weight NaN for a row without an order."""
+    from pithtrain_b200.ops.router import router_replayed, router_topk
+
+    logits = torch.randn(5, E, device="cuda")
+    logits[1, E - 1], logits[3] = float("nan"), float("-inf")
+    w, idx, _ = router_replayed(logits, k, lambda i: i, True)
+    w0, idx0, _ = router_topk(logits, k, "softmax_topk", True)
+    assert torch.equal(idx, idx0) and torch.equal(w.isnan(), w0.isnan())
+    assert ((idx >= 0) & (idx < E)).all() and all(r.unique().numel() == k for r in idx)
+    assert torch.equal(w.isnan().all(-1), torch.tensor([False, True, False, True, False], device="cuda"))
+
+
 @pytest.mark.parametrize("k", [1, 3, 4, 6, 8])
 @pytest.mark.parametrize("n,H", [(1, 8), (3, 264), (64, 2048), (5000, 512)])
 def test_combine_rows(n, H, k):
