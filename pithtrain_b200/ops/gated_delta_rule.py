@@ -96,8 +96,10 @@ def chunk_state(w, u, qg, kd, a):
 
 def _rows_of_8(t: torch.Tensor) -> torch.Tensor:
     """``t [B,S,H,128]`` with rows the kernels can read in 16-byte pieces (a slice of a wider projection qualifies)."""
-    ok = t.stride(-1) == 1 and all(s % 8 == 0 for s in t.stride()[:3]) and t.data_ptr() % 16 == 0
-    return t if ok else t.contiguous()
+    if t.stride(-1) == 1 and all(s % 8 == 0 for s in t.stride()[:3]) and t.data_ptr() % 16 == 0:
+        return t
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()  # contiguous() hands a contiguous tensor back as it is
 
 
 class _GatedDeltaRule(torch.autograd.Function):

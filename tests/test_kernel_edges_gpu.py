@@ -217,6 +217,26 @@ def test_gated_delta_rule_with_gates_beyond_the_range_of_exp():
         assert _rel(got[:, :, h], want[:, :, h].double()) < BF16_NORM + 2.0 ** -12, h
 
 
+def _shifted(t, by=4):
+    """The same values, contiguous, ``by`` elements into their storage."""
+    return torch.cat([t.new_zeros(by), t.flatten()])[by:].view(t.shape)
+
+
+def test_gated_delta_rule_on_misaligned_inputs():
+    from pithtrain_b200.ops.gated_delta_rule import gated_delta_rule
+
+    torch.manual_seed(2)
+    ts = [torch.nn.functional.normalize(torch.randn(2, 67, 2, 128, device="cuda"), dim=-1).bfloat16() for _ in range(4)]
+    g, beta = -torch.rand(2, 67, 2, device="cuda"), torch.rand(2, 67, 2, device="cuda").bfloat16()
+    outs = []
+    for move in (lambda t: t.clone(), _shifted):
+        leaves = [move(t).requires_grad_() for t in (*ts[:3], g, beta)]
+        o = gated_delta_rule(*leaves)
+        outs.append([o, *torch.autograd.grad(o, leaves, move(ts[3]))])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("B,S,nk,nv", [(1, 1, 1, 1), (2, 3, 1, 2), (1, 31, 2, 2), (2, 33, 2, 4), (1, 97, 3, 9)])
 def test_gdn_conv(B, S, nk, nv):
     """Convolution + SiLU + l2 norm + repetition and its gradients against tensor ops in 64 bits: one bf16 rounding each."""

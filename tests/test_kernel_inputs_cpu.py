@@ -1,0 +1,30 @@
+"""What the host hands to kernels that read 16 bytes at a time, checked on the CPU: base addresses and row pitches."""
+
+import pytest
+import torch
+
+
+def _views(n, *shape):
+    """bf16 tensors of one shape: aligned, contiguous 4 elements into their storage, transposed, with an odd row pitch, expanded."""
+    numel = torch.Size(shape).numel()
+    base = torch.arange(numel + 64, dtype=torch.float32).bfloat16()
+    yield base[:numel].view(shape)
+    yield base[4:4 + numel].view(shape)
+    yield base[:numel].view(*shape[:-2], shape[-1], shape[-2]).transpose(-1, -2)
+    yield torch.zeros(*shape[:-1], shape[-1] + n).bfloat16()[..., :shape[-1]]
+    yield base[1:1 + shape[-1]].expand(shape)
+
+
+def _readable(t):
+    return t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(s % 8 == 0 for s, n in zip(t.stride()[:-1], t.shape) if n > 1)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 128), (2, 3, 2, 128), (1, 65, 4, 128)])
+def test_delta_rule_inputs_are_readable_in_16_byte_pieces(shape):
+    from pithtrain_b200.ops.gated_delta_rule import _rows_of_8
+
+    for t in _views(4, *shape):
+        got = _rows_of_8(t)
+        assert torch.equal(got, t) and _readable(got)
+    wide = torch.zeros(*shape[:2], 3 * shape[2] * 128).bfloat16()[..., 128 * shape[2]:256 * shape[2]].unflatten(-1, shape[2:])
+    assert _rows_of_8(wide).data_ptr() == wide.data_ptr()  # a slice of a projection is read in place
