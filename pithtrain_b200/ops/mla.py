@@ -13,10 +13,11 @@ from .common import sp, use_native
 
 def _rows(t: torch.Tensor) -> torch.Tensor:
     """2-D with rows readable in 16-byte pieces (a column slice of a wider projection qualifies)."""
-    return t if t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 else t.contiguous()
+    return t if t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 else _dense(t)
 
 
 def _dense(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous and 16-byte aligned."""
     t = t.contiguous()
     return t if t.data_ptr() % 16 == 0 else t.clone()
 

@@ -437,6 +437,17 @@ def test_mla_assembly(n, S, H, dn, dr, dv, positions):
         assert ((a - b).abs() <= BF16_MAX * b.abs() + 1e-6 * H * 5).all()
 
 
+def test_mla_assembly_on_misaligned_inputs():
+    from pithtrain_b200.ops import mla
+
+    torch.manual_seed(6)
+    q, kp, kv = (torch.randn(3, c, device="cuda").bfloat16() for c in (2 * 192, 64, 2 * 256))
+    cos, sin = (torch.rand(3, 64, device="cuda").bfloat16() for _ in range(2))
+    got = mla.mla_assemble(*(_shifted(t) for t in (q, kp, kv)), cos, sin, None, 3, 2, 128, 64, 128)
+    for a, b in zip(got, mla.mla_assemble(q, kp, kv, cos, sin, None, 3, 2, 128, 64, 128)):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("sizes", [[16], [0, 48, 16], [272, 0, 16, 528]])
 @pytest.mark.parametrize("H", [8, 264, 2880])
 def test_segment_sum_and_row_bias_dot(sizes, H):

@@ -28,3 +28,17 @@ def test_delta_rule_inputs_are_readable_in_16_byte_pieces(shape):
         assert torch.equal(got, t) and _readable(got)
     wide = torch.zeros(*shape[:2], 3 * shape[2] * 128).bfloat16()[..., 128 * shape[2]:256 * shape[2]].unflatten(-1, shape[2:])
     assert _rows_of_8(wide).data_ptr() == wide.data_ptr()  # a slice of a projection is read in place
+
+
+@pytest.mark.parametrize("n", [1, 5])
+def test_mla_inputs_are_readable_in_16_byte_pieces(n):
+    from pithtrain_b200.ops import mla
+
+    for t in _views(4, n, 64):
+        got = mla._rows(t)
+        assert torch.equal(got, t) and _readable(got)
+    wide = torch.zeros(n, 200).bfloat16()[:, 72:136]
+    assert mla._rows(wide).data_ptr() == wide.data_ptr()
+    # one token: the blocks of a projection of odd width are contiguous where they lie
+    for block in mla.split_columns(torch.zeros(1, 128 + 20 + 64).bfloat16(), (128, 20, 64)):
+        assert mla._rows(block).data_ptr() % 16 == 0
