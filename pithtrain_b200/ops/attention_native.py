@@ -88,6 +88,13 @@ def _as_token_major(t: torch.Tensor) -> torch.Tensor:
     return t if _token_major(t) else t.contiguous()
 
 
+def _aligned_gradient(do: torch.Tensor) -> torch.Tensor:
+    """``do`` as the pass over its rows reads it, in 16-byte pieces. Unlike q, k and v it comes to no tensor map of the forward
+    that would have refused a misaligned base, and ``contiguous()`` hands a contiguous piece of a larger gradient back as it is."""
+    do = _as_token_major(do)
+    return do if do.data_ptr() % 16 == 0 else do.clone()
+
+
 def forward(q, k, v, scale: float, causal: bool, q_off: int, row_lo: Optional[torch.Tensor],
             sinks: Optional[torch.Tensor]) -> Tuple[torch.Tensor, torch.Tensor]:
     """Launch the forward kernel: returns ``out [B,Sq,Hq,Dv]`` bf16 and ``lse [B,Hq,Sq]`` fp32."""
@@ -113,7 +120,7 @@ def backward(do, q, k, v, out, lse, scale: float, causal: bool, q_off: int, row_
     which the sink gradient needs)."""
     from .. import _native
 
-    q, k, v, do, out = (_as_token_major(t) for t in (q, k, v, do, out))
+    q, k, v, out, do = *(_as_token_major(t) for t in (q, k, v, out)), _aligned_gradient(do)
     lse = lse.contiguous()  # ring attention hands in halves of a longer sequence's statistics
     B, Sq, Hq, D = q.shape
     Sk, Hkv, Dv = k.shape[1], k.shape[2], v.shape[-1]
@@ -140,7 +147,7 @@ def backward_split(do, q, k, v, out, lse, scale: float, causal: bool, q_off: int
     of the forward kernel and any length. Same results; ``delta`` is a strided view."""
     from .. import _native
 
-    q, k, v, do, out = (_as_token_major(t) for t in (q, k, v, do, out))
+    q, k, v, out, do = *(_as_token_major(t) for t in (q, k, v, out)), _aligned_gradient(do)
     lse = lse.contiguous()
     B, Sq, Hq, D = q.shape
     Sk, Hkv, Dv = k.shape[1], k.shape[2], v.shape[-1]

@@ -448,6 +448,17 @@ def test_mla_assembly_on_misaligned_inputs():
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("S,Dqk,Dv", [(67, 128, 128), (128, 192, 128), (64, 256, 256), (68, 64, 64)])
+def test_attention_backward_of_a_misaligned_gradient(S, Dqk, Dv):
+    """A contiguous piece of a larger gradient that starts 8 bytes into it."""
+    torch.manual_seed(7)
+    q, k, v, do = (torch.randn(1, S, 2, d, device="cuda").bfloat16() for d in (Dqk, Dqk, Dv, Dv))
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    out = N.attention(*leaves, True, None, None, None, None)
+    for a, b in zip(torch.autograd.grad(out, leaves, _shifted(do), retain_graph=True), torch.autograd.grad(out, leaves, do)):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("sizes", [[16], [0, 48, 16], [272, 0, 16, 528]])
 @pytest.mark.parametrize("H", [8, 264, 2880])
 def test_segment_sum_and_row_bias_dot(sizes, H):

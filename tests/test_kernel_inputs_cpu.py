@@ -42,3 +42,12 @@ def test_mla_inputs_are_readable_in_16_byte_pieces(n):
     # one token: the blocks of a projection of odd width are contiguous where they lie
     for block in mla.split_columns(torch.zeros(1, 128 + 20 + 64).bfloat16(), (128, 20, 64)):
         assert mla._rows(block).data_ptr() % 16 == 0
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 2, 128), (2, 5, 3, 64), (1, 63, 1, 256)])
+def test_output_gradients_of_attention_are_readable_in_16_byte_pieces(shape):
+    from pithtrain_b200.ops import attention_native as N
+
+    for t in _views(4, *shape):
+        got = N._aligned_gradient(t)
+        assert torch.equal(got, t) and N._token_major(got)
