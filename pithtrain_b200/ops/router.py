@@ -119,7 +119,7 @@ def router_replayed(logits: torch.Tensor, k: int, replay, renorm: bool = False, 
                                               1.0, sp())
         _native.check(rc, "pt_router_topk_fwd")
         idx = replay(picks if getattr(replay, "any_int", False) else picks.long()).int().contiguous()
-        if idx.dim() == 2 and idx.shape[0] == n and 0 < idx.shape[1] <= 16:
+        if idx.device == lg.device and idx.dim() == 2 and idx.shape[0] == n and 0 < idx.shape[1] <= 16:
             w, probs = _RouterGivenFn.apply(logits, idx, renorm, scale)
             return w, idx, probs
     else:

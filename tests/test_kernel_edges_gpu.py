@@ -350,6 +350,13 @@ def test_router_picks_of_a_nan_row_are_experts(E, k):
     assert torch.equal(w.isnan().all(-1), torch.tensor([False, True, False, True, False], device="cuda"))
 
 
+def test_router_replayed_refuses_picks_on_another_device():
+    from pithtrain_b200.ops.router import router_replayed
+
+    with pytest.raises(RuntimeError):
+        router_replayed(torch.randn(3, 8, device="cuda"), 2, lambda idx: idx.cpu())
+
+
 @pytest.mark.parametrize("k", [1, 3, 4, 6, 8])
 @pytest.mark.parametrize("n,H", [(1, 8), (3, 264), (64, 2048), (5000, 512)])
 def test_combine_rows(n, H, k):
