@@ -155,7 +155,7 @@ def _fused_ok(q, k, v, g, beta, chunk_size: int) -> bool:
     """The fused kernels hold 64 x 128 tiles of bf16 inputs; everything else takes the general path below."""
     return (q.is_cuda and chunk_size == 64 and all(t.dtype == torch.bfloat16 for t in (q, k, v)) and q.shape[1] > 0
             and q.shape[0] > 0 and q.shape == k.shape == v.shape and q.shape[-1] == 128 and g.shape == beta.shape == q.shape[:3]
-            and q.shape[0] * q.shape[2] <= 65535)
+            and q.shape[0] * q.shape[2] <= 65535 and all(t.device == q.device for t in (k, v, g, beta)))
 
 
 def gated_delta_rule(q, k, v, g, beta, chunk_size: int = 64):

@@ -237,6 +237,16 @@ def test_gated_delta_rule_on_misaligned_inputs():
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("elsewhere", [1, 2, 3, 4])
+def test_gated_delta_rule_refuses_inputs_on_another_device(elsewhere):
+    from pithtrain_b200.ops.gated_delta_rule import gated_delta_rule
+
+    ts = [torch.rand(1, 9, 2, 128, device="cuda").bfloat16() for _ in range(3)] + [torch.rand(1, 9, 2, device="cuda") for _ in range(2)]
+    ts[elsewhere] = ts[elsewhere].cpu()
+    with pytest.raises(RuntimeError):
+        gated_delta_rule(*ts)
+
+
 @pytest.mark.parametrize("B,S,nk,nv", [(1, 1, 1, 1), (2, 3, 1, 2), (1, 31, 2, 2), (2, 33, 2, 4), (1, 97, 3, 9)])
 def test_gdn_conv(B, S, nk, nv):
     """Convolution + SiLU + l2 norm + repetition and its gradients against tensor ops in 64 bits: one bf16 rounding each."""
