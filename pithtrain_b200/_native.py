@@ -166,6 +166,12 @@ def stream_ptr() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
+def on_current_device(t: torch.Tensor) -> bool:
+    """Whether launches of this module, which go to the current device, reach the memory of ``t``. Operations that take a kernel
+    in place of tensor operations ask it, because those run on the device of their tensors."""
+    return t.is_cuda and t.get_device() == torch._C._cuda_getDevice()
+
+
 def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 

@@ -121,7 +121,7 @@ def zigzag_positions(S_local: int, cp_size: int, cp_rank: int, device) -> torch.
 
 def packed_positions(S: int, cu_seqlens: torch.Tensor) -> torch.Tensor:
     """Position of each of ``S`` packed tokens within its document."""
-    if (cu_seqlens.is_cuda and cu_seqlens.dim() == 1 and cu_seqlens.numel() >= 2 and 0 < S < 2 ** 31
+    if (_native.on_current_device(cu_seqlens) and cu_seqlens.dim() == 1 and cu_seqlens.numel() >= 2 and 0 < S < 2 ** 31
             and cu_seqlens.dtype in (torch.int32, torch.int64)):
         cu = cu_seqlens.to(torch.int32).contiguous()
         out = torch.empty(S, dtype=torch.int64, device=cu.device)

@@ -152,7 +152,7 @@ def force_balance(num_experts: int) -> Callable[[torch.Tensor], torch.Tensor]:
     def replay(topk_idx: torch.Tensor) -> torch.Tensor:
         n, k = topk_idx.shape
         stride = num_experts // k
-        if topk_idx.is_cuda and topk_idx.dtype in (torch.int32, torch.int64) and 0 < n * k < 2 ** 31 and 0 < num_experts < 2 ** 31:
+        if _native.on_current_device(topk_idx) and topk_idx.dtype in (torch.int32, torch.int64) and 0 < n * k < 2 ** 31 and 0 < num_experts < 2 ** 31:
             out = torch.empty((n, k), dtype=topk_idx.dtype, device=topk_idx.device)
             rc = _native.lib().pt_balanced_replay(out.data_ptr(), int(out.dtype == torch.int64), n, k, num_experts, _native.stream_ptr())
             _native.check(rc, "pt_balanced_replay")

@@ -55,10 +55,10 @@ def row_lower_bounds(B: int, Sq: int, q_off: int, window_left: Optional[int], cu
     has_w = window_left is not None and window_left >= 0
     if not has_w and cu_seqlens is None:
         return None
-    if (cu_seqlens is not None and cu_seqlens.is_cuda and cu_seqlens.dim() == 1 and cu_seqlens.numel() >= 2 and B * Sq > 0
-            and cu_seqlens.device == torch.device(device)):
-        from .. import _native
+    from .. import _native
 
+    if (cu_seqlens is not None and _native.on_current_device(cu_seqlens) and cu_seqlens.dim() == 1 and cu_seqlens.numel() >= 2
+            and B * Sq > 0 and cu_seqlens.device == torch.device(device)):
         cu = cu_seqlens.to(torch.int32).contiguous()
         lo = torch.empty(B * Sq, dtype=torch.int32, device=device)
         rc = _native.lib().pt_row_lower_bounds(cu.data_ptr(), cu.numel(), lo.data_ptr(), B, Sq, int(q_off), min(int(window_left), 1 << 30) if has_w else -1,

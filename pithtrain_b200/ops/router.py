@@ -111,7 +111,7 @@ def router_replayed(logits: torch.Tensor, k: int, replay, renorm: bool = False, 
     """:func:`router_topk` (``softmax_topk``) with the picks exchanged by ``replay(top-k indices) -> indices``: the weights are the
     softmax scores of the replayed experts. The indices are int64, or int32 for a ``replay`` with a true ``any_int``."""
     n, E = logits.shape
-    if logits.is_cuda and logits.dtype in (torch.float32, torch.bfloat16) and E <= 512 and k <= 16 and n > 0:
+    if _native.on_current_device(logits) and logits.dtype in (torch.float32, torch.bfloat16) and E <= 512 and k <= 16 and n > 0:
         lg = logits.detach().contiguous()
         picks = torch.empty((n, k), dtype=torch.int32, device=lg.device)
         w = torch.empty((n, k), dtype=torch.float32, device=lg.device)

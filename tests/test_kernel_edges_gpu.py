@@ -654,3 +654,25 @@ def test_packed_positions(docs):
         S = docs[-1] - docs[0]
         got = packed_positions(S, cu.cuda())
         assert got.dtype == torch.int64 and torch.equal(got.cpu(), packed_positions(S, cu))
+
+
+def test_tensors_of_another_device_take_the_tensor_operations(monkeypatch):
+    """Launches go to the current device: with the tensors on another one, no kernel may be handed their memory."""
+    from pithtrain_b200.models.common import packed_positions
+    from pithtrain_b200.modules.load_balance import force_balance
+    from pithtrain_b200.ops.router import router_replayed
+
+    cu, dev = torch.tensor([0, 3, 3, 9], dtype=torch.int32, device="cuda"), torch.device("cuda", torch.cuda.current_device())
+    picks, logits = torch.zeros(9, 2, dtype=torch.int32, device="cuda"), torch.randn(9, 8, device="cuda")
+    calls = [lambda: (packed_positions(9, cu),), lambda: (N.row_lower_bounds(1, 9, 0, 4, cu, dev),), lambda: (force_balance(8)(picks),),
+             lambda: router_replayed(logits, 2, force_balance(8), True)]
+    want = [c() for c in calls]
+
+    def no_launch(rc, what):
+        raise AssertionError(what)
+
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 99)
+    monkeypatch.setattr(_native, "check", no_launch)
+    for c, w in zip(calls, want):
+        for a, b in zip(c(), w):
+            torch.testing.assert_close(a, b, rtol=1e-6, atol=0)

@@ -1,5 +1,7 @@
 """What the host hands to kernels that read 16 bytes at a time, checked on the CPU: base addresses and row pitches."""
 
+from types import SimpleNamespace
+
 import pytest
 import torch
 
@@ -51,3 +53,12 @@ def test_output_gradients_of_attention_are_readable_in_16_byte_pieces(shape):
     for t in _views(4, *shape):
         got = N._aligned_gradient(t)
         assert torch.equal(got, t) and N._token_major(got)
+
+
+def test_current_device_predicate(monkeypatch):
+    from pithtrain_b200 import _native
+
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 1, raising=False)
+    on = [SimpleNamespace(is_cuda=True, get_device=lambda d=d: d) for d in (0, 1)]
+    assert [_native.on_current_device(t) for t in on] == [False, True]
+    assert not _native.on_current_device(torch.zeros(1))
