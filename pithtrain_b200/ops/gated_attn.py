@@ -21,7 +21,7 @@ def gated_attn_supported(qkv: torch.Tensor, q_w: torch.Tensor, k_w: torch.Tensor
     """bf16, heads of 64, 128 or 256 channels (8 to a lane) and a rotation of a multiple of 16 of them (a partner in another lane)."""
     return (use_native(qkv) and D in (64, 128, 256) and 0 < rope_dim <= D and rope_dim % 16 == 0 and qkv.dim() == 2 and qkv.shape[0] > 0
             and qkv.shape[1] == 2 * (Hq + Hkv) * D
-            and all(w.dtype == torch.bfloat16 and w.is_cuda and w.shape == (D,) and w.is_contiguous() and w.data_ptr() % 16 == 0
+            and all(w.dtype == torch.bfloat16 and w.device == qkv.device and w.shape == (D,) and w.is_contiguous() and w.data_ptr() % 16 == 0
                     for w in (q_w, k_w)))
 
 
@@ -66,6 +66,8 @@ class _Pre(torch.autograd.Function):
 def gated_attn_pre(qkv, q_w, k_w, cos, sin, Hq: int, Hkv: int, D: int, eps: float):
     """``qkv [n, 2*(Hq+Hkv)*D]`` (q and gate interleaved per head, then k, then v), ``cos``/``sin [n, R]`` ->
     ``q [n,Hq,D], k [n,Hkv,D], v [n,Hkv,D]`` and the gate ``[n,Hq,D]``, a view of the packed rows."""
+    if not cos.device == sin.device == qkv.device:
+        raise RuntimeError(f"qkv on {qkv.device}, rotary tables on {cos.device} and {sin.device}")
     return _Pre.apply(qkv, q_w, k_w, cos, sin, Hq, Hkv, D, eps)
 
 

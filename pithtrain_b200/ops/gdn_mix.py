@@ -19,7 +19,7 @@ def _dense(t: torch.Tensor) -> torch.Tensor:
 
 def conv_supported(x: torch.Tensor, weight: torch.Tensor, nk: int, nv: int, dk: int, dv: int) -> bool:
     """Heads of 128 channels, four taps, bf16: what a warp of the kernels holds in registers."""
-    return (use_native(x) and weight.dtype == torch.bfloat16 and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and dk == 128
+    return (use_native(x) and weight.device == x.device and weight.dtype == torch.bfloat16 and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and dk == 128
             and dv == 128 and nv % nk == 0 and weight.shape == ((2 * nk + nv) * 128, 1, 4) and x.dim() == 3
             and 0 < x.shape[0] <= 65535 and 0 < x.shape[1] <= 65535 * 32)
 
@@ -86,8 +86,9 @@ class _GatedNorm(torch.autograd.Function):
 
 
 def gated_norm_supported(x: torch.Tensor, z: torch.Tensor, weight: torch.Tensor) -> bool:
-    return (use_native(x) and z.dtype == weight.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[1] == 128 and z.shape == x.shape
-            and x.shape[0] > 0 and weight.is_contiguous() and weight.data_ptr() % 16 == 0)
+    return (use_native(x) and z.device == weight.device == x.device and _native.on_current_device(x)
+            and z.dtype == weight.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[1] == 128 and z.shape == x.shape
+            and x.shape[0] > 0 and weight.shape == (128,) and weight.is_contiguous() and weight.data_ptr() % 16 == 0)
 
 
 def gated_norm(x: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:

@@ -84,5 +84,8 @@ def supported(x: torch.Tensor, cos: torch.Tensor, H: int, dn: int, dr: int, dv: 
 def mla_assemble(q, k_pe, kv, cos, sin, positions: Optional[torch.Tensor], S: int, H: int, dn: int, dr: int, dv: int):
     """``q [n, H*(dn+dr)]``, ``k_pe [n, dr]``, ``kv [n, H*(dn+dv)]`` -> ``q, k [n,H,dn+dr]``, ``v [n,H,dv]`` with the rotary parts
     rotated (interleaved pairs in, halves out) and the rotary key shared by every head. ``positions`` int32 ``[n]`` or None (row % S)."""
+    for t in (k_pe, kv, cos, sin, *(() if positions is None else (positions,))):
+        if t.device != q.device:
+            raise RuntimeError(f"q on {q.device}, another input on {t.device}")
     pos = None if positions is None else positions.int().contiguous()
     return _Assemble.apply(q, k_pe, kv, cos, sin.contiguous(), pos, S, H, dn, dr, dv)

@@ -676,3 +676,27 @@ def test_tensors_of_another_device_take_the_tensor_operations(monkeypatch):
     for c, w in zip(calls, want):
         for a, b in zip(c(), w):
             torch.testing.assert_close(a, b, rtol=1e-6, atol=0)
+
+
+def test_layer_passes_refuse_inputs_on_another_device():
+    """Weights, gates and rotary tables elsewhere, or a weight that the general form would repeat over the channels, do not
+    reach the kernels as addresses."""
+    from pithtrain_b200.ops import gated_attn as GA, gdn_mix, mla
+
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    x, w = mk(4, 128), mk(128)
+    assert gdn_mix.gated_norm_supported(x, x, w)
+    for z, u in ((x.cpu(), w), (x, w.cpu()), (x, w[:1])):
+        assert not gdn_mix.gated_norm_supported(x, z, u)
+    taps = mk(3 * 128, 1, 4)
+    assert gdn_mix.conv_supported(mk(1, 5, 384), taps, 1, 1, 128, 128) and not gdn_mix.conv_supported(mk(1, 5, 384), taps.cpu(), 1, 1, 128, 128)
+    qkv, c = mk(4, 512), mk(4, 32)
+    assert GA.gated_attn_supported(qkv, w, w, 32, 1, 1, 128)
+    assert not GA.gated_attn_supported(qkv, w, w.cpu(), 32, 1, 1, 128)
+    args = (mk(4, 192), mk(4, 64), mk(4, 256), mk(4, 64), mk(4, 64), torch.arange(4, device="cuda"))
+    for i in range(2):
+        with pytest.raises(RuntimeError):
+            GA.gated_attn_pre(qkv, w, w, *(t.cpu() if i == j else t for j, t in enumerate((c, c))), 1, 1, 128, 1e-6)
+    for i in range(1, 6):
+        with pytest.raises(RuntimeError):
+            mla.mla_assemble(*(t.cpu() if i == j else t for j, t in enumerate(args)), 4, 1, 128, 64, 128)
