@@ -134,8 +134,8 @@ SIGS = {
     "pt_attn_bwd_split": "PPPPPPPPPPPPP" + "IIIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_attn_bwd": "PPPPPPPPPPPPPPP" + "IIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_gemm2cta_nt": "PPPIIILLLP",
-    "pt_mla_fwd": "PPPLLLPPPPPPIIIIIIP",
-    "pt_mla_bwd": "PPPPPPPPPIIIIIIP",
+    "pt_mla_fwd": "PPPLLLPPPPPPIIIIIIIP",
+    "pt_mla_bwd": "PPPPPPPPPIIIIIIIP",
     "pt_row_bias_dot": "PPPIPPPIIP",
     "pt_gdn_conv_fwd": "PPPPPIIIIP",
     "pt_gdn_conv_parts": "II",

@@ -6,6 +6,7 @@
 //   16 bytes. The rotary dims arrive as (x0, y0, x1, y1, ..) pairs and leave as (x.., y..) halves; rotated in fp32, rounded once.
 #include "elementwise.cuh"
 #include "host_common.h"
+#include "ptx.cuh"
 
 namespace pt {
 namespace mla {
@@ -13,10 +14,26 @@ namespace mla {
 struct Args {
   const __nv_bfloat16 *q, *kpe, *kv;  // row pitches ldq, ldk, ldkv
   long long ldq, ldk, ldkv;
-  const __nv_bfloat16 *cosb, *sinb;   // [max_pos, dr]
+  const __nv_bfloat16 *cosb, *sinb;   // [rows, dr]
   const int* pos;                     // optional [n]; else row % S
-  int n, S, H, dn, dr, dv;
+  int n, S, H, dn, dr, dv, rows;
+  int* err;
 };
+
+// Row of the rotary tables for token t, counted from their end if negative. A position outside them is recorded and reads as
+// row 0 (false): its rotated values are NaN.
+__device__ __forceinline__ bool table_row(const Args& p, int t, long long& row) {
+  const int pos = p.pos ? p.pos[t] : t % p.S;
+  row = pos < 0 ? pos + p.rows : pos;
+  if (row >= 0 && row < p.rows) return true;
+  if (threadIdx.x == 0 && p.err) atomicCAS(p.err, 0, PT_ERR_BOUNDS);
+  row = 0;
+  return false;
+}
+__device__ __forceinline__ void spoil(float (&a)[8], float (&b)[8]) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) a[e] = b[e] = NAN;
+}
 
 // 16 interleaved values -> 8 of the first and 8 of the second half, rotated; i0 = 8 j is the first pair
 __device__ __forceinline__ void rotate(const __nv_bfloat16* src, const __nv_bfloat16* c, const __nv_bfloat16* s, int i0, int half,
@@ -53,8 +70,9 @@ __global__ void __launch_bounds__(256) fwd_kernel(const Args p, __nv_bfloat16* _
                                                   __nv_bfloat16* __restrict__ vo) {
   const int t = blockIdx.x, half = p.dr / 2, d = p.dn + p.dr;
   const __nv_bfloat16 *q = p.q + t * p.ldq, *kv = p.kv + t * p.ldkv, *kpe = p.kpe + t * p.ldk;
-  const int pos = p.pos ? p.pos[t] : t % p.S;
-  const __nv_bfloat16 *c = p.cosb + (long long)pos * p.dr, *s = p.sinb + (long long)pos * p.dr;
+  long long row;
+  const bool known = table_row(p, t, row);
+  const __nv_bfloat16 *c = p.cosb + row * p.dr, *s = p.sinb + row * p.dr;
   __nv_bfloat16 *qt = qo + (long long)t * p.H * d, *kt = ko + (long long)t * p.H * d, *vt = vo + (long long)t * p.H * p.dv;
   const int nn = p.dn / 8, nv = p.dv / 8, nr = p.dr / 16;
   for (int i = threadIdx.x; i < p.H * nn; i += blockDim.x) {
@@ -70,9 +88,11 @@ __global__ void __launch_bounds__(256) fwd_kernel(const Args p, __nv_bfloat16* _
     const int h = i / nr, i0 = (i - h * nr) * 8;
     float a[8], b[8];
     rotate(q + h * d + p.dn, c, s, i0, half, a, b);
+    if (!known) spoil(a, b);
     store8(qt + h * d + p.dn + i0, a);
     store8(qt + h * d + p.dn + half + i0, b);
     rotate(kpe, c, s, i0, half, a, b);
+    if (!known) spoil(a, b);
     store8(kt + h * d + p.dn + i0, a);
     store8(kt + h * d + p.dn + half + i0, b);
   }
@@ -83,8 +103,9 @@ __global__ void __launch_bounds__(256) bwd_kernel(const Args p, const __nv_bfloa
                                                   __nv_bfloat16* __restrict__ dkpe, __nv_bfloat16* __restrict__ dkv) {
   extern __shared__ float part[];  // [H][dr]: the heads' gradients of the shared rotary key
   const int t = blockIdx.x, half = p.dr / 2, d = p.dn + p.dr;
-  const int pos = p.pos ? p.pos[t] : t % p.S;
-  const __nv_bfloat16 *c = p.cosb + (long long)pos * p.dr, *s = p.sinb + (long long)pos * p.dr;
+  long long row;
+  const bool known = table_row(p, t, row);
+  const __nv_bfloat16 *c = p.cosb + row * p.dr, *s = p.sinb + row * p.dr;
   const __nv_bfloat16 *qt = gq + (long long)t * p.H * d, *kt = gk + (long long)t * p.H * d, *vt = gv + (long long)t * p.H * p.dv;
   __nv_bfloat16 *dqt = dq + (long long)t * p.H * d, *dkvt = dkv + (long long)t * p.H * (p.dn + p.dv);
   const int nn = p.dn / 8, nv = p.dv / 8, nr = p.dr / 16;
@@ -92,9 +113,11 @@ __global__ void __launch_bounds__(256) bwd_kernel(const Args p, const __nv_bfloa
     const int h = i / nr, i0 = (i - h * nr) * 8;
     float lo[8], hi[8];
     rotate_back(qt + h * d + p.dn, c, s, i0, half, lo, hi);
+    if (!known) spoil(lo, hi);
     store8(dqt + h * d + p.dn + 2 * i0, lo);
     store8(dqt + h * d + p.dn + 2 * i0 + 8, hi);
     rotate_back(kt + h * d + p.dn, c, s, i0, half, lo, hi);
+    if (!known) spoil(lo, hi);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       part[h * p.dr + 2 * i0 + e] = lo[e];
@@ -119,7 +142,7 @@ __global__ void __launch_bounds__(256) bwd_kernel(const Args p, const __nv_bfloa
 }
 
 inline bool valid(const Args& a) {
-  return a.n > 0 && a.H > 0 && a.S > 0 && a.dn > 0 && a.dv > 0 && a.dr > 0 && a.dn % 8 == 0 && a.dv % 8 == 0 && a.dr % 16 == 0 &&
+  return a.n > 0 && a.H > 0 && a.S > 0 && a.rows > 0 && a.dn > 0 && a.dv > 0 && a.dr > 0 && a.dn % 8 == 0 && a.dv % 8 == 0 && a.dr % 16 == 0 &&
          a.H * a.dr * 4 <= 48 * 1024;
 }
 
@@ -129,13 +152,13 @@ inline bool valid(const Args& a) {
 using namespace pt;
 
 // q [n, H (dn + dr)], kpe [n, dr], kv [n, H (dn + dv)] bf16 with row pitches (elements, multiples of 8, 16-byte aligned bases); cosb,
-// sinb [max_pos, dr] bf16; pos int32 [n] or null (then row % S). Outputs contiguous. dn, dv multiples of 8, dr of 16.
+// sinb [rows, dr] bf16; pos int32 [n] or null (then row % S). Outputs contiguous. dn, dv multiples of 8, dr of 16.
 PT_API int pt_mla_fwd(const void* q, const void* kpe, const void* kv, long long ldq, long long ldk, long long ldkv, const void* cosb,
                       const void* sinb, const int* pos, void* qo, void* ko, void* vo, int n, int S, int H, int dn, int dr, int dv,
-                      void* stream_) {
+                      int rows, void* stream_) {
   using B = __nv_bfloat16;
   const mla::Args a{static_cast<const B*>(q), static_cast<const B*>(kpe), static_cast<const B*>(kv), ldq, ldk, ldkv, static_cast<const B*>(cosb),
-                    static_cast<const B*>(sinb), pos, n, S, H, dn, dr, dv};
+                    static_cast<const B*>(sinb), pos, n, S, H, dn, dr, dv, rows, device_status_word()};
   if (!mla::valid(a)) return -2;
   mla::fwd_kernel<<<n, 256, 0, static_cast<cudaStream_t>(stream_)>>>(a, static_cast<B*>(qo), static_cast<B*>(ko), static_cast<B*>(vo));
   return (int)cudaGetLastError();
@@ -143,9 +166,10 @@ PT_API int pt_mla_fwd(const void* q, const void* kpe, const void* kv, long long 
 
 // Gradients gq, gk, gv of the outputs (contiguous) -> dq [n, H (dn + dr)], dkpe [n, dr], dkv [n, H (dn + dv)], contiguous.
 PT_API int pt_mla_bwd(const void* gq, const void* gk, const void* gv, const void* cosb, const void* sinb, const int* pos, void* dq, void* dkpe,
-                      void* dkv, int n, int S, int H, int dn, int dr, int dv, void* stream_) {
+                      void* dkv, int n, int S, int H, int dn, int dr, int dv, int rows, void* stream_) {
   using B = __nv_bfloat16;
-  const mla::Args a{nullptr, nullptr, nullptr, 0, 0, 0, static_cast<const B*>(cosb), static_cast<const B*>(sinb), pos, n, S, H, dn, dr, dv};
+  const mla::Args a{nullptr, nullptr, nullptr, 0, 0, 0, static_cast<const B*>(cosb), static_cast<const B*>(sinb), pos, n, S, H, dn, dr, dv, rows,
+                    device_status_word()};
   if (!mla::valid(a)) return -2;
   mla::bwd_kernel<<<n, 256, H * dr * 4, static_cast<cudaStream_t>(stream_)>>>(
       a, static_cast<const B*>(gq), static_cast<const B*>(gk), static_cast<const B*>(gv), static_cast<B*>(dq), static_cast<B*>(dkpe),

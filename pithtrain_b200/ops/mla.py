@@ -52,7 +52,7 @@ class _Assemble(torch.autograd.Function):
         vo = torch.empty((n, H, dv), dtype=q.dtype, device=dev)
         rc = _native.lib().pt_mla_fwd(q.data_ptr(), k_pe.data_ptr(), kv.data_ptr(), q.stride(0), k_pe.stride(0), kv.stride(0), cos.data_ptr(),
                                       sin.data_ptr(), _native.ptr(positions), qo.data_ptr(), ko.data_ptr(), vo.data_ptr(), n, S, H, dn, dr, dv,
-                                      sp())
+                                      cos.shape[0], sp())
         _native.check(rc, "pt_mla_fwd")
         ctx.save_for_backward(cos, sin, positions)
         ctx.cfg = (S, H, dn, dr, dv)
@@ -70,7 +70,7 @@ class _Assemble(torch.autograd.Function):
         dkpe = torch.empty((n, dr), dtype=like.dtype, device=dev)
         dkv = torch.empty((n, H * (dn + dv)), dtype=like.dtype, device=dev)
         rc = _native.lib().pt_mla_bwd(gq.data_ptr(), gk.data_ptr(), gv.data_ptr(), cos.data_ptr(), sin.data_ptr(), _native.ptr(positions),
-                                      dq.data_ptr(), dkpe.data_ptr(), dkv.data_ptr(), n, S, H, dn, dr, dv, sp())
+                                      dq.data_ptr(), dkpe.data_ptr(), dkv.data_ptr(), n, S, H, dn, dr, dv, cos.shape[0], sp())
         _native.check(rc, "pt_mla_bwd")
         return (dq, dkpe, dkv) + (None,) * 8
 
@@ -88,4 +88,4 @@ def mla_assemble(q, k_pe, kv, cos, sin, positions: Optional[torch.Tensor], S: in
         if t.device != q.device:
             raise RuntimeError(f"q on {q.device}, another input on {t.device}")
     pos = None if positions is None else positions.int().contiguous()
-    return _Assemble.apply(q, k_pe, kv, cos, sin.contiguous(), pos, S, H, dn, dr, dv)
+    return _Assemble.apply(q, k_pe, kv, cos, _dense(sin), pos, S, H, dn, dr, dv)

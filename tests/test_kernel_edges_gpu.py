@@ -700,3 +700,29 @@ def test_layer_passes_refuse_inputs_on_another_device():
     for i in range(1, 6):
         with pytest.raises(RuntimeError):
             mla.mla_assemble(*(t.cpu() if i == j else t for j, t in enumerate(args)), 4, 1, 128, 64, 128)
+
+
+@pytest.mark.parametrize("positions", [None, [0, 1, 7, 3], [2, -8, 0, -1], [2, -9, 0, 1]])
+def test_mla_positions_outside_the_rotary_tables(positions):
+    """Negative positions count from the end of the tables, as an index does; one outside them is never read, shows as NaN both
+    ways and is reported."""
+    from pithtrain_b200.ops import mla
+
+    torch.manual_seed(4)
+    n, rows = 4, 3 if positions is None else 8
+    bad = next((i for i, x in enumerate(positions or range(n)) if not -rows <= x < rows), None)
+    q, kp, kv = (torch.randn(n, c, device="cuda").bfloat16().requires_grad_() for c in (2 * 32, 16, 2 * 32))
+    cos, sin = (torch.rand(rows, 16, device="cuda").bfloat16() for _ in range(2))
+    pos = None if positions is None else torch.tensor(positions, device="cuda")
+    out = mla.mla_assemble(q, kp, kv, cos, sin, pos, n, 2, 16, 16, 16)
+    grads = torch.autograd.grad(out, (q, kp, kv), [torch.ones_like(t) for t in out])
+    if bad is None:
+        _native.check_status()
+        same = mla.mla_assemble(q, kp, kv, cos, sin, pos % rows, n, 2, 16, 16, 16)
+        assert all(torch.equal(a, b) for a, b in zip(out, same))
+    else:
+        with pytest.raises(_native.KernelStatusError):
+            _native.check_status()
+    for t, part in ((out[0], slice(16, None)), (out[1], slice(16, None)), (grads[0].view(n, 2, 32), slice(16, None)), (grads[1][:, None], slice(None))):
+        assert [bool(x) for x in t[..., part].isnan().all(-1).all(-1)] == [i == bad for i in range(n)]
+    assert torch.isfinite(out[2]).all() and torch.isfinite(grads[2]).all()
