@@ -387,7 +387,7 @@ class _MoEExpertsFn(torch.autograd.Function):
         if ew.b2 is not None:
             # y = act @ W2.T + b2 ; the routing-weight gradient also sees the bias term
             row_bias_dot(dyg, ew.b2.detach(), offs, slot_of_row, d_w_flat, n_rows)
-            row_w = w.reshape(-1).float()[slot_of_row.clamp(min=0)]  # pad rows of dyg are zero, whatever their weight
+            row_w = torch.cat([w.reshape(-1).float(), w.new_zeros(1, dtype=torch.float32)])[slot_of_row]  # -1 (pad) picks the zero
             accumulate_grad(ew.b2, segment_sum(dyg, offs, E, row_w=row_w))
         if ew.b1 is not None:
             accumulate_grad(ew.b1, segment_sum(dgu, offs, E))

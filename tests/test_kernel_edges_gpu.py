@@ -506,6 +506,24 @@ def test_segment_sum_and_row_bias_dot(sizes, H):
     assert (dw.double() - want).abs().max() < 2.0 ** -24 * H * 25 * 16
 
 
+@pytest.mark.parametrize("biased", [False, True])
+def test_experts_without_tokens(biased):
+    """A rank of an expert-parallel group that receives nothing: only pad rows, and no slot that they could take a weight from."""
+    from pithtrain_b200.ops import moe as M
+
+    k, E, H, I = 2, 4, 128, 64
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    x, w = mk(0, H).requires_grad_(), torch.rand(0, k, device="cuda").requires_grad_()
+    g1, g2 = torch.zeros(E, 2 * I, H, device="cuda"), torch.zeros(E, H, I, device="cuda")
+    b1, b2 = (torch.nn.Parameter(mk(E, c)) for c in (2 * I, H)) if biased else (None, None)
+    ew = M.ExpertWeights(mk(E, 2 * I, H), mk(E, H, I), lambda: g1, lambda: g2, b1=b1, b2=b2)
+    out = M.moe_experts(x, w, torch.zeros(0, k, dtype=torch.int32, device="cuda"), ew)
+    out.backward(torch.ones_like(out))
+    _native.check_status()
+    assert out.shape == x.grad.shape == (0, H) and w.grad.shape == (0, k)
+    assert all(not t.any() for t in (g1, g2, *((b1.grad, b2.grad) if biased else ())))
+
+
 @pytest.mark.parametrize("window", [None, 0, 5, 300])
 @pytest.mark.parametrize("docs", [[0, 1], [0, 7, 7, 8, 300], [0, 128, 256, 300], [0, 100, 200]])
 def test_row_lower_bounds(docs, window):

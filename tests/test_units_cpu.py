@@ -245,6 +245,23 @@ def test_moe_experts_cpu_vs_loop():
             assert torch.allclose(a, b, atol=1e-4, rtol=1e-4)
 
 
+def test_pad_rows_of_biased_experts_take_no_weight():
+    """An infinite weight of the first slot stays with its expert: every group has pad rows here."""
+    from pithtrain_b200.ops import moe as M
+
+    torch.manual_seed(0)
+    n, k, E, H, I = 5, 2, 4, 16, 8
+    x, w = torch.randn(n, H, requires_grad=True), torch.rand(n, k)
+    w[0, 0] = float("inf")
+    eids = (torch.arange(n)[:, None] * 2 % E + torch.arange(k)).int()  # slot 0 goes to expert 0
+    b1, b2 = torch.nn.Parameter(torch.randn(E, 2 * I)), torch.nn.Parameter(torch.randn(E, H))
+    g1, g2 = torch.zeros(E, 2 * I, H), torch.zeros(E, H, I)
+    ew = M.ExpertWeights(torch.randn(E, 2 * I, H) * 0.2, torch.randn(E, H, I) * 0.2, lambda: g1, lambda: g2, b1=b1, b2=b2)
+    out = M.moe_experts(x, w.requires_grad_(), eids, ew)
+    out.backward(torch.ones_like(out))
+    assert not torch.isfinite(b2.grad[0]).any() and torch.isfinite(b2.grad[1:]).all()
+
+
 # ------------------------------------------------------------------------------------------------ data
 def test_datasets(tmp_path):
     from pithtrain_b200.modules.dataset import ConcatDataset, MemmapDataset, SyntheticDataset
