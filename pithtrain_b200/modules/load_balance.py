@@ -157,11 +157,9 @@ def force_balance(num_experts: int) -> Callable[[torch.Tensor], torch.Tensor]:
             rc = _native.lib().pt_balanced_replay(out.data_ptr(), int(out.dtype == torch.int64), n, k, num_experts, _native.stream_ptr())
             _native.check(rc, "pt_balanced_replay")
             return out
-        t = torch.arange(n, device=topk_idx.device, dtype=topk_idx.dtype).unsqueeze(1)
-        if stride == 0:  # more slots than experts: every slot of a token goes to the same one
-            return (t % num_experts).expand(n, k).clone()
-        j = torch.arange(0, k * stride, stride, device=topk_idx.device, dtype=topk_idx.dtype).unsqueeze(0)
-        return (t + j) % num_experts
+        t = torch.arange(n, device=topk_idx.device).unsqueeze(1)
+        j = torch.arange(k, device=topk_idx.device).unsqueeze(0)
+        return ((t + j * stride) % num_experts).to(topk_idx.dtype)
 
     replay.any_int = True  # takes the picks in the type that the router kernel writes
     return replay

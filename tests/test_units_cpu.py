@@ -245,6 +245,16 @@ def test_moe_experts_cpu_vs_loop():
             assert torch.allclose(a, b, atol=1e-4, rtol=1e-4)
 
 
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.int8, torch.int16, torch.int32, torch.int64, torch.float32])
+@pytest.mark.parametrize("n,E,k", [(300, 100, 4), (1, 1, 1), (257, 6, 3), (40, 4, 8)])
+def test_balanced_replay_in_every_type(n, E, k, dtype):
+    """More tokens than the type counts: the sums are made in 64 bits."""
+    from pithtrain_b200.modules.load_balance import force_balance
+
+    got = force_balance(E)(torch.zeros(n, k, dtype=dtype))
+    assert got.dtype == dtype and got.tolist() == [[(t + j * (E // k)) % E for j in range(k)] for t in range(n)]
+
+
 def test_pad_rows_of_biased_experts_take_no_weight():
     """An infinite weight of the first slot stays with its expert: every group has pad rows here."""
     from pithtrain_b200.ops import moe as M
