@@ -1,8 +1,12 @@
-// Attention backward that keeps P and dS at fp32 accuracy, for sm_100a (tcgen05 / TMEM / TMA): head dims 64, 128, 192/128
+// Attention backward that keeps all 24 bits of P and dS, for sm_100a (tcgen05 / TMEM / TMA): head dims 64, 128, 192/128
 // (MLA) and 256, any sequence length, with the masks of the forward kernel. It covers what csrc/attention_bwd.cu does
 // not (wider heads, lengths that are no multiple of 4), where gradients come from unrounded probabilities:
-//   P = hi + lo and dS = hi + lo as two bf16 numbers each (16 mantissa bits and more; error 2^-17 of the value), so every
-//   product with them is two MMAs into the same fp32 accumulator. S and dP need no split: their operands are bf16.
+//   P = hi + mid + lo and dS likewise, three bf16 numbers of 8 bits each (what is left is below 2^-25 of the value), so every
+//   product with them is three MMAs into the same fp32 accumulator. S and dP need no split: their operands are bf16.
+// Error of the fp32 sums of dV against 64 bits, causal, 64 / 517 / 2048 rows: 5e-7 / 2.6e-6 / 9e-6 (two terms: 2.2e-6 / 3.0e-6 /
+// 7.9e-6; fp32 tensor ops: 2.4e-7 / 5.4e-7 / 1.1e-6). At short lengths the terms decide, at long ones that the tensor core cuts
+// its fp32 sums off where FMAs round them. The bf16 gradients do not tell the three apart: 1.655e-3 +- 1e-7 each at 3072 rows.
+// Two terms did show where the keys share a large common part (it cancels in dQ): 1.6602e-3 against 1.6586e-3 (tensor ops 1.6589e-3).
 //
 // What bounds the shapes is on-chip memory: at head dim 256 a 128-row dK and dV tile alone fill the 512 TMEM columns, and
 // two stationary plus two streamed 128-row tiles do not fit in shared memory. Hence one accumulator per launch and
@@ -11,13 +15,14 @@
 //   DK : X1 = K, X2 = V   Y1 = Q, Y2 = dO    dK += dS^T Q
 //   DQ : X1 = Q, X2 = dO  Y1 = K, Y2 = V     dQ += dS K
 //     S = X1 Y1^T, dP = X2 Y2^T -> TMEM (two buffers of 64 columns each); P = exp2(S c - lse2), dS = P o (dP - delta);
-//     hi / lo go back over S's own columns in TMEM and are the A operand of the accumulating MMA (B = Y1 or Y2 read
-//     MN-major). S and dP of step n+1 are issued before the accumulation of step n, so they run under its exponentials.
-// Recomputing S twice and dP once costs 11 products of the tile instead of 5, all on the tensor core; the tensor-op
-// backward it replaces ran fp32 SIMT products over [heads, S, S] matrices in memory. Measured, causal, DQ + DK + DV:
-//   1 x 2048, 16 heads x 192/128    :  80 +  74 +  53 us  (tensor ops: about 3 ms)
-//   1 x 3072, 16/2 heads x 256      : 200 + 202 + 156 us  (tensor ops: about 9 ms)
-//   1 x 4093 in 9 documents, 32/4 heads x 128, with forward and the passes around it: 0.61 ms (tensor ops: 21 ms)
+//     hi and mid go back over S's own columns in TMEM, lo over dP's, and are the A operand of the accumulating MMA (B = Y1 or
+//     Y2 read MN-major). S and dP of step n+1 are issued before the accumulation of step n, so they run under its exponentials.
+// Recomputing S twice and dP once and splitting costs 14 products of the tile instead of 5, all on the tensor core; the
+// tensor-op backward it replaces ran fp32 SIMT products over [heads, S, S] matrices in memory. Measured, causal, DQ + DK + DV
+// (with two terms):
+//   1 x 2048, 16 heads x 192/128         :  90 +  81 +  62 us  ( 83 +  75 +  55; tensor ops: about 3 ms)
+//   1 x 3072, 16/2 heads x 256           : 222 + 219 + 174 us  (201 + 199 + 155; tensor ops: about 9 ms)
+//   1 x 4093 in 9 documents, 32/4 x 128  : 147 + 169 + 150 us  (136 + 159 + 139; tensor ops: 21 ms)
 //
 // No atomics: dQ rows belong to one CTA; dK / dV of a query head are written once, directly when there is no GQA group,
 // else to per-head fp32 partials that attn_split_group_sum_kernel adds in head order. Results are reproducible.
@@ -86,7 +91,7 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   uint64_t* y2_full = bars + 5;     // NST2
   uint64_t* y2_empty = bars + 7;    // NST2
   uint64_t* s_full = bars + 9;      // 2: S (and dP) of a step are in TMEM
-  uint64_t* a_ready = bars + 11;    // 2: compute (8 warps) -> MMA: hi / lo are in TMEM, dP has been read
+  uint64_t* a_ready = bars + 11;    // 2: compute (8 warps) -> MMA: hi / mid / lo are in TMEM, dP has been read
   uint64_t* acc_done = bars + 13;   // 1
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 14);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
@@ -270,12 +275,14 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         if (!ok) break;
         tc_fence_after();
         const uint32_t yb = ym + (MODE == ASP_DV ? s2 * (Cfg::Y2_BYTES >> 4) : s1 * (Cfg::Y1_BYTES >> 4));
-        // columns of the buffer, per half h of 32 streamed rows: hi 16 columns at 32 h, lo 16 columns at 32 h + 16
+        // columns of the buffer, per half h of 32 streamed rows: hi 16 columns at 32 h, mid 16 columns at 32 h + 16; lo 16
+        // columns at 32 h of the dP buffer of the step
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint32_t a = tmem_base + (n & 1) * 64 + (k >> 1) * 32 + (k & 1) * 8;
           umma_f16_ts_lh(tACC, a, yb + ((k * 2048) >> 4), HI, IDESC_A, (k != 0 || n != 0) ? 1u : 0u);
           umma_f16_ts_lh(tACC, a + 16, yb + ((k * 2048) >> 4), HI, IDESC_A, 1u);
+          umma_f16_ts_lh(tACC, a + 128, yb + ((k * 2048) >> 4), HI, IDESC_A, 1u);
         }
         umma_commit(&y1_empty[s1]);
         if (MODE == ASP_DV) umma_commit(&y2_empty[s2]);
@@ -334,7 +341,7 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       // element masks only where a lane needs them (warp-uniform: the stores below are collective)
       const bool masked = __any_sync(0xffffffffu, y0 < my_lo || y0 + 31 > my_hi);
       const float* st = reinterpret_cast<const float*>(sStat + (n % NST1) * 512) + g * 32;
-      uint32_t hi[16], lo[16];
+      uint32_t hi[16], mid[16], lo[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         float v[2];
@@ -349,10 +356,14 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         }
         hi[i] = pack_bf16x2(v[0], v[1]);
         const float2 h = unpack_bf16x2(hi[i]);
-        lo[i] = pack_bf16x2(v[0] - h.x, v[1] - h.y);
+        v[0] -= h.x; v[1] -= h.y;  // exact: what a rounding leaves fits in fewer bits
+        mid[i] = pack_bf16x2(v[0], v[1]);
+        const float2 m = unpack_bf16x2(mid[i]);
+        lo[i] = pack_bf16x2(v[0] - m.x, v[1] - m.y);
       }
       tmem_st_32x16(tS, hi);
-      tmem_st_32x16(tS + 16, lo);
+      tmem_st_32x16(tS + 16, mid);
+      tmem_st_32x16(tS + 128, lo);  // over dP, which this warp alone reads and has read (unused columns in DV)
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();

@@ -75,6 +75,29 @@ def test_attention_backward_split(Dqk, Dv, Hq, Hkv, B, Sq, Sk, causal, window, d
     assert _rel(got[3], want[3]) < 1e-5
 
 
+@pytest.mark.parametrize("Dqk,Dv", [(64, 64), (128, 128), (192, 128), (256, 256)])
+def test_attention_backward_split_holds_fp32_probabilities(Dqk, Dv):
+    """The fp32 partials of dV for each query head, before anything is rounded to bf16. One tile of queries: 12 products of the
+    tensor core into the accumulator, each cut off by at most 2^-24 of it, and an exponential good to 2^-22; P in two bf16 terms
+    (2^-17) would show as 2e-6."""
+    torch.manual_seed(Dqk)
+    S, Hq, Hkv = 64, 4, 2
+    q, k, v, do = (torch.randn(1, S, h, d, device="cuda").bfloat16() for h, d in ((Hq, Dqk), (Hkv, Dqk), (Hkv, Dv), (Hq, Dv)))
+    scale = Dqk ** -0.5
+    out, lse = N.forward(q, k, v, scale, True, 0, None, None)
+    dq, dk, dv = (torch.empty_like(t) for t in (q, k, v))
+    delta, lse2 = (torch.empty(Hq * S + 128, device="cuda") for _ in range(2))
+    part = torch.empty(S * Hq * Dqk, device="cuda")  # holds dV's partials last
+    rc = _native.lib().pt_attn_bwd_split(*(t.data_ptr() for t in (q, k, v, out, do, lse)), None,
+                                         *(t.data_ptr() for t in (dq, dk, dv, delta, lse2, part)), 1, S, S, Hq, Hkv, Dqk, Dv,
+                                         q.stride(1), k.stride(1), v.stride(1), out.stride(1), do.stride(1), scale, 1, 0, _native.stream_ptr())
+    _native.check(rc, "pt_attn_bwd_split")
+    _native.check_status()
+    qd, dod, kd = (t.double().permute(0, 2, 1, 3) for t in (q, do, k.repeat_interleave(Hq // Hkv, 2)))
+    p = torch.exp(qd @ kd.mT * scale - lse.double()[..., None]).tril()
+    assert _rel(part[:S * Hq * Dv].view(1, S, Hq, Dv), (p.mT @ dod).permute(0, 2, 1, 3)) < 2.0 ** -20
+
+
 def test_attention_backward_split_keeps_batch_entries_apart():
     """Rows past the end of a batch entry read as zero: an infinity in the next entry stays there."""
     q, k, v, do = (torch.randn(2, 70, 2, 256, device="cuda").bfloat16() for _ in range(4))
