@@ -21,7 +21,7 @@ from ..ops.embedding import Embedding
 from ..ops.linear import FusedWeights, Linear, fused_linear, linear
 from ..ops.moe import ExpertWeights, moe_experts, moe_experts_ref
 from ..ops.norm import RMSNorm, rmsnorm_ref
-from ..ops.router import router_replayed, router_topk, router_topk_ref
+from ..ops.router import router_replayed, router_replayed_ref, router_topk, router_topk_ref
 from ..parallel import ep as ep_mod
 from .interface import RoutingInfo
 
@@ -127,6 +127,10 @@ def packed_positions(S: int, cu_seqlens: torch.Tensor) -> torch.Tensor:
         out = torch.empty(S, dtype=torch.int64, device=cu.device)
         _native.check(_native.lib().pt_packed_positions(cu.data_ptr(), cu.numel(), out.data_ptr(), S, _native.stream_ptr()), "pt_packed_positions")
         return out
+    return packed_positions_ref(S, cu_seqlens)
+
+
+def packed_positions_ref(S: int, cu_seqlens: torch.Tensor) -> torch.Tensor:
     starts = cu_seqlens[:-1].long()
     lengths = (cu_seqlens[1:] - cu_seqlens[:-1]).long()
     return torch.arange(S, device=cu_seqlens.device) - torch.repeat_interleave(starts, lengths, output_size=S)
@@ -190,10 +194,11 @@ class Gate(nn.Module):
     def forward(self, tokens: torch.Tensor, reference: bool = False):
         """Returns ``(topk_idx[m,k] int32, topk_weight[m,k] fp32, lb_loss or None)``."""
         logits = self.logits(tokens)
-        fn = router_topk_ref if reference else router_topk
         if self.router_replay is not None and self.mode == "softmax_topk":
-            w, idx, scores = router_replayed(logits, self.num_experts_per_tok, self.router_replay, self.norm_topk_prob, self.scale)
+            fn = router_replayed_ref if reference else router_replayed
+            w, idx, scores = fn(logits, self.num_experts_per_tok, self.router_replay, self.norm_topk_prob, self.scale)
         else:
+            fn = router_topk_ref if reference else router_topk
             w, idx, scores = fn(logits, self.num_experts_per_tok, self.mode, self.norm_topk_prob, self.scale)
         lb_loss = None
         if self.load_balance_loss_fn is not None:
@@ -379,7 +384,11 @@ class PipelineChunk(nn.Module):
     def reference_forward(self, hidden_states: torch.Tensor, cu_seqlens: Optional[torch.Tensor] = None) -> torch.Tensor:
         if self.stage_index == 0:
             hidden_states = torch.nn.functional.embedding(hidden_states, self.embed_tokens.weight)
-        rotary = self.forward_posemb(hidden_states.shape[1], cu_seqlens)
+        S = hidden_states.shape[1]
+        if cu_seqlens is not None and self.supports_packed:  # as forward_posemb, without its kernel
+            rotary = RotaryPos(self.rotary_emb.cos, self.rotary_emb.sin, packed_positions_ref(S, cu_seqlens), S)
+        else:
+            rotary = self.forward_posemb(S, cu_seqlens)
         for layer in self.layers.values():
             hidden_states = layer.reference_forward(hidden_states, rotary, cu_seqlens)
         if self.stage_index == self.stage_count - 1:

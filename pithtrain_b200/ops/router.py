@@ -106,6 +106,18 @@ class _RouterGivenFn(torch.autograd.Function):
         return _RouterFn.backward(ctx, dw, None, dprobs)[0], None, None, None
 
 
+def _given_ref(logits, idx, renorm, scale):
+    scores = logits.float().softmax(-1)
+    w = scores.gather(-1, idx.long())
+    if renorm:
+        w = w / w.sum(-1, keepdim=True)
+    return w * scale, idx.int(), scores
+
+
+def router_replayed_ref(logits, k, replay, renorm=False, scale=1.0):
+    return _given_ref(logits, replay(torch.topk(logits.float().softmax(-1), k, dim=-1).indices), renorm, scale)
+
+
 def router_replayed(logits: torch.Tensor, k: int, replay, renorm: bool = False, scale: float = 1.0
                     ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """:func:`router_topk` (``softmax_topk``) with the picks exchanged by ``replay(top-k indices) -> indices``: the weights are the
@@ -122,13 +134,8 @@ def router_replayed(logits: torch.Tensor, k: int, replay, renorm: bool = False, 
         if idx.device == lg.device and idx.dim() == 2 and idx.shape[0] == n and 0 < idx.shape[1] <= 16:
             w, probs = _RouterGivenFn.apply(logits, idx, renorm, scale)
             return w, idx, probs
-    else:
-        idx = replay(torch.topk(logits.float().softmax(-1), k, dim=-1).indices)
-    scores = logits.float().softmax(-1)
-    w = scores.gather(-1, idx.long())
-    if renorm:
-        w = w / w.sum(-1, keepdim=True)
-    return w * scale, idx.int(), scores
+        return _given_ref(logits, idx, renorm, scale)
+    return router_replayed_ref(logits, k, replay, renorm, scale)
 
 
 class _RouterTopkSoftmax(torch.autograd.Function):

@@ -154,3 +154,55 @@ def test_family_staged_vs_reference(family):
         if d > (8e-2 if ".router." in n or ".gate." in n else 3e-2):
             bad.append((n, d))
     assert not bad, bad
+
+
+@pytest.mark.parametrize("family", ["qwen3_moe", "deepseek_v2"])
+def test_replayed_routing_and_packed_documents_vs_reference(family):
+    """The balanced replay and packed documents: the kernels' routing weights and positions against the tensor operations of
+    ``reference_forward``."""
+    from pithtrain_b200 import _native
+    from pithtrain_b200.contexts import distributed
+    from pithtrain_b200.dualpipe.execution import ChunkRecord, model_backward, model_forward
+    from pithtrain_b200.models import MODEL_CLASSES
+    from pithtrain_b200.modules.load_balance import force_balance
+
+    distributed.reset_single_process()
+    distributed.device = torch.device("cuda", 0)
+    torch.manual_seed(0)
+    qwen3 = dict(model_type="qwen3_moe", hidden_size=512, num_attention_heads=8, num_key_value_heads=2, head_dim=128, rms_norm_eps=1e-6,
+                 num_experts=16, num_experts_per_tok=4, moe_intermediate_size=256, norm_topk_prob=True, vocab_size=1024,
+                 num_hidden_layers=2, max_position_embeddings=256, rope_theta=1e6, attention_bias=False)
+    cfg = SimpleNamespace(**(qwen3 if family == "qwen3_moe" else FAMILY_CONFIGS[family]))
+    prev = torch.get_default_dtype()
+    torch.set_default_dtype(torch.bfloat16)
+    try:
+        with torch.device("cuda"):
+            m = MODEL_CLASSES[cfg.model_type](cfg, -1)
+    finally:
+        torch.set_default_dtype(prev)
+    with torch.no_grad():
+        for p in m.parameters():
+            if p.dim() >= 2:
+                p.normal_(0, 0.03)
+    for mod in m.modules():
+        if hasattr(mod, "router_replay"):
+            mod.router_replay = force_balance(mod.num_experts)
+    ids, labels = torch.randint(0, 1024, (1, 253), device="cuda"), torch.randint(0, 1024, (253,), device="cuda")
+    cu = torch.tensor([0, 1, 70, 70, 253], dtype=torch.int32, device="cuda")
+    rec = ChunkRecord(len(m.layers))
+    loss = torch.nn.functional.cross_entropy(model_forward(m, ids, rec, cu)[0].float(), labels, reduction="sum")
+    model_backward(m, rec, None, loss)
+    _native.check_status()
+    got = {n: p.grad.float().clone() for n, p in m.named_parameters() if p.grad is not None}
+    for p in m.parameters():
+        p.grad = None
+    for mod in m.modules():
+        for v in vars(mod).values():
+            if type(v).__name__ == "FusedWeights":
+                v.fused_grad = None
+    want = torch.nn.functional.cross_entropy(m.reference_forward(ids, cu)[0].float(), labels, reduction="sum")
+    want.backward()
+    assert abs(float(loss.detach()) - float(want.detach())) / float(want.detach()) < 5e-3
+    bad = {n: d for n, p in m.named_parameters() if p.grad is not None
+           for d in [calc_diff(got[n], p.grad.float())] if d > (8e-2 if ".gate." in n else 3e-2)}
+    assert not bad, bad

@@ -245,6 +245,33 @@ def test_moe_experts_cpu_vs_loop():
             assert torch.allclose(a, b, atol=1e-4, rtol=1e-4)
 
 
+def test_oracle_of_replayed_routing_and_packed_positions_is_tensor_operations(monkeypatch):
+    """``reference_forward`` must not run the kernels that it checks: neither for a router replay nor for packed documents."""
+    from types import SimpleNamespace
+
+    from pithtrain_b200.contexts import distributed
+    from pithtrain_b200.models import MODEL_CLASSES, common
+
+    distributed.reset_single_process()
+    distributed.device = torch.device("cpu")
+    torch.manual_seed(0)
+    cfg = SimpleNamespace(model_type="qwen3_moe", hidden_size=32, num_attention_heads=2, num_key_value_heads=1, head_dim=16, rms_norm_eps=1e-6,
+                          num_experts=4, num_experts_per_tok=2, moe_intermediate_size=16, norm_topk_prob=True, vocab_size=64,
+                          num_hidden_layers=1, max_position_embeddings=32, rope_theta=1e4, attention_bias=False)
+    m = MODEL_CLASSES["qwen3_moe"](cfg, -1)
+    m.rotary_emb.float()
+    seen = []
+    for mod in m.modules():
+        if hasattr(mod, "router_replay"):
+            mod.router_replay = lambda idx: (seen.append(idx), (idx + 1) % 4)[1]
+    ids, cu = torch.randint(0, 64, (1, 32)), torch.tensor([0, 5, 32], dtype=torch.int32)
+    want = m.reference_forward(ids, cu)
+    for name in ("router_replayed", "packed_positions"):
+        monkeypatch.setattr(common, name, lambda *a, **k: pytest.fail("a kernel's dispatch in the oracle"))
+    monkeypatch.setattr(common._native, "lib", lambda: pytest.fail("a kernel in the oracle"))
+    assert torch.equal(m.reference_forward(ids, cu), want) and len(seen) == 2
+
+
 @pytest.mark.parametrize("dtype", [torch.uint8, torch.int8, torch.int16, torch.int32, torch.int64, torch.float32])
 @pytest.mark.parametrize("n,E,k", [(300, 100, 4), (1, 1, 1), (257, 6, 3), (40, 4, 8)])
 def test_balanced_replay_in_every_type(n, E, k, dtype):
