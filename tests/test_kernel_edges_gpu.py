@@ -49,6 +49,7 @@ def _rel(a, b):
     (1, 127, 127, True, None, None), (2, 130, 130, True, None, None), (1, 257, 257, False, None, None),
     (1, 64, 320, True, None, None), (2, 96, 200, False, None, None), (1, 515, 515, True, 100, None),
     (1, 517, 517, True, None, [0, 1, 130, 131, 400, 517]), (1, 640, 640, True, 64, [0, 128, 129, 512, 640]),
+    (2, 325, 325, True, 70, None), (3, 200, 200, True, None, [0, 1, 64, 130, 200]), (2, 66, 200, True, 40, None),
 ])
 def test_attention_backward_split(Dqk, Dv, Hq, Hkv, B, Sq, Sk, causal, window, docs):
     """dq, dk, dv are the 64-bit gradients rounded to bf16: P and dS lose nothing on the way (rounding them too would show as
@@ -340,7 +341,12 @@ def test_router_replayed(n, E, k, renorm, dtype):
     want = p.gather(1, picks)
     want = (want / want.sum(-1, keepdim=True) if renorm else want) * 2.5
     torch.autograd.backward((want, p), (dw.double(), dp.double()))
-    assert seen[0].dtype == torch.int64 and torch.equal(seen[0], p.topk(k).indices) or dtype == torch.bfloat16  # bf16 logits tie
+    assert seen[0].dtype == torch.int64
+    if dtype == torch.float32:
+        assert torch.equal(seen[0], p.topk(k).indices)
+    else:  # bf16 logits tie: other picks of the same scores, no pick twice
+        assert torch.equal(ld.detach().gather(1, seen[0]), ld.detach().topk(k).values)
+        assert all(r.unique().numel() == k for r in seen[0])
     assert torch.equal(idx.long(), picks)
     assert _rel(w.detach(), want.detach()) < 1e-6 and _rel(probs.detach(), p.detach()) < 1e-6
     # a logit's gradient is p times a difference that may cancel: fp32 error of its terms, then the rounding of the result
@@ -381,6 +387,31 @@ def test_router_picks_of_a_nan_row_are_experts(E, k):
     assert torch.equal(idx, idx0) and torch.equal(w.isnan(), w0.isnan())
     assert ((idx >= 0) & (idx < E)).all() and all(r.unique().numel() == k for r in idx)
     assert torch.equal(w.isnan().all(-1), torch.tensor([False, True, False, True, False], device="cuda"))
+
+
+@pytest.mark.parametrize("renorm", [False, True])
+@pytest.mark.parametrize("E", [16, 40, 512])
+def test_router_replayed_picks_out_of_range(E, renorm):
+    """A pick outside [0, E) has the weight NaN (renormalised, so has its row) and is read nowhere; other rows are untouched."""
+    from pithtrain_b200.ops.router import router_replayed
+
+    torch.manual_seed(E)
+    logits = torch.randn(4, E, device="cuda")
+    picks = torch.tensor([[0, 1, 2], [3, -1, 4], [E, 5, 6], [7, 8, E - 1]], device="cuda")
+    lg, ld = logits.clone().requires_grad_(), logits.double().requires_grad_()
+    w, idx, probs = router_replayed(lg, 3, lambda i: picks, renorm)
+    out = torch.zeros_like(w, dtype=torch.bool)
+    out[1, 1] = out[2, 0] = True
+    assert torch.equal(idx.long(), picks) and torch.equal(w.isnan(), out.any(-1, keepdim=True).expand_as(out) if renorm else out)
+    w[[0, 3]].sum(1).dot(torch.tensor([1.0, 2.0], device="cuda")).backward()
+    p = ld.softmax(-1)
+    wd = p.gather(1, picks.clamp(0, E - 1))
+    wd = wd / wd.sum(-1, keepdim=True) if renorm else wd
+    wd[[0, 3]].sum(1).dot(torch.tensor([1.0, 2.0], dtype=torch.float64, device="cuda")).backward()
+    assert _rel(probs.detach(), p.detach()) < 1e-6 and _rel(w[[0, 3]].detach(), wd[[0, 3]].detach()) < 1e-6
+    assert (lg.grad.double() - ld.grad)[[0, 3]].abs().max() <= 1e-6 * 2 * 3
+    if not renorm:  # the weights that were not used carry no gradient
+        assert not lg.grad[[1, 2]].any()
 
 
 def test_router_replayed_refuses_picks_on_another_device():
