@@ -687,6 +687,9 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMa
 // a_idx (optional, K-major A only): row r of the GEMM's A is source row a_idx[r] / a_idx_div of the
 // tensor described by a_rows/a_cols/lda (negative index or r >= a_idx_len: a zero row), fetched with
 // TMA gather4 straight into the swizzled operand tile.
+// Accumulation into one D is ordered by the caller: two launches that accumulate into the same elements must be on one stream
+// or ordered by events. Only bf16 reduce-adds would not lose updates to each other; fp32 in the K-grouped mode and every
+// epilogue without TMA read D, add to it and store it.
 // Returns 0 on success.
 PT_API int pt_gemm_bf16(const void* A, const void* B, void* D, int mode, int M, int N, int K,
                         int a_mn, int b_mn, long long a_rows, long long a_cols, long long lda,
@@ -772,7 +775,8 @@ PT_API int pt_gemm_bf16(const void* A, const void* B, void* D, int mode, int M, 
 
 // Expert weight gradients of two micro-batches in one launch: for every group g,
 //   D_g += A1[offs1[g]:offs1[g+1]]^T B1[...] + A2[offs2[g]:offs2[g+1]]^T B2[...]
-// (A* [R*, M], B* [R*, N] bf16 row-major, read MN-major; D [G, M, N] bf16 or fp32, accumulated with TMA reduce-add).
+// (A* [R*, M], B* [R*, N] bf16 row-major, read MN-major; D [G, M, N] bf16, accumulated with TMA reduce-add, or fp32, read,
+// added to and stored: see pt_gemm_bf16 on launches that overlap).
 // One pass over the gradient buffer instead of two: the launch is bound by that read-modify-write, not by its FLOPs.
 // Group sizes must be multiples of 16 in both operand pairs.
 PT_API int pt_gemm_bf16_kgroup2(const void* A1, const void* B1, const int* offs1, long long rows1, const void* A2,

@@ -215,7 +215,8 @@ def grouped_gemm_tn(dy: torch.Tensor, x: torch.Tensor, offs: torch.Tensor, out: 
                     accumulate: bool = True) -> torch.Tensor:
     """``out[g] (+)= dy[rows_g].T @ x[rows_g]`` with ``out[G,N,K]`` (expert wgrad).
 
-    Group sizes must be multiples of 16; pad rows must be zero in ``dy`` (or ``x``).
+    Group sizes must be multiples of 16; pad rows must be zero in ``dy`` (or ``x``). Like any ``+=`` on a tensor, calls that
+    accumulate into one ``out`` have to be ordered: on one stream, or by events. An fp32 ``out`` is read, added to and stored.
     """
     G, N, K = out.shape
     if not _native_ok(dy, x):
@@ -238,7 +239,8 @@ def grouped_gemm_tn_pair(dy1: torch.Tensor, x1: torch.Tensor, offs1: torch.Tenso
                          offs2: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """``out[g] += dy1[rows1_g].T @ x1[rows1_g] + dy2[rows2_g].T @ x2[rows2_g]``: the expert weight gradients of two
     micro-batches in one launch. The launch is bound by the read-modify-write of ``out`` (the whole ``[G, N, K]``
-    gradient buffer), not by its FLOPs, so one pass for two micro-batches nearly halves its cost."""
+    gradient buffer), not by its FLOPs, so one pass for two micro-batches nearly halves its cost. Calls that accumulate into
+    one ``out`` have to be ordered, as for :func:`grouped_gemm_tn`."""
     G, N, K = out.shape
     if not (_native_ok(dy1, x1) and _native_ok(dy2, x2)) or N % 8 != 0 or K % 8 != 0:
         grouped_gemm_tn(dy1, x1, offs1, out, accumulate=True)

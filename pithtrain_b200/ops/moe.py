@@ -308,7 +308,8 @@ class ExpertWeights:
     """What :func:`moe_experts` needs from the owning module.
 
     ``w1`` is the fused gate/up projection ``[E, 2I, H]`` (gate rows first, or interleaved), ``w2`` the
-    down projection ``[E, H, I]``; ``g1``/``g2`` return the gradient buffers to accumulate into.
+    down projection ``[E, H, I]``; ``g1``/``g2`` return the gradient buffers to accumulate into, which backward passes on
+    several streams must not do at the same time (the engine keeps all weight gradients on its compute stream).
     ``b1``/``b2`` are optional per-expert biases (``[E, 2I]``, ``[E, H]``) as parameters.
     """
 
