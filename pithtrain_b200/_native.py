@@ -178,14 +178,15 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 # Number of kernel launches issued through this module since it was last reset (bench bookkeeping).
 LAUNCHES = 0
-_LAUNCHES_PER_CALL = {"pt_route_sort": 4, "pt_attn_bwd": 3, "pt_attn_bwd_split": 6, "pt_gdr_fwd": 3, "pt_gdr_bwd": 3, "pt_merge_partial": 2}
+_LAUNCHES_PER_CALL = {"pt_route_sort": 4, "pt_attn_bwd": 3, "pt_gdr_fwd": 3, "pt_gdr_bwd": 3, "pt_merge_partial": 2}
 
 
-def check(rc: int, what: str) -> None:
+def check(rc: int, what: str, launches: int | None = None) -> None:
+    """Raise if ``rc`` is an error; ``launches``: the kernels that this call issued, where that depends on its arguments."""
     global LAUNCHES
     if rc != 0:
         raise RuntimeError(f"{what} failed with code {rc}")
-    LAUNCHES += _LAUNCHES_PER_CALL.get(what, 1)
+    LAUNCHES += _LAUNCHES_PER_CALL.get(what, 1) if launches is None else launches
 
 
 def set_peer_wait_limit(seconds: float) -> None:

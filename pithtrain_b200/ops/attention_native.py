@@ -164,7 +164,7 @@ def backward_split(do, q, k, v, out, lse, scale: float, causal: bool, q_off: int
                                          lse2.data_ptr(), _native.ptr(part), B, Sq, Sk, Hq, Hkv, D, Dv, q.stride(1), k.stride(1),
                                          v.stride(1), out.stride(1), do.stride(1), float(scale), int(bool(causal)), int(q_off),
                                          _native.stream_ptr())
-    _native.check(rc, "pt_attn_bwd_split")
+    _native.check(rc, "pt_attn_bwd_split", launches=4 if part is None else 6)  # a group sum each for dK and dV
     return dq, dk, dv, delta[:ns].view(B, Hq, Sp)[..., :Sq]
 
 

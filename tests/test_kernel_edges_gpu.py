@@ -798,3 +798,14 @@ def test_mla_positions_outside_the_rotary_tables(positions):
     for t, part in ((out[0], slice(16, None)), (out[1], slice(16, None)), (grads[0].view(n, 2, 32), slice(16, None)), (grads[1][:, None], slice(None))):
         assert [bool(x) for x in t[..., part].isnan().all(-1).all(-1)] == [i == bad for i in range(n)]
     assert torch.isfinite(out[2]).all() and torch.isfinite(grads[2]).all()
+
+
+@pytest.mark.parametrize("Hkv,launches", [(4, 4), (2, 6)])
+def test_launch_count_of_the_split_backward(Hkv, launches):
+    """The row sums, dQ, dK and dV, and the sums of dK and dV over a group of heads where there are groups."""
+    q, do = (torch.randn(1, 5, 4, 64, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(1, 5, Hkv, 64, device="cuda").bfloat16() for _ in range(2))
+    out, lse = N.forward(q, k, v, 0.125, True, 0, None, None)
+    before = _native.LAUNCHES
+    N.backward_split(do, q, k, v, out, lse, 0.125, True, 0, None)
+    assert _native.LAUNCHES - before == launches
