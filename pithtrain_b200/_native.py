@@ -87,7 +87,6 @@ SIGS = {
     "pt_sumsq_grid": "",
     "pt_sumsq": "PILPP",
     "pt_adamw": "PIPIPPLPFFFFFFFP",
-    "pt_muon_momentum": "PIPIPLFPP",
     "pt_muon_slabs": "LL",
     "pt_muon_momentum_sumsq": "PIPIPLLFPPP",
     "pt_frobenius_scales": "PIIPPP",

@@ -215,11 +215,6 @@ PT_API int pt_muon_momentum_sumsq(const void* g, int g_fp32, void* buf, int buf_
   return (int)cudaGetLastError();
 }
 
-PT_API int pt_muon_momentum(const void* g, int g_fp32, void* buf, int buf_fp32, void* upd, long long numel,
-                            float beta, const float* grad_scale, void* stream_) {
-  return pt_muon_momentum_sumsq(g, g_fp32, buf, buf_fp32, upd, 1, numel, beta, grad_scale, nullptr, stream_);
-}
-
 // s1, s2: bf16 [E] from the partial sums of pt_muon_momentum_sumsq.
 PT_API int pt_frobenius_scales(const float* partial, int E, int slabs, void* s1, void* s2, void* stream_) {
   if (E <= 0) return 0;
