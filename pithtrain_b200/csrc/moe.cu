@@ -308,7 +308,7 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict_
 // combine: out[t] = (res ? res[t] : 0) + sum_{j<k, row>=0} (w ? w[t,j] : 1) * y[row_of_slot[t*k+j]]
 // One warp per token; fp32 accumulation; k rows gathered per token.
 // ----------------------------------------------------------------------------------------------
-// One warp per token, one row at a time: the better one where there are tokens for every warp of the chip (see pt_combine).
+// One warp per token, one row at a time: the better one where there are tokens for the warps of the chip (see pt_combine).
 __global__ void __launch_bounds__(256)
 combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_slot,
                const float* __restrict__ w, const __nv_bfloat16* __restrict__ res,
@@ -339,7 +339,7 @@ combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_
   }
 }
 
-// Fewer tokens than that are a latency problem: k random 4 KB rows each. One thread per 8 columns of a token, so that at 64
+// Fewer tokens than that are a latency problem: k random rows each. One thread per 8 columns of a token, so that at 64
 // tokens of 2048 columns 512 warps ask for rows instead of 64, and the k row loads of a thread are independent: indices and
 // weights first, then four rows in flight at a time, added in slot order (the same sums as above).
 __global__ void __launch_bounds__(256)
@@ -894,10 +894,16 @@ PT_API int pt_combine(const void* y, const int* row_of_slot, const float* w, con
   cudaStream_t st = (cudaStream_t)stream_;
   if (n_max <= 0) return 0;
   if (H % 8 != 0) return -1;
-  // Measured, cold cache, 8 rows a token, 2048 columns, wide / warp per token: 64 tokens 12 / 44 us, 512 17 / 46, 2048 (6 rows)
-  // 31 / 41, 3001 41 / 45, 4096 68 / 57, 8192 117 / 100: beyond the L2's size more rows in flight only queue up in memory.
+  // A warp walks its token's k rows one after the other, so up to some 3000 tokens (20 warps an SM) its kernel takes the time of
+  // one such chain whatever the size; from there on it keeps memory busy with fewer requests in flight than the wide one. The line
+  // is the same at every width and k. Measured, cold cache, wide / warp per token, us:
+  //   columns x k       64 tokens   1024      2048      3072      4096      8192
+  //   2048 x 8          12 / 45     25 / 48   39 / 53   53 / 55   68 / 57   121 / 100
+  //   2048 x 4           9 / 27     16 / 29   25 / 31   33 / 33   43 / 35    76 / 60
+  //   2880 x 4          10 / 37     21 / 39   33 / 41   45 / 45   59 / 49   102 / 84
+  //    512 x 8          11 / 16     12 / 18   18 / 18   18 / 18   25 / 21    39 / 33
   const long long vecs = (long long)n_max * (H / 8);
-  if (vecs <= 3072ll * 256)
+  if (n_max <= 3072)
     combine_wide_kernel<<<grid_for(vecs, 256, 64), 256, 0, st>>>((const __nv_bfloat16*)y, row_of_slot, w,
         (const __nv_bfloat16*)res, (__nv_bfloat16*)out, n_ptr, n_max, k, H);
   else

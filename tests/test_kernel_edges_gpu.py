@@ -422,7 +422,7 @@ def test_router_replayed_refuses_picks_on_another_device():
 
 
 @pytest.mark.parametrize("k", [1, 3, 4, 6, 8])
-@pytest.mark.parametrize("n,H", [(1, 8), (3, 264), (64, 2048), (5000, 512)])
+@pytest.mark.parametrize("n,H", [(1, 8), (3, 264), (64, 2048), (3072, 264), (3073, 264), (5000, 512)])
 def test_combine_rows(n, H, k):
     from pithtrain_b200.ops.moe import combine_rows
 
