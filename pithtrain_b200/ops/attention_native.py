@@ -92,9 +92,10 @@ def _as_token_major(t: torch.Tensor) -> torch.Tensor:
 
 def _aligned_gradient(do: torch.Tensor) -> torch.Tensor:
     """``do`` as the pass over its rows reads it, in 16-byte pieces. Unlike q, k and v it comes to no tensor map of the forward
-    that would have refused a misaligned base, and ``contiguous()`` hands a contiguous piece of a larger gradient back as it is."""
+    that would have refused a misaligned base or pitch, and ``contiguous()`` hands a contiguous piece of a larger gradient back
+    as it is (one of a single row with whatever pitch it has)."""
     do = _as_token_major(do)
-    return do if do.data_ptr() % 16 == 0 else do.clone()
+    return do if _token_major(do) else do.clone(memory_format=torch.contiguous_format)
 
 
 def forward(q, k, v, scale: float, causal: bool, q_off: int, row_lo: Optional[torch.Tensor],

@@ -46,7 +46,7 @@ def test_mla_inputs_are_readable_in_16_byte_pieces(n):
         assert mla._rows(block).data_ptr() % 16 == 0
 
 
-@pytest.mark.parametrize("shape", [(1, 1, 2, 128), (2, 5, 3, 64), (1, 63, 1, 256)])
+@pytest.mark.parametrize("shape", [(1, 1, 2, 128), (1, 1, 1, 64), (2, 5, 3, 64), (1, 63, 1, 256)])
 def test_output_gradients_of_attention_are_readable_in_16_byte_pieces(shape):
     from pithtrain_b200.ops import attention_native as N
 
