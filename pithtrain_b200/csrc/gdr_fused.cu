@@ -1,4 +1,4 @@
-// Gated delta rule (Gated DeltaNet) for bf16 q, k, v with head dims 128: the whole chunked evaluation in five kernels, forward
+// Gated delta rule (Gated DeltaNet) for bf16 q, k, v with head dims 128: the whole chunked evaluation in six kernels, forward
 // and backward, chunk C = 64. (csrc/gdr.cu holds only the pass over the chunks, for the other dtypes and head dims.)
 //
 //   per chunk, b = cumulative log gate, D_ij = exp(b_i - b_j) for j <= i, qs = q / sqrt(dk):
@@ -16,16 +16,17 @@
 //
 // All arithmetic is fp32 FMA on fp32 values (q, k, v and do are bf16 and enter exactly), as in the tensor-op form: splitting
 // operands over tensor-core products was not taken because the state recurrence carries every rounding to the end of the
-// sequence. What bounds it is the FMA pipe: 5.2 M FMA per chunk and head forward, 12 M backward. Two things follow. Only the
-// products that need the running state stay in the sequential kernels (w S and k^T v' forward); and every product reads its
-// operands from shared memory in 16-byte pieces, 8 to 11 FMA per piece, tiles padded to 132 or 68 columns so that the eight
-// threads of a phase hit different banks. The sequential kernels prefetch the next chunk with cp.async.
+// sequence. 5.8 M FMA per chunk and head forward, 12 M backward; two to an instruction they keep the FMA pipe 38 to 55 % busy.
+// What bounds the kernels is the shared memory that the operands come from (63 to 82 % of its pipe) and the wait for it. Two
+// things follow. Only the products that need the running state stay in the sequential kernels (w S and k^T v' forward); and every
+// product reads its operands from shared memory in 16-byte pieces, 8 to 11 FMA per piece, tiles padded to 132 or 68 columns so
+// that the eight threads of a phase hit different banks. The sequential kernels prefetch the next chunk with cp.async.
 //
 // A product phase of a chunk kernel has eight warps and nothing beside it, so what it needs is fetched before it: tiles by
 // cp.async under the phase in front, rows of q, k and v into registers.
-// Measured, 1 x 3072, 32 heads (48 chunks): chunk_fwd 202, scan_fwd 280, out 129, dvp 50, scan_bwd 383, chunk_bwd 802 us; with
-// plain loads between the phases out took 242 and chunk_bwd 1122. The tensor-op form with the recurrence kernels of csrc/gdr.cu
-// took about 8 ms for the two directions. Counters of chunk_bwd before: issue slots 28 %, waits for global memory 2.7 per issue.
+// Measured, 1 x 3072, 32 heads (48 chunks): chunk_fwd 211, scan_fwd 291, out 136, dvp 49, scan_bwd 397, chunk_bwd 816 us; with
+// plain loads between the phases out took 242 and chunk_bwd 1122 (issue slots 28 %, waits for global memory 2.7 per issue; now
+// 42 % and 0.3). The tensor-op form with the recurrence kernels of csrc/gdr.cu took about 8 ms for the two directions.
 // The sums of a row or column are made in a fixed order: results are reproducible.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
