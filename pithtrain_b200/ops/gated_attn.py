@@ -68,6 +68,8 @@ def gated_attn_pre(qkv, q_w, k_w, cos, sin, Hq: int, Hkv: int, D: int, eps: floa
     ``q [n,Hq,D], k [n,Hkv,D], v [n,Hkv,D]`` and the gate ``[n,Hq,D]``, a view of the packed rows."""
     if not cos.device == sin.device == qkv.device:
         raise RuntimeError(f"qkv on {qkv.device}, rotary tables on {cos.device} and {sin.device}")
+    if not (cos.shape == sin.shape and cos.shape[0] == qkv.shape[0] and cos.dtype == sin.dtype == qkv.dtype):
+        raise RuntimeError(f"rotary rows {tuple(cos.shape)}, {tuple(sin.shape)} of {cos.dtype}, {sin.dtype} for qkv {tuple(qkv.shape)} of {qkv.dtype}")
     return _Pre.apply(qkv, q_w, k_w, cos, sin, Hq, Hkv, D, eps)
 
 
@@ -96,4 +98,6 @@ class _Post(torch.autograd.Function):
 
 def gated_attn_post(o, gate):
     """``o [n,H,D] * sigmoid(gate)``; ``gate`` is the view that :func:`gated_attn_pre` returned."""
+    if gate.shape != o.shape:
+        raise RuntimeError(f"gate {tuple(gate.shape)} for an output {tuple(o.shape)}")
     return _Post.apply(o, gate)

@@ -20,7 +20,7 @@ def _dense(t: torch.Tensor) -> torch.Tensor:
 def conv_supported(x: torch.Tensor, weight: torch.Tensor, nk: int, nv: int, dk: int, dv: int) -> bool:
     """Heads of 128 channels, four taps, bf16: what a warp of the kernels holds in registers."""
     return (use_native(x) and weight.device == x.device and weight.dtype == torch.bfloat16 and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and dk == 128
-            and dv == 128 and nv % nk == 0 and weight.shape == ((2 * nk + nv) * 128, 1, 4) and x.dim() == 3
+            and dv == 128 and nv % nk == 0 and weight.shape == ((2 * nk + nv) * 128, 1, 4) and x.dim() == 3 and x.shape[2] == weight.shape[0]
             and 0 < x.shape[0] <= 65535 and 0 < x.shape[1] <= 65535 * 32)
 
 

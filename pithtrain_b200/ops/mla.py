@@ -87,5 +87,12 @@ def mla_assemble(q, k_pe, kv, cos, sin, positions: Optional[torch.Tensor], S: in
     for t in (k_pe, kv, cos, sin, *(() if positions is None else (positions,))):
         if t.device != q.device:
             raise RuntimeError(f"q on {q.device}, another input on {t.device}")
+    n = q.shape[0]
+    if not (q.shape == (n, H * (dn + dr)) and k_pe.shape == (n, dr) and kv.shape == (n, H * (dn + dv)) and cos.shape == sin.shape
+            and cos.shape[1] == dr and (positions is None or positions.shape == (n,))):
+        raise RuntimeError(f"MLA inputs of {H} heads {dn} + {dr} / {dv}: q {tuple(q.shape)}, rotary key {tuple(k_pe.shape)}, kv {tuple(kv.shape)}, "
+                           f"tables {tuple(cos.shape)}, {tuple(sin.shape)}, positions {None if positions is None else tuple(positions.shape)}")
+    if not q.dtype == k_pe.dtype == kv.dtype == cos.dtype == sin.dtype:
+        raise RuntimeError(f"MLA inputs of types {q.dtype}, {k_pe.dtype}, {kv.dtype}, {cos.dtype}, {sin.dtype}")
     pos = None if positions is None else positions.int().contiguous()
     return _Assemble.apply(q, k_pe, kv, cos, _dense(sin), pos, S, H, dn, dr, dv)

@@ -809,3 +809,26 @@ def test_launch_count_of_the_split_backward(Hkv, launches):
     before = _native.LAUNCHES
     N.backward_split(do, q, k, v, out, lse, 0.125, True, 0, None)
     assert _native.LAUNCHES - before == launches
+
+
+def test_layer_passes_refuse_other_shapes():
+    """What a reshape or a broadcast of the tensor operations refused: rows or widths that the kernels would read past."""
+    from pithtrain_b200.ops import gated_attn as GA, gdn_mix, mla
+
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    taps, w, qkv, c = mk(3 * 128, 1, 4), mk(128), mk(4, 512), mk(4, 32)
+    assert gdn_mix.conv_supported(mk(1, 5, 384), taps, 1, 1, 128, 128) and not gdn_mix.conv_supported(mk(1, 5, 256), taps, 1, 1, 128, 128)
+    for bad in ((c[:3], c[:3]), (c, c[:, :16]), (c.float(), c.float())):
+        with pytest.raises(RuntimeError):
+            GA.gated_attn_pre(qkv, w, w, *bad, 1, 1, 128, 1e-6)
+    o = mk(4, 1, 128)
+    with pytest.raises(RuntimeError):
+        GA.gated_attn_post(o, GA.gated_attn_pre(qkv, w, w, c, c, 1, 1, 128, 1e-6)[3][:3])
+    args = [mk(4, 192), mk(4, 64), mk(4, 256), mk(4, 64), mk(4, 64), torch.arange(4, device="cuda")]
+    mla.mla_assemble(*args, 4, 1, 128, 64, 128)
+    for i in range(6):
+        for bad in (args[i][:3], args[i][..., :-1], args[i].double()) if i < 5 else (args[i][:3],):
+            if i in (3, 4) and bad.shape == (3, 64):
+                continue  # shorter tables: checked position by position
+            with pytest.raises(RuntimeError):
+                mla.mla_assemble(*(bad if i == j else t for j, t in enumerate(args)), 4, 1, 128, 64, 128)
