@@ -89,9 +89,8 @@ SIGS = {
     "pt_adamw": "PIPIPPLPFFFFFFFP",
     "pt_muon_slabs": "LL",
     "pt_muon_momentum_sumsq": "PIPIPLLFPPP",
-    "pt_frobenius_scales": "PIIPPP",
-    "pt_gram_scale_copy": "PPPIIP",
-    "pt_gram_shift_scale": "PPIIFP",
+    "pt_frobenius_scales": "PIIPP",
+    "pt_muon_orthogonalize": "PPPPPPIIIIPPIFFP",
     "pt_symm_malloc": "PL",
     "pt_symm_free": "P",
     "pt_ipc_export": "PP",

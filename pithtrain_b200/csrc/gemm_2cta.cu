@@ -1,9 +1,7 @@
-// Dense bf16 NT GEMM with 2-CTA tcgen05 tiles (cta_group::2).
+// bf16 GEMMs with 2-CTA tcgen05 tiles (cta_group::2): dense products and stacks of equal products.
 //
-// Default path of ops/gemm.py: gemm_nt for fresh bf16 outputs (q/k/v/o projections, lm_head, dense MLPs); the
-// single-CTA family in gemm.cu serves the accumulating, fp32-output, NN / TN and grouped forms.
-//
-//   D[M,N] = A[M,K] * B[N,K]^T, bf16 in, fp32 accumulate in TMEM, bf16 out through TMA stores.
+//   D_e[M,N] = A_e * B_e, bf16 in, fp32 accumulate in TMEM. Either operand is K-major (reduction contiguous) or MN-major, so
+//   the forward (NT), input-gradient (NN) and weight-gradient (TN) forms read the tensors as they sit in memory.
 //   A pair of CTAs (cluster 2x1x1) owns a 256 x 256 output tile: CTA r loads rows [m0 + 128 r, +128) of A and rows
 //   [n0 + 128 r, +128) of B (its half of N) with ordinary, non-multicast TMA loads issued in the .cta_group::2 form,
 //   whose completion lands on the leader's (CTA 0) mbarrier. The leader's MMA thread issues
@@ -11,14 +9,21 @@
 //   memory, so each B byte is loaded from L2 once per pair and each shared-memory byte feeds twice the FLOPs of the
 //   single-CTA kernel. Each CTA keeps its 128 accumulator rows in its own TMEM and runs its own epilogue.
 //
-//   per CTA: warp 0 producer, warp 1 MMA (leader only issues; both allocate TMEM), warps 2..5 epilogue.
+//   per CTA: warp 0 producer, warp 1 MMA (leader only issues; both allocate TMEM), warps 2..5 or 2..9 epilogue.
 //   Barriers live at the same shared-memory offset in both CTAs:
 //     full[s]       used in CTA 0: leader producer arrives with expect_tx(both CTAs' bytes)
-//     empty[s]      in each CTA: leader MMA commits once to its own copy and once to the peer's (mapa address)
+//     empty[s]      in each CTA: one commit of the leader's MMA thread arrives on both copies
 //     tmem_full[b]  in each CTA: same
-//     tmem_empty[b] used in CTA 0: the 8 epilogue warps of the pair arrive there (remote arrive from CTA 1)
+//     tmem_empty[b] used in CTA 0: the epilogue warps of the pair arrive there (remote arrive from CTA 1)
 //
-// PTX forms follow the vendored CUTLASS headers (cute/arch/copy_sm100_tma.hpp: SM100_TMA_2SM_LOAD_2D,
+// Epilogues:
+//   T2_STORE   bf16 through TMA stores: the q/k/v/o projections, lm_head and dense MLPs (ops/gemm.py)
+//   T2_FUSED   bf16 of s_e * (alpha * acc + beta * C + diag * I): the products of the Newton-Schulz iteration with the addend,
+//              the diagonal, the normalisation and the weight update in them. With `sym` (D symmetric) only the tiles on and
+//              above the diagonal are computed, and each is stored a second time, transposed.
+//   T2_REDUCE  D += acc in bf16 or fp32 by TMA reduce-add (dense weight gradients)
+//
+// PTX forms follow the vendored CUTLASS headers (cute/arch/copy_sm100_tma.hpp: SM100_TMA_2SM_LOAD_3D,
 // cute/arch/mma_sm100_umma.hpp: SM100_MMA_F16BF16_2x1SM_SS, cute/arch/tmem_allocator_sm100.hpp: Allocator2Sm,
 // cutlass/arch/barrier.h: umma_arrive_2x1SM, umma_arrive_2x1SM_sm0).
 #include "host_common.h"
@@ -33,11 +38,20 @@ constexpr int T2_STAGES = 5;
 constexpr int T2_A_BYTES = T2_BM * T2_BK * 2;        // 16 KB
 constexpr int T2_B_BYTES = (T2_BN / 2) * T2_BK * 2;  // 16 KB (this CTA's half)
 constexpr int T2_STAGE_BYTES = T2_A_BYTES + T2_B_BYTES;
-constexpr int T2_STAGING = 4 * 2 * 4096;
 constexpr uint32_t T2_PEER_MASK = 0xFEFFFFFFu;  // clears the pair-rank bit of a shared::cluster address -> CTA 0
+
+enum Gemm2Epi : int { T2_STORE = 0, T2_FUSED = 1, T2_REDUCE = 2 };
 
 struct Gemm2Args {
   int M, N, K;
+  int batch;     // stacked products (dense: 1)
+  int sym;       // T2_FUSED: D is symmetric (M == N)
+  int out_fp32;  // T2_REDUCE
+  float alpha, beta, diag;
+  const float* scale;  // T2_FUSED: one factor per product (null: 1), applied scale_pow times
+  int scale_pow;
+  const __nv_bfloat16* C;  // T2_FUSED addend, laid out as D (null: none)
+  long long ldc, c_stride;
   int* err;
 };
 
@@ -61,11 +75,11 @@ __device__ __forceinline__ void tmem_dealloc_2cta(uint32_t taddr, uint32_t ncols
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 // TMA load of this CTA's box; completion bytes go to the mbarrier at the same offset in CTA 0.
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y) {
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(smem_dst)),
-      "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar) & T2_PEER_MASK), "r"(x), "r"(y)
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar) & T2_PEER_MASK), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
 __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -77,28 +91,52 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, u
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
-// Arrive (once the MMAs issued so far have completed) on the barrier at this offset in both CTAs of the pair: one commit
-// per CTA, the peer's copy addressed through mapa (both commits track the same preceding MMAs).
+// Arrive (once the MMAs issued so far have completed) on the barrier at this offset in both CTAs of the pair. One commit for
+// both: with one a CTA the tensor pipe lost 20 of 330 ns a k-block (8192^3 1415 -> 1470 TFLOP/s, 8192 x 5120 x 2048 1387 ->
+// 1435); one commit for two or three k-blocks gained nothing more and delays the loads.
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  const uint32_t own = smem_u32(bar);
-  uint32_t peer;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(own), "r"(1u));
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(own) : "memory");
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(peer) : "memory");
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"(static_cast<uint16_t>(3))
+               : "memory");
 }
 // Plain arrive on CTA 0's copy of a barrier (from either CTA).
 __device__ __forceinline__ void mbar_arrive_leader(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(smem_u32(bar) & T2_PEER_MASK) : "memory");
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+// Epilogue warps of a CTA: four, one for each 32-row quarter of the accumulator, or eight, the two of a quarter taking its
+// 64-column chunks in turn. Eight pay where a short reduction meets an addend (A^2 of 128 x [768, 768]: 102 -> 84 us); elsewhere
+// the products of a tile hide four, and eight cost 4 to 5 % (polling beside a power-capped tensor core: A of 128 x [768, 2048] 166
+// -> 173 us, B X 246 -> 261).
+template <int EPI, int EW>
+constexpr int t2_slabs() { return EPI == T2_STORE || EW == 8 ? 2 : 4; }  // 4 KB staging slabs of an epilogue warp
+template <int EPI, int EW>
+constexpr int t2_smem_bytes() { return T2_STAGES * T2_STAGE_BYTES + EW * t2_slabs<EPI, EW>() * 4096 + 256 + 1024; }
+
+// Eight bf16 pairs -> one 128-byte row of a swizzled slab (64 columns).
+__device__ __forceinline__ void t2_store_row(uint8_t* rowp, int lane, const float (&v)[64]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    uint4 w;
+    w.x = pack_bf16x2(v[8 * j + 0], v[8 * j + 1]);
+    w.y = pack_bf16x2(v[8 * j + 2], v[8 * j + 3]);
+    w.z = pack_bf16x2(v[8 * j + 4], v[8 * j + 5]);
+    w.w = pack_bf16x2(v[8 * j + 6], v[8 * j + 7]);
+    *reinterpret_cast<uint4*>(rowp + ((j ^ (lane & 7)) << 4)) = w;
+  }
+}
+
+template <bool A_MN, bool B_MN, int EPI, int EW>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EW, 1)
 gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                const __grid_constant__ CUtensorMap tmD, const Gemm2Args args) {
-  constexpr uint32_t IDESC = make_idesc(1, 1, 2 * T2_BM, T2_BN, false, false);
+                const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmT, const Gemm2Args args) {
+  constexpr uint32_t IDESC = make_idesc(1, 1, 2 * T2_BM, T2_BN, A_MN, B_MN);
+  constexpr int NSLAB = t2_slabs<EPI, EW>();
+  constexpr int SPLIT = EW / 4;  // warps that share a quarter
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* staging = smem + T2_STAGES * T2_STAGE_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(staging + T2_STAGING);
+  uint64_t* full = reinterpret_cast<uint64_t*>(staging + EW * NSLAB * 4096);
   uint64_t* empty = full + T2_STAGES;
   uint64_t* tmem_full = empty + T2_STAGES;
   uint64_t* tmem_empty = tmem_full + 2;
@@ -110,12 +148,14 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int m_tiles = (args.M + 2 * T2_BM - 1) / (2 * T2_BM), n_tiles = (args.N + T2_BN - 1) / T2_BN;
-  const int num_tiles = m_tiles * n_tiles;
+  const bool sym = EPI == T2_FUSED && args.sym;
+  const int per_matrix = sym ? m_tiles * (m_tiles + 1) / 2 : m_tiles * n_tiles;
+  const int num_tiles = per_matrix * args.batch;
   const int num_kb = (args.K + T2_BK - 1) / T2_BK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < T2_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 8); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 2 * EW); }
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); tma_prefetch_desc(&tmD);
@@ -130,14 +170,29 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
 
-  auto tile_origin = [&](int t, int& m0, int& n0) {
-    const int GROUP = 8;
-    int per = GROUP * n_tiles;
-    int gid = t / per, first_m = gid * GROUP;
-    int gsz = min(m_tiles - first_m, GROUP);
-    int local = t - gid * per;
-    m0 = (first_m + local % gsz) * 2 * T2_BM;
-    n0 = (local / gsz) * T2_BN;
+  // Tile t of the launch: product e, origin (m0, n0).
+  auto tile_origin = [&](int t, int& e, int& m0, int& n0) {
+    e = t / per_matrix;
+    const int r = t - e * per_matrix;
+    int mt, nt;
+    if (sym) {
+      // columns of the upper triangle one after the other: column nt holds rows 0 .. nt
+      nt = 0;
+      int left = r;
+      while (left > nt) { left -= nt + 1; ++nt; }
+      mt = left;
+    } else {
+      // 8-row supergroups: concurrently running pairs share A rows and B columns in L2
+      const int GROUP = 8;
+      const int per = GROUP * n_tiles;
+      const int gid = r / per, first_m = gid * GROUP;
+      const int gsz = min(m_tiles - first_m, GROUP);
+      const int local = r - gid * per;
+      mt = first_m + local % gsz;
+      nt = local / gsz;
+    }
+    m0 = mt * 2 * T2_BM;
+    n0 = nt * T2_BN;
   };
 
   if (warp == 0) {
@@ -146,8 +201,10 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       uint32_t it = 0;
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-        int m0, n0;
-        tile_origin(t, m0, n0);
+        int e, m0, n0;
+        tile_origin(t, e, m0, n0);
+        m0 += (int)rank * T2_BM;
+        n0 += (int)rank * (T2_BN / 2);
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % T2_STAGES;
           const uint32_t ph = (it / T2_STAGES) & 1;
@@ -155,8 +212,33 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           if (!ok) break;
           if (leader) mbar_expect_tx(&full[s], 2 * T2_STAGE_BYTES);
           uint8_t* sa = smem + s * T2_STAGE_BYTES;
-          tma_load_2d_pair(sa, &tmA, &full[s], kb * T2_BK, m0 + (int)rank * T2_BM);
-          tma_load_2d_pair(sa + T2_A_BYTES, &tmB, &full[s], kb * T2_BK, n0 + (int)rank * (T2_BN / 2));
+          uint8_t* sb = sa + T2_A_BYTES;
+          if (!A_MN) {
+            tma_load_3d_pair(sa, &tmA, &full[s], kb * T2_BK, m0, e);
+          } else {
+#pragma unroll
+            for (int j = 0; j < T2_BM / 64; ++j) tma_load_3d_pair(sa + j * (T2_BK * 128), &tmA, &full[s], m0 + 64 * j, kb * T2_BK, e);
+          }
+          if (!B_MN) {
+            tma_load_3d_pair(sb, &tmB, &full[s], kb * T2_BK, n0, e);
+          } else {
+#pragma unroll
+            for (int j = 0; j < T2_BN / 128; ++j) tma_load_3d_pair(sb + j * (T2_BK * 128), &tmB, &full[s], n0 + 64 * j, kb * T2_BK, e);
+          }
+        }
+      }
+      if (leader && *abort_flag) {
+        // gave up somewhere: let the copies already in flight land before the pair retires (bounded)
+        const uint32_t n = it < (uint32_t)T2_STAGES ? it : (uint32_t)T2_STAGES;
+        const uint64_t t0 = globaltimer_ns();
+        for (uint32_t j = 1; j <= n; ++j) {
+          const uint32_t jt = it - j;
+          while (!mbar_try_wait(&full[jt % T2_STAGES], (jt / T2_STAGES) & 1)) {
+            if (globaltimer_ns() - t0 > 20000000ull) {
+              if (args.err) atomicCAS(args.err, 0, PT_ERR_TIMEOUT_DRAIN);
+              break;
+            }
+          }
         }
       }
     }
@@ -179,9 +261,13 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           const uint32_t a_addr = smem_u32(smem + s * T2_STAGE_BYTES);
           const uint32_t b_addr = a_addr + T2_A_BYTES;
 #pragma unroll
-          for (int k = 0; k < T2_BK / 16; ++k)
-            umma_f16_pair(d_tmem, make_smem_desc_sw128(a_addr + k * 32, 16, 1024), make_smem_desc_sw128(b_addr + k * 32, 16, 1024),
-                          IDESC, (kb | k) != 0 ? 1u : 0u);
+          for (int k = 0; k < T2_BK / 16; ++k) {
+            const uint64_t ad = A_MN ? make_smem_desc_sw128(a_addr + k * 2048, T2_BK * 128, 1024)
+                                     : make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
+            const uint64_t bd = B_MN ? make_smem_desc_sw128(b_addr + k * 2048, T2_BK * 128, 1024)
+                                     : make_smem_desc_sw128(b_addr + k * 32, 16, 1024);
+            umma_f16_pair(d_tmem, ad, bd, IDESC, (kb | k) != 0 ? 1u : 0u);
+          }
           umma_commit_pair(&empty[s]);
         }
         if (!ok) break;
@@ -190,56 +276,137 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
   } else {
     // ------------------------------------------------------------------ epilogue (both CTAs, own 128 rows)
-    const int q = warp & 3;
-    uint32_t tc = 0;
+    const int q = warp & 3;            // TMEM lane quarter this warp may read
+    const int first = (warp - 2) >> 2;  // chunks first, first + SPLIT, ...
+    uint8_t* slabs = staging + (warp - 2) * NSLAB * 4096;
+    uint32_t tc = 0, slab = 0;
     bool used_tma = false;
     for (int t = pair; t < num_tiles; t += num_pairs, ++tc) {
-      int m0, n0;
-      tile_origin(t, m0, n0);
+      int e, m0, n0;
+      tile_origin(t, e, m0, n0);
       const int acc = tc & 1;
-      int good = 1;
-      if (lane == 0) good = mbar_wait_bounded(&tmem_full[acc], (tc >> 1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE) ? 1 : 0;
-      good = __shfl_sync(0xffffffffu, good, 0);
-      if (!good) break;
-      tc_fence_after();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * T2_BN;
       const int row0 = m0 + (int)rank * T2_BM + q * 32;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * T2_BN;
+      const int cols_per = (EPI == T2_REDUCE && args.out_fp32) ? 32 : 64;
+      const int chunks = (min(args.N - n0, T2_BN) + cols_per - 1) / cols_per;
+      float sc = 1.f;
+      const __nv_bfloat16* cbase = nullptr;
+      bool mirror = false;
+      uint4 cv[8];
+      // addend of chunk cc, four rows of 128 bytes an instruction: lane -> row 4 i + lane / 8, piece lane % 8
+      auto load_c = [&](int cc) {
+        if (cbase == nullptr) return;
+        const int col = cc * 64 + (lane & 7) * 8;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int row = row0 + 4 * i + (lane >> 3);
+          cv[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (row < args.M && n0 + col < args.N) cv[i] = *reinterpret_cast<const uint4*>(cbase + (long long)row * args.ldc + col);
+        }
+      };
+      if (EPI == T2_FUSED) {
+        if (args.scale) {
+          const float s = args.scale[e];
+          sc = args.scale_pow == 2 ? s * s : s;
+        }
+        if (args.C) cbase = args.C + (long long)e * args.c_stride + n0;
+        mirror = sym && m0 != n0;
+        if (first < chunks) load_c(first);  // in flight while the products of this tile finish
+      }
+      if (!mbar_wait_bounded_warp(&tmem_full[acc], (tc >> 1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE)) break;
+      tc_fence_after();
+      if (SPLIT > 1 && first >= chunks && lane == 0) mbar_arrive_leader(&tmem_empty[acc]);  // a single chunk: nothing for the second warp
 #pragma unroll 1
-      for (int cc = 0; cc < T2_BN / 64; ++cc) {
-        if (n0 + cc * 64 >= args.N) break;
-        uint8_t* st = staging + (q * 2 + (cc & 1)) * 4096;
-        if (lane == 0) tma_store_wait_read<1>();
-        __syncwarp();
+      for (int cc = first; cc < chunks; cc += SPLIT) {
         uint32_t r0[32], r1[32];
-        tmem_ld_32x32(taddr + cc * 64, r0);
-        tmem_ld_32x32(taddr + cc * 64 + 32, r1);
+        tmem_ld_32x32(taddr + cc * cols_per, r0);
+        if (cols_per == 64) tmem_ld_32x32(taddr + cc * 64 + 32, r1);
         tmem_ld_wait();
-        if (cc == T2_BN / 64 - 1 || n0 + (cc + 1) * 64 >= args.N) {
-          // the accumulator has left TMEM: hand the buffer back to the leader's MMA thread
+        if (cc + SPLIT >= chunks) {
+          // this warp's part of the accumulator has left TMEM: hand the buffer back to the leader's MMA thread
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_leader(&tmem_empty[acc]);
         }
-        uint8_t* rowp = st + lane * 128;
+        if (EPI == T2_REDUCE && args.out_fp32) {
+          uint8_t* st = slabs + (slab % NSLAB) * 4096;
+          ++slab;
+          if (lane == 0) tma_store_wait_read<NSLAB - 1>();
+          __syncwarp();
+          uint8_t* rowp = st + lane * 128;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint4 v, w;
-          v.x = pack_bf16x2(__uint_as_float(r0[8 * j + 0]), __uint_as_float(r0[8 * j + 1]));
-          v.y = pack_bf16x2(__uint_as_float(r0[8 * j + 2]), __uint_as_float(r0[8 * j + 3]));
-          v.z = pack_bf16x2(__uint_as_float(r0[8 * j + 4]), __uint_as_float(r0[8 * j + 5]));
-          v.w = pack_bf16x2(__uint_as_float(r0[8 * j + 6]), __uint_as_float(r0[8 * j + 7]));
-          w.x = pack_bf16x2(__uint_as_float(r1[8 * j + 0]), __uint_as_float(r1[8 * j + 1]));
-          w.y = pack_bf16x2(__uint_as_float(r1[8 * j + 2]), __uint_as_float(r1[8 * j + 3]));
-          w.z = pack_bf16x2(__uint_as_float(r1[8 * j + 4]), __uint_as_float(r1[8 * j + 5]));
-          w.w = pack_bf16x2(__uint_as_float(r1[8 * j + 6]), __uint_as_float(r1[8 * j + 7]));
-          *reinterpret_cast<uint4*>(rowp + ((j ^ (lane & 7)) << 4)) = v;
-          *reinterpret_cast<uint4*>(rowp + (((j + 4) ^ (lane & 7)) << 4)) = w;
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(rowp + ((j ^ (lane & 7)) << 4)) = make_uint4(r0[4 * j], r0[4 * j + 1], r0[4 * j + 2], r0[4 * j + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_reduce_add_3d(&tmD, st, n0 + cc * 32, row0, e);  // past the tensor's extent: clipped by TMA
+            tma_store_commit();
+            used_tma = true;
+          }
+          continue;
+        }
+        uint8_t* st = slabs + (slab % NSLAB) * 4096;
+        ++slab;
+        if (lane == 0) tma_store_wait_read<NSLAB - 1>();
+        __syncwarp();
+        float v[64];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) { v[j] = __uint_as_float(r0[j]); v[32 + j] = __uint_as_float(r1[j]); }
+        if (EPI == T2_FUSED) {
+          const int d = row0 + lane - n0 - cc * 64;  // column of the diagonal in this chunk, if inside
+#pragma unroll
+          for (int j = 0; j < 64; ++j) v[j] *= args.alpha;
+          if (cbase) {
+            // through the slab, so that each lane gets its own row
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int r = 4 * i + (lane >> 3);
+              *reinterpret_cast<uint4*>(st + r * 128 + (((lane & 7) ^ (r & 7)) << 4)) = cv[i];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const uint4 c8 = *reinterpret_cast<const uint4*>(st + lane * 128 + ((j ^ (lane & 7)) << 4));
+              const uint32_t w[4] = {c8.x, c8.y, c8.z, c8.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float2 f = unpack_bf16x2(w[i]);
+                v[8 * j + 2 * i] = fmaf(args.beta, f.x, v[8 * j + 2 * i]);
+                v[8 * j + 2 * i + 1] = fmaf(args.beta, f.y, v[8 * j + 2 * i + 1]);
+              }
+            }
+            if (cc + SPLIT < chunks) load_c(cc + SPLIT);
+          }
+          if (args.diag != 0.f) {
+#pragma unroll
+            for (int j = 0; j < 64; ++j) v[j] += j == d ? args.diag : 0.f;
+          }
+#pragma unroll
+          for (int j = 0; j < 64; ++j) v[j] *= sc;
+        }
+        t2_store_row(st + lane * 128, lane, v);
+        uint8_t* mt = nullptr;
+        if (EPI == T2_FUSED && mirror) {
+          // the transposed copy: 64 rows (columns of the chunk) x 32 columns (rows of this warp), 64 bytes a row
+          mt = slabs + (slab % NSLAB) * 4096;
+          ++slab;
+          if (lane == 0) tma_store_wait_read<NSLAB - 2>();
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 64; ++j) *reinterpret_cast<__nv_bfloat16*>(mt + j * 64 + lane * 2) = __float2bfloat16(v[j]);
         }
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          tma_store_2d(&tmD, st, n0 + cc * 64, row0);  // rows or columns past the tensor's extent are clipped by TMA
+          // rows or columns past the tensor's extent are clipped by TMA
+          if (EPI == T2_REDUCE) tma_reduce_add_3d(&tmD, st, n0 + cc * 64, row0, e);
+          else tma_store_3d(&tmD, st, n0 + cc * 64, row0, e);
           tma_store_commit();
+          if (EPI == T2_FUSED && mt) {
+            tma_store_3d(&tmT, mt, row0, n0 + cc * 64, e);
+            tma_store_commit();
+          }
           used_tma = true;
         }
       }
@@ -256,6 +423,48 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   }
 }
 
+// One operand: a stack of row-major matrices [rows, cols], pitch ld, `stride` elements apart.
+struct T2Mat {
+  const void* p;
+  long long rows, cols, ld, stride;
+};
+
+// D_e = A_e B_e for args.batch products. A is [M, K] (or [K, M] with A_MN), B [N, K] (or [K, N] with B_MN), D [M, N].
+template <bool A_MN, bool B_MN, int EPI, int EW = 4>
+int t2_launch(const T2Mat& A, const T2Mat& B, const T2Mat& D, Gemm2Args& a, cudaStream_t stream) {
+  CUtensorMap tmA, tmB, tmD, tmT;
+  const int mn_rows = T2_BK, mn_cols = 64;
+  if (encode_tmap_3d(&tmA, A.p, TM_BF16, a.batch, A.rows, A.cols, A.ld, A.stride, 1, A_MN ? mn_rows : T2_BM, A_MN ? mn_cols : T2_BK, TM_SW_128)) return -3;
+  if (encode_tmap_3d(&tmB, B.p, TM_BF16, a.batch, B.rows, B.cols, B.ld, B.stride, 1, B_MN ? mn_rows : T2_BN / 2, B_MN ? mn_cols : T2_BK, TM_SW_128)) return -3;
+  const bool f32 = EPI == T2_REDUCE && a.out_fp32;
+  if (encode_tmap_3d(&tmD, D.p, f32 ? TM_F32 : TM_BF16, a.batch, D.rows, D.cols, D.ld, D.stride, 1, 32, f32 ? 32 : 64, TM_SW_128)) return -3;
+  tmT = tmD;
+  if (EPI == T2_FUSED && a.sym && encode_tmap_3d(&tmT, D.p, TM_BF16, a.batch, D.rows, D.cols, D.ld, D.stride, 1, 64, 32, TM_SW_NONE)) return -3;
+  a.err = device_status_word();
+  auto kern = gemm2cta_kernel<A_MN, B_MN, EPI, EW>;
+  constexpr int smem = t2_smem_bytes<EPI, EW>();
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
+    configured = true;
+  }
+  const long long m_tiles = (a.M + 2 * T2_BM - 1) / (2 * T2_BM), n_tiles = (a.N + T2_BN - 1) / T2_BN;
+  const long long tiles = a.batch * (EPI == T2_FUSED && a.sym ? m_tiles * (m_tiles + 1) / 2 : m_tiles * n_tiles);
+  if (tiles > 0x3fffffffLL) return -2;
+  long long pairs = sm_count() / 2;
+  if (pairs > tiles) pairs = tiles;
+  kern<<<(unsigned)(2 * pairs), 64 + 32 * EW, smem, stream>>>(tmA, tmB, tmD, tmT, a);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+inline Gemm2Args t2_args(int M, int N, int K, int batch) {
+  Gemm2Args a;
+  a.M = M; a.N = N; a.K = K; a.batch = batch; a.sym = 0; a.out_fp32 = 0;
+  a.alpha = 1.f; a.beta = 0.f; a.diag = 0.f;
+  a.scale = nullptr; a.scale_pow = 1; a.C = nullptr; a.ldc = 0; a.c_stride = 0; a.err = nullptr;
+  return a;
+}
+
 }  // namespace pt
 
 // x [M, K], w [N, K] bf16 row-major with pitches lda / ldb, out [M, N] bf16 with pitch ldd; K a multiple of 8.
@@ -263,22 +472,72 @@ PT_API int pt_gemm2cta_nt(const void* x, const void* w, void* out, int M, int N,
                           long long ldd, void* stream_) {
   using namespace pt;
   if (M <= 0 || N <= 0 || K <= 0 || K % 8 != 0) return -2;
-  CUtensorMap tmA, tmB, tmD;
-  if (encode_tmap_2d(&tmA, x, TM_BF16, M, K, lda, T2_BM, T2_BK, TM_SW_128)) return -3;
-  if (encode_tmap_2d(&tmB, w, TM_BF16, N, K, ldb, T2_BN / 2, T2_BK, TM_SW_128)) return -3;
-  if (encode_tmap_2d(&tmD, out, TM_BF16, M, N, ldd, 32, 64, TM_SW_128)) return -3;
-  Gemm2Args a;
-  a.M = M; a.N = N; a.K = K;
-  a.err = device_status_word();
-  const int smem = T2_STAGES * T2_STAGE_BYTES + T2_STAGING + 256 + 1024;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm2cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
-    configured = true;
+  Gemm2Args a = t2_args(M, N, K, 1);
+  return t2_launch<false, false, T2_STORE>({x, M, K, lda, lda * M}, {w, N, K, ldb, ldb * N}, {out, M, N, ldd, ldd * M}, a,
+                                           static_cast<cudaStream_t>(stream_));
+}
+
+// Orthogonalisation of Muon's updates: `steps` >= 1 quintic Newton-Schulz steps X <- (s_i (bA + cA^2 + aI)) X, A = X X^T, on a stack
+// Y [E, r, c] (bf16, contiguous, r and c multiples of 8), starting from s_e Y_e with the factors s [E] (fp32). Y
+// keeps its orientation: a wide one takes A = Y Y^T and B Y, a tall one A = Y^T Y and Y B, B being symmetric. The first step's
+// normalisation goes into the epilogues (A by s^2, B by s). Scratch: Z and Z2 like Y (Z2 may be Y itself),
+// A and B [E, min, min].
+// The last product updates weights: outs[i] holds the next counts[i] matrices, w = decay * w + alpha * X (decay 0: w = alpha * X).
+//
+// Bound by the tensor cores. Both Gram products are symmetric, so a third (three tiles a side) to 7/16 (eight) of their tiles
+// need not be computed, and the addend, diagonal, scaling and weight update ride in the epilogues instead of in passes of
+// their own. Five steps, library batched products with separate passes / here: 128 x [768, 2048] 3627 -> 2734 us, 64 x [1408, 2048]
+// 7767 -> 4539, 64 x [2880, 2880] 41.5 -> 28.8 ms, 32 x [256, 512] 300 -> 184, one [2048, 4096] 575 -> 555 (36 tiles for 74 pairs).
+PT_API int pt_muon_orthogonalize(const void* Y, void* Z, void* Z2, void* A, void* B, const float* s, int E, int r, int c, int steps,
+                                 const long long* outs, const int* counts, int n_outs, float decay, float alpha, void* stream_) {
+  using namespace pt;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (E <= 0 || r <= 0 || c <= 0) return 0;
+  if (r % 8 != 0 || c % 8 != 0 || steps < 1) return -2;
+  const bool wide = r <= c;
+  const int m = wide ? r : c;
+  const float ka = 3.4445f, kb = -4.7750f, kc = 2.0315f;
+  const long long yy = (long long)r * c, mm = (long long)m * m;
+  const T2Mat tA{A, m, m, m, mm}, tB{B, m, m, m, mm};
+  const void* X = Y;
+  for (int it = 0; it < steps; ++it) {
+    const T2Mat tX{X, r, c, c, yy};
+    Gemm2Args g = t2_args(m, m, wide ? c : r, E);
+    g.sym = 1;
+    if (it == 0) { g.scale = s; g.scale_pow = 2; }
+    int rc = wide ? t2_launch<false, false, T2_FUSED>(tX, tX, tA, g, stream) : t2_launch<true, true, T2_FUSED>(tX, tX, tA, g, stream);
+    if (rc) return rc;
+    g = t2_args(m, m, m, E);
+    g.sym = 1; g.alpha = kc; g.beta = kb; g.diag = ka;
+    g.C = static_cast<const __nv_bfloat16*>(A); g.ldc = m; g.c_stride = mm;
+    if (it == 0) g.scale = s;
+    rc = t2_launch<false, false, T2_FUSED, 8>(tA, tA, tB, g, stream);
+    if (rc) return rc;
+    if (it < steps - 1) {
+      g = t2_args(r, c, m, E);
+      void* next = it % 2 == 0 ? Z : Z2;
+      const T2Mat tN{next, r, c, c, yy};
+      rc = wide ? t2_launch<false, true, T2_STORE>(tB, tX, tN, g, stream) : t2_launch<false, false, T2_STORE>(tX, tB, tN, g, stream);
+      if (rc) return rc;
+      X = next;
+      continue;
+    }
+    long long first = 0;
+    for (int i = 0; i < n_outs; ++i) {
+      if (counts[i] <= 0) continue;
+      g = t2_args(r, c, m, counts[i]);
+      g.alpha = alpha; g.beta = decay;
+      void* w = reinterpret_cast<void*>(outs[i]);
+      if (decay != 0.f) { g.C = static_cast<const __nv_bfloat16*>(w); g.ldc = c; g.c_stride = yy; }
+      T2Mat xi = tX, bi = tB;
+      xi.p = static_cast<const __nv_bfloat16*>(X) + first * yy;
+      bi.p = static_cast<const __nv_bfloat16*>(B) + first * mm;
+      const T2Mat tW{w, r, c, c, yy};
+      rc = wide ? t2_launch<false, true, T2_FUSED, 8>(bi, xi, tW, g, stream) : t2_launch<false, false, T2_FUSED, 8>(xi, bi, tW, g, stream);
+      if (rc) return rc;
+      first += counts[i];
+    }
+    if (first != E) return -2;
   }
-  const int m_tiles = (M + 2 * T2_BM - 1) / (2 * T2_BM), n_tiles = (N + T2_BN - 1) / T2_BN;
-  int pairs = sm_count() / 2;
-  if (pairs > m_tiles * n_tiles) pairs = m_tiles * n_tiles;
-  gemm2cta_kernel<<<2 * pairs, 192, smem, static_cast<cudaStream_t>(stream_)>>>(tmA, tmB, tmD, a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  return 0;
 }

@@ -115,54 +115,14 @@ muon_momentum_kernel(const TG* __restrict__ g, TB* __restrict__ buf, __nv_bfloat
   }
 }
 
-// s = 1 / (|G|_F + 1e-7) of each matrix from its slabs: s1 = bf16(s), s2 = bf16(s^2).
+// s = 1 / (|G|_F + 1e-7) of each matrix from its slabs.
 __global__ void __launch_bounds__(32)
-frobenius_scales_kernel(const float* __restrict__ partial, int slabs, __nv_bfloat16* __restrict__ s1, __nv_bfloat16* __restrict__ s2) {
+frobenius_scales_kernel(const float* __restrict__ partial, int slabs, float* __restrict__ s) {
   double t = 0.0;
   for (int i = threadIdx.x; i < slabs; i += 32) t += partial[(long long)blockIdx.x * slabs + i];
 #pragma unroll
   for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (threadIdx.x == 0) {
-    const float s = 1.f / ((float)sqrt(t) + 1e-7f);
-    s1[blockIdx.x] = __float2bfloat16(s);
-    s2[blockIdx.x] = __float2bfloat16(s * s);
-  }
-}
-
-// First step of the orthogonalisation on the Gram matrices A [E, m, m]: A *= s2 (in place) and C = A, the addend of the next
-// product. One pass for a scaling (a broadcast elementwise operation, 3.5 TB/s) and a copy: 64 x [768, 768] 69 -> 40 us.
-__global__ void __launch_bounds__(256)
-gram_scale_copy_kernel(__nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ C, const __nv_bfloat16* __restrict__ s2, long long nvec, long long per_vec) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
-    const float s = __bfloat162float(s2[i / per_vec]);
-    float f[8];
-    load8(A + i * 8, f);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] *= s;
-    store8(A + i * 8, f);
-    store8(C + i * 8, f);
-  }
-}
-
-// B = (B + a I) * s1 on [E, m, m], rounded to bf16 after the sum and after the product.
-__global__ void __launch_bounds__(256)
-gram_shift_scale_kernel(__nv_bfloat16* __restrict__ B, const __nv_bfloat16* __restrict__ s1, long long nvec, int m, float a) {
-  const int row_vec = m / 8;
-  const long long per_vec = (long long)m * row_vec;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
-    const long long e0 = i / per_vec;
-    const unsigned in = (unsigned)(i - e0 * per_vec);
-    const float s = __bfloat162float(s1[e0]);
-    const int row = in / row_vec, d = row - (int)(in % row_vec) * 8;  // the diagonal is element d of this vector, if inside
-    float f[8];
-    load8(B + i * 8, f);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float x = e == d ? __bfloat162float(__float2bfloat16(f[e] + a)) : f[e];
-      f[e] = x * s;
-    }
-    store8(B + i * 8, f);
-  }
+  if (threadIdx.x == 0) s[blockIdx.x] = 1.f / ((float)sqrt(t) + 1e-7f);
 }
 
 // w = w * decay + alpha * x  (bf16 weights, bf16 update)
@@ -215,28 +175,11 @@ PT_API int pt_muon_momentum_sumsq(const void* g, int g_fp32, void* buf, int buf_
   return (int)cudaGetLastError();
 }
 
-// s1, s2: bf16 [E] from the partial sums of pt_muon_momentum_sumsq.
-PT_API int pt_frobenius_scales(const float* partial, int E, int slabs, void* s1, void* s2, void* stream_) {
+// s: fp32 [E] from the partial sums of pt_muon_momentum_sumsq.
+PT_API int pt_frobenius_scales(const float* partial, int E, int slabs, float* s, void* stream_) {
   if (E <= 0) return 0;
   if (slabs < 1) return -1;
-  frobenius_scales_kernel<<<E, 32, 0, (cudaStream_t)stream_>>>(partial, slabs, (__nv_bfloat16*)s1, (__nv_bfloat16*)s2);
-  return (int)cudaGetLastError();
-}
-
-// A, C: bf16 [E, m, m] contiguous, m a multiple of 8.
-PT_API int pt_gram_scale_copy(void* A, void* C, const void* s2, int E, int m, void* stream_) {
-  if (E <= 0 || m <= 0) return 0;
-  if (m % 8 != 0 || m > 65536) return -1;
-  const long long per_vec = (long long)m * m / 8, nvec = per_vec * E;
-  gram_scale_copy_kernel<<<flat_grid(nvec), 256, 0, (cudaStream_t)stream_>>>((__nv_bfloat16*)A, (__nv_bfloat16*)C, (const __nv_bfloat16*)s2, nvec, per_vec);
-  return (int)cudaGetLastError();
-}
-
-PT_API int pt_gram_shift_scale(void* B, const void* s1, int E, int m, float a, void* stream_) {
-  if (E <= 0 || m <= 0) return 0;
-  if (m % 8 != 0 || m > 65536) return -1;
-  const long long nvec = (long long)m * m / 8 * E;
-  gram_shift_scale_kernel<<<flat_grid(nvec), 256, 0, (cudaStream_t)stream_>>>((__nv_bfloat16*)B, (const __nv_bfloat16*)s1, nvec, m, a);
+  frobenius_scales_kernel<<<E, 32, 0, (cudaStream_t)stream_>>>(partial, slabs, s);
   return (int)cudaGetLastError();
 }
 

@@ -9,8 +9,9 @@ publishes the result; the reference's gather-per-weight and owner broadcasts hav
 
 Implementation notes. Work is done on contiguous *units*: a plain parameter, or the fused
 ``[E, 2, I, H]`` storage behind an expert gate/up pair (each ``[I, H]`` matrix is still
-orthogonalised on its own). On CUDA the momentum update and the final ``w = w*(1-lr*wd) - lr*s*O``
-are single kernels over the unit; the matmuls of the iteration go to batched GEMMs. The momentum
+orthogonalised on its own). On CUDA the momentum update is one kernel over the unit; units of one matrix
+shape are orthogonalised as one stack on the 2-CTA products, the last of which also makes
+``w = w*(1-lr*wd) - lr*s*O``. The momentum
 buffers can live in pinned host memory (``offload_state``): chunks are prefetched on a copy
 stream while the previous chunk is being orthogonalised and written back on another, which is what
 lets a 30B-parameter model train on one 180 GB GPU.
@@ -45,7 +46,8 @@ def _owned(p: torch.Tensor) -> bool:
 
 
 def zeropower_via_newtonschulz5(Gm: torch.Tensor, steps: int = 5) -> torch.Tensor:
-    """Quintic Newton-Schulz iteration towards the orthogonal polar factor, batched over leading dims.
+    """Quintic Newton-Schulz iteration towards the orthogonal polar factor, batched over leading dims. CUDA stacks whose sides are
+    multiples of 8 run on the 2-CTA products (:func:`_orthogonalize`).
 
     The iteration is ``X <- aX + (bA + cA^2)X`` with ``A = X X^T`` on the wide orientation of
     ``X0 = G / (|G|_F + 1e-7)``, in bf16 (pithtrain/modules/optimizer.py:34-57 of the reference). It is
@@ -62,12 +64,47 @@ def zeropower_via_newtonschulz5(Gm: torch.Tensor, steps: int = 5) -> torch.Tenso
     assert Gm.ndim >= 2
     if _own_gemm_usable(Gm):
         return newtonschulz5_own_gemm(Gm, steps)
-    return _newton_schulz(Gm, steps, None)
+    if steps >= 1 and Gm.numel() > 0 and _fused_shape(Gm) and _native.on_current_device(Gm) and not _transformed(Gm):
+        G = Gm.to(torch.bfloat16).contiguous()
+        G3 = G.view(-1, *G.shape[-2:])
+        s = 1.0 / (torch.linalg.vector_norm(G3, dim=(-2, -1), dtype=torch.float32) + 1e-7)
+        out = torch.empty_like(G3)
+        if G3.data_ptr() % 16 != 0:
+            G3 = G3.clone()
+        _orthogonalize(G3, torch.empty_like(G3), s, steps, [out], 0.0, 1.0)
+        return out.view(G.shape)
+    return _newton_schulz(Gm, steps)
 
 
-def _newton_schulz(Gm: torch.Tensor, steps: int, scales) -> torch.Tensor:
-    """``scales``: None, or bf16 ``(s, s^2)`` of every matrix of a CUDA stack whose smaller side is a multiple of 8; the
-    first step's scalings, copy and diagonal then take two passes over the Gram matrices instead of five."""
+def _transformed(t: torch.Tensor) -> bool:
+    """Whether autograd, forward-mode differentiation or a functorch transform looks at what is done with ``t``; kernels on raw
+    pointers would pass them by."""
+    return ((t.requires_grad and torch.is_grad_enabled()) or torch._C._functorch.is_functorch_wrapped_tensor(t)
+            or torch.autograd.forward_ad._current_level >= 0)
+
+
+def _fused_shape(t: torch.Tensor) -> bool:
+    """Whether the matrices of ``t`` fit the 2-CTA products: whole 16-byte rows in both orientations."""
+    return t.shape[-2] % 8 == 0 and t.shape[-1] % 8 == 0
+
+
+def _orthogonalize(Y, spare, s, steps, outs, decay, alpha) -> None:
+    """Newton-Schulz on the stack ``Y`` [E, r, c] (bf16, CUDA) from ``s * Y``; the next ``len(w)`` results go to each ``w`` of
+    ``outs`` as ``w * decay + alpha * X``. ``spare`` is overwritten and may be ``Y`` itself."""
+    import ctypes
+
+    E, r, c = Y.shape
+    m, L = min(r, c), _native.lib()
+    Z = torch.empty_like(Y)
+    A, B = torch.empty((2, E, m, m), dtype=Y.dtype, device=Y.device)
+    ptrs, counts = (ctypes.c_longlong * len(outs))(*(w.data_ptr() for w in outs)), (ctypes.c_int * len(outs))(*(w.shape[0] for w in outs))
+    rc = L.pt_muon_orthogonalize(Y.data_ptr(), Z.data_ptr(), spare.data_ptr(), A.data_ptr(), B.data_ptr(), s.data_ptr(), E, r, c, steps,
+                                 ptrs, counts, len(outs), float(decay), float(alpha), _native.stream_ptr())
+    _native.check(rc, "pt_muon_orthogonalize", 3 * steps - 1 + len(outs))
+
+
+def _newton_schulz(Gm: torch.Tensor, steps: int) -> torch.Tensor:
+    """The same on tensor operations: other devices, and matrices whose sides are not multiples of 8."""
     a, b, c = 3.4445, -4.7750, 2.0315
     G = Gm.to(torch.bfloat16)
     squeeze = G.ndim == 2
@@ -81,28 +118,18 @@ def _newton_schulz(Gm: torch.Tensor, steps: int, scales) -> torch.Tensor:
         nrm = torch.linalg.vector_norm(G, dim=(-2, -1), keepdim=True, dtype=torch.float32)
         out = G / (nrm + 1e-7).to(G.dtype)
     else:
-        if scales is None:
-            nrm = torch.linalg.vector_norm(G, dim=(-2, -1), keepdim=True, dtype=torch.float32)
-            s = 1.0 / (nrm + 1e-7)
-            s1, s2 = s.to(G.dtype), (s * s).to(G.dtype)
+        nrm = torch.linalg.vector_norm(G, dim=(-2, -1), keepdim=True, dtype=torch.float32)
+        s = 1.0 / (nrm + 1e-7)
+        s1, s2 = s.to(G.dtype), (s * s).to(G.dtype)
         out = None
         for it in range(steps):
             A = torch.bmm(X, X.mT)
-            if it == 0 and scales is not None:
-                B = torch.empty_like(A)
-                L, E, m = _native.lib(), A.shape[0], A.shape[1]
-                _native.check(L.pt_gram_scale_copy(A.data_ptr(), B.data_ptr(), scales[1].data_ptr(), E, m, _native.stream_ptr()),
-                              "pt_gram_scale_copy")
-                B.baddbmm_(A, A, beta=b, alpha=c)
-                _native.check(L.pt_gram_shift_scale(B.data_ptr(), scales[0].data_ptr(), E, m, a, _native.stream_ptr()),
-                              "pt_gram_shift_scale")
-            else:
-                if it == 0:
-                    A.mul_(s2)
-                B = torch.baddbmm(A, A, A, beta=b, alpha=c)
-                B.diagonal(dim1=-2, dim2=-1).add_(a)
-                if it == 0:
-                    B.mul_(s1)
+            if it == 0:
+                A.mul_(s2)
+            B = torch.baddbmm(A, A, A, beta=b, alpha=c)
+            B.diagonal(dim1=-2, dim2=-1).add_(a)
+            if it == 0:
+                B.mul_(s1)
             last = it == steps - 1
             if last and tall:
                 out = torch.bmm(X.mT, B)  # [n, m]: the input's own orientation
@@ -185,6 +212,18 @@ def orthogonalized_updates(params: List[torch.Tensor], updates: List[torch.Tenso
         o = zeropower_via_newtonschulz5(u, steps=steps).to(p.dtype)
         out.append(o * muon_scale_factor(u.size(-2), u.size(-1)))
     return out
+
+
+def _native_update(w, g, buf) -> bool:
+    """Whether the momentum and update kernels take this unit."""
+    return (w.is_cuda and w.dtype == torch.bfloat16 and w.is_contiguous() and g.is_contiguous() and buf.is_contiguous()
+            and w.numel() % 8 == 0 and g.dtype in (torch.float32, torch.bfloat16) and buf.dtype in (torch.float32, torch.bfloat16))
+
+
+def _stackable(w, g, buf) -> bool:
+    """Whether the unit's matrices can be orthogonalised with the update of ``w`` in the last product."""
+    return (w.numel() > 0 and _native_update(w, g, buf) and _fused_shape(w) and not _own_gemm_usable(w)
+            and _native.on_current_device(w) and w.data_ptr() % 16 == 0 and g.data_ptr() % 16 == 0 and buf.data_ptr() % 16 == 0)
 
 
 class _Unit:
@@ -296,43 +335,69 @@ class Muon(torch.optim.Optimizer):
                 if host:
                     self._run_offloaded(host, beta, lr, wd, tail=resident)
                 else:
-                    for w, g, st, gs in resident:
-                        self._update_chunk(w, g, st, beta, lr, wd, gs)
+                    self._update_all(resident, beta, lr, wd)
             else:
-                for w, g, st, gs in work:
-                    self._update_chunk(w, g, st, beta, lr, wd, gs)
+                self._update_all(work, beta, lr, wd)
         return loss
+
+    def _update_all(self, work, beta, lr, wd) -> None:
+        """Items ``(w, g, momentum, gradient scale)``; matrices of one shape are orthogonalised as one stack of at most
+        ``max_chunk_elems`` elements. One layer's small projections leave most SMs idle: of a [512, 2048] matrix the products
+        have 3 to 16 tiles for 74 CTA pairs."""
+        stacks: Dict[tuple, list] = {}
+        for item in work:
+            w, g, buf, gs = item
+            if not _stackable(w, g, buf):
+                self._update_chunk(w, g, buf, beta, lr, wd, gs)
+                continue
+            key = (w.shape[-2], w.shape[-1], w.device)
+            batch = stacks.setdefault(key, [])
+            if batch and sum(i[0].numel() for i in batch) + w.numel() > self.max_chunk_elems:
+                self._update_stack(batch, beta, lr, wd)
+                batch.clear()
+            batch.append(item)
+        for batch in stacks.values():
+            self._update_stack(batch, beta, lr, wd)
+
+    def _update_stack(self, items, beta, lr, wd) -> None:
+        """Matrices of one shape: momentum and norms by item, the orthogonalisation and the weight update on all of them."""
+        n, m = items[0][0].shape[-2:]
+        dev, L = items[0][0].device, _native.lib()
+        counts = [w.numel() // (n * m) for w, _, _, _ in items]
+        E = sum(counts)
+        upd = torch.empty((E, n, m), dtype=torch.bfloat16, device=dev)
+        s = torch.empty(E, dtype=torch.float32, device=dev)
+        first = 0
+        for (w, g, buf, gscale), count in zip(items, counts):
+            partial = torch.empty((count, L.pt_muon_slabs(count, n * m)), dtype=torch.float32, device=dev)
+            rc = L.pt_muon_momentum_sumsq(g.data_ptr(), int(g.dtype == torch.float32), buf.data_ptr(),
+                                          int(buf.dtype == torch.float32), upd[first].data_ptr(), count, n * m, float(beta),
+                                          None if gscale is None else gscale.data_ptr(), partial.data_ptr(), _native.stream_ptr())
+            _native.check(rc, "pt_muon_momentum_sumsq")
+            rc = L.pt_frobenius_scales(partial.data_ptr(), count, partial.shape[1], s[first:].data_ptr(), _native.stream_ptr())
+            _native.check(rc, "pt_frobenius_scales")
+            first += count
+        _orthogonalize(upd, upd, s, 5, [w.view(-1, n, m) for w, _, _, _ in items], 1 - lr * wd, -lr * muon_scale_factor(n, m))
 
     def _update_chunk(self, w, g, buf, beta, lr, wd, gscale=None) -> None:
         """``buf`` is on the same device as ``w`` here."""
+        if _stackable(w, g, buf):
+            return self._update_stack([(w, g, buf, gscale)], beta, lr, wd)
         n, m = w.shape[-2], w.shape[-1]
-        scales = None
-        native = (w.is_cuda and w.dtype == torch.bfloat16 and w.is_contiguous() and g.is_contiguous()
-                  and buf.is_contiguous() and w.numel() % 8 == 0 and g.dtype in (torch.float32, torch.bfloat16)
-                  and buf.dtype in (torch.float32, torch.bfloat16))
+        native = _native_update(w, g, buf)
         if native:
             L = _native.lib()
             upd = torch.empty(w.shape, dtype=torch.bfloat16, device=w.device)
-            # the fused norm and the passes over the Gram matrices work on whole 16-byte vectors of one matrix's rows
-            fused = w.numel() > 0 and min(n, m) % 8 == 0 and min(n, m) <= 65536 and not _own_gemm_usable(upd)
-            E, per = (w.numel() // (n * m), n * m) if fused else (1, w.numel())
-            partial = torch.empty((E, L.pt_muon_slabs(E, per)), dtype=torch.float32, device=w.device) if fused else None
             rc = L.pt_muon_momentum_sumsq(g.data_ptr(), int(g.dtype == torch.float32), buf.data_ptr(),
-                                          int(buf.dtype == torch.float32), upd.data_ptr(), E, per, float(beta),
-                                          None if gscale is None else gscale.data_ptr(),
-                                          None if partial is None else partial.data_ptr(), _native.stream_ptr())
+                                          int(buf.dtype == torch.float32), upd.data_ptr(), 1, w.numel(), float(beta),
+                                          None if gscale is None else gscale.data_ptr(), None, _native.stream_ptr())
             _native.check(rc, "pt_muon_momentum_sumsq")
-            if fused:
-                scales = torch.empty((2, E), dtype=torch.bfloat16, device=w.device)
-                rc = L.pt_frobenius_scales(partial.data_ptr(), E, partial.shape[1], scales[0].data_ptr(), scales[1].data_ptr(),
-                                           _native.stream_ptr())
-                _native.check(rc, "pt_frobenius_scales")
         else:
             g32 = g.float() if gscale is None else g.float() * gscale.to(g.device)
             b32 = buf.float().lerp_(g32, 1 - beta)
             buf.copy_(b32)
             upd = g32.lerp(b32, beta)
-        orth = zeropower_via_newtonschulz5(upd, steps=5) if scales is None else _newton_schulz(upd, 5, scales)
+        orth = zeropower_via_newtonschulz5(upd, steps=5)
         scale = muon_scale_factor(n, m)
         if native:
             orth = orth.contiguous()

@@ -616,6 +616,65 @@ def test_muon_update_with_fused_norm(shape, gdt, bdt):
     assert float((got - want).norm()) <= bound
 
 
+@pytest.mark.parametrize("shape", [(8, 8), (3, 8, 520), (2, 520, 8), (2, 248, 264), (1, 264, 248), (3, 256, 256), (2, 512, 776), (1, 1032, 520)])
+def test_newton_schulz_products(shape):
+    """Against the iteration in 64 bits, at the edges of the 256-wide tiles and of their mirrored halves. The kernels round the
+    Gram matrices, the polynomial and the factors to bf16 once each, the tensor operations up to three times, so they may not be
+    further off than those; 5 % for chance, since both errors are sums over random roundings."""
+    from pithtrain_b200.modules.optimizer import _newton_schulz, zeropower_via_newtonschulz5
+
+    torch.manual_seed(11)
+    G = torch.randn(shape, device="cuda").bfloat16()
+    before = G.clone()
+    got, ops = zeropower_via_newtonschulz5(G), _newton_schulz(G, 5)
+    _native.check_status()
+    assert torch.equal(G, before) and got.shape == G.shape and got.dtype == torch.bfloat16
+    X = G.double() / (torch.linalg.vector_norm(G.double(), dim=(-2, -1), keepdim=True) + 1e-7)
+    for _ in range(5):
+        A = X @ X.mT if shape[-2] <= shape[-1] else X.mT @ X
+        B = -4.7750 * A + 2.0315 * A @ A
+        X = 3.4445 * X + (B @ X if shape[-2] <= shape[-1] else X @ B)
+    assert float((got.double() - X).norm()) <= 1.05 * float((ops.double() - X).norm())
+
+
+def test_newton_schulz_under_transforms():
+    """Autograd, forward mode and vmap see the tensor operations."""
+    from pithtrain_b200.modules.optimizer import _newton_schulz, zeropower_via_newtonschulz5
+
+    torch.manual_seed(13)
+    G = torch.randn(2, 16, 24, device="cuda").bfloat16()
+    leaf = G.clone().requires_grad_()
+    assert torch.equal(torch.autograd.grad(zeropower_via_newtonschulz5(leaf).sum(), leaf)[0],
+                       torch.autograd.grad(_newton_schulz(leaf, 5).sum(), leaf)[0])
+    assert torch.equal(torch.func.vmap(zeropower_via_newtonschulz5)(G), torch.func.vmap(lambda g: _newton_schulz(g, 5))(G))
+    one = torch.ones_like(G)
+    assert torch.equal(torch.func.jvp(zeropower_via_newtonschulz5, (G,), (one,))[1],
+                       torch.func.jvp(lambda g: _newton_schulz(g, 5), (G,), (one,))[1])
+
+
+def test_muon_stacks_matrices_of_one_shape():
+    """Parameters of one shape are orthogonalised together, others by themselves; both as one at a time."""
+    from pithtrain_b200.modules.optimizer import Muon
+
+    torch.manual_seed(12)
+    shapes = [(64, 136), (64, 136), (3, 64, 136), (136, 64), (20, 12), (64, 136)]
+    weights = [torch.randn(s, device="cuda").bfloat16() for s in shapes]
+    grads = [torch.randn(s, device="cuda") for s in shapes]
+
+    def run(groups, **kw):
+        params = [torch.nn.Parameter(w.clone()) for w in weights]
+        for p, g in zip(params, grads):
+            p.main_grad = g
+        for idx in groups:
+            Muon([params[i] for i in idx], lr=0.1, **kw).step()
+        _native.check_status()
+        return params
+
+    together = run([range(6)])
+    for other in (run([[i] for i in range(6)]), run([range(6)], max_chunk_elems=2 * 64 * 136)):
+        assert all(torch.equal(a, b) for a, b in zip(together, other))
+
+
 @pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
 @pytest.mark.parametrize("n,E,k", [(1, 1, 1), (3, 4, 8), (257, 130, 6), (5000, 512, 16)])
 def test_balanced_replay(n, E, k, dtype):
