@@ -132,6 +132,8 @@ SIGS = {
     "pt_attn_bwd_split": "PPPPPPPPPPPPP" + "IIIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_attn_bwd": "PPPPPPPPPPPPPPP" + "IIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_gemm2cta_nt": "PPPIIILLLP",
+    "pt_gemm2cta_nn": "PPPIIILLLP",
+    "pt_gemm2cta_tn": "PPPIIIIILLLP",
     "pt_mla_fwd": "PPPLLLPPPPPPIIIIIIIP",
     "pt_mla_bwd": "PPPPPPPPPIIIIIIIP",
     "pt_row_bias_dot": "PPPIPPPIIP",

@@ -22,6 +22,8 @@
 //              the diagonal, the normalisation and the weight update in them. With `sym` (D symmetric) only the tiles on and
 //              above the diagonal are computed, and each is stored a second time, transposed.
 //   T2_REDUCE  D += acc in bf16 or fp32 by TMA reduce-add (dense weight gradients)
+//   T2_SUM     the same with the sums of an fp32 product: the tensor core cuts its sums off, so every T2_PROMOTE k-blocks they
+//              move to registers and are added there with rounding
 //
 // PTX forms follow the vendored CUTLASS headers (cute/arch/copy_sm100_tma.hpp: SM100_TMA_2SM_LOAD_3D,
 // cute/arch/mma_sm100_umma.hpp: SM100_MMA_F16BF16_2x1SM_SS, cute/arch/tmem_allocator_sm100.hpp: Allocator2Sm,
@@ -40,13 +42,13 @@ constexpr int T2_B_BYTES = (T2_BN / 2) * T2_BK * 2;  // 16 KB (this CTA's half)
 constexpr int T2_STAGE_BYTES = T2_A_BYTES + T2_B_BYTES;
 constexpr uint32_t T2_PEER_MASK = 0xFEFFFFFFu;  // clears the pair-rank bit of a shared::cluster address -> CTA 0
 
-enum Gemm2Epi : int { T2_STORE = 0, T2_FUSED = 1, T2_REDUCE = 2 };
+enum Gemm2Epi : int { T2_STORE = 0, T2_FUSED = 1, T2_REDUCE = 2, T2_SUM = 3 };
 
 struct Gemm2Args {
   int M, N, K;
   int batch;     // stacked products (dense: 1)
   int sym;       // T2_FUSED: D is symmetric (M == N)
-  int out_fp32;  // T2_REDUCE
+  int out_fp32;  // T2_REDUCE, T2_SUM
   float alpha, beta, diag;
   const float* scale;  // T2_FUSED: one factor per product (null: 1), applied scale_pow times
   int scale_pow;
@@ -108,6 +110,10 @@ __device__ __forceinline__ void mbar_arrive_leader(uint64_t* bar) {
 // 64-column chunks in turn. Eight pay where a short reduction meets an addend (A^2 of 128 x [768, 768]: 102 -> 84 us); elsewhere
 // the products of a tile hide four, and eight cost 4 to 5 % (polling beside a power-capped tensor core: A of 128 x [768, 2048] 166
 // -> 173 us, B X 246 -> 261).
+// T2_SUM: k-blocks that the tensor core sums up before the sum moves to registers. Relative error (2-norm) of [5120, 2048] over
+// 3001 rows / [768, 1024] over 1001 and time of the former, cold: never 3.2e-6 / 9.8e-7, every 8 blocks 4.7e-7 / 4.6e-7 76 us, 4
+// 2.4e-7 / 2.3e-7 83, 2 1.5e-7 / 1.3e-7 97, 1 1.4e-7 / 1.0e-7 113; the library's fp32 product 5.0e-7 / 2.5e-7, about 1000 us.
+constexpr int T2_PROMOTE = 2;
 template <int EPI, int EW>
 constexpr int t2_slabs() { return EPI == T2_STORE || EW == 8 ? 2 : 4; }  // 4 KB staging slabs of an epilogue warp
 template <int EPI, int EW>
@@ -152,6 +158,7 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   const int per_matrix = sym ? m_tiles * (m_tiles + 1) / 2 : m_tiles * n_tiles;
   const int num_tiles = per_matrix * args.batch;
   const int num_kb = (args.K + T2_BK - 1) / T2_BK;
+  const int parts = (num_kb + T2_PROMOTE - 1) / T2_PROMOTE;  // T2_SUM: accumulators of a tile
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < T2_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -247,13 +254,18 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (leader && lane == 0) {
       uint32_t it = 0, tc = 0;
       bool ok = true;
-      for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tc) {
+      for (int item = 0; ok; ++item, ++tc) {
+        // an accumulator's work: a tile, or for T2_SUM a tile's next T2_PROMOTE k-blocks
+        const int t = pair + (EPI == T2_SUM ? item / parts : item) * num_pairs;
+        if (t >= num_tiles) break;
+        const int kb0 = EPI == T2_SUM ? (item % parts) * T2_PROMOTE : 0;
+        const int kb1 = EPI == T2_SUM ? min(num_kb, kb0 + T2_PROMOTE) : num_kb;
         const int acc = tc & 1;
         ok = mbar_wait_bounded(&tmem_empty[acc], ((tc >> 1) & 1) ^ 1, abort_flag, args.err, PT_ERR_TIMEOUT_MMA);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * T2_BN;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % T2_STAGES;
           ok = mbar_wait_bounded(&full[s], (it / T2_STAGES) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_MMA);
           if (!ok) break;
@@ -266,7 +278,7 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                                      : make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
             const uint64_t bd = B_MN ? make_smem_desc_sw128(b_addr + k * 2048, T2_BK * 128, 1024)
                                      : make_smem_desc_sw128(b_addr + k * 32, 16, 1024);
-            umma_f16_pair(d_tmem, ad, bd, IDESC, (kb | k) != 0 ? 1u : 0u);
+            umma_f16_pair(d_tmem, ad, bd, IDESC, (kb != kb0 || k != 0) ? 1u : 0u);
           }
           umma_commit_pair(&empty[s]);
         }
@@ -281,13 +293,82 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     uint8_t* slabs = staging + (warp - 2) * NSLAB * 4096;
     uint32_t tc = 0, slab = 0;
     bool used_tma = false;
+    if constexpr (EPI == T2_SUM) {
+      // half of the tile's columns in registers, 32 at a time from TMEM
+      static_assert(EPI != T2_SUM || EW == 8, "two warps a quarter");
+      bool good = true;
+      for (int t = pair; t < num_tiles && good; t += num_pairs) {
+        int e, m0, n0;
+        tile_origin(t, e, m0, n0);
+        const int row0 = m0 + (int)rank * T2_BM + q * 32, col0 = n0 + first * (T2_BN / 2);
+        float sum[T2_BN / 2];
+#pragma unroll
+        for (int j = 0; j < T2_BN / 2; ++j) sum[j] = 0.f;
+        for (int part = 0; part < parts; ++part, ++tc) {
+          const int acc = tc & 1;
+          good = mbar_wait_bounded_warp(&tmem_full[acc], (tc >> 1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE);
+          if (!good) break;
+          tc_fence_after();
+          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * T2_BN + first * (T2_BN / 2);
+#pragma unroll
+          for (int c = 0; c < T2_BN / 32; ++c) {
+            uint32_t r[16];
+            tmem_ld_32x16(taddr + c * 16, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sum[16 * c + j] += __uint_as_float(r[j]);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_leader(&tmem_empty[acc]);
+        }
+        if (!good) break;
+        const int cols_per = args.out_fp32 ? 32 : 64;
+#pragma unroll
+        for (int c = 0; c < T2_BN / 64; ++c) {
+          // 32 columns: a slab of fp32, half a slab of bf16
+          if (col0 + c * 32 / cols_per * cols_per >= args.N) break;
+          uint8_t* st = slabs + (slab % NSLAB) * 4096;
+          if (args.out_fp32 || c % 2 == 0) {
+            if (lane == 0) tma_store_wait_read<NSLAB - 1>();
+            __syncwarp();
+          }
+          uint8_t* rowp = st + lane * 128;
+          if (args.out_fp32) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<float4*>(rowp + ((j ^ (lane & 7)) << 4)) =
+                  make_float4(sum[32 * c + 4 * j], sum[32 * c + 4 * j + 1], sum[32 * c + 4 * j + 2], sum[32 * c + 4 * j + 3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint4 w;
+              w.x = pack_bf16x2(sum[32 * c + 8 * j], sum[32 * c + 8 * j + 1]);
+              w.y = pack_bf16x2(sum[32 * c + 8 * j + 2], sum[32 * c + 8 * j + 3]);
+              w.z = pack_bf16x2(sum[32 * c + 8 * j + 4], sum[32 * c + 8 * j + 5]);
+              w.w = pack_bf16x2(sum[32 * c + 8 * j + 6], sum[32 * c + 8 * j + 7]);
+              *reinterpret_cast<uint4*>(rowp + (((j + (c % 2) * 4) ^ (lane & 7)) << 4)) = w;
+            }
+            if (c % 2 == 0) continue;
+          }
+          ++slab;
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_reduce_add_3d(&tmD, st, col0 + c * 32 / cols_per * cols_per, row0, e);  // past the tensor's extent: clipped by TMA
+            tma_store_commit();
+            used_tma = true;
+          }
+        }
+      }
+    } else
     for (int t = pair; t < num_tiles; t += num_pairs, ++tc) {
       int e, m0, n0;
       tile_origin(t, e, m0, n0);
       const int acc = tc & 1;
       const int row0 = m0 + (int)rank * T2_BM + q * 32;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * T2_BN;
-      const int cols_per = (EPI == T2_REDUCE && args.out_fp32) ? 32 : 64;
+      const int cols_per = EPI == T2_REDUCE && args.out_fp32 ? 32 : 64;
       const int chunks = (min(args.N - n0, T2_BN) + cols_per - 1) / cols_per;
       float sc = 1.f;
       const __nv_bfloat16* cbase = nullptr;
@@ -328,11 +409,11 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           __syncwarp();
           if (lane == 0) mbar_arrive_leader(&tmem_empty[acc]);
         }
+        uint8_t* st = slabs + (slab % NSLAB) * 4096;
+        ++slab;
+        if (lane == 0) tma_store_wait_read<NSLAB - 1>();
+        __syncwarp();
         if (EPI == T2_REDUCE && args.out_fp32) {
-          uint8_t* st = slabs + (slab % NSLAB) * 4096;
-          ++slab;
-          if (lane == 0) tma_store_wait_read<NSLAB - 1>();
-          __syncwarp();
           uint8_t* rowp = st + lane * 128;
 #pragma unroll
           for (int j = 0; j < 8; ++j)
@@ -340,16 +421,12 @@ gemm2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            tma_reduce_add_3d(&tmD, st, n0 + cc * 32, row0, e);  // past the tensor's extent: clipped by TMA
+            tma_reduce_add_3d(&tmD, st, n0 + cc * 32, row0, e);
             tma_store_commit();
             used_tma = true;
           }
           continue;
         }
-        uint8_t* st = slabs + (slab % NSLAB) * 4096;
-        ++slab;
-        if (lane == 0) tma_store_wait_read<NSLAB - 1>();
-        __syncwarp();
         float v[64];
 #pragma unroll
         for (int j = 0; j < 32; ++j) { v[j] = __uint_as_float(r0[j]); v[32 + j] = __uint_as_float(r1[j]); }
@@ -436,7 +513,7 @@ int t2_launch(const T2Mat& A, const T2Mat& B, const T2Mat& D, Gemm2Args& a, cuda
   const int mn_rows = T2_BK, mn_cols = 64;
   if (encode_tmap_3d(&tmA, A.p, TM_BF16, a.batch, A.rows, A.cols, A.ld, A.stride, 1, A_MN ? mn_rows : T2_BM, A_MN ? mn_cols : T2_BK, TM_SW_128)) return -3;
   if (encode_tmap_3d(&tmB, B.p, TM_BF16, a.batch, B.rows, B.cols, B.ld, B.stride, 1, B_MN ? mn_rows : T2_BN / 2, B_MN ? mn_cols : T2_BK, TM_SW_128)) return -3;
-  const bool f32 = EPI == T2_REDUCE && a.out_fp32;
+  const bool f32 = (EPI == T2_REDUCE || EPI == T2_SUM) && a.out_fp32;
   if (encode_tmap_3d(&tmD, D.p, f32 ? TM_F32 : TM_BF16, a.batch, D.rows, D.cols, D.ld, D.stride, 1, 32, f32 ? 32 : 64, TM_SW_128)) return -3;
   tmT = tmD;
   if (EPI == T2_FUSED && a.sym && encode_tmap_3d(&tmT, D.p, TM_BF16, a.batch, D.rows, D.cols, D.ld, D.stride, 1, 64, 32, TM_SW_NONE)) return -3;
@@ -475,6 +552,30 @@ PT_API int pt_gemm2cta_nt(const void* x, const void* w, void* out, int M, int N,
   Gemm2Args a = t2_args(M, N, K, 1);
   return t2_launch<false, false, T2_STORE>({x, M, K, lda, lda * M}, {w, N, K, ldb, ldb * N}, {out, M, N, ldd, ldd * M}, a,
                                            static_cast<cudaStream_t>(stream_));
+}
+
+// dy [M, N], w [N, K] -> out [M, K] bf16, reduction over N (input gradient of a dense layer). K a multiple of 8.
+PT_API int pt_gemm2cta_nn(const void* dy, const void* w, void* out, int M, int K, int N, long long lda, long long ldb,
+                          long long ldd, void* stream_) {
+  using namespace pt;
+  if (M <= 0 || N <= 0 || K <= 0 || K % 8 != 0) return -2;
+  Gemm2Args a = t2_args(M, K, N, 1);
+  return t2_launch<false, true, T2_STORE>({dy, M, N, lda, lda * M}, {w, N, K, ldb, ldb * N}, {out, M, K, ldd, ldd * M}, a,
+                                          static_cast<cudaStream_t>(stream_));
+}
+
+// dy [M, N], x [M, K] -> D [N, K] += dy^T x in fp32 or bf16 (weight gradient of a dense layer). N and K multiples of 8.
+// fp32_sums: the error of an fp32 product, at about half the rate. Launches that add to the same elements are ordered by the
+// caller, as for pt_gemm_bf16.
+PT_API int pt_gemm2cta_tn(const void* dy, const void* x, void* D, int out_fp32, int fp32_sums, int N, int K, int M, long long lda,
+                          long long ldb, long long ldd, void* stream_) {
+  using namespace pt;
+  if (M <= 0 || N <= 0 || K <= 0 || N % 8 != 0 || K % 8 != 0) return -2;
+  Gemm2Args a = t2_args(N, K, M, 1);
+  a.out_fp32 = out_fp32;
+  const T2Mat tA{dy, M, N, lda, lda * M}, tB{x, M, K, ldb, ldb * M}, tD{D, N, K, ldd, ldd * N};
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  return fp32_sums ? t2_launch<true, true, T2_SUM, 8>(tA, tB, tD, a, stream) : t2_launch<true, true, T2_REDUCE>(tA, tB, tD, a, stream);
 }
 
 // Orthogonalisation of Muon's updates: `steps` >= 1 quintic Newton-Schulz steps X <- (s_i (bA + cA^2 + aI)) X, A = X X^T, on a stack

@@ -616,6 +616,34 @@ def test_muon_update_with_fused_norm(shape, gdt, bdt):
     assert float((got - want).norm()) <= bound
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 512, 8), (255, 776, 264), (257, 1032, 520), (1024, 520, 256), (1032, 8, 1032), (1999, 520, 264), (2056, 264, 776)])
+def test_dense_products_on_cta_pairs(M, N, K):
+    """Input and weight gradients at the edges of the 256-wide tiles and of the 64-long reduction blocks, against 64 bits: one
+    rounding of the result on top of fp32 sums. The tensor core cuts each of its additions off (about n / 64 of 2^-24 a sum of n
+    terms, measured 1e-9 n); ``fp32_sums`` has to stay within what the library's fp32 product shows."""
+    from pithtrain_b200.ops import gemm as G
+    from pithtrain_b200.ops.linear import _wgrad_into
+
+    torch.manual_seed(M)
+    dy, x, w = (torch.randn(s, device="cuda").bfloat16() for s in ((M, N), (M, K), (N, K)))
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm())  # noqa: E731
+    # a rounding is at most 2^-8 of its value; the 2-norm's bound needs values enough to average over
+    assert rel(G.gemm_nn(dy, w), dy.double() @ w.double()) <= (BF16_NORM if M * K > 64 else BF16_MAX)
+    want = dy.double().t() @ x.double()
+    assert rel(G.gemm_tn(dy, x, out=torch.zeros(N, K, device="cuda"), accumulate=True), want) <= 6e-8 + 2e-9 * M
+    simt = rel(dy.float().t() @ x.float(), want)
+    got = G.gemm_tn(dy, x, out=torch.zeros(N, K, device="cuda"), accumulate=True, fp32_sums=True)
+    assert rel(got, want) <= max(simt, 1.5e-7)  # 128 rows a sum of the tensor core
+    start = torch.randn(N, K, device="cuda")
+    for target in (start.clone(), start.bfloat16()):
+        before = target.double()
+        _wgrad_into(dy, x, target)
+        sum_ = before + want
+        bound = 2e-7 + 2e-9 * M if target.dtype == torch.float32 else 2 * BF16_NORM  # the product and the sum are rounded
+        assert rel(target, sum_) <= bound
+    _native.check_status()
+
+
 @pytest.mark.parametrize("shape", [(8, 8), (3, 8, 520), (2, 520, 8), (2, 248, 264), (1, 264, 248), (3, 256, 256), (2, 512, 776), (1, 1032, 520)])
 def test_newton_schulz_products(shape):
     """Against the iteration in 64 bits, at the edges of the 256-wide tiles and of their mirrored halves. The kernels round the
