@@ -14,15 +14,19 @@
 //   DV : X1 = K           Y1 = Q, Y2 = dO    dV += P^T dO
 //   DK : X1 = K, X2 = V   Y1 = Q, Y2 = dO    dK += dS^T Q
 //   DQ : X1 = Q, X2 = dO  Y1 = K, Y2 = V     dQ += dS K
-//     S = X1 Y1^T, dP = X2 Y2^T -> TMEM (two buffers of 64 columns each); P = exp2(S c - lse2), dS = P o (dP - delta);
+//     S = X1 Y1^T, dP = X2 Y2^T -> TMEM (buffers of 64 columns each); P = exp2(S c - lse2), dS = P o (dP - delta);
 //     hi and mid go back over S's own columns in TMEM, lo over dP's, and are the A operand of the accumulating MMA (B = Y1 or
-//     Y2 read MN-major). S and dP of step n+1 are issued before the accumulation of step n, so they run under its exponentials.
+//     Y2 read MN-major). With two buffers S and dP of step n+1 run under the exponentials of step n; where one CTA leaves room for
+//     another (head dims 64 and 128) there is one buffer, and the other CTA fills the tensor core meanwhile.
 // Recomputing S twice and dP once and splitting costs 14 products of the tile instead of 5, all on the tensor core; the
-// tensor-op backward it replaces ran fp32 SIMT products over [heads, S, S] matrices in memory. Measured, causal, DQ + DK + DV
-// (with two terms):
-//   1 x 2048, 16 heads x 192/128         :  90 +  81 +  62 us  ( 83 +  75 +  55; tensor ops: about 3 ms)
-//   1 x 3072, 16/2 heads x 256           : 222 + 219 + 174 us  (201 + 199 + 155; tensor ops: about 9 ms)
-//   1 x 4093 in 9 documents, 32/4 x 128  : 147 + 169 + 150 us  (136 + 159 + 139; tensor ops: 21 ms)
+// tensor-op backward it replaces ran fp32 SIMT products over [heads, S, S] matrices in memory. Measured, causal, DQ + DK + DV, us
+// (before: two stages a streamed tile and a fixed order of the MMAs, binary searches for the row bounds, scalar fp32):
+//   1 x 2048, 16 heads x 192/128         :  68 +  70 +  54   ( 91 +  81 +  61; tensor ops: about 3 ms)
+//   1 x 3072, 16/2 heads x 256           : 202 + 210 + 145   (219 + 217 + 174; tensor ops: about 9 ms)
+//   1 x 4093 in 9 documents, 32/4 x 128  : 123 + 143 + 121   (148 + 169 + 150; tensor ops: 21 ms)
+//   1 x 3001, 32/4 x 128                 : 234 + 236 + 196   (288 + 289 + 235)
+// What is left: 28 MMAs a 64-row step at 64 cycles or more (also where N = 64 should take 32), and the split's arithmetic (without
+// it and the exponentials a step takes three quarters of its time).
 //
 // No atomics: dQ rows belong to one CTA; dK / dV of a query head are written once, directly when there is no GQA group,
 // else to per-head fp32 partials that attn_split_group_sum_kernel adds in head order. Results are reproducible.
@@ -55,24 +59,34 @@ struct AttnSplitCfg {
   static constexpr int DA = MODE == ASP_DV ? D2 : D1;     // columns of the accumulator
   static constexpr int X1_BYTES = (D1 / 64) * ASP_XSLAB, X2_BYTES = HAS_DP ? (D2 / 64) * ASP_XSLAB : 0;
   static constexpr int Y1_BYTES = (D1 / 64) * ASP_YSLAB, Y2_BYTES = (D2 / 64) * ASP_YSLAB;
-  // stages of the streamed tiles: at head dim 256 with dP (128 KB stationary) only one of Y2 fits, which is enough: its
-  // only reader is the dP product, issued a step ahead
-  static constexpr int NST1 = 2, NST2 = (HAS_DP && D1 + D2 > 320) ? 1 : 2;
-  static constexpr int STAT_BYTES = NST1 * 512;           // lse2[64] | delta[64] per Y1 stage (DV, DK)
+  // Two CTAs an SM where 256 TMEM columns hold the accumulator and one buffer of S and dP: the chain of a step (scores, softmax,
+  // split, accumulation) is then hidden by the other CTA, and so are the first loads and the last stores of a tile, which count
+  // where documents are short (8191 rows in 128 documents, 32/4 heads of 128: 149 + 180 + 162 us alone, 122 + 151 + 133 paired;
+  // one document of 3001 rows is even).
+  static constexpr bool PAIRED = D1 <= 128;
+  static constexpr int NBUF = PAIRED ? 1 : 2;             // buffers of S and dP (64 columns each)
+  static constexpr int T_DP = 64 * NBUF, T_ACC = 128 * NBUF, T_COLS = 256 * NBUF;
+  // stages of the streamed tiles: what fits. Where only one of Y2 does, its only reader is the dP product (the scores of the
+  // step run meanwhile), or a partner CTA covers the load.
+  static constexpr int NST1 = PAIRED ? (D1 == 64 ? 4 : 2) : D1 + D2 <= 320 ? 4 : (HAS_DP ? 2 : 3);
+  static constexpr int NST2 = PAIRED ? (D1 == 64 ? 3 : HAS_DP ? 1 : 2) : D1 + D2 <= 320 ? 3 : (HAS_DP ? 1 : 2);
+  // lse2[64] | delta[64] (DV, DK): with each Y1 stage, or one copy that follows the steps where two CTAs share the memory
+  static constexpr int STAT_BYTES = (PAIRED ? 1 : NST1) * 512;
   static constexpr int BAR_BYTES = 256;
   static constexpr int SMEM = X1_BYTES + X2_BYTES + NST1 * Y1_BYTES + NST2 * Y2_BYTES + STAT_BYTES + BAR_BYTES;
-  static_assert(SMEM <= 227 * 1024, "shared memory");
-  static_assert(256 + DA <= 512, "TMEM columns");
-  static constexpr int THREADS = 12 * 32;
+  static_assert(SMEM <= (PAIRED ? 113 * 1024 : 227 * 1024), "shared memory");
+  static_assert(T_ACC + DA <= T_COLS, "TMEM columns");
+  static constexpr int THREADS = 10 * 32;
 };
 
 template <int D1, int D2, int MODE>
-__global__ void __launch_bounds__(384, 1)
+__global__ void __launch_bounds__(320, (AttnSplitCfg<D1, D2, MODE>::PAIRED ? 2 : 1))
 attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
                       const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2, const AttnSplitArgs args) {
   using Cfg = AttnSplitCfg<D1, D2, MODE>;
   constexpr bool HAS_DP = Cfg::HAS_DP;
-  constexpr int DA = Cfg::DA, NST1 = Cfg::NST1, NST2 = Cfg::NST2;
+  constexpr int DA = Cfg::DA, NST1 = Cfg::NST1, NST2 = Cfg::NST2, NBUF = Cfg::NBUF;
+  constexpr bool PAIRED = Cfg::PAIRED;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if ((smem_u32(smem) & 1023u) != 0) {  // uniform over the CTA
@@ -86,14 +100,15 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   uint8_t* sStat = sY2 + NST2 * Cfg::Y2_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + Cfg::STAT_BYTES);
   uint64_t* x_full = bars;          // 1
-  uint64_t* y1_full = bars + 1;     // NST1
-  uint64_t* y1_empty = bars + 3;    // NST1
-  uint64_t* y2_full = bars + 5;     // NST2
-  uint64_t* y2_empty = bars + 7;    // NST2
-  uint64_t* s_full = bars + 9;      // 2: S (and dP) of a step are in TMEM
-  uint64_t* a_ready = bars + 11;    // 2: compute (8 warps) -> MMA: hi / mid / lo are in TMEM, dP has been read
-  uint64_t* acc_done = bars + 13;   // 1
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* y1_full = bars + 1;     // NST1 (at most 4)
+  uint64_t* y1_empty = bars + 5;    // NST1
+  uint64_t* y2_full = bars + 9;     // NST2 (at most 4)
+  uint64_t* y2_empty = bars + 13;   // NST2
+  uint64_t* s_full = bars + 17;     // 2: S (and dP) of a step are in TMEM
+  uint64_t* a_ready = bars + 19;    // 2: compute (8 warps) -> MMA: hi / mid / lo are in TMEM, dP has been read
+  uint64_t* acc_done = bars + 21;   // 1
+  uint64_t* st_full = bars + 22;    // 1: the single copy of the statistics (PAIRED)
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 23);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -121,16 +136,18 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       t_lo = need > 0 ? (need + 63) / 64 : 0;
     }
     if (args.row_lo && t_lo <= t_hi) {
-      // largest i with row_lo[first row of tile i] <= k_last
-      int a = t_lo, z = t_hi;
-      if (args.row_lo[row_base + a * 64] > k_last) {
-        t_hi = t_lo - 1;
-      } else {
-        while (a < z) {
-          const int mid = (a + z + 1) >> 1;
-          if (args.row_lo[row_base + mid * 64] <= k_last) a = mid; else z = mid - 1;
-        }
-        t_hi = a;
+      // the tiles before the first one whose first row has row_lo > k_last: 32 probes a round (each warp for itself), since a
+      // binary search is a chain of loads that nothing hides
+      int n_t = t_hi - t_lo + 1, first = t_lo;
+      t_hi = t_lo - 1;
+      while (n_t > 0) {
+        const int step = (n_t + 31) / 32;
+        const bool seen = lane * step < n_t && args.row_lo[row_base + (first + lane * step) * 64] <= k_last;
+        const int c = __popc(__ballot_sync(0xffffffffu, seen));  // the probes that are seen come first
+        if (c == 0) break;
+        t_hi = first + (c - 1) * step;
+        n_t = min(step - 1, first + n_t - 1 - t_hi);
+        first = t_hi + 1;
       }
     }
   }
@@ -162,20 +179,21 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
     for (int s = 0; s < NST2; ++s) { mbar_init(&y2_full[s], 1); mbar_init(&y2_empty[s], 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&a_ready[s], 8); }
     mbar_init(acc_done, 1);
+    mbar_init(st_full, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmX1); tma_prefetch_desc(&tmY1); tma_prefetch_desc(&tmY2);
     if (HAS_DP) tma_prefetch_desc(&tmX2);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_ptr, 512);
+    tmem_alloc(tmem_ptr, Cfg::T_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
-  const uint32_t tACC = tmem_base + 256;  // S: columns 0..127 (two buffers), dP: 128..255
+  const uint32_t tACC = tmem_base + Cfg::T_ACC;  // S: NBUF buffers of 64 columns, then dP, then the accumulator
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
@@ -188,18 +206,19 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         for (int db = 0; db < D2 / 64; ++db) tma_load_3d(sX2 + db * ASP_XSLAB, &tmX2, x_full, hx * D2 + 64 * db, x0, b);
       }
       bool ok = true;
-      int n1 = 0, n2 = 0;
+      int n1 = 0, n2 = 0, n3 = 0;
       for (int n = 0; n < N && ok; ++n) {
         const int s1 = n % NST1, s2 = n % NST2;
         const int y0 = (t_lo + n) * 64;
         ok = mbar_wait_bounded(&y1_empty[s1], ((n / NST1) & 1) ^ 1, abort_flag, args.err, PT_ERR_TIMEOUT_PRODUCER);
         if (!ok) break;
-        mbar_expect_tx(&y1_full[s1], Cfg::Y1_BYTES + (MODE == ASP_DQ ? 0 : (MODE == ASP_DK ? 512 : 256)));
+        constexpr int STATS = MODE == ASP_DQ ? 0 : (MODE == ASP_DK ? 512 : 256);
+        mbar_expect_tx(&y1_full[s1], Cfg::Y1_BYTES + (PAIRED ? 0 : STATS));
 #pragma unroll
         for (int db = 0; db < D1 / 64; ++db)
           tma_load_3d(sY1 + s1 * Cfg::Y1_BYTES + db * ASP_YSLAB, &tmY1, &y1_full[s1], hy * D1 + 64 * db, y0, b);
-        if (MODE != ASP_DQ) {
-          const long long so = ((long long)b * args.Hq + hq) * args.Sp + y0;
+        const long long so = ((long long)b * args.Hq + hq) * args.Sp + y0;
+        if (MODE != ASP_DQ && !PAIRED) {
           bulk_load_1d(sStat + s1 * 512, args.lse2 + so, 256, &y1_full[s1]);
           if (MODE == ASP_DK) bulk_load_1d(sStat + s1 * 512 + 256, args.delta + so, 256, &y1_full[s1]);
         }
@@ -211,14 +230,23 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         for (int db = 0; db < D2 / 64; ++db)
           tma_load_3d(sY2 + s2 * Cfg::Y2_BYTES + db * ASP_YSLAB, &tmY2, &y2_full[s2], hy * D2 + 64 * db, y0, b);
         ++n2;
+        if (MODE != ASP_DQ && PAIRED) {
+          // the compute warps have read the statistics of step n-1; the scores of step n come after that step's accumulation
+          if (n > 0) ok = mbar_wait_bounded(&a_ready[0], (n - 1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_PRODUCER);
+          if (!ok) break;
+          mbar_expect_tx(st_full, STATS);
+          bulk_load_1d(sStat, args.lse2 + so, 256, st_full);
+          if (MODE == ASP_DK) bulk_load_1d(sStat + 256, args.delta + so, 256, st_full);
+          ++n3;
+        }
       }
       if (*abort_flag) {
         // let copies in flight land before the CTA retires (bounded)
         const uint64_t t0 = globaltimer_ns();
         bool drained = false;
         while (!drained && globaltimer_ns() - t0 < 20000000ull) {
-          drained = mbar_try_wait(x_full, 0);
-          for (int i = 0; i < 2 && drained; ++i) {
+          drained = mbar_try_wait(x_full, 0) && (n3 == 0 || mbar_try_wait(st_full, (n3 - 1) & 1));
+          for (int i = 0; i < 4 && drained; ++i) {
             const int c1 = n1 - 1 - i, c2 = n2 - 1 - i;
             if (c1 >= 0 && i < NST1) drained = drained && mbar_try_wait(&y1_full[c1 % NST1], (c1 / NST1) & 1);
             if (c2 >= 0 && i < NST2) drained = drained && mbar_try_wait(&y2_full[c2 % NST2], (c2 / NST2) & 1);
@@ -236,62 +264,72 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       const uint32_t x1 = smem_desc_lo(smem_u32(sX1), 16), x2 = smem_desc_lo(smem_u32(sX2), 16);
       const uint32_t y1k = smem_desc_lo(smem_u32(sY1), 16), y2k = smem_desc_lo(smem_u32(sY2), 16);
       const uint32_t ym = MODE == ASP_DV ? smem_desc_lo(smem_u32(sY2), ASP_YSLAB) : smem_desc_lo(smem_u32(sY1), ASP_YSLAB);
-      // S(n) and dP(n). Buffer n & 1 was last read by the accumulation of step n-2 (issued earlier by this thread) and its dP
-      // half by the compute warps of step n-2 (their arrival was awaited before that accumulation).
-      auto scores = [&](int n) -> bool {
-        const int s1 = n % NST1, s2 = n % NST2;
-        if (!mbar_wait_bounded(&y1_full[s1], (n / NST1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_MMA)) return false;
-        tc_fence_after();
-        const uint32_t d = tmem_base + (n & 1) * 64, yb = y1k + s1 * (Cfg::Y1_BYTES >> 4);
+      // Buffer n % NBUF of S was last read by the accumulation of step n - NBUF (issued earlier by this thread), its dP half by the
+      // compute warps of that step (their arrival was awaited before the accumulation).
+      // S and dP take turns: two independent accumulators, where one alone waits for its own previous sum (N = 64: 2 to 4 %)
+      auto scores = [&](int n) {
+        const uint32_t d = tmem_base + (n % NBUF) * 64, yb = y1k + (n % NST1) * (Cfg::Y1_BYTES >> 4);
+        const uint32_t yc = y2k + (n % NST2) * (Cfg::Y2_BYTES >> 4);
 #pragma unroll
         for (int db = 0; db < D1 / 64; ++db)
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
+          for (int k = 0; k < 4; ++k) {
             umma_f16_lh(d, x1 + ((db * ASP_XSLAB + k * 32) >> 4), HI, yb + ((db * ASP_YSLAB + k * 32) >> 4), HI, IDESC_S,
                         (db | k) != 0 ? 1u : 0u);
-        if (HAS_DP) {
-          if (!mbar_wait_bounded(&y2_full[s2], (n / NST2) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_MMA)) return false;
-          tc_fence_after();
-          const uint32_t yc = y2k + s2 * (Cfg::Y2_BYTES >> 4);
-#pragma unroll
-          for (int db = 0; db < D2 / 64; ++db)
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_f16_lh(d + 128, x2 + ((db * ASP_XSLAB + k * 32) >> 4), HI, yc + ((db * ASP_YSLAB + k * 32) >> 4), HI, IDESC_S,
+            if (HAS_DP && db < D2 / 64)
+              umma_f16_lh(d + Cfg::T_DP, x2 + ((db * ASP_XSLAB + k * 32) >> 4), HI, yc + ((db * ASP_YSLAB + k * 32) >> 4), HI, IDESC_S,
                           (db | k) != 0 ? 1u : 0u);
-          umma_commit(&y2_empty[s2]);
-        }
-        umma_commit(&s_full[n & 1]);
-        return true;
+          }
+        if (HAS_DP) umma_commit(&y2_empty[n % NST2]);
+        umma_commit(&s_full[n % NBUF]);
       };
-      bool ok = mbar_wait_bounded(x_full, 0, abort_flag, args.err, PT_ERR_TIMEOUT_MMA);
-      if (ok) ok = scores(0);
-      for (int n = 0; n < N && ok; ++n) {
-        if (n + 1 < N) ok = scores(n + 1);
-        if (!ok) break;
+      auto accumulate = [&](int n) {
         const int s1 = n % NST1, s2 = n % NST2;
-        if (MODE == ASP_DV) ok = mbar_wait_bounded(&y2_full[s2], (n / NST2) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_MMA);
-        if (ok) ok = mbar_wait_bounded(&a_ready[n & 1], (n >> 1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_MMA);
-        if (!ok) break;
-        tc_fence_after();
         const uint32_t yb = ym + (MODE == ASP_DV ? s2 * (Cfg::Y2_BYTES >> 4) : s1 * (Cfg::Y1_BYTES >> 4));
-        // columns of the buffer, per half h of 32 streamed rows: hi 16 columns at 32 h, mid 16 columns at 32 h + 16; lo 16
-        // columns at 32 h of the dP buffer of the step
+        // columns of the buffer for the k-th 16 streamed rows: hi 8 columns at 16 k, mid at 16 k + 8, lo at 16 k of the dP half
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const uint32_t a = tmem_base + (n & 1) * 64 + (k >> 1) * 32 + (k & 1) * 8;
+          const uint32_t a = tmem_base + (n % NBUF) * 64 + k * 16;
           umma_f16_ts_lh(tACC, a, yb + ((k * 2048) >> 4), HI, IDESC_A, (k != 0 || n != 0) ? 1u : 0u);
-          umma_f16_ts_lh(tACC, a + 16, yb + ((k * 2048) >> 4), HI, IDESC_A, 1u);
-          umma_f16_ts_lh(tACC, a + 128, yb + ((k * 2048) >> 4), HI, IDESC_A, 1u);
+          umma_f16_ts_lh(tACC, a + 8, yb + ((k * 2048) >> 4), HI, IDESC_A, 1u);
+          umma_f16_ts_lh(tACC, a + Cfg::T_DP, yb + ((k * 2048) >> 4), HI, IDESC_A, 1u);
         }
         umma_commit(&y1_empty[s1]);
         if (MODE == ASP_DV) umma_commit(&y2_empty[s2]);
+      };
+      // Whatever is ready, the scores of the next step (at most NBUF - 1 ahead of the accumulation) first: in a fixed order
+      // a late load of step n + 1 holds up the accumulation of step n and with it the stage that the load after it waits for.
+      bool ok = mbar_wait_bounded(x_full, 0, abort_flag, args.err, PT_ERR_TIMEOUT_MMA);
+      int ns = 0, na = 0;  // steps whose scores, accumulation have been issued
+      uint32_t idle = 0;
+      uint64_t t0 = 0;
+      while (ok && na < N) {
+        if (ns < N && ns < na + NBUF && mbar_test_wait(&y1_full[ns % NST1], (ns / NST1) & 1) &&
+            (!HAS_DP || mbar_test_wait(&y2_full[ns % NST2], (ns / NST2) & 1))) {
+          tc_fence_after();
+          scores(ns++);
+          idle = 0;
+        } else if (na < ns && mbar_test_wait(&a_ready[na % NBUF], (na / NBUF) & 1) &&
+                   (MODE != ASP_DV || mbar_test_wait(&y2_full[na % NST2], (na / NST2) & 1))) {
+          tc_fence_after();
+          accumulate(na++);
+          idle = 0;
+        } else if ((++idle & 255u) == 0) {  // bounded as in mbar_wait_bounded
+          if (*abort_flag) { ok = false; break; }
+          const uint64_t now = globaltimer_ns();
+          if (idle == 256u) t0 = now;
+          if (now - t0 > PT_WAIT_LIMIT_NS) {
+            *abort_flag = 1;
+            if (args.err) atomicCAS(args.err, 0, PT_ERR_TIMEOUT_MMA);
+            ok = false;
+          }
+        }
       }
       if (ok) umma_commit(acc_done);
     }
-  } else if (warp >= 4) {
+  } else {
     // ---------------------------------------------------------------- compute: thread = stationary row, 32 streamed rows
-    const int g = (warp - 4) >> 2;            // half of the streamed rows
+    const int g = (warp - 2) >> 2;            // half of the streamed rows
     const int qd = warp & 3;                  // TMEM lane quarter
     const int r = qd * 32 + lane;
     const int xr = x0 + r;                    // my row within the batch entry: a query (DQ) or a key (DK, DV)
@@ -311,63 +349,98 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
     if (MODE != ASP_DQ && x_valid) {
       my_lo = args.causal ? xr - args.q_off : 0;
       my_hi = args.Sq - 1;
-      if (args.row_lo) {
-        int c = -1, z = my_hi;  // largest c with row_lo[c] <= xr
-        while (c < z) {
-          const int mid = (c + z + 1) >> 1;
-          if (args.row_lo[row_base + mid] <= xr) c = mid; else z = mid - 1;
-        }
-        my_hi = c;
-      }
     }
+    // DK, DV with lower bounds: those of this warp's 32 streamed rows, one a lane, loaded a step ahead
+    const bool bounds = MODE != ASP_DQ && args.row_lo != nullptr;
+    auto load_bound = [&](int n) {
+      const int y = (t_lo + n) * 64 + g * 32 + lane;
+      return bounds && n < N && y < args.Sq ? args.row_lo[row_base + y] : 0x7fffffff;
+    };
+    int bound = load_bound(0);
     bool ok = true;
     for (int n = 0; n < N; ++n) {
       const int y0 = (t_lo + n) * 64 + g * 32;
+      int hi_n = my_hi;
+      if (bounds) {
+        // streamed rows of this step that see my key: the bounds do not decrease, so they are the first c of the 32
+        int c = 0;
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1)
+          if (__shfl_sync(0xffffffffu, bound, c + w - 1) <= xr) c += w;
+        if (__shfl_sync(0xffffffffu, bound, c) <= xr) ++c;  // c <= 31 here
+        hi_n = min(my_hi, y0 + c - 1);
+        bound = load_bound(n + 1);
+      }
       int good = 1;
       if (lane == 0) {
-        good = mbar_wait_bounded(&s_full[n & 1], (n >> 1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE) ? 1 : 0;
-        // the statistics came with Y1, which the S product has already read: complete, but this thread has to observe it
+        good = mbar_wait_bounded(&s_full[n % NBUF], (n / NBUF) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE) ? 1 : 0;
+        // the statistics that came with Y1, which the S product has already read, are complete, but this thread has to observe it
         if (MODE != ASP_DQ && good)
-          good = mbar_wait_bounded(&y1_full[n % NST1], (n / NST1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE) ? 1 : 0;
+          good = (PAIRED ? mbar_wait_bounded(st_full, n & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE)
+                         : mbar_wait_bounded(&y1_full[n % NST1], (n / NST1) & 1, abort_flag, args.err, PT_ERR_TIMEOUT_EPILOGUE)) ? 1 : 0;
       }
       good = __shfl_sync(0xffffffffu, good, 0);
       if (!good) { ok = false; break; }
       tc_fence_after();
-      const uint32_t tS = tmem_base + lane_off + (n & 1) * 64 + g * 32;
-      uint32_t sv[32], dp[32];
-      tmem_ld_32x32(tS, sv);
-      if (HAS_DP) tmem_ld_32x32(tS + 128, dp);
-      tmem_ld_wait();
+      const uint32_t tS = tmem_base + lane_off + (n % NBUF) * 64 + g * 32;
       // element masks only where a lane needs them (warp-uniform: the stores below are collective)
-      const bool masked = __any_sync(0xffffffffu, y0 < my_lo || y0 + 31 > my_hi);
-      const float* st = reinterpret_cast<const float*>(sStat + (n % NST1) * 512) + g * 32;
-      uint32_t hi[16], mid[16], lo[16];
+      const bool masked = __any_sync(0xffffffffu, y0 < my_lo || y0 + 31 > hi_n);
+      const float* st = reinterpret_cast<const float*>(sStat + (PAIRED ? 0 : n % NST1) * 512) + g * 32;
+      const uint64_t scale2 = f2_pack(args.scale_log2, args.scale_log2), minus1 = f2_pack(-1.f, -1.f);
+      constexpr int CH = PAIRED ? 16 : 32;  // streamed rows at a time: two CTAs leave 96 registers a thread
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        float v[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int c = 2 * i + e;
-          const float l2 = MODE == ASP_DQ ? my_lse : st[c];
-          float p = ex2_approx(fmaf(__uint_as_float(sv[c]), args.scale_log2, -l2));
-          if (HAS_DP) p *= __uint_as_float(dp[c]) - (MODE == ASP_DQ ? my_delta : st[64 + c]);
-          if (masked) p = (y0 + c >= my_lo && y0 + c <= my_hi) ? p : 0.f;
-          v[e] = p;
+      for (int j = 0; j < 32; j += CH) {
+        uint32_t sv[CH], dp[CH];
+        if constexpr (CH == 32) {
+          tmem_ld_32x32(tS, sv);
+          if (HAS_DP) tmem_ld_32x32(tS + Cfg::T_DP, dp);
+        } else {
+          tmem_ld_32x16(tS + j, sv);
+          if (HAS_DP) tmem_ld_32x16(tS + j + Cfg::T_DP, dp);
         }
-        hi[i] = pack_bf16x2(v[0], v[1]);
-        const float2 h = unpack_bf16x2(hi[i]);
-        v[0] -= h.x; v[1] -= h.y;  // exact: what a rounding leaves fits in fewer bits
-        mid[i] = pack_bf16x2(v[0], v[1]);
-        const float2 m = unpack_bf16x2(mid[i]);
-        lo[i] = pack_bf16x2(v[0] - m.x, v[1] - m.y);
+        tmem_ld_wait();
+#pragma unroll
+        for (int h = 0; h < CH; h += 16) {
+          uint32_t hi[8], mid[8], lo[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            // two elements at a time, in packed fp32
+            const int c = h + 2 * i, r = j + c;
+            const uint64_t l2 = MODE == ASP_DQ ? f2_pack(-my_lse, -my_lse) : f2_pack(-st[r], -st[r + 1]);
+            float p0, p1;
+            f2_unpack(f2_fma(f2_pack(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), scale2, l2), p0, p1);
+            p0 = ex2_approx(p0);
+            p1 = ex2_approx(p1);
+            if (HAS_DP) {
+              const uint64_t de = MODE == ASP_DQ ? f2_pack(my_delta, my_delta) : f2_pack(st[64 + r], st[64 + r + 1]);
+              const uint64_t d = f2_fma(de, minus1, f2_pack(__uint_as_float(dp[c]), __uint_as_float(dp[c + 1])));
+              f2_unpack(f2_mul(f2_pack(p0, p1), d), p0, p1);
+            }
+            if (masked) {
+              p0 = (y0 + r >= my_lo && y0 + r <= hi_n) ? p0 : 0.f;
+              p1 = (y0 + r + 1 >= my_lo && y0 + r + 1 <= hi_n) ? p1 : 0.f;
+            }
+            // rounded, not cut off: cut-off terms all have one sign, which adds to what the tensor core cuts off (1.04e-5 for 9e-6)
+            hi[i] = pack_bf16x2(p0, p1);
+            const float2 hf = unpack_bf16x2(hi[i]);
+            float r0, r1;  // exact: what a rounding leaves fits in fewer bits
+            const uint64_t rest = f2_fma(f2_pack(hf.x, hf.y), minus1, f2_pack(p0, p1));
+            f2_unpack(rest, r0, r1);
+            mid[i] = pack_bf16x2(r0, r1);
+            const float2 mf = unpack_bf16x2(mid[i]);
+            f2_unpack(f2_fma(f2_pack(mf.x, mf.y), minus1, rest), r0, r1);
+            lo[i] = pack_bf16x2(r0, r1);
+          }
+          // over the columns just read: those 16 of S, and 8 of dP (unused columns in DV), which this warp alone reads
+          tmem_st_32x8(tS + j + h, hi);
+          tmem_st_32x8(tS + j + h + 8, mid);
+          tmem_st_32x8(tS + j + h + Cfg::T_DP, lo);
+        }
       }
-      tmem_st_32x16(tS, hi);
-      tmem_st_32x16(tS + 16, mid);
-      tmem_st_32x16(tS + 128, lo);  // over dP, which this warp alone reads and has read (unused columns in DV)
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&a_ready[n & 1]);
+      if (lane == 0) mbar_arrive(&a_ready[n % NBUF]);
     }
     if (ok) {
       int good = 1;
@@ -410,7 +483,7 @@ attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, Cfg::T_COLS);
   }
 }
 

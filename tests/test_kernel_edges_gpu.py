@@ -76,6 +76,29 @@ def test_attention_backward_split(Dqk, Dv, Hq, Hkv, B, Sq, Sk, causal, window, d
     assert _rel(got[3], want[3]) < 1e-5
 
 
+@pytest.mark.parametrize("Dqk,Dv,Hq,Hkv", [(64, 64, 2, 1), (128, 128, 2, 1), (192, 128, 1, 1), (256, 256, 1, 1)])
+@pytest.mark.parametrize("Sq,docs", [(2113, 1), (2113, 40), (4201, 300), (2305, 2304)])
+def test_attention_backward_split_finds_its_tiles(Dqk, Dv, Hq, Hkv, Sq, docs):
+    """More than 32 tiles of 64 rows, so that the search for the last tile takes two rounds of probes; documents of one row
+    upwards, many in one tile."""
+    torch.manual_seed(docs)
+    q, k = (torch.randn(1, Sq, h, Dqk, device="cuda").bfloat16() for h in (Hq, Hkv))
+    v, do = torch.randn(1, Sq, Hkv, Dv, device="cuda").bfloat16(), torch.randn(1, Sq, Hq, Dv, device="cuda").bfloat16()
+    cuts = sorted((torch.randperm(Sq - 1)[:docs - 1] + 1).tolist())
+    cu = torch.tensor([0, *cuts, Sq], dtype=torch.int32, device="cuda")
+    row_lo = N.row_lower_bounds(1, Sq, 0, None, cu, q.device)
+    out, lse = N.forward(q, k, v, Dqk ** -0.5, True, 0, row_lo, None)
+    got = N.backward_split(do, q, k, v, out, lse, Dqk ** -0.5, True, 0, row_lo)
+    _native.check_status()
+    want = _backward64(do, q, k, v, out, lse, Dqk ** -0.5, True, 0, row_lo)
+    bound = BF16_NORM + 2.0 ** -12
+    assert _rel(got[2], want[2]) < bound  # dv has no cancellation
+    for a, b in zip(got[:2], want[:2]):
+        # rows that see one key have dS = dP - delta = 0 up to the rounding of out, 2^-8 of terms of size 3 D^0.5
+        slack = BF16_MAX * 3 * Dv ** 0.5 * Dqk ** -0.5 * 4 * (a.numel() * min(1.0, 2 * docs / Sq)) ** 0.5
+        assert float((a.double() - b).norm()) < bound * float(b.norm()) + slack
+
+
 @pytest.mark.parametrize("Dqk,Dv", [(64, 64), (128, 128), (192, 128), (256, 256)])
 def test_attention_backward_split_holds_fp32_probabilities(Dqk, Dv):
     """The fp32 partials of dV for each query head, before anything is rounded to bf16. One tile of queries: 12 products of the
