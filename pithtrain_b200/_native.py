@@ -9,6 +9,9 @@ silently fall back to eager PyTorch.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
+import sys
+import types
 from ctypes import c_int, c_longlong, c_void_p, c_float
 from functools import lru_cache
 from pathlib import Path
@@ -54,6 +57,22 @@ def lib() -> ctypes.CDLL:
     L = ctypes.CDLL(str(_LIB_PATH))
     _declare(L)
     return L
+
+
+_HOST_PATH = _LIB_PATH.with_name("pith_host_ops.so")
+
+
+@lru_cache(maxsize=1)
+def host():
+    """The operators whose host side is C++ (``csrc/host_ops.cpp``), bound to the kernels of :func:`lib`."""
+    lib()
+    if not _HOST_PATH.exists():
+        raise NativeLibraryMissing(f"{_HOST_PATH} not found: run `python -m pithtrain_b200.build` (or __graft_entry__.build())")
+    spec = importlib.util.spec_from_file_location("pith_host_ops", _HOST_PATH)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    module.bind(str(_LIB_PATH))
+    return module
 
 
 SIGS = {
@@ -132,8 +151,8 @@ SIGS = {
     "pt_attn_bwd_split": "PPPPPPPPPPPPP" + "IIIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_attn_bwd": "PPPPPPPPPPPPPPP" + "IIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_gemm2cta_nt": "PPPIIILLLP",
-    "pt_gemm2cta_nn": "PPPIIILLLP",
-    "pt_gemm2cta_tn": "PPPIIIIILLLP",
+    "pt_dense_nn": "PPPIIILLLP",
+    "pt_dense_tn": "PPPIIIIILLLP",
     "pt_mla_fwd": "PPPLLLPPPPPPIIIIIIIP",
     "pt_mla_bwd": "PPPPPPPPPIIIIIIIP",
     "pt_row_bias_dot": "PPPIPPPIIP",
@@ -176,17 +195,16 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
-# Number of kernel launches issued through this module since it was last reset (bench bookkeeping).
-LAUNCHES = 0
+_launches = 0
 _LAUNCHES_PER_CALL = {"pt_route_sort": 4, "pt_attn_bwd": 3, "pt_gdr_fwd": 3, "pt_gdr_bwd": 3, "pt_merge_partial": 2}
 
 
 def check(rc: int, what: str, launches: int | None = None) -> None:
     """Raise if ``rc`` is an error; ``launches``: the kernels that this call issued, where that depends on its arguments."""
-    global LAUNCHES
+    global _launches
     if rc != 0:
         raise RuntimeError(f"{what} failed with code {rc}")
-    LAUNCHES += _LAUNCHES_PER_CALL.get(what, 1) if launches is None else launches
+    _launches += _LAUNCHES_PER_CALL.get(what, 1) if launches is None else launches
 
 
 def set_peer_wait_limit(seconds: float) -> None:
@@ -213,3 +231,19 @@ def check_status() -> None:
         raise KernelStatusError(STATUS_NAMES.get(v, f"status {v}"))
     if v < 0:
         raise RuntimeError(f"status word unavailable ({v})")
+
+
+class _Module(types.ModuleType):
+    """This module, with ``LAUNCHES``: kernels launched through it and through :func:`host` since it was last set to 0."""
+
+    @property
+    def LAUNCHES(self) -> int:
+        return _launches + (host().launches() if host.cache_info().currsize else 0)
+
+    @LAUNCHES.setter
+    def LAUNCHES(self, value: int) -> None:
+        global _launches
+        _launches = value - (host().launches() if host.cache_info().currsize else 0)
+
+
+sys.modules[__name__].__class__ = _Module

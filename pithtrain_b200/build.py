@@ -1,8 +1,9 @@
-"""Build the native sm_100a library in-tree with nvcc (no torch headers, no JIT cache).
+"""Build the native sm_100a library in-tree with nvcc (no JIT cache).
 
 Every ``csrc/*.cu`` file is compiled to an object with
 ``-gencode arch=compute_100a,code=sm_100a -lineinfo`` and linked into
-``pithtrain_b200/_lib/libpithb200.so``, which :mod:`pithtrain_b200._native` loads with ctypes.
+``pithtrain_b200/_lib/libpithb200.so``, which :mod:`pithtrain_b200._native` loads with ctypes. ``csrc/host_ops.cpp`` (the host side
+of the operators that run in every layer, with torch's headers) becomes ``_lib/pith_host_ops.so``.
 Objects are rebuilt only when their source (or a header) is newer.
 """
 
@@ -47,6 +48,19 @@ def lib_path() -> Path:
     return LIBDIR / LIBNAME
 
 
+def host_ops_command(out: Path) -> list:
+    """Compiler command of ``csrc/host_ops.cpp`` (torch's headers; no CUDA code)."""
+    import sysconfig
+
+    from torch.utils import cpp_extension
+
+    # nvcc's host compiler, not $CXX: one that links its own libstdc++ in cannot share exceptions and streams with torch's
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=pith_host_ops",
+            *(f"-I{p}" for p in cpp_extension.include_paths()), "-I/usr/local/cuda/include", f"-I{sysconfig.get_paths()['include']}",
+            str(CSRC / "host_ops.cpp"), "-o", str(out), f"-L{cpp_extension.library_paths()[0]}",
+            "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python"]
+
+
 def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False, bounds_check: bool = False) -> Path:
     """Compile and link the library; returns its path. ``bounds_check`` builds ``libpithb200_checked.so`` with
     ``-DPT_BOUNDS_CHECK`` (index validation in the kernels that address memory through device-computed indices)."""
@@ -65,6 +79,10 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False, 
                 cmd[1:1] = ["-Xptxas", "-v"]
             jobs.append((src, cmd))
 
+    host_out, host_src = LIBDIR / "pith_host_ops.so", CSRC / "host_ops.cpp"
+    if force or not host_out.exists() or host_out.stat().st_mtime < host_src.stat().st_mtime:
+        jobs.append((host_src, host_ops_command(host_out)))
+
     def run(job):
         src, cmd = job
         res = subprocess.run(cmd, capture_output=True, text=True)
@@ -79,7 +97,7 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False, 
                     raise RuntimeError(f"nvcc failed for {src}")
     out = LIBDIR / "libpithb200_checked.so" if bounds_check else lib_path()
     objs = [str(objdir / (s.stem + ".o")) for s in sources]
-    need_link = bool(jobs) or not out.exists()
+    need_link = any(src.suffix == ".cu" for src, _ in jobs) or not out.exists()
     if need_link:
         cmd = [_nvcc(), "-shared", "-o", str(out), *objs, "-lcudart_static", "-lrt", "-lpthread", "-ldl"]
         res = subprocess.run(cmd, capture_output=True, text=True)

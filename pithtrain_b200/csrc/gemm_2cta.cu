@@ -554,23 +554,36 @@ PT_API int pt_gemm2cta_nt(const void* x, const void* w, void* out, int M, int N,
                                            static_cast<cudaStream_t>(stream_));
 }
 
+extern "C" int pt_gemm_bf16(const void* A, const void* B, void* D, int mode, int M, int N, int K, int a_mn, int b_mn, long long a_rows,
+                            long long a_cols, long long lda, long long b_rows, long long b_cols, long long ldb, long long d_rows, long long ldd,
+                            const int* offs, int num_groups, int b_group_rows, long long d_group_stride, int out_fp32, int accumulate,
+                            int use_tma_store, int epi, int bn, int max_ctas, const int* a_idx, int a_idx_div, long long a_idx_len, void* stream_);
+
 // dy [M, N], w [N, K] -> out [M, K] bf16, reduction over N (input gradient of a dense layer). K a multiple of 8.
-PT_API int pt_gemm2cta_nn(const void* dy, const void* w, void* out, int M, int K, int N, long long lda, long long ldb,
-                          long long ldd, void* stream_) {
+// Reductions below 512 take the single-CTA kernel: the launch of the pair costs what its tiles save (64 and 128 columns 9 us for
+// 11, from 512 on even or behind: csrc/gemm.cu 40, here 35 at 512 rows of [5120, 2048]).
+PT_API int pt_dense_nn(const void* dy, const void* w, void* out, int M, int K, int N, long long lda, long long ldb, long long ldd,
+                       void* stream_) {
   using namespace pt;
   if (M <= 0 || N <= 0 || K <= 0 || K % 8 != 0) return -2;
+  if (N < 512)
+    return pt_gemm_bf16(dy, w, out, 0, M, K, N, 0, 1, M, N, lda, N, K, ldb, M, ldd, nullptr, 0, 0, 0, 0, 0, 1, 2, 0, 0, nullptr, 1, 0, stream_);
   Gemm2Args a = t2_args(M, K, N, 1);
   return t2_launch<false, true, T2_STORE>({dy, M, N, lda, lda * M}, {w, N, K, ldb, ldb * N}, {out, M, K, ldd, ldd * M}, a,
                                           static_cast<cudaStream_t>(stream_));
 }
 
 // dy [M, N], x [M, K] -> D [N, K] += dy^T x in fp32 or bf16 (weight gradient of a dense layer). N and K multiples of 8.
-// fp32_sums: the error of an fp32 product, at about half the rate. Launches that add to the same elements are ordered by the
-// caller, as for pt_gemm_bf16.
-PT_API int pt_gemm2cta_tn(const void* dy, const void* x, void* D, int out_fp32, int fp32_sums, int N, int K, int M, long long lda,
-                          long long ldb, long long ldd, void* stream_) {
+// fp32_sums: the error of an fp32 product, at about half the rate. Other reductions below 1024 rows take the single-CTA kernel
+// ([5120, 2048] into fp32, single / pair: 64 rows 24 / 28 us, 512 rows 31 / 32, 2048 rows 57 / 51). Launches that add to the same
+// elements are ordered by the caller, as for pt_gemm_bf16.
+PT_API int pt_dense_tn(const void* dy, const void* x, void* D, int out_fp32, int fp32_sums, int N, int K, int M, long long lda,
+                       long long ldb, long long ldd, void* stream_) {
   using namespace pt;
   if (M <= 0 || N <= 0 || K <= 0 || N % 8 != 0 || K % 8 != 0) return -2;
+  if (!fp32_sums && M < 1024)
+    return pt_gemm_bf16(dy, x, D, 0, N, K, M, 1, 1, M, N, lda, M, K, ldb, N, ldd, nullptr, 0, 0, 0, out_fp32, 1, 1, 2, 0, 0, nullptr, 1, 0,
+                        stream_);
   Gemm2Args a = t2_args(N, K, M, 1);
   a.out_fp32 = out_fp32;
   const T2Mat tA{dy, M, N, lda, lda * M}, tB{x, M, K, ldb, ldb * M}, tD{D, N, K, ldd, ldd * N};

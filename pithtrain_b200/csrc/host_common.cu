@@ -27,6 +27,18 @@ int* g_status[kMaxDevices] = {nullptr};
 int g_sms[kMaxDevices] = {0};
 std::mutex g_mu;
 
+// A thread that has made no runtime call yet (the autograd engine's, with an operator's backward as its first work) has no current
+// context, which the driver's encoder wants: bind that of the current device and try again.
+template <class Encode>
+CUresult with_context(Encode encode) {
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+  }
+  return r;
+}
+
 CUtensorMapDataType to_cu(TmDtype dt) {
   switch (dt) {
     case TM_BF16: return CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -88,9 +100,10 @@ int encode_tmap_2d(CUtensorMap* out, const void* base, TmDtype dt, uint64_t rows
   cuuint64_t strides[1] = {ld_elems * (uint64_t)elem_size(dt)};
   cuuint32_t box[2] = {box_cols, box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, to_cu(dt), 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, to_cu(sw), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = with_context([&] {
+    return fn(out, to_cu(dt), 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, to_cu(sw),
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
   if (r != CUDA_SUCCESS) {
     fprintf(stderr,
             "[pithtrain_b200] cuTensorMapEncodeTiled(2d) failed: %d base=%p rows=%llu cols=%llu "
@@ -111,9 +124,10 @@ int encode_tmap_3d(CUtensorMap* out, const void* base, TmDtype dt, uint64_t d2, 
   cuuint64_t strides[2] = {ld_elems * (uint64_t)elem_size(dt), ld2_elems * (uint64_t)elem_size(dt)};
   cuuint32_t box[3] = {box_cols, box_rows, box_d2};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(out, to_cu(dt), 3, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, to_cu(sw), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = with_context([&] {
+    return fn(out, to_cu(dt), 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, to_cu(sw),
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
   if (r != CUDA_SUCCESS) {
     fprintf(stderr, "[pithtrain_b200] cuTensorMapEncodeTiled(3d) failed: %d\n", (int)r);
     return (int)r;

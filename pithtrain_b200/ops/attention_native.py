@@ -21,11 +21,7 @@ import torch
 
 ENABLED = True
 _DIMS = {(64, 64), (128, 128), (192, 128), (256, 256)}
-# Head-dim pairs of csrc/attention_bwd.cu, for lengths that are a multiple of 4 (its row statistics move in 16-byte pieces
-# without a padded pitch): five tile products, P and dS rounded to bf16, gradients 2.3e-3 to 2.9e-3 off the 64-bit ones. All
-# other gradients came from fp32 products before they had kernels (1.7e-3, the rounding of the result) and keep that in
-# csrc/attention_bwd_split.cu with 14 tile products. 32/4 heads x 128 at 4096 / 4093 tokens: 439 / 1465 us.
-_BWD_DIMS = {(64, 64), (128, 128)}
+_BWD_DIMS = {(64, 64), (128, 128)}  # of csrc/attention_bwd.cu, for lengths that are a multiple of 4 (why: csrc/host_ops.cpp)
 _ROW_LO_CACHE: dict = {}
 
 
@@ -169,31 +165,6 @@ def backward_split(do, q, k, v, out, lse, scale: float, causal: bool, q_off: int
     return dq, dk, dv, delta[:ns].view(B, Hq, Sp)[..., :Sq]
 
 
-class _Attention(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, sinks, row_lo, scale, causal, q_off):
-        out, lse = forward(q, k, v, scale, causal, q_off, row_lo, sinks)
-        ctx.save_for_backward(q, k, v, out, lse, sinks if sinks is not None else q.new_empty(0),
-                              row_lo if row_lo is not None else q.new_empty(0))
-        ctx.has_sinks, ctx.has_lo = sinks is not None, row_lo is not None
-        ctx.scale, ctx.causal, ctx.q_off = scale, causal, q_off
-        ctx.mark_non_differentiable(lse)
-        return out, lse
-
-    @staticmethod
-    def backward(ctx, do, _dlse):
-        q, k, v, out, lse, sinks, row_lo = ctx.saved_tensors
-        sinks = sinks if ctx.has_sinks else None
-        row_lo = row_lo if ctx.has_lo else None
-        fast = (q.shape[-1], v.shape[-1]) in _BWD_DIMS and q.shape[1] % 4 == 0
-        dq, dk, dv, delta = (backward if fast else backward_split)(do, q, k, v, out, lse, ctx.scale, ctx.causal, ctx.q_off, row_lo)
-        d_sinks = None
-        if sinks is not None:
-            # d lse-normalised weight of the sink column: -exp(sink - lse) * delta, summed over batch and rows
-            d_sinks = -(torch.exp(sinks.float().view(1, -1, 1) - lse) * delta).sum((0, 2)).to(sinks.dtype)
-        return dq, dk, dv, d_sinks, None, None, None, None
-
-
 def attention(q, k, v, causal, scale, window_left, sinks, cu_seqlens, return_lse=False, q_off: Optional[int] = None):
     """Attention of ``q [B,Sq,Hq,D]`` against ``k [B,Sk,Hkv,D]``, ``v [B,Sk,Hkv,Dv]`` on the own kernels (autograd-aware).
     ``q_off`` is the position of query 0 relative to key 0 (default ``Sk - Sq``: the last query sees the last key)."""
@@ -203,7 +174,9 @@ def attention(q, k, v, causal, scale, window_left, sinks, cu_seqlens, return_lse
         q_off = Sk - Sq
     sc = float(scale) if scale is not None else q.shape[-1] ** -0.5
     row_lo = row_lower_bounds(B, Sq, q_off, window_left, cu_seqlens, q.device)
-    out, lse = _Attention.apply(q, k, v, sinks, row_lo, sc, bool(causal), int(q_off))
+    from .. import _native
+
+    out, lse = _native.host().attention(q, k, v, sinks, row_lo, sc, bool(causal), int(q_off))
     return (out, lse) if return_lse else out
 
 

@@ -63,9 +63,6 @@ def _chk2d(t: torch.Tensor, name: str):
 # projection shapes 7 to 16 % faster than the single-CTA family in all three forms (us, single / pair: [5120, 2048] 77 / 66 NT,
 # 75 / 67 NN, 91 / 82 TN into fp32; [10944, 2048] 146 / 122, 144 / 126, 151 / 134).
 USE_2CTA = True
-# Below these reduction lengths the launch of the pair costs what its tiles save: NN over 64 and 128 columns 9 / 11 us, from 512
-# on even or ahead; TN over 64 rows [5120, 2048] 24 / 28, over 512 rows 31 / 32, from 2048 rows 57 / 51.
-MIN_NN_2CTA, MIN_TN_2CTA = 512, 1024
 
 
 def _gemm2cta_nt(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
@@ -119,11 +116,11 @@ def gemm_nn(dy: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None,
     M, N = dy.shape
     K = w.shape[1]
     assert w.shape[0] == N
-    if USE_2CTA and out is None and not accumulate and out_dtype == torch.bfloat16 and K % 8 == 0 and M > 0 and N >= MIN_NN_2CTA:
+    if USE_2CTA and out is None and not accumulate and out_dtype == torch.bfloat16 and K % 8 == 0 and M > 0 and N > 0:
         out = torch.empty((M, K), dtype=torch.bfloat16, device=dy.device)
-        rc = _native.lib().pt_gemm2cta_nn(dy.data_ptr(), w.data_ptr(), out.data_ptr(), M, K, N, dy.stride(0), w.stride(0),
+        rc = _native.lib().pt_dense_nn(dy.data_ptr(), w.data_ptr(), out.data_ptr(), M, K, N, dy.stride(0), w.stride(0),
                                           out.stride(0), _native.stream_ptr())
-        _native.check(rc, "pt_gemm2cta_nn")
+        _native.check(rc, "pt_dense_nn")
         return out
     if out is None:
         out = torch.empty((M, K), dtype=out_dtype, device=dy.device)
@@ -153,10 +150,10 @@ def gemm_tn(dy: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None = None,
         assert not accumulate
         out = torch.empty((N, K), dtype=out_dtype, device=dy.device)
     assert not fp32_sums or (accumulate and N % 8 == 0 and K % 8 == 0 and out.is_contiguous())
-    if accumulate and (fp32_sums or USE_2CTA and M >= MIN_TN_2CTA) and N % 8 == 0 and K % 8 == 0 and out.is_contiguous() and out.data_ptr() % 16 == 0:
-        rc = _native.lib().pt_gemm2cta_tn(dy.data_ptr(), x.data_ptr(), out.data_ptr(), int(out.dtype == torch.float32), int(fp32_sums),
+    if accumulate and (fp32_sums or USE_2CTA) and M > 0 and N % 8 == 0 and K % 8 == 0 and out.is_contiguous() and out.data_ptr() % 16 == 0:
+        rc = _native.lib().pt_dense_tn(dy.data_ptr(), x.data_ptr(), out.data_ptr(), int(out.dtype == torch.float32), int(fp32_sums),
                                           N, K, M, dy.stride(0), x.stride(0), out.stride(0), _native.stream_ptr())
-        _native.check(rc, "pt_gemm2cta_tn")
+        _native.check(rc, "pt_dense_tn")
         return out
     _launch(dy, x, out, DENSE, N, K, M, True, True, (M, N), dy.stride(0), (M, K), x.stride(0),
             N, out.stride(0), accumulate=accumulate)

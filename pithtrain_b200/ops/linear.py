@@ -16,7 +16,7 @@ from typing import List, Optional, Sequence
 import torch
 import torch.nn as nn
 
-from .._native import on_current_device
+from .._native import host, on_current_device
 from ..dualpipe.utils import WeightGradStore
 from . import gemm as G
 from .common import accumulate_grad, grad_buffer, use_native
@@ -26,59 +26,51 @@ def _wgrad_into(dy2: torch.Tensor, x2: torch.Tensor, target: torch.Tensor) -> No
     """target[N,K] += dy2[M,N].T @ x2[M,K]."""
     M, N = dy2.shape
     if use_native(dy2) and x2.dtype == torch.bfloat16 and target.is_contiguous() and N % 8 == 0 and x2.shape[1] % 8 == 0:
-        if M % 8 == 0:
-            G.gemm_tn(dy2, x2, out=target, accumulate=True)
-            return
         # Odd row counts keep the precision of the fp32 product below, at a tenth of its time (3001 rows of the Qwen3 widths: 12 of
         # 26 ms a step went into such products).
-        if (M > 0 and dy2.is_contiguous() and x2.is_contiguous() and target.dtype in (torch.float32, torch.bfloat16)
-                and all(t.data_ptr() % 16 == 0 and on_current_device(t) for t in (dy2, x2, target))):
-            G.gemm_tn(dy2, x2, out=target, accumulate=True, fp32_sums=True)
-            return
+        if M % 8 == 0 or (dy2.is_contiguous() and x2.is_contiguous() and on_current_device(dy2) and on_current_device(x2)):
+            if (M > 0 and G.USE_2CTA and on_current_device(target) and target.dtype in (torch.float32, torch.bfloat16)
+                    and (dy2.data_ptr() | x2.data_ptr() | target.data_ptr()) % 16 == 0):
+                host().wgrad_into(dy2, x2, target, M % 8 != 0)
+                return
+            if M % 8 == 0:
+                G.gemm_tn(dy2, x2, out=target, accumulate=True)
+                return
     target.add_((dy2.float().t() @ x2.float()).to(target.dtype))
 
 
+def _queue_wgrad(dy2: torch.Tensor, x2: torch.Tensor, get_wgrad) -> None:
+    """Accumulate a weight gradient now, or hand it to the pipeline's W phase."""
+    if WeightGradStore.enabled:
+        WeightGradStore.put(lambda: _wgrad_into(dy2, x2, get_wgrad()))
+    else:
+        _wgrad_into(dy2, x2, get_wgrad())
+
+
 class _LinearFn(torch.autograd.Function):
+    """On the library's product: other devices, types and widths than the kernels take."""
+
     @staticmethod
     def forward(ctx, x, w, b, grad_targets):
         """``grad_targets`` = (weight_grad_buffer_getter, bias_param) resolved lazily at backward."""
         K = x.shape[-1]
         x2 = x.reshape(-1, K)
-        if use_native(x2) and w.dtype == torch.bfloat16 and K % 8 == 0 and w.shape[0] % 8 == 0:
-            x2 = x2.contiguous()
-            y = G.gemm_nt(x2, w)
-            if b is not None:
-                y += b
-        else:
-            y = torch.nn.functional.linear(x2, w, b)
         ctx.save_for_backward(x2, w)
         ctx.grad_targets = grad_targets
         ctx.has_bias = b is not None
         ctx.in_shape = x.shape
-        return y.view(*x.shape[:-1], w.shape[0])
+        return torch.nn.functional.linear(x2, w, b).view(*x.shape[:-1], w.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
         x2, w = ctx.saved_tensors
-        N = w.shape[0]
-        dy2 = dy.reshape(-1, N)
-        if use_native(dy2) and w.dtype == torch.bfloat16 and N % 8 == 0 and w.shape[1] % 8 == 0:
-            dy2 = dy2.contiguous()
-            dx = G.gemm_nn(dy2, w) if ctx.needs_input_grad[0] else None
-        else:
-            dx = (dy2 @ w) if ctx.needs_input_grad[0] else None
+        dy2 = dy.reshape(-1, w.shape[0])
+        dx = (dy2 @ w).view(ctx.in_shape) if ctx.needs_input_grad[0] else None
         get_wgrad, bias_param = ctx.grad_targets
-
-        def wgrad_fn(dy2=dy2, x2=x2):
-            _wgrad_into(dy2, x2, get_wgrad())
-
         if ctx.has_bias and bias_param is not None:
             accumulate_grad(bias_param, dy2.float().sum(0))
-        if WeightGradStore.enabled:
-            WeightGradStore.put(wgrad_fn)
-        else:
-            wgrad_fn()
-        return (dx.view(ctx.in_shape) if dx is not None else None), None, None, None
+        _queue_wgrad(dy2, x2, get_wgrad)
+        return dx, None, None, None
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -99,6 +91,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
 
     if fp8_linear.eligible(x, weight, fp8):
         return fp8_linear.fp8_linear_apply(x, weight, bias, (grad_getter, bias))
+    if use_native(x) and weight.dtype is torch.bfloat16 and x.shape[-1] % 8 == 0 and weight.shape[0] % 8 == 0 and weight.dim() == 2:
+        return host().linear(x, weight, bias, grad_getter, bias)
     return _LinearFn.apply(x, weight, bias, (grad_getter, bias))
 
 
@@ -199,13 +193,26 @@ class FusedWeights:
     def _in_place(self, tensors, fused) -> bool:
         if fused is None:
             return False
-        for t, view in zip(tensors, self.views(fused)):
-            if t is None or t.data_ptr() != view.data_ptr() or t.stride() != view.stride() or t.dtype != view.dtype:
+        base, size, dtype = fused.data_ptr(), fused.element_size(), fused.dtype
+        for t, (offset, stride) in zip(tensors, self._layout(fused)):
+            if t is None or t.data_ptr() != base + offset * size or t.stride() != stride or t.dtype != dtype:
                 return False
         return True
 
+    def _layout(self, fused: torch.Tensor) -> List[tuple]:
+        """(offset in elements, strides) of the parameters' views of ``fused``."""
+        out, off = [], 0
+        for p in self.params:
+            if self.layout == "rows":
+                out.append((off, fused.stride()))
+                off += p.shape[0] * fused.stride(0)
+            else:
+                out.append((off, (fused.stride(0), *fused.stride()[2:])))
+                off += fused.stride(1)
+        return out
+
     def weight(self) -> Optional[torch.Tensor]:
-        if not self._in_place([p.data for p in self.params], self.fused):
+        if not self._in_place(self.params, self.fused):
             return None
         return self.gemm_view(self.fused)
 

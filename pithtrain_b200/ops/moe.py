@@ -285,6 +285,12 @@ _PENDING_WGRAD: dict = {}
 
 def _run_expert_wgrad(ew: "ExpertWeights", k: int, a, b) -> None:
     dyg, act_s, dgu, x, slot_of_row, offs, n_rows = a
+    if b is None and use_native(dyg, x) and x.shape[1] % 8 == 0 and act_s.shape[1] % 8 == 0 and x.stride(-1) == 1:
+        g1, g2 = ew.g1(), ew.g2()
+        if (g1.is_contiguous() and g2.is_contiguous() and (g1.data_ptr() | g2.data_ptr()) % 16 == 0
+                and all(g.dtype in (torch.float32, torch.bfloat16) for g in (g1, g2))):
+            _native.host().expert_wgrads(dyg, act_s, dgu, x, slot_of_row, offs, n_rows, k, g1, g2)
+            return
     xs = gather_rows(x, slot_of_row, div=k, n_rows=n_rows)
     if b is None:
         G.grouped_gemm_tn(dyg, act_s, offs, ew.g2(), accumulate=True)
@@ -294,6 +300,29 @@ def _run_expert_wgrad(ew: "ExpertWeights", k: int, a, b) -> None:
     xs2 = gather_rows(x2, sor2, div=k, n_rows=n2)
     G.grouped_gemm_tn_pair(dyg, act_s, offs, dyg2, act2, offs2, ew.g2())
     G.grouped_gemm_tn_pair(dgu, xs, offs, dgu2, xs2, offs2, ew.g1())
+
+
+def _queue_expert_wgrad(ew: "ExpertWeights", k: int, mine) -> None:
+    """Accumulate the weight gradients of an expert block now, or hand them to the pipeline's W phase."""
+
+    def wgrad_fn():
+        if PAIR_EXPERT_WGRADS and use_native(mine[0]):
+            # an expert block is known by its down projection's storage: the owning module builds a new
+            # ExpertWeights view on every call
+            key = ew.w2.data_ptr()
+            other = _PENDING_WGRAD.pop(key, None)
+            if other is None:
+                # wait for the next micro-batch of this expert block: both share one pass over the gradients
+                _PENDING_WGRAD[key] = (ew, k, mine)
+                return
+            _run_expert_wgrad(ew, k, other[2], mine)
+        else:
+            _run_expert_wgrad(ew, k, mine, None)
+
+    if WeightGradStore.enabled:
+        WeightGradStore.put(wgrad_fn)
+    else:
+        wgrad_fn()
 
 
 def flush_pending_expert_wgrads() -> None:
@@ -403,25 +432,7 @@ class _MoEExpertsFn(torch.autograd.Function):
         d_x = combine_rows(dxs, row_of_slot, k) if ctx.needs_input_grad[0] else None
         del dxs
 
-        def wgrad_fn(dyg=dyg, act_s=act_s, dgu=dgu, x=x, slot_of_row=slot_of_row, offs=offs, n_rows=n_rows):
-            mine = (dyg, act_s, dgu, x, slot_of_row, offs, n_rows)
-            if PAIR_EXPERT_WGRADS and use_native(dyg):
-                # an expert block is known by its down projection's storage: the owning module builds a new
-                # ExpertWeights view on every call
-                key = ew.w2.data_ptr()
-                other = _PENDING_WGRAD.pop(key, None)
-                if other is None:
-                    # wait for the next micro-batch of this expert block: both share one pass over the gradients
-                    _PENDING_WGRAD[key] = (ew, k, mine)
-                    return
-                _run_expert_wgrad(ew, k, other[2], mine)
-            else:
-                _run_expert_wgrad(ew, k, mine, None)
-
-        if WeightGradStore.enabled:
-            WeightGradStore.put(wgrad_fn)
-        else:
-            wgrad_fn()
+        _queue_expert_wgrad(ew, k, (dyg, act_s, dgu, x, slot_of_row, offs, n_rows))
         return d_x, d_w, None, None, None
 
 
@@ -430,7 +441,29 @@ def moe_experts(x: torch.Tensor, w: torch.Tensor, eids: torch.Tensor, ew: Expert
     """Weighted expert outputs for received tokens: ``out[t] = sum_j w[t,j] * expert_{eids[t,j]}(x[t])``."""
     if not x.requires_grad and torch.is_grad_enabled():
         x = x.detach().requires_grad_()
-    return _MoEExpertsFn.apply(x.contiguous(), w, eids, ew, n_valid)
+    x = x.contiguous()
+    if x.is_cuda and x.data_ptr() % 16 != 0:  # rows are read in 16-byte vectors
+        x = x.clone()
+    if n_valid is None and _host_block(x, w, eids, ew):
+        n, k = eids.shape
+        E = ew.w1.shape[0]
+        return _native.host().moe_experts(x, w, eids, ew.w1, ew.w2, ALIGN, sorted_capacity(n * k, E), ew.interleaved, float(ew.alpha),
+                                          float(ew.limit), lambda *mine: _queue_expert_wgrad(ew, k, mine))
+    return _MoEExpertsFn.apply(x, w, eids, ew, n_valid)
+
+
+def _host_block(x, w, eids, ew: ExpertWeights) -> bool:
+    """Whether the whole block runs in one C++ operator (csrc/host_ops.cpp): bf16 products without biases. fp8, biases, a count of
+    valid slots (expert parallelism), no tokens and widths that a kernel refuses take :class:`_MoEExpertsFn`."""
+    from . import fp8_linear as F8
+
+    w1, w2 = ew.w1, ew.w2
+    return (use_native(x) and ew.b1 is None and ew.b2 is None and not GATHER_IN_GEMM and not F8.enabled() and eids.numel() > 0
+            and w1.dtype is torch.bfloat16 and w2.dtype is torch.bfloat16 and w1.is_contiguous() and w2.is_contiguous()
+            and x.dim() == 2 and w1.dim() == 3 and w2.dim() == 3 and x.shape[1] == w1.shape[2] == w2.shape[1] and w1.shape[1] == 2 * w2.shape[2]
+            and x.shape[1] % 64 == 0 and w1.shape[1] % 64 == 0 and w2.shape[2] % 8 == 0 and w1.shape[0] == w2.shape[0]
+            and w.is_cuda and eids.is_cuda and w.shape == eids.shape and x.shape[0] == eids.shape[0]
+            and (x.data_ptr() | w1.data_ptr() | w2.data_ptr()) % 16 == 0)
 
 
 def moe_experts_ref(x, w, eids, w1, w2, b1=None, b2=None, interleaved=False, alpha=1.0, limit=0.0):

@@ -15,7 +15,7 @@ from typing import Optional
 import torch
 
 from .. import _native
-from .common import accumulate_colsum_pair, sp, use_native
+from .common import use_native
 
 
 def rotate_half(x):
@@ -49,55 +49,6 @@ def qk_norm_rope_ref(qkv, q_w, k_w, cos, sin, Hq, Hkv, D, eps, positions=None, S
     return apply_rope_ref(q, c, s), apply_rope_ref(k, c, s), v
 
 
-class _QKNormRopeFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, qkv, q_w, k_w, cos, sin, positions, Hq, Hkv, D, eps, S, zero_centered):
-        n = qkv.shape[0]
-        dev = qkv.device
-        q = torch.empty((n, Hq, D), dtype=qkv.dtype, device=dev)
-        k = torch.empty((n, Hkv, D), dtype=qkv.dtype, device=dev)
-        has_norm = q_w is not None
-        rq = torch.empty((n, Hq), dtype=torch.float32, device=dev) if has_norm else None
-        rk = torch.empty((n, Hkv), dtype=torch.float32, device=dev) if has_norm else None
-        pos = None if positions is None else positions.int().contiguous()
-        rc = _native.lib().pt_qk_norm_rope_fwd(
-            qkv.data_ptr(), q.data_ptr(), k.data_ptr(), None if not has_norm else q_w.data_ptr(),
-            None if not has_norm else k_w.data_ptr(), cos.data_ptr(), sin.data_ptr(),
-            None if pos is None else pos.data_ptr(), None if rq is None else rq.data_ptr(),
-            None if rk is None else rk.data_ptr(), n, S, Hq, Hkv, D, qkv.stride(0), float(eps), int(zero_centered), sp())
-        _native.check(rc, "pt_qk_norm_rope_fwd")
-        v = qkv[:, (Hq + Hkv) * D:].view(n, Hkv, D)
-        ctx.save_for_backward(qkv, q_w, k_w, cos, sin, pos, rq, rk)
-        ctx.cfg = (Hq, Hkv, D, S, zero_centered)
-        ctx.qw_ref, ctx.kw_ref = q_w, k_w
-        return q, k, v
-
-    @staticmethod
-    def backward(ctx, dq, dk, dv):
-        qkv, q_w, k_w, cos, sin, pos, rq, rk = ctx.saved_tensors
-        Hq, Hkv, D, S, zc = ctx.cfg
-        n = qkv.shape[0]
-        L = _native.lib()
-        dqkv = torch.empty_like(qkv)
-        has_norm = q_w is not None
-        grid = L.pt_qk_norm_rope_bwd_grid(n, Hq, Hkv, D)
-        part = torch.empty((grid, 2 * D), dtype=torch.float32, device=qkv.device) if has_norm else None
-        dq = dq.contiguous() if dq is not None else torch.zeros((n, Hq, D), dtype=qkv.dtype, device=qkv.device)
-        dk = dk.contiguous() if dk is not None else torch.zeros((n, Hkv, D), dtype=qkv.dtype, device=qkv.device)
-        if dv is not None:
-            dv = dv.contiguous()
-            dv = dv if dv.data_ptr() % 16 == 0 else dv.clone()
-        rc = L.pt_qk_norm_rope_bwd(
-            dq.data_ptr(), dk.data_ptr(), None if dv is None else dv.data_ptr(), qkv.data_ptr(), dqkv.data_ptr(), None if not has_norm else q_w.data_ptr(),
-            None if not has_norm else k_w.data_ptr(), cos.data_ptr(), sin.data_ptr(), None if pos is None else pos.data_ptr(),
-            None if rq is None else rq.data_ptr(), None if rk is None else rk.data_ptr(),
-            None if part is None else part.data_ptr(), n, S, Hq, Hkv, D, qkv.stride(0), dqkv.stride(0), int(zc), sp())
-        _native.check(rc, "pt_qk_norm_rope_bwd")
-        if has_norm:
-            accumulate_colsum_pair(ctx.qw_ref, ctx.kw_ref, part, D)
-        return (dqkv,) + (None,) * 11
-
-
 def qk_norm_rope(qkv: torch.Tensor, q_w: Optional[torch.Tensor], k_w: Optional[torch.Tensor],
                  cos: torch.Tensor, sin: torch.Tensor, Hq: int, Hkv: int, D: int, eps: float = 1e-6,
                  positions: Optional[torch.Tensor] = None, S: Optional[int] = None, zero_centered: bool = False):
@@ -106,5 +57,5 @@ def qk_norm_rope(qkv: torch.Tensor, q_w: Optional[torch.Tensor], k_w: Optional[t
         S = qkv.shape[0]
     if (use_native(qkv) and D in (64, 128) and cos.dtype == torch.bfloat16 and cos.shape[-1] == D
             and qkv.stride(1) == 1 and (q_w is None or q_w.dtype == torch.bfloat16)):
-        return _QKNormRopeFn.apply(qkv, q_w, k_w, cos.contiguous(), sin.contiguous(), positions, Hq, Hkv, D, eps, S, zero_centered)
+        return _native.host().qk_norm_rope(qkv, q_w, k_w, cos, sin, positions, Hq, Hkv, D, eps, S, zero_centered)
     return qk_norm_rope_ref(qkv, q_w, k_w, cos, sin, Hq, Hkv, D, eps, positions, S, zero_centered)

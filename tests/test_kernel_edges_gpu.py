@@ -942,3 +942,117 @@ def test_layer_passes_refuse_other_shapes():
                 continue  # shorter tables: checked position by position
             with pytest.raises(RuntimeError):
                 mla.mla_assemble(*(bad if i == j else t for j, t in enumerate(args)), 4, 1, 128, 64, 128)
+
+
+# ------------------------------------------------------------------------------------------------
+# operators with their host side in C++
+# ------------------------------------------------------------------------------------------------
+def _host_operators():
+    """(name, function of its differentiable inputs, inputs): outputs as a tuple of differentiable tensors."""
+    from pithtrain_b200.ops.attention import attention
+    from pithtrain_b200.ops.linear import linear
+    from pithtrain_b200.ops.moe import ExpertWeights, moe_experts
+    from pithtrain_b200.ops.norm import rmsnorm
+    from pithtrain_b200.ops.rope import qk_norm_rope
+    from pithtrain_b200.ops.router import router_topk
+
+    torch.manual_seed(21)
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    w, nw, hw = torch.nn.Parameter(mk(64, 128)), torch.nn.Parameter(mk(128)), torch.nn.Parameter(mk(64))
+    cos, sin = mk(16, 64), mk(16, 64)
+    w1, w2 = mk(4, 128, 64), mk(4, 64, 64)
+    ew = ExpertWeights(w1, w2, lambda: torch.zeros(4, 128, 64, device="cuda"), lambda: torch.zeros(4, 64, 64, device="cuda"))
+    eids = torch.randint(0, 4, (9, 2), dtype=torch.int32, device="cuda")
+    return [
+        ("linear", lambda x: (linear(x, w),), (mk(9, 128),)),
+        ("rmsnorm", lambda x, r: rmsnorm(x, nw, 1e-6, r), (mk(9, 128), mk(9, 128))),
+        ("rope", lambda x: qk_norm_rope(x, hw, hw, cos, sin, 2, 1, 64, S=9), (mk(9, 256),)),
+        ("attention", lambda q, k, v: (attention(q, k, v),), (mk(1, 9, 2, 64), mk(1, 9, 1, 64), mk(1, 9, 1, 64))),
+        ("router", lambda x: router_topk(x, 2, "softmax_topk", True)[::2], (mk(9, 16).float(),)),
+        ("experts", lambda x, p: (moe_experts(x, p, eids, ew),), (mk(9, 64), torch.rand(9, 2, device="cuda"))),
+    ]
+
+
+@pytest.mark.parametrize("name", ["linear", "rmsnorm", "rope", "attention", "router", "experts"])
+def test_host_operators_in_autograd(name):
+    """Each output alone, strided and misaligned inputs and gradients, saved-tensor hooks, a changed input and transforms: as for an
+    operator written in Python."""
+    fn, inputs = next((f, i) for n, f, i in _host_operators() if n == name)
+    leaves = [t.clone().requires_grad_() for t in inputs]
+    outs = fn(*leaves)
+    grads = [torch.randn(o.shape, device="cuda").to(o.dtype) for o in outs]
+    want = torch.autograd.grad(outs, leaves, grads, retain_graph=True, allow_unused=True)
+    # one output at a time; gradients are linear in them up to the rounding of each pass
+    total = None
+    for o, g in zip(outs, grads):
+        part = [torch.zeros_like(t) if p is None else p for p, t in zip(torch.autograd.grad(o, leaves, g, retain_graph=True, allow_unused=True), leaves)]
+        total = part if total is None else [a.float() + b.float() for a, b in zip(total, part)]
+    for a, b in zip(total, want):
+        assert float((a.float() - b.float()).norm()) <= 4 * BF16_NORM * float(b.float().norm()) + 1e-6
+
+    def elsewhere(t):  # the same values, every other row (token) of a larger tensor that starts off a 16-byte boundary
+        rows = 1 if t.dim() == 4 else 0
+        shape = [2 * n if i == rows else n for i, n in enumerate(t.shape)]
+        big = torch.zeros(1 + 2 * t.numel(), dtype=t.dtype, device="cuda")[1:].view(shape)
+        part = big[:, ::2] if rows else big[::2]
+        part.copy_(t)
+        return part
+
+    moved = [elsewhere(t.detach()).requires_grad_() for t in leaves]
+    got_outs = fn(*moved)
+    got = torch.autograd.grad(got_outs, moved, [elsewhere(g) for g in grads], allow_unused=True)
+    for a, b in zip((*got_outs, *got), (*outs, *want)):
+        torch.testing.assert_close(a, b, rtol=0, atol=0 if name != "attention" else 2e-2)  # its fp32 sums come by atomics
+    saved = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (saved.append(1), t)[1], lambda t: t):
+        hooked = fn(*leaves)
+    for a, b in zip(torch.autograd.grad(hooked, leaves, grads, allow_unused=True), want):
+        torch.testing.assert_close(a, b, rtol=0, atol=0 if name != "attention" else 2e-2)
+    assert saved
+    with torch.no_grad():
+        assert not any(o.requires_grad for o in fn(*leaves))
+    if name != "router":  # keeps only what it computed
+        mine = [t.clone().requires_grad_() for t in inputs]
+        temp = [t * 1 for t in mine]
+        outs = fn(*temp)
+        with torch.no_grad():
+            temp[0 if name != "rmsnorm" else 1].add_(1)
+        if name != "rmsnorm":  # with a residual it keeps their sum
+            with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+                torch.autograd.grad(outs, mine, grads, allow_unused=True)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda *a: fn(*a))(*[torch.stack([t, t]) for t in inputs])
+    with pytest.raises(RuntimeError):
+        torch.func.jvp(lambda *a: fn(*a), tuple(inputs), tuple(torch.ones_like(t) for t in inputs))
+    _native.check_status()
+
+
+@pytest.mark.parametrize("bias", [False, True])
+def test_host_linear_defers_and_finds_its_gradients(bias):
+    """Weight gradients go to the W phase while it is on, to ``main_grad`` where a parameter has one and to ``.grad`` otherwise."""
+    from pithtrain_b200.dualpipe.utils import WeightGradStore
+    from pithtrain_b200.ops.linear import linear
+    from pithtrain_b200.ops.norm import rmsnorm
+
+    torch.manual_seed(22)
+    x = torch.randn(24, 64, device="cuda").bfloat16().requires_grad_()
+    for flat in (False, True):
+        w, b = (torch.nn.Parameter(torch.randn(s, device="cuda").bfloat16()) for s in ((32, 64), (32,)))
+        nw = torch.nn.Parameter(torch.randn(64, device="cuda").bfloat16())
+        if flat:
+            for p in (w, b, nw):
+                p.main_grad = torch.zeros(p.shape, device="cuda")
+        y = linear(rmsnorm(x, nw), w, b if bias else None)
+        WeightGradStore.enabled = True
+        try:
+            y.backward(torch.ones_like(y))
+        finally:
+            WeightGradStore.enabled = False
+        of = (lambda p: p.main_grad) if flat else (lambda p: p.grad)
+        assert of(w) is None or not of(w).any()
+        WeightGradStore.flush()
+        WeightGradStore.pop()
+        h = rmsnorm(x.detach(), nw.detach()).double()
+        assert _rel(of(w), torch.ones(32, 24, device="cuda", dtype=torch.float64) @ h) <= BF16_NORM
+        assert of(nw).any() and (not bias or _rel(of(b), torch.full((32,), 24.0, device="cuda", dtype=torch.float64)) == 0)
+    _native.check_status()
