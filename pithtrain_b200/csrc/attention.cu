@@ -70,25 +70,28 @@ struct AttnFwdCfg {
 // element pairs are evaluated by polynomial on the FMA pipe instead of the special-function unit.
 template <uint32_t POLY, int C0, int C1>
 __device__ __forceinline__ float softmax_exp_store(const uint32_t (&sv)[128], float scale_log2, float m_use, uint32_t tS) {
-  float l4[4] = {0.f, 0.f, 0.f, 0.f};
-  const float nm = -m_use;
+  // two scores an instruction where the FMA pipe works (scaling, row sum): 2227 -> 2171 us at 1 x 16384 x 32/4 heads x 128, causal,
+  // 180 -> 176 at 4096. (The same in the backward kernels, whose exponentials wait less on issue slots: 5520 -> 5600, not there.)
+  uint64_t l2[2] = {f2_pack(0.f, 0.f), f2_pack(0.f, 0.f)};
+  const uint64_t scale2 = f2_pack(scale_log2, scale_log2), nm2 = f2_pack(-m_use, -m_use);
 #pragma unroll
   for (int c = C0; c < C1; ++c) {
     uint32_t w[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const float x0 = fmaf(__uint_as_float(sv[c * 32 + 2 * i]), scale_log2, nm);
-      const float x1 = fmaf(__uint_as_float(sv[c * 32 + 2 * i + 1]), scale_log2, nm);
+      float x0, x1;
+      f2_unpack(f2_fma(f2_pack(__uint_as_float(sv[c * 32 + 2 * i]), __uint_as_float(sv[c * 32 + 2 * i + 1])), scale2, nm2), x0, x1);
       // POLY bit (2i mod 8) / (2i+1 mod 8): which elements of every 8 go to the FMA pipe
       const float e0 = (POLY & (1u << ((2 * i) & 7))) ? exp2_poly(x0) : ex2_approx(x0);
       const float e1 = (POLY & (1u << ((2 * i + 1) & 7))) ? exp2_poly(x1) : ex2_approx(x1);
-      l4[(2 * i) & 3] += e0;
-      l4[(2 * i + 1) & 3] += e1;
+      l2[i & 1] = f2_add(l2[i & 1], f2_pack(e0, e1));
       w[i] = pack_bf16x2(e0, e1);
     }
     tmem_st_32x16(tS + c * 16, w);
   }
-  return (l4[0] + l4[1]) + (l4[2] + l4[3]);
+  float a, b;
+  f2_unpack(f2_add(l2[0], l2[1]), a, b);
+  return a + b;
 }
 
 template <int DQK, int DV, int NQ, int KST>
