@@ -196,7 +196,7 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 _launches = 0
-_LAUNCHES_PER_CALL = {"pt_route_sort": 4, "pt_attn_bwd": 3, "pt_gdr_fwd": 3, "pt_gdr_bwd": 3, "pt_merge_partial": 2}
+_LAUNCHES_PER_CALL = {"pt_attn_bwd": 3, "pt_gdr_fwd": 3, "pt_gdr_bwd": 3, "pt_merge_partial": 2}
 
 
 def check(rc: int, what: str, launches: int | None = None) -> None:

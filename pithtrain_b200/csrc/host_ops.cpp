@@ -683,13 +683,13 @@ Tensor moe_experts(const Tensor& x, const Tensor& w, const Tensor& eids, const T
     check_aligned(w1, "w1");
     check_aligned(w2, "w2");
     const Tensor flat = eids.to(at::kInt).contiguous();
-    const Tensor counts = empty({((slots + 511) / 512 + 1) * E}, flat, at::kInt);  // workspace of the chunked sort
+    const Tensor counts = E > 1024 ? empty({E}, flat, at::kInt) : Tensor();  // scratch of the sort beyond that many experts
     offs = empty({E + 1}, flat, at::kInt);
     row_of_slot = empty({slots}, flat, at::kInt);
     slot_of_row = empty({r_cap}, flat, at::kInt);
-    check(api.pt_route_sort(ptr(flat), nullptr, slots, E, align, ptr(counts), counts.numel(), ptr(offs), ptr(row_of_slot), ptr(slot_of_row), r_cap,
+    check(api.pt_route_sort(ptr(flat), nullptr, slots, E, align, ptr(counts), E, ptr(offs), ptr(row_of_slot), ptr(slot_of_row), r_cap,
                             current_stream()),
-          "pt_route_sort", 4);
+          "pt_route_sort", E > 1024 ? 3 : 1);
     const Tensor n_rows = offs.narrow(0, E, 1);
     gu = grouped(gather(x, slot_of_row, k, n_rows), w1, offs, false);
     const int64_t inter = gu.size(1) / 2;

@@ -85,15 +85,14 @@ def route_sort(eids: torch.Tensor, num_experts: int, r_cap: Optional[int] = None
     flat = flat.int() if flat.dtype != torch.int32 else flat
     flat = flat.contiguous()
     dev = flat.device
-    chunks = (n + 511) // 512
-    counts = torch.empty((chunks + 1) * num_experts, dtype=torch.int32, device=dev)  # workspace of the chunked sort
+    counts = torch.empty(num_experts, dtype=torch.int32, device=dev) if num_experts > 1024 else None  # scratch of the per-expert sort
     offs = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)
     row_of_slot = torch.empty(n, dtype=torch.int32, device=dev)
     slot_of_row = torch.empty(r_cap, dtype=torch.int32, device=dev)
     rc = L.pt_route_sort(flat.data_ptr(), None if n_valid is None else n_valid.data_ptr(), n, num_experts,
-                         ALIGN, counts.data_ptr(), counts.numel(), offs.data_ptr(), row_of_slot.data_ptr(),
+                         ALIGN, _native.ptr(counts), num_experts, offs.data_ptr(), row_of_slot.data_ptr(),
                          slot_of_row.data_ptr(), r_cap, sp())
-    _native.check(rc, "pt_route_sort")
+    _native.check(rc, "pt_route_sort", launches=1 if counts is None else 3)
     return offs, row_of_slot, slot_of_row
 
 

@@ -1056,3 +1056,29 @@ def test_host_linear_defers_and_finds_its_gradients(bias):
         assert _rel(of(w), torch.ones(32, 24, device="cuda", dtype=torch.float64) @ h) <= BF16_NORM
         assert of(nw).any() and (not bias or _rel(of(b), torch.full((32,), 24.0, device="cuda", dtype=torch.float64)) == 0)
     _native.check_status()
+
+
+@pytest.mark.parametrize("slots,E,valid", [(0, 4, None), (1, 1, None), (31, 33, None), (8191, 3, 5000), (8193, 256, None), (70001, 1024, 69000), (300000, 129, None), (64, 1025, None)])
+def test_route_sort_runs_and_capacity(slots, E, valid):
+    """At the edges of the warps' runs (32 slots and up) and of the experts a thread scans; slots without an expert; too few rows."""
+    from pithtrain_b200.ops import moe as M
+
+    torch.manual_seed(slots)
+    eids = torch.randint(-1, E + 1, (slots,), dtype=torch.int32, device="cuda")
+    if E > 2:
+        eids[torch.rand(slots, device="cuda") < 0.5] = 1  # one expert takes most
+    nv = None if valid is None else torch.tensor([valid], dtype=torch.int32, device="cuda")
+    cap = M.sorted_capacity(slots, E)
+    got = M.route_sort(eids, E, cap, nv)
+    _native.check_status()
+    want_in = eids.cpu().clone()
+    if valid is not None:
+        want_in[valid:] = -1
+    for a, b in zip(got, M.route_sort_ref(want_in, E, cap)):
+        assert torch.equal(a.cpu(), b)
+    rows = int(got[0][-1])
+    if rows and E <= 1024:
+        offs, row_of_slot, slot_of_row = M.route_sort(eids, E, rows - 1, nv)
+        with pytest.raises(_native.KernelStatusError):
+            _native.check_status()
+        assert torch.equal(offs, got[0]) and bool((row_of_slot == -1).all()) and bool((slot_of_row == -1).all())
