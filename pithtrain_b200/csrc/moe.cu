@@ -308,86 +308,116 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict_
 
 // ----------------------------------------------------------------------------------------------
 // combine: out[t] = (res ? res[t] : 0) + sum_{j<k, row>=0} (w ? w[t,j] : 1) * y[row_of_slot[t*k+j]]
-// One warp per token; fp32 accumulation; k rows gathered per token.
+// fp32 accumulation in slot order. Bound by the bytes of the rows, if enough of them are on their way: a row is contiguous, so
+// one warp of the block fetches rows by bulk copies into a ring in shared memory, four rows of a token to a stage, a lane to a
+// row; the other warps add them up, a thread 8 columns wide. Rows in flight then cost shared memory and no registers. A block
+// has a run of tokens that follow one another, so that a load of 32 indices is several tokens' worth and is asked for one load
+// ahead. Tokens of more than CB_COLS columns are walked in slices of equal width, one after the other.
 // ----------------------------------------------------------------------------------------------
-// One warp per token, one row at a time: the better one where there are tokens for the warps of the chip (see pt_combine).
-__global__ void __launch_bounds__(256)
-combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_slot,
-               const float* __restrict__ w, const __nv_bfloat16* __restrict__ res,
-               __nv_bfloat16* __restrict__ out, const int* __restrict__ n_ptr, int n_max, int k,
-               int H) {
-  const int n = n_ptr ? min(*n_ptr, n_max) : n_max;
-  const int lane = threadIdx.x & 31;
-  const int wpb = blockDim.x >> 5;
-  for (int t = blockIdx.x * wpb + (threadIdx.x >> 5); t < n; t += gridDim.x * wpb) {
-    for (int c0 = lane * 8; c0 < H; c0 += 256) {
-      float acc[8];
-      if (res) load8(res + (size_t)t * H + c0, acc);
-      else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-      }
-      for (int j = 0; j < k; ++j) {
-        int r = row_of_slot[(size_t)t * k + j];
-        if (r < 0) continue;
-        float wt = w ? w[(size_t)t * k + j] : 1.f;
-        float v[8];
-        load8(y + (size_t)r * H + c0, v);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] += wt * v[e];
-      }
-      store8(out + (size_t)t * H + c0, acc);
-    }
-  }
-}
+constexpr int CB_ROWS = 4, CB_STAGES = 8, CB_COLS = 4096;
 
-// Fewer tokens than that are a latency problem: k random rows each. One thread per 8 columns of a token, so that at 64
-// tokens of 2048 columns 512 warps ask for rows instead of 64, and the k row loads of a thread are independent: indices and
-// weights first, then four rows in flight at a time, added in slot order (the same sums as above).
-__global__ void __launch_bounds__(256)
-combine_wide_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_slot,
-               const float* __restrict__ w, const __nv_bfloat16* __restrict__ res,
-               __nv_bfloat16* __restrict__ out, const int* __restrict__ n_ptr, int n_max, int k,
-               int H) {
+__global__ void __launch_bounds__(CB_COLS / 8 + 32)
+combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_slot, const float* __restrict__ w,
+               const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ out, const int* __restrict__ n_ptr, int n_max,
+               int k, int H, int slices, int W, int stages, int* __restrict__ err) {
+  extern __shared__ __align__(128) uint8_t ring[];
+  __shared__ uint64_t full[CB_STAGES], empty[CB_STAGES];
+  __shared__ float weight_of[CB_STAGES][CB_ROWS];
+  __shared__ int present[CB_STAGES][CB_ROWS];
+  __shared__ int abort_flag;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, adders = (blockDim.x >> 5) - 1;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], adders); }
+    abort_flag = 0;
+    mbar_fence_init();
+  }
+  __syncthreads();
   const int n = n_ptr ? min(*n_ptr, n_max) : n_max;
-  const int vec = H / 8;
-  const long long total = (long long)n * vec;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int t = (int)(i / vec), c0 = (int)(i - (long long)t * vec) * 8;
-    const int* rows = row_of_slot + (size_t)t * k;
-    const float* wt = w ? w + (size_t)t * k : nullptr;
-    float acc[8];
-    if (res) load8(res + (size_t)t * H + c0, acc);
-    else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-    }
-    int j = 0;
-    for (; j + 4 <= k; j += 4) {
-      int r[4];
-      float f[4], v[4][8];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) { r[u] = rows[j + u]; f[u] = wt ? wt[j + u] : 1.f; }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (r[u] >= 0) load8(y + (size_t)r[u] * H + c0, v[u]);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (r[u] < 0) continue;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] += f[u] * v[u][e];
+  const long long items = (long long)n * slices;
+  const size_t row_bytes = (size_t)W * 2;
+  int stage = 0;
+  uint32_t phase = 0;
+  const long long first = items * blockIdx.x / gridDim.x, last = items * (blockIdx.x + 1) / gridDim.x;
+  if (warp == adders) {
+    int id = -1, next_id = -1;  // slots base + lane, base + 32 + lane
+    float f = 1.f, next_f = 1.f;
+    const long long slots = (long long)n * k;
+    long long base = 0, armed = 0;
+    auto fetch = [&](long long slot, int& i, float& v) {
+      i = slot < slots ? row_of_slot[slot] : -1;
+      v = slot < slots && w ? w[slot] : 1.f;
+    };
+    bool ok = true;
+    for (long long item = first; ok && item < last; ++item) {
+      const int s = (int)(item / n), c0 = s * W;
+      const long long t = item - (long long)s * n;
+      const uint32_t bytes = (uint32_t)min(W, H - c0) * 2;
+      if (item == first || t == 0) {
+        base = t * k;
+        fetch(base + lane, id, f);
+        fetch(base + 32 + lane, next_id, next_f);
+      }
+      for (int j0 = 0; j0 < k; j0 += CB_ROWS) {
+        if (t * k + j0 - base >= 32) {
+          base += 32;
+          id = next_id;
+          f = next_f;
+          fetch(base + 32 + lane, next_id, next_f);
+        }
+        ok = mbar_wait_bounded_warp(&empty[stage], phase ^ 1, &abort_flag, err, PT_ERR_TIMEOUT_PRODUCER);
+        if (!ok) break;
+        const int at = (int)(t * k + j0 - base) + lane;  // below 64 in the lanes that count
+        const int near = __shfl_sync(0xffffffffu, id, at & 31), far = __shfl_sync(0xffffffffu, next_id, at & 31);
+        const float near_f = __shfl_sync(0xffffffffu, f, at & 31), far_f = __shfl_sync(0xffffffffu, next_f, at & 31);
+        const int row = lane >= min(CB_ROWS, k - j0) ? -1 : at < 32 ? near : far;
+        if (lane < CB_ROWS) {
+          weight_of[stage][lane] = at < 32 ? near_f : far_f;
+          present[stage][lane] = row >= 0;
+        }
+        const uint32_t rows = __popc(__ballot_sync(0xffffffffu, row >= 0));
+        __syncwarp();
+        if (lane == 0) mbar_expect_tx(&full[stage], rows * bytes);
+        __syncwarp();
+        if (row >= 0) bulk_load_1d(ring + (stage * CB_ROWS + lane) * row_bytes, y + (size_t)row * H + c0, bytes, &full[stage]);
+        ++armed;
+        if (++stage == stages) { stage = 0; phase ^= 1; }
       }
     }
-    for (; j < k; ++j) {
-      const int r = rows[j];
-      if (r < 0) continue;
-      const float f = wt ? wt[j] : 1.f;
-      float v[8];
-      load8(y + (size_t)r * H + c0, v);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] += f * v[e];
+    if (!ok) {  // the copies that are still on their way end before the block does
+      for (int back = 0; back < stages && back < armed; ++back) {
+        if (--stage < 0) { stage = stages - 1; phase ^= 1; }
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try_wait(&full[stage], phase) && globaltimer_ns() - t0 < PT_WAIT_LIMIT_NS) {}
+      }
     }
-    store8(out + (size_t)t * H + c0, acc);
+    return;
+  }
+  const int c = threadIdx.x * 8;
+  for (long long item = first; item < last; ++item) {
+    const int s = (int)(item / n), c0 = s * W;
+    const long long t = item - (long long)s * n;
+    const bool in = c < min(W, H - c0);
+    const size_t at = (size_t)t * H + c0 + c;
+    float acc[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+    if (res && in) load8(res + at, acc);
+    for (int j0 = 0; j0 < k; j0 += CB_ROWS) {
+      if (!mbar_wait_bounded(&full[stage], phase, &abort_flag, err, PT_ERR_TIMEOUT_EPILOGUE)) return;
+#pragma unroll
+      for (int u = 0; u < CB_ROWS; ++u) {
+        if (!in || !present[stage][u]) continue;
+        const float f = weight_of[stage][u];
+        float v[8];
+        load8(reinterpret_cast<const __nv_bfloat16*>(ring + (stage * CB_ROWS + u) * row_bytes) + c, v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += f * v[e];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[stage]);
+      if (++stage == stages) { stage = 0; phase ^= 1; }
+    }
+    if (in) store8(out + at, acc);
   }
 }
 
@@ -894,21 +924,28 @@ PT_API int pt_combine(const void* y, const int* row_of_slot, const float* w, con
   cudaStream_t st = (cudaStream_t)stream_;
   if (n_max <= 0) return 0;
   if (H % 8 != 0) return -1;
-  // A warp walks its token's k rows one after the other, so up to some 3000 tokens (20 warps an SM) its kernel takes the time of
-  // one such chain whatever the size; from there on it keeps memory busy with fewer requests in flight than the wide one. The line
-  // is the same at every width and k. Measured, cold cache, wide / warp per token, us:
-  //   columns x k       64 tokens   1024      2048      3072      4096      8192
-  //   2048 x 8          12 / 45     25 / 48   39 / 53   53 / 55   68 / 57   121 / 100
-  //   2048 x 4           9 / 27     16 / 29   25 / 31   33 / 33   43 / 35    76 / 60
-  //   2880 x 4          10 / 37     21 / 39   33 / 41   45 / 45   59 / 49   102 / 84
-  //    512 x 8          11 / 16     12 / 18   18 / 18   18 / 18   25 / 21    39 / 33
-  const long long vecs = (long long)n_max * (H / 8);
-  if (n_max <= 3072)
-    combine_wide_kernel<<<grid_for(vecs, 256, 64), 256, 0, st>>>((const __nv_bfloat16*)y, row_of_slot, w,
-        (const __nv_bfloat16*)res, (__nv_bfloat16*)out, n_ptr, n_max, k, H);
-  else
-    combine_kernel<<<grid_for(n_max, 8, 16), 256, 0, st>>>((const __nv_bfloat16*)y, row_of_slot, w,
-        (const __nv_bfloat16*)res, (__nv_bfloat16*)out, n_ptr, n_max, k, H);
+  const int pieces = H / 8, W = (pieces + (pieces + 511) / 512 - 1) / ((pieces + 511) / 512) * 8, slices = (H + W - 1) / W;
+  const int adders = (W / 8 + 31) / 32;
+  // Some sixteen adding warps an SM, in two to sixteen blocks, share 200 KB of rings: 3 to 8 stages each. Rows wider than the 2048
+  // columns of eight warps are better left whole (two blocks of twelve warps and 4 stages for 2880 columns: 70 us for 12288 tokens
+  // of 4, as two slices of six warps 84). Measured, cold cache, us; before: one thread for 8 columns of a token with four loads in
+  // flight up to 3072 tokens, one warp a token above that:
+  //   columns x k       64 tokens   1024      2048      3072      4096      8192      12288
+  //   2048 x 8          12 -> 10    25 -> 16  39 -> 23  51 -> 31  57 -> 37  100 -> 61 109 -> 88
+  //   2048 x 4           9 -> 8     16 -> 12  25 -> 16  33 -> 21  34 -> 25  59 -> 38   66 -> 51
+  //   2880 x 4          10 -> 8     21 -> 14  33 -> 20  45 -> 25  47 -> 30  84 -> 49   90 -> 70
+  //    512 x 8          11 -> 8     12 -> 10  17 -> 13  18 -> 15  19 -> 16  33 -> 23   37 -> 31
+  const int blocks = adders > 8 ? 2 : 16 / adders;
+  const int stage_bytes = CB_ROWS * W * 2, room = 200 * 1024 / blocks / stage_bytes, stages = room < CB_STAGES ? room : CB_STAGES;
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  combine_kernel<<<grid_for((long long)n_max * slices, 1, blocks), adders * 32 + 32, stages * stage_bytes, st>>>(
+      (const __nv_bfloat16*)y, row_of_slot, w, (const __nv_bfloat16*)res, (__nv_bfloat16*)out, n_ptr, n_max, k, H, slices, W, stages,
+      device_status_word());
   return (int)cudaGetLastError();
 }
 

@@ -460,6 +460,29 @@ def test_combine_rows(n, H, k):
         assert ((got.double() - want).abs() <= BF16_MAX * want.abs() + 2.0 ** -20 * (k + 1) * 5).all()
 
 
+@pytest.mark.parametrize("n,H,k", [(37, 2056, 5), (300, 2880, 4), (40, 4104, 8), (3, 12296, 2), (700, 64, 40), (2500, 256, 33), (65, 72, 16)])
+def test_combine_rows_runs_and_slices(n, H, k):
+    """Rows wider than one block's columns, runs of tokens past several loads of 32 indices, tokens of more slots than one load, and
+    tokens without a row; an absent row is skipped, not multiplied: infinities next to it stay out."""
+    from pithtrain_b200.ops.moe import combine_rows
+
+    torch.manual_seed(n)
+    y = torch.randn(2 * n, H, device="cuda").bfloat16()
+    y[0] = float("inf")
+    rows = torch.randint(1, 2 * n, (n, k), device="cuda", dtype=torch.int32)
+    rows[torch.rand(n, k, device="cuda") < 0.3] = -1
+    rows[:: 5] = -1
+    w = torch.rand(n, k, device="cuda")
+    w[rows < 0] = float("nan")
+    got = combine_rows(y, rows.reshape(-1), k, w).double()
+    want = torch.zeros(n, H, device="cuda", dtype=torch.double)
+    for j in range(k):
+        want += torch.where(rows[:, j : j + 1] >= 0, y[rows[:, j].long().clamp(min=0)].double() * w[:, j : j + 1].double(), 0.0)
+    # fp32 sums of k terms below 5, one bf16 rounding
+    assert ((got - want).abs() <= BF16_MAX * want.abs() + 2.0 ** -24 * k * k * 5).all()
+    assert (got[::5] == 0).all()
+
+
 @pytest.mark.parametrize("pair", [False, True])
 @pytest.mark.parametrize("sizes,N,K", [([16], 8, 8), ([0, 16, 80], 136, 40), ([48, 0, 0, 64], 264, 296), ([32] * 40, 392, 776)])
 def test_grouped_weight_gradient_into_fp32(sizes, N, K, pair):
