@@ -4,75 +4,125 @@
 // kernel (pithtrain/operators/cross_entropy.py:15-125).
 #include "elementwise.cuh"
 #include "host_common.h"
+#include "ptx.cuh"
 
 namespace pt {
 
-constexpr int CE_THREADS = 1024;
+// Exponentials are 2^(v log2(e) - c): one fused multiply-add and one instruction of the special function unit each, so that the
+// two passes over a row (39 M logits: 17 us of that unit) fit beside its read and write. c = max * log2(e) is the same rounded
+// number in every term of the sum and in lse2 = c + log2(sum), so its rounding cancels in the gradient; the loss takes it out.
+constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 
-__global__ void __launch_bounds__(CE_THREADS)
-cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels,
-                     float* __restrict__ loss, int n, int V, long long ld, int ignore_index) {
+__device__ __forceinline__ float max8(const uint4& v) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+  const __nv_bfloat162 a = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
+  return fmaxf(__low2float(a), __high2float(a));
+}
+__device__ __forceinline__ void exp8(const uint4& v, float c, float (&e)[8]) {
+  const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 p = unpack_bf16x2(q[i]);
+    e[2 * i] = ex2_approx(fmaf(p.x, LOG2E, -c));
+    e[2 * i + 1] = ex2_approx(fmaf(p.y, LOG2E, -c));
+  }
+}
+__device__ __forceinline__ void minus_one_at(float (&e)[8], int c, long long label) {
+  if (c != label >> 3) return;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (i == (label & 7)) e[i] -= 1.f;
+}
+// Stops the compiler from carrying a vector's fp32 form from one pass to the next.
+__device__ __forceinline__ void keep_packed(uint4& v) { asm volatile("" : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)); }
+
+// A block of T threads to a row. NV > 0: the row is held in registers, NV vectors of 8 columns a thread. NV = 0: it is read
+// twice, the first time with a running maximum. The reductions of a row leave its warps idle, so small blocks beat wide ones as
+// long as all rows of an SM have 1536 threads or more; with 8 vectors a thread (55 us for 9496 columns, 150 for 32000) they have
+// too few, and a ring of rows in shared memory (50 us) pays for its waits.
+template <int T, int NV>
+__global__ void __launch_bounds__(T, (NV > 2 ? 1536 : 2048) / T)
+cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels, float* __restrict__ loss, int V,
+                     long long ld, int ignore_index) {
   __shared__ float red[32];
-  const int row = blockIdx.x;
-  if (row >= n) return;
+  const int row = blockIdx.x, tid = threadIdx.x, nvec = V / 8;
   __nv_bfloat16* x = logits + (size_t)row * ld;
+  uint4* xv = reinterpret_cast<uint4*>(x);
   const long long label = labels[row];
-  const int nvec = V / 8;
+  const int rest = nvec * 8 + tid;  // a column past the last whole vector, in the first V % 8 threads
   if (label == ignore_index) {
-    for (int c = threadIdx.x; c < nvec; c += CE_THREADS) *reinterpret_cast<uint4*>(x + c * 8) = make_uint4(0, 0, 0, 0);
-    for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) x[c] = __float2bfloat16(0.f);
-    if (threadIdx.x == 0) loss[row] = 0.f;
+    for (int c = tid; c < nvec; c += T) xv[c] = make_uint4(0, 0, 0, 0);
+    if (rest < V) x[rest] = __float2bfloat16(0.f);
+    if (tid == 0) loss[row] = 0.f;
     return;
   }
-  // pass 1: online max / sum-exp
-  float m = -INFINITY, s = 0.f;
-  for (int c = threadIdx.x; c < nvec; c += CE_THREADS) {
-    float v[8];
-    load8(x + c * 8, v);
-    float lm = v[0];
+  const float last = rest < V ? __bfloat162float(x[rest]) : -INFINITY;
+  const float xl = tid == 0 ? __bfloat162float(x[label]) : 0.f;
+  uint4 raw[NV > 0 ? NV : 1];
+  float m = last, s = 0.f, gm, shift;  // shift: c of the block
+  if (NV > 0) {
 #pragma unroll
-    for (int e = 1; e < 8; ++e) lm = fmaxf(lm, v[e]);
-    float nm = fmaxf(m, lm);
-    float acc = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc += __expf(v[e] - nm);
-    s = s * __expf(m - nm) + acc;
-    m = nm;
-  }
-  for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) {
-    float v = __bfloat162float(x[c]);
-    float nm = fmaxf(m, v);
-    s = s * __expf(m - nm) + __expf(v - nm);
-    m = nm;
-  }
-  float gm = block_max(m, red);
-  s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
-  float gs = block_sum(s, red);
-  float lse = gm + __logf(gs);
-  float xl = __bfloat162float(x[label]);
-  __syncthreads();  // everyone has read x[label] before it is overwritten
-  if (threadIdx.x == 0) loss[row] = lse - xl;
-  // pass 2: gradient in place
-  for (int c = threadIdx.x; c < nvec; c += CE_THREADS) {
-    float v[8];
-    load8(x + c * 8, v);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      v[e] = __expf(v[e] - lse);
-      if (c * 8 + e == label) v[e] -= 1.f;
+    for (int i = 0; i < NV; ++i) {
+      const int c = tid + i * T;
+      raw[i] = c < nvec ? xv[c] : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);  // -inf
     }
-    store8(x + c * 8, v);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) m = fmaxf(m, max8(raw[i]));
+    gm = block_max(m, red);
+    shift = __fmul_rn(gm, LOG2E);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      keep_packed(raw[i]);
+      float e[8];
+      exp8(raw[i], shift, e);
+      s += ((e[0] + e[1]) + (e[2] + e[3])) + ((e[4] + e[5]) + (e[6] + e[7]));
+    }
+  } else {
+    shift = -INFINITY;
+#pragma unroll 4
+    for (int c = tid; c < nvec; c += T) {
+      const uint4 v = xv[c];
+      const float up = fmaxf(m, max8(v)), scaled = __fmul_rn(up, LOG2E), c_up = up == -INFINITY ? 0.f : scaled;
+      float e[8];
+      exp8(v, c_up, e);
+      s = s * ex2_approx(shift - c_up) + (((e[0] + e[1]) + (e[2] + e[3])) + ((e[4] + e[5]) + (e[6] + e[7])));
+      m = up;
+      shift = scaled;
+    }
+    gm = block_max(m, red);
+    const float own = shift;
+    shift = __fmul_rn(gm, LOG2E);
+    if (m != gm) s *= ex2_approx(own - shift);
   }
-  for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) {
-    float v = __expf(__bfloat162float(x[c]) - lse);
-    if (c == label) v -= 1.f;
-    x[c] = __float2bfloat16(v);
+  s += ex2_approx(fmaf(last, LOG2E, -shift));
+  const float gs = block_sum(gm == -INFINITY ? 0.f : s, red);
+  // x[label] was read ahead of the barriers above, it is written after them. The logarithm of the loss is taken in 64 bits: the fast one
+  // is off by 3e-7 on average.
+  const float lse2 = shift + __log2f(gs);
+  auto gradient = [&](const uint4& v, int c) {
+    float e[8];
+    exp8(v, lse2, e);
+    minus_one_at(e, c, label);
+    store8(x + c * 8, e);
+  };
+  if (NV > 0) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      keep_packed(raw[i]);
+      if (tid + i * T < nvec) gradient(raw[i], tid + i * T);
+    }
+  } else {
+#pragma unroll 4
+    for (int c = tid; c < nvec; c += T) gradient(xv[c], c);
   }
+  if (rest < V) x[rest] = __float2bfloat16(ex2_approx(fmaf(last, LOG2E, -lse2)) - (rest == label ? 1.f : 0.f));
+  if (tid == 0) loss[row] = (float)((double)gm - xl + (log((double)gs) - fmaf(gm, LOG2E, -shift) * LN2));
 }
 
 // x *= s[0] over a flat bf16 buffer (s on the device).
 __global__ void scale_bf16_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ s, long long nvec) {
   const float sc = *s;
+  if (sc == 1.f) return;  // a summed loss: nothing to change
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += (long long)gridDim.x * blockDim.x) {
     float f[8];
     load8(x + v * 8, f);
@@ -91,8 +141,22 @@ PT_API int pt_cross_entropy(void* logits, const long long* labels, float* loss, 
   cudaStream_t st = (cudaStream_t)stream_;
   if (n <= 0) return 0;
   if (ld % 8 != 0) return -1;
-  cross_entropy_kernel<<<n, CE_THREADS, 0, st>>>((__nv_bfloat16*)logits, labels, loss, n, V, ld, ignore_index);
-  return (int)cudaGetLastError();
+  auto launch = [&](auto kernel, int threads) {
+    kernel<<<n, threads, 0, st>>>((__nv_bfloat16*)logits, labels, loss, V, ld, ignore_index);
+    return (int)cudaGetLastError();
+  };
+  // Cold cache, us, before (1024 threads and two reads for every row) -> now, and one read and one write at 6.5 TB/s. 4096 rows:
+  // 1000 columns 37 -> 12 (3), 4096: 44 -> 18 (10), 8192: 53 -> 31 (21), 9496: 61 -> 42 (24), 12288: 63 -> 45 (31), 15520: 74 -> 59 (39).
+  // 2048 rows: 20000 columns 46 -> 37 (25), 32000: 60 -> 51 (40), 50304: 87 -> 86 (63), 151936: 265 -> 252 (192); the last four read
+  // their rows twice, up to 32768 columns by 512 threads (by 1024: 47 and 57 us).
+  const int nvec = V / 8;
+  if (nvec <= 128 * 2) return launch(cross_entropy_kernel<128, 2>, 128);
+  if (nvec <= 128 * 4) return launch(cross_entropy_kernel<128, 4>, 128);
+  if (nvec <= 256 * 4) return launch(cross_entropy_kernel<256, 4>, 256);
+  if (nvec <= 512 * 3) return launch(cross_entropy_kernel<512, 3>, 512);
+  if (nvec <= 512 * 4) return launch(cross_entropy_kernel<512, 4>, 512);
+  if (nvec <= 4096) return launch(cross_entropy_kernel<512, 0>, 512);
+  return launch(cross_entropy_kernel<1024, 0>, 1024);
 }
 
 PT_API int pt_scale_bf16(void* x, const float* s, long long numel, void* stream_) {

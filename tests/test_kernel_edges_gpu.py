@@ -1105,3 +1105,31 @@ def test_route_sort_runs_and_capacity(slots, E, valid):
         with pytest.raises(_native.KernelStatusError):
             _native.check_status()
         assert torch.equal(offs, got[0]) and bool((row_of_slot == -1).all()) and bool((slot_of_row == -1).all())
+
+
+@pytest.mark.parametrize("n,V", [(1, 1), (5, 7), (3, 8), (300, 2047), (300, 2048), (9, 2056), (300, 4096), (9, 4104), (9, 8192), (9, 8201), (300, 12288), (9, 12296),
+                                 (300, 16384), (300, 16392), (9, 40003)])
+def test_cross_entropy_rows(n, V):
+    """One block size and one row length after the other, whole vectors and rests, masked columns (minus infinity), shifted rows."""
+    from pithtrain_b200.ops.cross_entropy import cross_entropy
+
+    torch.manual_seed(V)
+    ld = (V + 7) // 8 * 8
+    buf = (torch.randn(n, ld, device="cuda") * 3 + 40 * torch.randn(n, 1, device="cuda")).bfloat16()
+    if V > 32:
+        buf[:, : V // 3] = float("-inf")  # whole threads without a finite column
+    labels = torch.randint(V // 3 if V > 32 else 0, V, (n,), device="cuda")
+    labels[0] = V - 1
+    if n > 2:
+        labels[1] = -100
+    want_in = buf[:, :V].double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(want_in, labels, ignore_index=-100, reduction="none")
+    want.sum().backward()
+    logits = buf[:, :V].detach().requires_grad_()
+    got = cross_entropy(logits * 1.0 if ld == V else logits.as_strided((n, V), (ld, 1)), labels)
+    got.backward()
+    # the arguments of 2^x are rounded at |logit| log2(e) < 400, the sum of V terms in blocks, each loss of about |logit| once
+    assert abs(float(got.detach().double() - want.detach().sum())) <= 2.0 ** -14 * float(want.detach().abs().sum()) + 2.0 ** -16 * n
+    g, w = logits.grad.double(), want_in.grad
+    assert ((g - w).abs() <= BF16_MAX * w.abs() + 2.0 ** -14 * (w.abs() + 2.0 ** -8)).all()
+    assert (g[labels == -100] == 0).all()
