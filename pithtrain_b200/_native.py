@@ -96,6 +96,7 @@ SIGS = {
     "pt_route_sort": "PPIIIPLPPPIP",
     "pt_route_sort_noalloc": "PIIIPPPIP",
     "pt_gather_rows": "PPIPPIILP",
+    "pt_embedding_bwd": "PPPIILP",
     "pt_indexed_bias_add": "PPPIPPIIP",
     "pt_segment_sum": "PIPPIPIP",
     "pt_combine": "PPPPPPIIIP",

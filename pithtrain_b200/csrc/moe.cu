@@ -307,6 +307,31 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict_
 }
 
 // ----------------------------------------------------------------------------------------------
+// embedding gradient: grad[ids[r]] += dy[r], fp32 from bf16. Bound by the rows of dy once and the touched rows of grad twice; a warp
+// walks a row, 8 columns a lane in two four-wide reductions, which the L2 performs, so that equal ids need no order. An id outside
+// the table is recorded and skipped.
+// ----------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const long long* __restrict__ ids, float* __restrict__ grad, int n, int H,
+                     long long V, int* __restrict__ err) {
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int r = blockIdx.x * warps + (threadIdx.x >> 5); r < n; r += gridDim.x * warps) {
+    const long long id = ids[r];
+    if (id < 0 || id >= V) {
+      if (lane == 0) atomicCAS(err, 0, PT_ERR_BOUNDS);
+      continue;
+    }
+    for (int c = lane * 8; c < H; c += 256) {
+      float v[8];
+      load8(dy + (size_t)r * H + c, v);
+      float* g = grad + (size_t)id * H + c;
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g + 4), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+    }
+  }
+}
+
+// ----------------------------------------------------------------------------------------------
 // combine: out[t] = (res ? res[t] : 0) + sum_{j<k, row>=0} (w ? w[t,j] : 1) * y[row_of_slot[t*k+j]]
 // fp32 accumulation in slot order. Bound by the bytes of the rows, if enough of them are on their way: a row is contiguous, so
 // one warp of the block fetches rows by bulk copies into a ring in shared memory, four rows of a token to a stage, a lane to a
@@ -916,6 +941,14 @@ PT_API int pt_gather_rows(const void* src, const int* idx, int div, void* dst, c
   if (H % 8 != 0) return -1;
   gather_rows_kernel<<<grid_for(n_rows_max, 8, 16), 256, 0, st>>>((const __nv_bfloat16*)src, idx, div,
       (__nv_bfloat16*)dst, n_rows_ptr, n_rows_max, H, src_stride);
+  return (int)cudaGetLastError();
+}
+
+// Into a table of 9496 x 2048: 4096 rows 77 -> 20 us, 256 rows 15 -> 9 us, against a conversion of dy and an indexed addition of one element a thread.
+PT_API int pt_embedding_bwd(const void* dy, const long long* ids, float* grad, int n, int H, long long V, void* stream_) {
+  if (n <= 0 || H <= 0) return 0;
+  if (H % 8 != 0) return -1;
+  embedding_bwd_kernel<<<grid_for(n, 8, 8), 256, 0, (cudaStream_t)stream_>>>((const __nv_bfloat16*)dy, ids, grad, n, H, V, device_status_word());
   return (int)cudaGetLastError();
 }
 

@@ -4,7 +4,8 @@ from __future__ import annotations
 
 import torch
 
-from .common import grad_buffer
+from .. import _native
+from .common import grad_buffer, sp, use_native
 from .moe import gather_rows
 
 
@@ -25,6 +26,15 @@ class _EmbeddingFn(torch.autograd.Function):
         (ids,) = ctx.saved_tensors
         w = ctx.w_ref
         g = grad_buffer(w)
+        n, H = ids.numel(), dy.shape[-1]
+        # fp32 gradients of bf16 rows; the additions into one row have no order, as those of index_add_
+        if (use_native(dy) and dy.dtype == torch.bfloat16 and g.dtype == torch.float32 and g.device == dy.device == ids.device
+                and ids.dtype == torch.int64 and H % 8 == 0 and g.is_contiguous() and g.data_ptr() % 16 == 0
+                and not dy.requires_grad and not torch.are_deterministic_algorithms_enabled()):
+            rows, flat = dy.reshape(n, H).contiguous(), ids.reshape(-1).contiguous()
+            if rows.data_ptr() % 16 == 0:
+                _native.check(_native.lib().pt_embedding_bwd(rows.data_ptr(), flat.data_ptr(), g.data_ptr(), n, H, g.shape[0], sp()), "pt_embedding_bwd")
+                return None, None
         g.index_add_(0, ids.reshape(-1), dy.reshape(-1, dy.shape[-1]).to(g.dtype))
         return None, None
 

@@ -1133,3 +1133,26 @@ def test_cross_entropy_rows(n, V):
     g, w = logits.grad.double(), want_in.grad
     assert ((g - w).abs() <= BF16_MAX * w.abs() + 2.0 ** -14 * (w.abs() + 2.0 ** -8)).all()
     assert (g[labels == -100] == 0).all()
+
+
+@pytest.mark.parametrize("n,V,H", [(1, 1, 8), (0, 5, 64), (37, 3, 264), (700, 90, 2048), (5000, 4, 8)])
+def test_embedding_gradient(n, V, H):
+    """Rows of one id add up, onto what the buffer holds; strided and misaligned gradients; fp32 buffers and bf16 ones."""
+    from pithtrain_b200.ops.embedding import embedding
+
+    torch.manual_seed(n)
+    ids = torch.randint(0, V, (n,), device="cuda")
+    for dy in (torch.randn(n, H, device="cuda").bfloat16(), torch.randn(n * H + 1, device="cuda").bfloat16()[1:].view(n, H),
+               torch.randn(n, 1, device="cuda").bfloat16().expand(n, H), torch.randn(H, n, device="cuda").bfloat16().t()):
+        start = torch.randn(V, H, device="cuda")
+        want = start.double().index_add(0, ids, dy.double())
+        size = start.abs().double().index_add(0, ids, dy.abs().double())
+        w = torch.nn.Parameter(torch.randn(V, H, device="cuda").bfloat16())
+        w.main_grad = start.clone()
+        embedding(ids, w).backward(dy)
+        assert ((w.main_grad.double() - want).abs() <= 2.0 ** -24 * (n + 1) * size).all()  # n fp32 additions at most, in any order
+    w = torch.nn.Parameter(torch.zeros(V, H, device="cuda").bfloat16())
+    embedding(ids, w).backward(torch.ones(n, H, device="cuda").bfloat16())
+    # a bf16 .grad: counts are whole numbers, exact up to 256
+    assert torch.equal(w.grad[:, 0].float().clamp(max=256), torch.bincount(ids, minlength=V).float().clamp(max=256))
+    _native.check_status()
