@@ -28,6 +28,7 @@
 // PTX forms follow the vendored CUTLASS headers (cute/arch/copy_sm100_tma.hpp: SM100_TMA_2SM_LOAD_3D,
 // cute/arch/mma_sm100_umma.hpp: SM100_MMA_F16BF16_2x1SM_SS, cute/arch/tmem_allocator_sm100.hpp: Allocator2Sm,
 // cutlass/arch/barrier.h: umma_arrive_2x1SM, umma_arrive_2x1SM_sm0).
+#include "gemm_skinny.h"
 #include "host_common.h"
 #include "ptx.cuh"
 
@@ -549,6 +550,7 @@ PT_API int pt_gemm2cta_nt(const void* x, const void* w, void* out, int M, int N,
                           long long ldd, void* stream_) {
   using namespace pt;
   if (M <= 0 || N <= 0 || K <= 0 || K % 8 != 0) return -2;
+  if (gemm_skinny_better(M, N, K)) return gemm_skinny_nt(x, w, out, M, N, K, lda, ldb, ldd, static_cast<cudaStream_t>(stream_));
   Gemm2Args a = t2_args(M, N, K, 1);
   return t2_launch<false, false, T2_STORE>({x, M, K, lda, lda * M}, {w, N, K, ldb, ldb * N}, {out, M, N, ldd, ldd * M}, a,
                                            static_cast<cudaStream_t>(stream_));

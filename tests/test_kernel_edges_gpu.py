@@ -1156,3 +1156,23 @@ def test_embedding_gradient(n, V, H):
     # a bf16 .grad: counts are whole numbers, exact up to 256
     assert torch.equal(w.grad[:, 0].float().clamp(max=256), torch.bincount(ids, minlength=V).float().clamp(max=256))
     _native.check_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 5120, 2048), (3, 136, 72), (64, 128, 64), (64, 2048, 4096), (64, 9496, 520), (65, 264, 1032), (127, 2048, 512), (128, 648, 4096),
+                                   (129, 128, 2048), (200, 2048, 4096), (300, 376, 1024), (1000, 128, 2048), (64, 20000, 128)])
+def test_dense_few_rows(M, N, K):
+    """Row counts up to a tile and past it, feature and reduction remainders, every split of the reduction from one CTA to eight; rows
+    of a wider tensor; the same bits in every run."""
+    from pithtrain_b200.ops import gemm as G
+
+    torch.manual_seed(M + N + K)
+    wide = torch.randn(M, K + 16, device="cuda").bfloat16()
+    for x in (torch.randn(M, K, device="cuda").bfloat16(), wide[:, 8 : K + 8]):
+        w = torch.randn(N, K, device="cuda").bfloat16()
+        got = G.gemm_nt(x, w)
+        want = x.double() @ w.double().t()
+        size = x.double().abs() @ w.double().abs().t()
+        # the tensor core cuts sums off at 24 bits or so, K / 16 times at most, then one bf16 rounding
+        assert ((got.double() - want).abs() <= BF16_MAX * want.abs() + 2.0 ** -22 * (K // 16 + 9) * size).all()
+        assert torch.equal(got, G.gemm_nt(x, w))
+    _native.check_status()
