@@ -1176,3 +1176,29 @@ def test_dense_few_rows(M, N, K):
         assert ((got.double() - want).abs() <= BF16_MAX * want.abs() + 2.0 ** -22 * (K // 16 + 9) * size).all()
         assert torch.equal(got, G.gemm_nt(x, w))
     _native.check_status()
+
+
+@pytest.mark.parametrize("extra", [False, True])
+@pytest.mark.parametrize("n,H", [(1, 8), (591, 2048), (592, 2056), (593, 4096), (1185, 520), (1777, 6152), (3, 8192)])
+def test_rmsnorm_backward_rows(n, H, extra):
+    """One row a block, one more than the blocks, several rows each; every number of vectors a thread; with and without a residual."""
+    from pithtrain_b200.ops.norm import rmsnorm
+
+    torch.manual_seed(n)
+    x = torch.randn(n, H, device="cuda").bfloat16().requires_grad_()
+    res = torch.randn(n, H, device="cuda").bfloat16().requires_grad_() if extra else None
+    w = torch.nn.Parameter(torch.randn(H, device="cuda").bfloat16())
+    w.main_grad = torch.zeros(H, device="cuda")
+    out = rmsnorm(x, w, 1e-6, res) if extra else rmsnorm(x, w, 1e-6)
+    y, h = out if isinstance(out, tuple) else (out, None)
+    dy, dh = torch.randn_like(y), torch.randn_like(y)
+    torch.autograd.backward([y, h] if extra else [y], [dy, dh] if extra else [dy])
+    hd = (h.detach() if extra else x.detach()).double()
+    rstd = (hd.square().mean(-1, keepdim=True) + 1e-6).rsqrt()
+    g = dy.double() * w.detach().double()
+    dx = rstd * (g - hd * rstd * (g * hd * rstd).mean(-1, keepdim=True)) + (dh.double() if extra else 0)
+    dw = (dy.double() * hd * rstd).sum(0)
+    # fp32 terms of size rstd (|g| + |xhat| |dot|) and |dh|, one bf16 rounding; dw: n fp32 additions at most
+    size = rstd * (g.abs() + (hd * rstd).abs() * (g * hd * rstd).abs().mean(-1, keepdim=True)) + (dh.double().abs() if extra else 0)
+    assert ((x.grad.double() - dx).abs() <= BF16_MAX * dx.abs() + 2.0 ** -16 * size).all()
+    assert ((w.main_grad.double() - dw).abs() <= 2.0 ** -24 * (n + 8) * (dy.double() * hd * rstd).abs().sum(0)).all()
