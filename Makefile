@@ -4,7 +4,7 @@ NPROC  ?= 1
 
 .PHONY: build test test-gpu bench estimate clean
 
-build:            ## compile pithtrain_b200/csrc/*.cu for sm_100a into pithtrain_b200/_lib/libpithb200.so
+build:            ## compile pithtrain_b200/csrc/*.cu for sm_100a into pithtrain_b200/_lib/libpithb200.so, csrc/host_ops.cpp into pith_host_ops.so
 	$(PYTHON) -m pithtrain_b200.build
 
 test: build       ## CPU tier (unit tests and 2-4 rank gloo jobs)

@@ -59,7 +59,7 @@ def _chk2d(t: torch.Tensor, name: str):
     assert t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0, f"{name} must be 16-byte aligned"
 
 
-# Dense products run on the 2-CTA kernel of csrc/gemm_2cta.cu, whose CTA pair shares each B tile: at 4096 rows and the models'
+# Dense products run on the 2-CTA kernel of csrc/gemm_2cta.cu (few rows: csrc/gemm_skinny.cu), whose CTA pair shares each B tile: at 4096 rows and the models'
 # projection shapes 7 to 16 % faster than the single-CTA family in all three forms (us, single / pair: [5120, 2048] 77 / 66 NT,
 # 75 / 67 NN, 91 / 82 TN into fp32; [10944, 2048] 146 / 122, 144 / 126, 151 / 134).
 USE_2CTA = True
