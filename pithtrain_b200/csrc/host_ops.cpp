@@ -9,7 +9,8 @@
 // The kernels stay in libpithb200.so; their entry points are looked up by name (bind) in the library that Python has loaded. What
 // a user can replace or observe is asked from Python when it is needed: the gradient buffer of a parameter (main_grad, else .grad)
 // and the deferral of weight gradients. The nodes keep tensors (through SavedVariable: version checks and saved-tensor hooks as
-// for any operator), never raw pointers, and no state outlives a call.
+// for any operator), never raw pointers, and no state outlives a call. A parameter that a node adds gradients to is kept beside its
+// saved value: under hooks, the memory trace's or a checkpoint's, unpacking hands out another tensor, without main_grad and .grad.
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include <torch/csrc/autograd/function.h>
@@ -184,6 +185,7 @@ using Below = at::AutoDispatchBelowADInplaceOrView;
 // ------------------------------------------------------------------------------------------------
 struct RmsNormBackward : Node {
   SavedVariable h, w, rstd;
+  Tensor weight;  // the parameter
   bool residual = false, h_is_output = false, zero_centered = false;
 
   variable_list apply(variable_list&& grads) override {
@@ -200,7 +202,7 @@ struct RmsNormBackward : Node {
       part = empty({api.pt_rmsnorm_bwd_grid(n), H}, hv, at::kFloat);
       check(api.pt_rmsnorm_bwd(ptr(dy), ptr(dh), ptr(hv), ptr(wd), ptr(r), ptr(dx), ptr(part), n, H, zero_centered, current_stream()), "pt_rmsnorm_bwd");
     }
-    if (task_should_compute_output(1)) accumulate_colsum(wv, part);
+    if (task_should_compute_output(1)) accumulate_colsum(weight, part);
     return {dx, Tensor(), residual ? dx : Tensor()};
   }
   void release_variables() override {
@@ -208,6 +210,7 @@ struct RmsNormBackward : Node {
     h.reset_data();
     w.reset_data();
     rstd.reset_data();
+    weight.reset();
   }
 };
 
@@ -236,6 +239,7 @@ py::object rmsnorm(const Tensor& x, const Tensor& w, double eps, const OptTensor
     node->residual = node->h_is_output = h.defined();
     node->h = h.defined() ? SavedVariable(h, true) : SavedVariable(xc, false);
     node->w = SavedVariable(w, false);
+    node->weight = w;
     node->rstd = SavedVariable(rstd, false);
     node->zero_centered = zero_centered;
   }
@@ -324,6 +328,7 @@ void wgrad_into(const Tensor& dy, const Tensor& x, const Tensor& target, bool fp
 // ------------------------------------------------------------------------------------------------
 struct QkNormRopeBackward : Node {
   SavedVariable qkv, q_w, k_w, cos, sin, pos, rq, rk;
+  Tensor q_weight, k_weight;  // the parameters
   int64_t Hq = 0, Hkv = 0, D = 0, S = 0;
   bool norm = false, zero_centered = false;
 
@@ -345,12 +350,14 @@ struct QkNormRopeBackward : Node {
                                     ptr(part), n, S, Hq, Hkv, D, x.stride(0), dx.stride(0), zero_centered, current_stream()),
             "pt_qk_norm_rope_bwd");
     }
-    if (norm) accumulate_colsum_pair(qw, kw, part, D);
+    if (norm) accumulate_colsum_pair(q_weight, k_weight, part, D);
     return {dx, Tensor(), Tensor()};
   }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     for (SavedVariable* v : {&qkv, &q_w, &k_w, &cos, &sin, &pos, &rq, &rk}) v->reset_data();
+    q_weight.reset();
+    k_weight.reset();
   }
 };
 
@@ -387,6 +394,8 @@ py::tuple qk_norm_rope(const Tensor& qkv_, const OptTensor& q_w_, const OptTenso
     node->qkv = SavedVariable(qkv, false);
     node->q_w = SavedVariable(q_w, false);
     node->k_w = SavedVariable(k_w, false);
+    node->q_weight = q_w;
+    node->k_weight = k_w;
     node->cos = SavedVariable(cos, false);
     node->sin = SavedVariable(sin, false);
     node->pos = SavedVariable(pos, false);

@@ -1050,6 +1050,51 @@ def test_host_operators_in_autograd(name):
     _native.check_status()
 
 
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("hooks", ["identity", "copy", "memory trace", "checkpoint"])
+def test_weight_gradients_under_saved_tensor_hooks(hooks, flat):
+    """Hooks hand other tensors back than the parameters; the gradients reach the parameters all the same, and are the same."""
+    from contextlib import nullcontext
+
+    from torch.utils.checkpoint import checkpoint
+
+    from pithtrain_b200.ops.linear import linear
+    from pithtrain_b200.ops.norm import rmsnorm
+    from pithtrain_b200.ops.rope import qk_norm_rope
+    from pithtrain_b200.tools.memory_trace import SavedTensorBytes
+
+    torch.manual_seed(25)
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    start, cos, sin = [mk(*s) for s in ((128,), (128,), (256, 128), (64,), (64,))], mk(9, 64), mk(9, 64)
+    x, res, dy = mk(9, 128), mk(9, 128), [mk(9, n, 64) for n in (2, 1, 1)]
+    context = {"identity": lambda: torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t), "memory trace": SavedTensorBytes,
+               "copy": lambda: torch.autograd.graph.saved_tensors_hooks(lambda t: t.clone(), lambda t: t.clone())}
+
+    def gradients(hooked):
+        n1, n2, w, qw, kw = params = [torch.nn.Parameter(t.clone()) for t in start]
+        if flat:
+            for p in params:
+                p.main_grad = torch.zeros(p.shape, device="cuda")
+
+        def block(x, res):
+            y, h = rmsnorm(rmsnorm(x, n1), n2, 1e-6, res)
+            return qk_norm_rope(linear(y + h, w), qw, kw, cos, sin, 2, 1, 64, S=9)
+
+        leaves = [t.clone().requires_grad_() for t in (x, res)]
+        if hooked and hooks == "checkpoint":
+            outs = checkpoint(block, *leaves, use_reentrant=False)
+        else:
+            with context[hooks]() if hooked else nullcontext():
+                outs = block(*leaves)
+        torch.autograd.backward(outs, dy)
+        return [p.main_grad if flat else p.grad for p in params] + [t.grad for t in leaves]
+
+    for want, got in zip(gradients(False), gradients(True)):
+        assert want is not None and bool(want.any())
+        assert got is not None and torch.equal(got, want)
+    _native.check_status()
+
+
 @pytest.mark.parametrize("bias", [False, True])
 def test_host_linear_defers_and_finds_its_gradients(bias):
     """Weight gradients go to the W phase while it is on, to ``main_grad`` where a parameter has one and to ``.grad`` otherwise."""
