@@ -8,23 +8,32 @@
 
 namespace pt {
 
-// Exponentials are 2^(v log2(e) - c): one fused multiply-add and one instruction of the special function unit each, so that the
-// two passes over a row (39 M logits: 17 us of that unit) fit beside its read and write. c = max * log2(e) is the same rounded
-// number in every term of the sum and in lse2 = c + log2(sum), so its rounding cancels in the gradient; the loss takes it out.
-constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+// Exponentials are 2^((v - max) log2(e) - c), two of them in two packed instructions and one each of the special function unit, so
+// that the two passes over a row (39 M logits: 17 us of that unit) fit beside its read and write. c is 0 in the sum and log2(sum)
+// in the gradient. The maximum is taken off first: v log2(e) - max log2(e) costs as much, but the second product overflows for
+// the lowest bf16 value, a common mask, and from 1e9 on is rounded by whole numbers.
+constexpr float LOG2E = 1.4426950408889634f;
 
 __device__ __forceinline__ float max8(const uint4& v) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
   const __nv_bfloat162 a = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
   return fmaxf(__low2float(a), __high2float(a));
 }
-__device__ __forceinline__ void exp8(const uint4& v, float c, float (&e)[8]) {
+// What is subtracted for the maximum m: of minus infinities alone (a masked stretch), a finite number below every other logit.
+__device__ __forceinline__ float below(float m) { return fmaxf(m, -3.4028234e38f); }
+__device__ __forceinline__ float exp1(float v, float m, float c) { return ex2_approx(fmaf(v - m, LOG2E, -c)); }
+template <bool C>  // without c: it is 0
+__device__ __forceinline__ void exp8(const uint4& v, float m, float c, float (&e)[8]) {
   const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+  const uint64_t m2 = f2_pack(-m, -m), c2 = f2_pack(-c, -c), log2e2 = f2_pack(LOG2E, LOG2E);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float2 p = unpack_bf16x2(q[i]);
-    e[2 * i] = ex2_approx(fmaf(p.x, LOG2E, -c));
-    e[2 * i + 1] = ex2_approx(fmaf(p.y, LOG2E, -c));
+    const uint64_t d = f2_add(f2_pack(p.x, p.y), m2);
+    float a, b;
+    f2_unpack(C ? f2_fma(d, log2e2, c2) : f2_mul(d, log2e2), a, b);
+    e[2 * i] = ex2_approx(a);
+    e[2 * i + 1] = ex2_approx(b);
   }
 }
 __device__ __forceinline__ void minus_one_at(float (&e)[8], int c, long long label) {
@@ -59,7 +68,7 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __rest
   const float last = rest < V ? __bfloat162float(x[rest]) : -INFINITY;
   const float xl = tid == 0 ? __bfloat162float(x[label]) : 0.f;
   uint4 raw[NV > 0 ? NV : 1];
-  float m = last, s = 0.f, gm, shift;  // shift: c of the block
+  float m = last, s = 0.f, gm;  // gm: maximum of the row, later what is subtracted for it
   if (NV > 0) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -68,40 +77,36 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __rest
     }
 #pragma unroll
     for (int i = 0; i < NV; ++i) m = fmaxf(m, max8(raw[i]));
-    gm = block_max(m, red);
-    shift = __fmul_rn(gm, LOG2E);
+    gm = below(block_max(m, red));
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       keep_packed(raw[i]);
       float e[8];
-      exp8(raw[i], shift, e);
+      exp8<false>(raw[i], gm, 0.f, e);
       s += ((e[0] + e[1]) + (e[2] + e[3])) + ((e[4] + e[5]) + (e[6] + e[7]));
     }
   } else {
-    shift = -INFINITY;
+    m = below(m);
 #pragma unroll 4
     for (int c = tid; c < nvec; c += T) {
       const uint4 v = xv[c];
-      const float up = fmaxf(m, max8(v)), scaled = __fmul_rn(up, LOG2E), c_up = up == -INFINITY ? 0.f : scaled;
+      const float up = fmaxf(m, max8(v));
       float e[8];
-      exp8(v, c_up, e);
-      s = s * ex2_approx(shift - c_up) + (((e[0] + e[1]) + (e[2] + e[3])) + ((e[4] + e[5]) + (e[6] + e[7])));
+      exp8<false>(v, up, 0.f, e);
+      s = s * exp1(m, up, 0.f) + (((e[0] + e[1]) + (e[2] + e[3])) + ((e[4] + e[5]) + (e[6] + e[7])));
       m = up;
-      shift = scaled;
     }
     gm = block_max(m, red);
-    const float own = shift;
-    shift = __fmul_rn(gm, LOG2E);
-    if (m != gm) s *= ex2_approx(own - shift);
+    s *= exp1(m, gm, 0.f);
   }
-  s += ex2_approx(fmaf(last, LOG2E, -shift));
-  const float gs = block_sum(gm == -INFINITY ? 0.f : s, red);
+  s += exp1(last, gm, 0.f);
+  const float gs = block_sum(s, red);
   // x[label] was read ahead of the barriers above, it is written after them. The logarithm of the loss is taken in 64 bits: the fast one
   // is off by 3e-7 on average.
-  const float lse2 = shift + __log2f(gs);
+  const float log2_sum = __log2f(gs);
   auto gradient = [&](const uint4& v, int c) {
     float e[8];
-    exp8(v, lse2, e);
+    exp8<true>(v, gm, log2_sum, e);
     minus_one_at(e, c, label);
     store8(x + c * 8, e);
   };
@@ -115,8 +120,8 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __rest
 #pragma unroll 4
     for (int c = tid; c < nvec; c += T) gradient(xv[c], c);
   }
-  if (rest < V) x[rest] = __float2bfloat16(ex2_approx(fmaf(last, LOG2E, -lse2)) - (rest == label ? 1.f : 0.f));
-  if (tid == 0) loss[row] = (float)((double)gm - xl + (log((double)gs) - fmaf(gm, LOG2E, -shift) * LN2));
+  if (rest < V) x[rest] = __float2bfloat16(exp1(last, gm, log2_sum) - (rest == label ? 1.f : 0.f));
+  if (tid == 0) loss[row] = (float)((double)gm - xl + log((double)gs));
 }
 
 // x *= s[0] over a flat bf16 buffer (s on the device).

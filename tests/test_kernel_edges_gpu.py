@@ -1180,6 +1180,46 @@ def test_cross_entropy_rows(n, V):
     assert (g[labels == -100] == 0).all()
 
 
+@pytest.mark.parametrize("V", [5, 8, 1000, 2056, 4104, 9496, 12296, 16384, 16392, 40003])
+def test_cross_entropy_of_masked_and_large_logits(V):
+    """Masks of any size, the lowest bf16 value among them, over the leading columns, the rest or a whole row, and logits so large that
+    their product with log2(e) is none or is rounded off by whole numbers."""
+    from pithtrain_b200.ops.cross_entropy import cross_entropy
+
+    torch.manual_seed(V)
+    ld, lowest = (V + 7) // 8 * 8, torch.finfo(torch.bfloat16).min
+    masks = [lowest, -2.4e38, -1e30, -1e9, -1e4, float("-inf")]
+    rows, labels = [], []
+    for fill in masks:
+        for lo, hi in ((0, V // 2), (V // 2, V - 1), (0, V - 1)):  # leading columns, the following ones, all but the last
+            row = torch.randn(ld).mul_(3)
+            row[lo:hi] = fill
+            rows.append(row)
+            labels.append(V - 1)
+    for fill in (*masks[:5], 1e9, 1e30, 3e38):
+        rows.append(torch.full((ld,), fill))  # every column alike: the loss is log V
+        labels.append(V // 3)
+    for peak in (1e9, 1e30, 3e38):
+        row = torch.randn(ld)
+        row[V // 2] = peak
+        rows.append(row)
+        labels.append(V // 2)
+    buf = torch.stack(rows).cuda().bfloat16()
+    label = torch.tensor(labels, device="cuda")
+    want_in = buf[:, :V].double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(want_in, label, reduction="none")
+    want.sum().backward()
+    for i in range(len(rows)):  # two of a row at a time: a loss that is wrong is not hidden by the others
+        logits = buf[[i, i]].detach().requires_grad_()
+        got = cross_entropy((logits * 1.0)[:, :V], label[[i, i]])
+        got.backward()
+        loss = 2 * float(want[i].detach())
+        # as in the test above; differences of the logits are exact or off by 2^-24 of themselves
+        assert abs(float(got.detach().double()) - loss) <= 2.0 ** -20 * (abs(loss) + 8), i
+        g, w = logits.grad[:, :V].double(), want_in.grad[i]
+        assert ((g - w).abs() <= BF16_MAX * w.abs() + 2.0 ** -14 * (w.abs() + 2.0 ** -8)).all(), i
+
+
 @pytest.mark.parametrize("n,V,H", [(1, 1, 8), (0, 5, 64), (37, 3, 264), (700, 90, 2048), (5000, 4, 8)])
 def test_embedding_gradient(n, V, H):
     """Rows of one id add up, onto what the buffer holds; strided and misaligned gradients; fp32 buffers and bf16 ones."""
