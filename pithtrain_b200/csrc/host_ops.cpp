@@ -622,7 +622,8 @@ Tensor combine(const Tensor& y, const Tensor& row_of_slot, const Tensor& w, int6
 }
 
 struct ExpertsBackward : Node {
-  SavedVariable x, w, w1, w2, gu, offs, row_of_slot, slot_of_row;
+  SavedVariable x, w, gu, offs, row_of_slot, slot_of_row;
+  Tensor w1, w2;  // parameters, not activations: saved-tensor hooks would copy or count them for every micro-batch
   PyRef queue_wgrad;  // (dyg, act, dgu, x, slot_of_row, offs, n_rows)
   int64_t k = 0;
   bool interleaved = false;
@@ -631,16 +632,16 @@ struct ExpertsBackward : Node {
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     if (!grads[0].defined()) return {Tensor(), Tensor()};
-    const Tensor xv = x.unpack(), wv = w.unpack(), w1v = w1.unpack(), w2v = w2.unpack(), g = gu.unpack(), o = offs.unpack();
+    const Tensor xv = x.unpack(), wv = w.unpack(), g = gu.unpack(), o = offs.unpack();
     const Tensor ros = row_of_slot.unpack(), sor = slot_of_row.unpack();
     Tensor dx, dw, dyg, dgu, act, n_rows;
     {
       Below guard;
       const Tensor d_out = dense(grads[0]);
-      n_rows = o.narrow(0, w1v.size(0), 1);
+      n_rows = o.narrow(0, w1.size(0), 1);
       const int64_t R = g.size(0), inter = g.size(1) / 2;
       dyg = gather(d_out, sor, k, n_rows);  // output gradient of each sorted row, without its routing weight
-      const Tensor da = grouped(dyg, w2v, o, true);
+      const Tensor da = grouped(dyg, w2, o, true);
       // routing weights and their gradients are looked up and scattered through the slot index in the kernel
       dgu = at::empty_like(g);
       act = empty({R, inter}, g, at::kBFloat16);
@@ -649,7 +650,7 @@ struct ExpertsBackward : Node {
       check(api.pt_swiglu_bwd(ptr(g), ptr(da), ptr(wf), ptr(dgu), ptr(act), ptr(dw), ptr(n_rows), R, inter, interleaved, static_cast<float>(alpha),
                               static_cast<float>(limit), ptr(sor), current_stream()),
             "pt_swiglu_bwd");
-      const Tensor dxs = grouped(dgu, w1v, o, true);
+      const Tensor dxs = grouped(dgu, w1, o, true);
       if (task_should_compute_output(0)) dx = combine(dxs, ros, Tensor(), k);
       dw = dw.view(wv.sizes()).to(wv.scalar_type());
     }
@@ -659,7 +660,9 @@ struct ExpertsBackward : Node {
   }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable* s : {&x, &w, &w1, &w2, &gu, &offs, &row_of_slot, &slot_of_row}) s->reset_data();
+    for (SavedVariable* s : {&x, &w, &gu, &offs, &row_of_slot, &slot_of_row}) s->reset_data();
+    w1.reset();
+    w2.reset();
   }
 };
 
@@ -712,8 +715,8 @@ Tensor moe_experts(const Tensor& x, const Tensor& w, const Tensor& eids, const T
     torch::autograd::set_history(out, node);
     node->x = SavedVariable(x, false);
     node->w = SavedVariable(w, false);
-    node->w1 = SavedVariable(w1, false);
-    node->w2 = SavedVariable(w2, false);
+    node->w1 = w1;
+    node->w2 = w2;
     node->gu = SavedVariable(gu, false);
     node->offs = SavedVariable(offs, false);
     node->row_of_slot = SavedVariable(row_of_slot, false);

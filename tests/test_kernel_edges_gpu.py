@@ -1095,6 +1095,24 @@ def test_weight_gradients_under_saved_tensor_hooks(hooks, flat):
     _native.check_status()
 
 
+def test_expert_weights_are_not_saved():
+    """What the expert block saves are activations: hooks (offloading, the memory trace) do not see its weights."""
+    from pithtrain_b200.ops.moe import ExpertWeights, moe_experts
+
+    torch.manual_seed(26)
+    w1, w2 = (torch.nn.Parameter(torch.randn(s, device="cuda").bfloat16()) for s in ((4, 128, 64), (4, 64, 64)))
+    g1, g2 = torch.zeros(w1.shape, device="cuda"), torch.zeros(w2.shape, device="cuda")
+    ew = ExpertWeights(w1, w2, lambda: g1, lambda: g2)
+    x, p = torch.randn(9, 64, device="cuda").bfloat16().requires_grad_(), torch.rand(9, 2, device="cuda")
+    eids = torch.randint(0, 4, (9, 2), dtype=torch.int32, device="cuda")
+    storages, weights = set(), {t.untyped_storage().data_ptr() for t in (w1, w2)}
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (storages.add(t.untyped_storage().data_ptr()), t)[1], lambda t: t):
+        out = moe_experts(x, p, eids, ew)
+    assert x.untyped_storage().data_ptr() in storages and not weights & storages
+    out.backward(torch.ones_like(out))
+    assert g1.any() and g2.any()
+
+
 @pytest.mark.parametrize("bias", [False, True])
 def test_host_linear_defers_and_finds_its_gradients(bias):
     """Weight gradients go to the W phase while it is on, to ``main_grad`` where a parameter has one and to ``.grad`` otherwise."""
