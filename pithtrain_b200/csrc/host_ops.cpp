@@ -19,6 +19,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <atomic>
 
 namespace {
@@ -95,6 +96,14 @@ void refuse_transforms(std::initializer_list<Tensor> inputs) {
               "this operator does not support functorch transforms (vmap, grad, jvp, jacrev, ...)");
   for (const Tensor& t : inputs)
     TORCH_CHECK_NOT_IMPLEMENTED(!t.defined() || !t._fw_grad(0).defined(), "forward-mode differentiation is not implemented for this operator");
+}
+// The kernels take raw pointers. Operands on the host or on different devices are refused, and those without memory of their own
+// (fake tensors, subclasses that wrap others).
+void check_operands(const Tensor& x, std::initializer_list<Tensor> others) {
+  TORCH_CHECK(x.is_cuda(), "the first operand must be on a CUDA device, is on ", x.device());
+  for (const Tensor& t : others) TORCH_CHECK(!t.defined() || t.device() == x.device(), "operands on ", x.device(), " and ", t.device());
+  const auto has_memory = [](const Tensor& t) { return !t.defined() || t.numel() == 0 || t.const_data_ptr() != nullptr; };
+  TORCH_CHECK(has_memory(x) && std::all_of(others.begin(), others.end(), has_memory), "an operand has no memory");
 }
 Tensor opt(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 Tensor empty(at::IntArrayRef sizes, const Tensor& like, at::ScalarType type) { return at::empty(sizes, like.options().dtype(type)); }
@@ -217,6 +226,7 @@ struct RmsNormBackward : Node {
 py::object rmsnorm(const Tensor& x, const Tensor& w, double eps, const OptTensor& residual_, bool zero_centered) {
   const Tensor residual = opt(residual_);
   refuse_transforms({x, w, residual});
+  check_operands(x, {w, residual});
   auto node = make_node<RmsNormBackward>(x, w, residual);
   Tensor xc, h, y, rstd;
   {
@@ -224,8 +234,8 @@ py::object rmsnorm(const Tensor& x, const Tensor& w, double eps, const OptTensor
     const int64_t H = x.size(-1), n = H ? x.numel() / H : 0;
     xc = dense(x);
     const Tensor rc = residual.defined() ? dense(residual) : Tensor();
-    TORCH_CHECK(!rc.defined() || (rc.numel() == xc.numel() && rc.is_cuda() && rc.scalar_type() == at::kBFloat16), "rmsnorm: residual ", rc.sizes());
-    TORCH_CHECK(w.is_cuda() && w.numel() == H && w.is_contiguous(), "rmsnorm: weight ", w.sizes(), " for rows of ", H);
+    TORCH_CHECK(!rc.defined() || (rc.numel() == xc.numel() && rc.scalar_type() == at::kBFloat16), "rmsnorm: residual ", rc.sizes());
+    TORCH_CHECK(w.numel() == H && w.is_contiguous(), "rmsnorm: weight ", w.sizes(), " for rows of ", H);
     const Tensor wd = dense(w);
     y = at::empty_like(xc);
     if (rc.defined()) h = at::empty_like(xc);
@@ -288,6 +298,7 @@ struct LinearBackward : Node {
 Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, const py::object& grad_getter, const py::object& bias_param) {
   const Tensor bias = opt(bias_);
   refuse_transforms({x, w, bias});
+  check_operands(x, {w, bias});
   auto node = make_node<LinearBackward>(x, w, bias);
   Tensor xc, y;
   {
@@ -318,6 +329,7 @@ Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, const py
 void wgrad_into(const Tensor& dy, const Tensor& x, const Tensor& target, bool fp32_sums) {
   check_rows(dy, "dy");
   check_rows(x, "x");
+  check_operands(dy, {x, target});
   check(api.pt_dense_tn(ptr(dy), ptr(x), target.data_ptr(), target.scalar_type() == at::kFloat, fp32_sums, dy.size(1), x.size(1), dy.size(0),
                         dy.stride(0), x.stride(0), target.stride(0), current_stream()),
         "pt_dense_tn");
@@ -365,6 +377,7 @@ py::tuple qk_norm_rope(const Tensor& qkv_, const OptTensor& q_w_, const OptTenso
                        const OptTensor& positions, int64_t Hq, int64_t Hkv, int64_t D, double eps, int64_t S, bool zero_centered) {
   const Tensor q_w = opt(q_w_), k_w = opt(k_w_);
   refuse_transforms({qkv_, q_w, k_w});
+  check_operands(qkv_, {q_w, k_w, cos_, sin_, opt(positions)});
   auto node = make_node<QkNormRopeBackward>(qkv_, q_w, k_w);
   Tensor qkv = qkv_, cos, sin, q, k, v, rq, rk, pos;
   {
@@ -489,6 +502,7 @@ py::tuple attention(const Tensor& q, const Tensor& k, const Tensor& v, const Opt
                     int64_t q_off) {
   const Tensor sinks = opt(sinks_), row_lo = opt(row_lo_);
   refuse_transforms({q, k, v, sinks});
+  check_operands(q, {k, v, sinks, row_lo});
   auto node = make_node<AttentionBackward>(q, k, v, sinks);
   Tensor out, lse;
   {
@@ -553,6 +567,7 @@ struct RouterBackward : Node {
 // (weights [n, k] fp32, picks [n, k] int32, probabilities [n, E] fp32 or None); given: the picks, else they are the top k
 py::tuple router(const Tensor& logits, const OptTensor& given, int64_t k, int64_t mode, bool renorm, double scale) {
   refuse_transforms({logits});
+  check_operands(logits, {opt(given)});
   auto node = make_node<RouterBackward>(logits);
   Tensor probs, idx, w;
   const int64_t n = logits.size(0), E = logits.size(1);
@@ -588,6 +603,7 @@ py::tuple router(const Tensor& logits, const OptTensor& given, int64_t k, int64_
 // The top k alone, [n, k] int32: what a replay of the routing is handed.
 Tensor router_picks(const Tensor& logits, int64_t k) {
   refuse_transforms({logits});
+  check_operands(logits, {});
   Below guard;
   const Tensor lg = logits.contiguous();
   const int64_t n = lg.size(0), E = lg.size(1);
@@ -603,6 +619,7 @@ Tensor router_picks(const Tensor& logits, int64_t k) {
 // Rows of group g times w[g]: D = X W^T (w [E, N, K]) or, w_mn, D = X W (w [E, K, N]); K the reduction.
 Tensor grouped(const Tensor& x, const Tensor& w, const Tensor& offs, bool w_mn) {
   const int64_t R = x.size(0), K = x.size(1), E = w.size(0), N = w_mn ? w.size(2) : w.size(1);
+  TORCH_CHECK(w.is_contiguous(), "expert weights must be contiguous");
   Tensor out = empty({R, N}, x, at::kBFloat16);
   check(api.pt_gemm_bf16(ptr(x), ptr(w), ptr(out), 1, R, N, K, 0, w_mn, R, K, K, E * w.size(1), w.size(2), w.size(2), R, N, ptr(offs), E, w.size(1), 0, 0, 0,
                          1, 2, 0, 0, nullptr, 1, 0, current_stream()),
@@ -674,6 +691,7 @@ void expert_wgrads(const Tensor& dyg, const Tensor& act, const Tensor& dgu, cons
     const int64_t R = dy.size(0), N = dy.size(1), K = a.size(1), E = g.size(0);
     TORCH_CHECK(g.dim() == 3 && g.size(1) == N && g.size(2) == K && g.is_contiguous(), "expert_wgrads: gradient buffer ", g.sizes());
     check_aligned(g, "the gradient buffer");
+    check_operands(dy, {g});
     check(api.pt_gemm_bf16(ptr(dy), ptr(a), g.data_ptr(), 2, N, K, 0, 1, 1, R, N, dy.stride(0), R, K, a.stride(0), N, K, ptr(offs), E, 0, N * K,
                            g.scalar_type() == at::kFloat, 1, 1, 2, 0, 0, nullptr, 1, 0, current_stream()),
           "pt_gemm_bf16");
@@ -686,6 +704,7 @@ void expert_wgrads(const Tensor& dyg, const Tensor& act, const Tensor& dgu, cons
 Tensor moe_experts(const Tensor& x, const Tensor& w, const Tensor& eids, const Tensor& w1, const Tensor& w2, int64_t align, int64_t r_cap,
                    bool interleaved, double alpha, double limit, const py::object& queue_wgrad) {
   refuse_transforms({x, w, w1, w2});
+  check_operands(x, {w, eids, w1, w2});
   auto node = make_node<ExpertsBackward>(x, w);
   Tensor gu, out, offs, row_of_slot, slot_of_row;
   const int64_t n = eids.size(0), k = eids.size(1), E = w1.size(0), slots = n * k;

@@ -62,3 +62,54 @@ def test_current_device_predicate(monkeypatch):
     on = [SimpleNamespace(is_cuda=True, get_device=lambda d=d: d) for d in (0, 1)]
     assert [_native.on_current_device(t) for t in on] == [False, True]
     assert not _native.on_current_device(torch.zeros(1))
+
+
+def _fake(*shape, dtype=torch.bfloat16):
+    """A tensor that says it is on a CUDA device and has no memory."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    with FakeTensorMode():
+        return torch.empty(shape, device="cuda", dtype=dtype)
+
+
+def _host():
+    from pithtrain_b200 import _native
+
+    if not _native._HOST_PATH.exists():
+        pytest.skip("the host library is not built")
+    return _native.host()
+
+
+def test_host_operators_refuse_operands_elsewhere():
+    """A weight, table or index on the host beside activations on the device is refused before anything reads it."""
+    h, cpu = _host(), lambda *s: torch.zeros(s, dtype=torch.bfloat16)  # noqa: E731
+    x, ids = _fake(8, 64), torch.zeros(8, 2, dtype=torch.int32)
+    w1, w2 = _fake(4, 128, 64), _fake(4, 64, 64)
+    calls = [
+        lambda: h.linear(x, cpu(64, 64), None, None, None),
+        lambda: h.linear(x, _fake(64, 64), cpu(64), None, None),
+        lambda: h.rmsnorm(x, cpu(64), 1e-6, None, False),
+        lambda: h.rmsnorm(x, _fake(64), 1e-6, cpu(8, 64), False),
+        lambda: h.qk_norm_rope(_fake(8, 192), cpu(64), cpu(64), _fake(8, 64), _fake(8, 64), None, 1, 1, 64, 1e-6, 8, False),
+        lambda: h.qk_norm_rope(_fake(8, 192), None, None, cpu(8, 64), cpu(8, 64), None, 1, 1, 64, 1e-6, 8, False),
+        lambda: h.qk_norm_rope(_fake(8, 192), None, None, _fake(8, 64), _fake(8, 64), torch.zeros(8, dtype=torch.int32), 1, 1, 64, 1e-6, 8, False),
+        lambda: h.attention(_fake(1, 8, 1, 64), cpu(1, 8, 1, 64), _fake(1, 8, 1, 64), None, None, 1.0, True, 0),
+        lambda: h.attention(_fake(1, 8, 1, 64), _fake(1, 8, 1, 64), _fake(1, 8, 1, 64), None, torch.zeros(8, dtype=torch.int32), 1.0, True, 0),
+        lambda: h.router(x, ids, 2, 0, True, 1.0),
+        lambda: h.moe_experts(x, _fake(8, 2), _fake(8, 2, dtype=torch.int32), w1.new_zeros(w1.shape, device="cpu"), w2, 16, 96, False, 1.0, 0.0, None),
+        lambda: h.moe_experts(x, _fake(8, 2), _fake(8, 2, dtype=torch.int32), w1, w2.new_zeros(w2.shape, device="cpu"), 16, 96, False, 1.0, 0.0, None),
+        lambda: h.wgrad_into(_fake(8, 64), _fake(8, 64), torch.zeros(64, 64), False),
+    ]
+    for call in calls:
+        with pytest.raises(RuntimeError, match="operands on cuda"):
+            call()
+    with pytest.raises(RuntimeError, match="must be on a CUDA device"):
+        h.linear(cpu(8, 64), cpu(64, 64), None, None, None)
+
+
+def test_host_operators_refuse_operands_without_memory():
+    h, x = _host(), _fake(8, 64)
+    for call in (lambda: h.linear(x, _fake(64, 64), None, None, None), lambda: h.rmsnorm(x, _fake(64), 1e-6, None, False), lambda: h.router_picks(x, 2),
+                 lambda: h.wgrad_into(x, x, _fake(64, 64, dtype=torch.float32), False)):
+        with pytest.raises(RuntimeError, match="no memory"):
+            call()
