@@ -227,6 +227,7 @@ py::object rmsnorm(const Tensor& x, const Tensor& w, double eps, const OptTensor
   const Tensor residual = opt(residual_);
   refuse_transforms({x, w, residual});
   check_operands(x, {w, residual});
+  TORCH_CHECK(x.size(-1) > 0, "rmsnorm: rows of no elements");
   auto node = make_node<RmsNormBackward>(x, w, residual);
   Tensor xc, h, y, rstd;
   {
@@ -304,7 +305,7 @@ Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, const py
   {
     Below guard;
     const int64_t K = w.size(1), N = w.size(0);
-    TORCH_CHECK(x.size(-1) == K, "linear: ", x.sizes(), " x ", w.sizes());
+    TORCH_CHECK(x.size(-1) == K && K > 0, "linear: ", x.sizes(), " x ", w.sizes());
     xc = x.contiguous();
     check_aligned(xc, "x");
     check_rows(w, "w");

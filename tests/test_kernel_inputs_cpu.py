@@ -69,7 +69,7 @@ def _fake(*shape, dtype=torch.bfloat16):
     from torch._subclasses.fake_tensor import FakeTensorMode
 
     with FakeTensorMode():
-        return torch.empty(shape, device="cuda", dtype=dtype)
+        return torch.empty((*shape[:-1], shape[-1] or 8), device="cuda", dtype=dtype)[..., : shape[-1]]  # no elements: of rows that have some
 
 
 def _host():
@@ -113,3 +113,13 @@ def test_host_operators_refuse_operands_without_memory():
                  lambda: h.wgrad_into(x, x, _fake(64, 64, dtype=torch.float32), False)):
         with pytest.raises(RuntimeError, match="no memory"):
             call()
+
+
+def test_host_operators_refuse_widths_of_zero():
+    """Rows of no elements have no number; dividing by their width ended the process."""
+    h = _host()
+    for x in (_fake(8, 0), _fake(0, 0)):
+        with pytest.raises(RuntimeError, match="linear"):
+            h.linear(x, _fake(64, 0), None, None, None)
+        with pytest.raises(RuntimeError, match="no elements"):
+            h.rmsnorm(x, _fake(0), 1e-6, None, False)
