@@ -63,8 +63,7 @@ _HOST_PATH = _LIB_PATH.with_name("pith_host_ops.so")
 
 
 @lru_cache(maxsize=1)
-def host():
-    """The operators whose host side is C++ (``csrc/host_ops.cpp``), bound to the kernels of :func:`lib`."""
+def _host_module():
     lib()
     if not _HOST_PATH.exists():
         raise NativeLibraryMissing(f"{_HOST_PATH} not found: run `python -m pithtrain_b200.build` (or __graft_entry__.build())")
@@ -73,6 +72,41 @@ def host():
     spec.loader.exec_module(module)
     module.bind(str(_LIB_PATH))
     return module
+
+
+class _TracedStep(torch.autograd.Function):
+    """A host operator as one step of a ``torch.jit.trace``. The tracer sees the allocations of a C++ operator, but not its kernels: a
+    trace of them alone would replay as unwritten memory. A Python function it records as a call."""
+
+    @staticmethod
+    def forward(ctx, op, *args):
+        needed = ctx.needs_input_grad[1:]
+        ctx.inputs = [a if a.is_leaf else a.detach().requires_grad_() for a, grad in zip(args, needed) if grad]
+        leaves = iter(ctx.inputs)
+        with torch.set_grad_enabled(bool(ctx.inputs)):
+            outs = op(*(next(leaves) if grad else a for a, grad in zip(args, needed)))
+        ctx.outs = outs if isinstance(outs, tuple) else (outs,)
+        ctx.set_materialize_grads(False)
+        given = tuple(None if o is None else o.detach() for o in ctx.outs)
+        ctx.mark_non_differentiable(*(g for g, o in zip(given, ctx.outs) if o is not None and not o.requires_grad))
+        return given if isinstance(outs, tuple) else given[0]
+
+    @staticmethod
+    def backward(ctx, *grads):
+        outs, grads = zip(*((o, g) for o, g in zip(ctx.outs, grads) if g is not None))
+        got = iter(torch.autograd.grad(outs, ctx.inputs, grads, retain_graph=True, allow_unused=True))
+        return None, *(next(got) if grad else None for grad in ctx.needs_input_grad[1:])
+
+
+class _TracedHost:
+    def __getattr__(self, name):
+        op = getattr(_host_module(), name)
+        return lambda *args: _TracedStep.apply(op, *args)
+
+
+def host():
+    """The operators whose host side is C++ (``csrc/host_ops.cpp``), bound to the kernels of :func:`lib`."""
+    return _host_module() if torch._C._get_tracing_state() is None else _TracedHost()
 
 
 SIGS = {
@@ -239,12 +273,12 @@ class _Module(types.ModuleType):
 
     @property
     def LAUNCHES(self) -> int:
-        return _launches + (host().launches() if host.cache_info().currsize else 0)
+        return _launches + (_host_module().launches() if _host_module.cache_info().currsize else 0)
 
     @LAUNCHES.setter
     def LAUNCHES(self, value: int) -> None:
         global _launches
-        _launches = value - (host().launches() if host.cache_info().currsize else 0)
+        _launches = value - (_host_module().launches() if _host_module.cache_info().currsize else 0)
 
 
 sys.modules[__name__].__class__ = _Module

@@ -1050,6 +1050,50 @@ def test_host_operators_in_autograd(name):
     _native.check_status()
 
 
+@pytest.mark.filterwarnings("ignore::DeprecationWarning", "ignore::torch.jit.TracerWarning")
+@pytest.mark.parametrize("name", ["linear", "rmsnorm", "rope", "router", "router after top k", "experts"])
+def test_host_operators_in_a_trace(name):
+    """``torch.jit.trace`` records each operator as a call: other inputs, of other numbers of rows too, give the operator's outputs and
+    gradients, not unwritten memory."""
+    from pithtrain_b200.ops.linear import linear
+    from pithtrain_b200.ops.moe import ExpertWeights, moe_experts
+    from pithtrain_b200.ops.norm import rmsnorm
+    from pithtrain_b200.ops.rope import qk_norm_rope
+    from pithtrain_b200.ops.router import router_topk
+
+    torch.manual_seed(27)
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    w, nw, hw, w1, w2 = mk(64, 128), mk(128), mk(64), mk(4, 128, 64), mk(4, 64, 64)  # constants of the trace
+    for t in (w, nw, hw):
+        t.main_grad = torch.zeros(t.shape, device="cuda")
+    cos, sin = mk(32, 64), mk(32, 64)
+    ew = ExpertWeights(w1, w2, lambda: torch.zeros(4, 128, 64, device="cuda"), lambda: torch.zeros(4, 64, 64, device="cuda"))
+    picks = lambda n: torch.randint(0, 4, (n, 2), dtype=torch.int32, device="cuda")  # noqa: E731
+    fn, inputs = {
+        "linear": (lambda x: linear(x, w), lambda n: [mk(n, 128)]),
+        "rmsnorm": (lambda x, r: rmsnorm(x, nw, 1e-6, r), lambda n: [mk(n, 128), mk(n, 128)]),
+        "rope": (lambda x: qk_norm_rope(x, hw, hw, cos, sin, 2, 1, 64, S=32), lambda n: [mk(n, 256)]),
+        "router": (lambda x: router_topk(x, 2, "softmax_topk", True), lambda n: [mk(n, 16).float()]),
+        "router after top k": (lambda x: router_topk(x, 2, "topk_softmax")[:2], lambda n: [mk(n, 16).float()]),
+        "experts": (lambda x, p, e: moe_experts(x, p, e, ew), lambda n: [mk(n, 64), torch.rand(n, 2, device="cuda"), picks(n)]),
+    }[name]
+    for grad in (False, True):
+        with torch.set_grad_enabled(grad):
+            example = lambda n: tuple(t.requires_grad_(grad and t.is_floating_point()) for t in inputs(n))  # noqa: E731
+            traced = torch.jit.trace(fn, example(9), check_trace=False)
+            for n in (9, 30, 1):
+                args = example(n)
+                leaves = [t for t in args if t.requires_grad]
+                want, got = ((o,) if isinstance(o, torch.Tensor) else o for o in (fn(*args), traced(*args)))
+                assert all(torch.equal(a, b) for a, b in zip(got, want))
+                if grad:
+                    dy = [torch.randn_like(o) if o.is_floating_point() else None for o in want]
+                    grads = [torch.autograd.grad([o for o in outs if o.requires_grad], leaves, [d for o, d in zip(outs, dy) if o.requires_grad], retain_graph=True)
+                             for outs in (want, got)]
+                    assert all(torch.equal(a, b) for a, b in zip(*grads))
+    _native.check_status()
+
+
 @pytest.mark.parametrize("flat", [False, True])
 @pytest.mark.parametrize("hooks", ["identity", "copy", "memory trace", "checkpoint"])
 def test_weight_gradients_under_saved_tensor_hooks(hooks, flat):
