@@ -16,8 +16,8 @@
 //   DQ : X1 = Q, X2 = dO  Y1 = K, Y2 = V     dQ += dS K
 //     S = X1 Y1^T, dP = X2 Y2^T -> TMEM (buffers of 64 columns each); P = exp2(S c - lse2), dS = P o (dP - delta);
 //     hi and mid go back over S's own columns in TMEM, lo over dP's, and are the A operand of the accumulating MMA (B = Y1 or
-//     Y2 read MN-major). With two buffers S and dP of step n+1 run under the exponentials of step n; where one CTA leaves room for
-//     another (head dims 64 and 128) there is one buffer, and the other CTA fills the tensor core meanwhile.
+//     Y2 read MN-major). With two buffers S and dP of step n+1 run under the exponentials of step n; where two CTAs share an SM
+//     (head dims 64 and 128, attn_split_launch) there is one buffer, and the other CTA fills the tensor core meanwhile.
 // Recomputing S twice and dP once and splitting costs 14 products of the tile instead of 5, all on the tensor core; the
 // tensor-op backward it replaces ran fp32 SIMT products over [heads, S, S] matrices in memory. Measured, causal, DQ + DK + DV, us
 // (before: two stages a streamed tile and a fixed order of the MMAs, binary searches for the row bounds, scalar fp32):
@@ -44,6 +44,7 @@ struct AttnSplitArgs {
   int B, Sq, Sk, Hq, Hkv;
   int Sp;                // row pitch of lse2 / delta: Sq rounded up to 4 (their tiles move in 16-byte pieces)
   int causal, q_off;
+  int reach;             // keys that a query sees, about: what the host knows of row_lo
   float scale_log2, out_scale;
   const int* row_lo;     // optional [B*Sq]
   const float* lse2;     // [B, Hq, Sp] log2-domain log-sum-exp (+inf for rows that saw no key)
@@ -53,21 +54,18 @@ struct AttnSplitArgs {
   int* err;
 };
 
-template <int D1, int D2, int MODE>
+template <int D1, int D2, int MODE, bool PAIRED>
 struct AttnSplitCfg {
   static constexpr bool HAS_DP = MODE != ASP_DV;
   static constexpr int DA = MODE == ASP_DV ? D2 : D1;     // columns of the accumulator
   static constexpr int X1_BYTES = (D1 / 64) * ASP_XSLAB, X2_BYTES = HAS_DP ? (D2 / 64) * ASP_XSLAB : 0;
   static constexpr int Y1_BYTES = (D1 / 64) * ASP_YSLAB, Y2_BYTES = (D2 / 64) * ASP_YSLAB;
-  // Two CTAs an SM where 256 TMEM columns hold the accumulator and one buffer of S and dP: the chain of a step (scores, softmax,
-  // split, accumulation) is then hidden by the other CTA, and so are the first loads and the last stores of a tile, which count
-  // where documents are short (8191 rows in 128 documents, 32/4 heads of 128: 149 + 180 + 162 us alone, 122 + 151 + 133 paired;
-  // one document of 3001 rows is even).
-  static constexpr bool PAIRED = D1 <= 128;
+  // PAIRED: two CTAs an SM (attn_split_launch says when), where 256 TMEM columns hold the accumulator and one buffer of S and dP.
+  static_assert(!PAIRED || D1 <= 128, "TMEM columns of two CTAs");
   static constexpr int NBUF = PAIRED ? 1 : 2;             // buffers of S and dP (64 columns each)
   static constexpr int T_DP = 64 * NBUF, T_ACC = 128 * NBUF, T_COLS = 256 * NBUF;
   // stages of the streamed tiles: what fits. Where only one of Y2 does, its only reader is the dP product (the scores of the
-  // step run meanwhile), or a partner CTA covers the load.
+  // step run meanwhile), or a partner CTA covers the load. (Alone at head dim 128, two of each: 9 to 18 % slower than four and three.)
   static constexpr int NST1 = PAIRED ? (D1 == 64 ? 4 : 2) : D1 + D2 <= 320 ? 4 : (HAS_DP ? 2 : 3);
   static constexpr int NST2 = PAIRED ? (D1 == 64 ? 3 : HAS_DP ? 1 : 2) : D1 + D2 <= 320 ? 3 : (HAS_DP ? 1 : 2);
   // lse2[64] | delta[64] (DV, DK): with each Y1 stage, or one copy that follows the steps where two CTAs share the memory
@@ -79,14 +77,13 @@ struct AttnSplitCfg {
   static constexpr int THREADS = 10 * 32;
 };
 
-template <int D1, int D2, int MODE>
-__global__ void __launch_bounds__(320, (AttnSplitCfg<D1, D2, MODE>::PAIRED ? 2 : 1))
+template <int D1, int D2, int MODE, bool PAIRED>
+__global__ void __launch_bounds__(320, (PAIRED ? 2 : 1))
 attn_bwd_split_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
                       const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2, const AttnSplitArgs args) {
-  using Cfg = AttnSplitCfg<D1, D2, MODE>;
+  using Cfg = AttnSplitCfg<D1, D2, MODE, PAIRED>;
   constexpr bool HAS_DP = Cfg::HAS_DP;
   constexpr int DA = Cfg::DA, NST1 = Cfg::NST1, NST2 = Cfg::NST2, NBUF = Cfg::NBUF;
-  constexpr bool PAIRED = Cfg::PAIRED;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if ((smem_u32(smem) & 1023u) != 0) {  // uniform over the CTA
@@ -558,9 +555,9 @@ struct SplitTensors {
   long long ldq, ldk, ldv, lddo;
 };
 
-template <int D1, int D2, int MODE>
-int attn_split_launch(const SplitTensors& t, const AttnSplitArgs& a, cudaStream_t stream) {
-  using Cfg = AttnSplitCfg<D1, D2, MODE>;
+template <int D1, int D2, int MODE, bool PAIRED>
+int attn_split_launch_as(const SplitTensors& t, const AttnSplitArgs& a, cudaStream_t stream) {
+  using Cfg = AttnSplitCfg<D1, D2, MODE, PAIRED>;
   constexpr bool DQ = MODE == ASP_DQ;
   // [B, S, cols] maps: rows past the end of a batch entry read zeros, never the next entry's rows (0 x inf is not 0)
   const uint64_t B = a.B, Sq = a.Sq, Sk = a.Sk;
@@ -569,12 +566,33 @@ int attn_split_launch(const SplitTensors& t, const AttnSplitArgs& a, cudaStream_
   if (encode_tmap_3d(&g, t.dout, TM_BF16, B, Sq, (uint64_t)a.Hq * D2, t.lddo, Sq * t.lddo, 1, DQ ? 128 : 64, 64, TM_SW_128)) return -3;
   if (encode_tmap_3d(&k, t.k, TM_BF16, B, Sk, (uint64_t)a.Hkv * D1, t.ldk, Sk * t.ldk, 1, DQ ? 64 : 128, 64, TM_SW_128)) return -3;
   if (encode_tmap_3d(&v, t.v, TM_BF16, B, Sk, (uint64_t)a.Hkv * D2, t.ldv, Sk * t.ldv, 1, DQ ? 64 : 128, 64, TM_SW_128)) return -3;
-  if (cudaFuncSetAttribute(attn_bwd_split_kernel<D1, D2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
+  if (cudaFuncSetAttribute(attn_bwd_split_kernel<D1, D2, MODE, PAIRED>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
     return -4;
   dim3 grid(a.Hq * a.B, ((DQ ? a.Sq : a.Sk) + 127) / 128);
-  if (DQ) attn_bwd_split_kernel<D1, D2, MODE><<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(q, g, k, v, a);
-  else attn_bwd_split_kernel<D1, D2, MODE><<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(k, v, q, g, a);
+  if (DQ) attn_bwd_split_kernel<D1, D2, MODE, PAIRED><<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(q, g, k, v, a);
+  else attn_bwd_split_kernel<D1, D2, MODE, PAIRED><<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(k, v, q, g, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+// Two CTAs an SM hide each other's steps, loads and stores, but share the tensor core and have one buffer of S and dP and fewer
+// stages each. So a CTA has its SM for itself up to one CTA an SM, and beyond that while its range of keys is long and the CTAs of an
+// SM are few; many or short ones come in pairs. Whole backward, causal, us, alone / paired:
+//   heads x 128, rows           CTAs   one document   4 documents   9          32
+//   16/4, 1023                   128    115 / 153      71 / 85       63 / 72
+//    8/2, 4093                   256    342 / 554     185 / 222     136 / 144  103 / 97
+//   16/4, 2049                   272    216 / 319     127 / 137     111 / 113   89 / 81
+//   16/4, 4093                   512    624 / 672     278 / 328     210 / 221  178 / 158
+//   64/8, 1023                   512    252 / 242     179 / 173     167 / 149
+//   32/4, 4093                  1024   1199 / 1173    513 / 498     375 / 360  306 / 269
+// Head dim 64: 98 / 138, 323 / 480, 201 / 274, 525 / 574, 207 / 201, 996 / 994 for one document.
+template <int D1, int D2, int MODE>
+int attn_split_launch(const SplitTensors& t, const AttnSplitArgs& a, cudaStream_t stream) {
+  if constexpr (D1 <= 128) {
+    const long long ctas = (long long)a.Hq * a.B * (((MODE == ASP_DQ ? a.Sq : a.Sk) + 127) / 128);
+    const long long sms = sm_count();
+    if (ctas > (a.reach >= 768 ? 4 * sms : a.reach >= 192 ? 2 * sms : sms)) return attn_split_launch_as<D1, D2, MODE, true>(t, a, stream);
+  }
+  return attn_split_launch_as<D1, D2, MODE, false>(t, a, stream);
 }
 
 template <int D1, int D2>
@@ -615,13 +633,14 @@ int attn_split_all(const SplitTensors& t, AttnSplitArgs a, const void* out, cons
 // delta, lse2: fp32 scratch of B*Hq*Sp + 128 elements each, Sp = Sq rounded up to 4, 16-byte aligned (delta holds the row sums
 // of dO*O afterwards, row pitch Sp). part: fp32 scratch [B*Sk, Hq, max(dqk, dv)] when Hq > Hkv, else null. dq / dk / dv
 // receive contiguous bf16 results.
-PT_API int pt_attn_bwd_split(const void* q, const void* k, const void* v, const void* out, const void* dout, const void* lse,
-                             const void* row_lo, void* dq, void* dk, void* dv, void* delta, void* lse2, void* part, int B, int Sq,
-                             int Sk, int Hq, int Hkv, int dqk, int dvd, long long ldq, long long ldk, long long ldv, long long ldo,
-                             long long lddo, float scale, int causal, int q_off, void* stream_) {
+// reach: about how many keys a query sees, for the choice between kernels (row_lo lies on the device); Sk if nothing is known.
+PT_API int pt_attn_bwd_split_reach(const void* q, const void* k, const void* v, const void* out, const void* dout, const void* lse,
+                                   const void* row_lo, void* dq, void* dk, void* dv, void* delta, void* lse2, void* part, int B, int Sq,
+                                   int Sk, int Hq, int Hkv, int dqk, int dvd, long long ldq, long long ldk, long long ldv, long long ldo,
+                                   long long lddo, float scale, int causal, int q_off, int reach, void* stream_) {
   if (B <= 0 || Sq <= 0 || Sk <= 0 || Hkv <= 0 || Hq % Hkv != 0 || scale <= 0.f) return -2;
   AttnSplitArgs a{};
-  a.B = B; a.Sq = Sq; a.Sk = Sk; a.Hq = Hq; a.Hkv = Hkv; a.causal = causal; a.q_off = q_off;
+  a.B = B; a.Sq = Sq; a.Sk = Sk; a.Hq = Hq; a.Hkv = Hkv; a.causal = causal; a.q_off = q_off; a.reach = reach;
   a.Sp = (Sq + 3) & ~3;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.row_lo = static_cast<const int*>(row_lo);
@@ -634,4 +653,12 @@ PT_API int pt_attn_bwd_split(const void* q, const void* k, const void* v, const 
   if (dqk == 192 && dvd == 128) return attn_split_all<192, 128>(t, a, out, lse, de, l2, pa, dq, dk, dv, ldo, scale, stream);
   if (dqk == 256 && dvd == 256) return attn_split_all<256, 256>(t, a, out, lse, de, l2, pa, dq, dk, dv, ldo, scale, stream);
   return -2;
+}
+
+PT_API int pt_attn_bwd_split(const void* q, const void* k, const void* v, const void* out, const void* dout, const void* lse,
+                             const void* row_lo, void* dq, void* dk, void* dv, void* delta, void* lse2, void* part, int B, int Sq,
+                             int Sk, int Hq, int Hkv, int dqk, int dvd, long long ldq, long long ldk, long long ldv, long long ldo,
+                             long long lddo, float scale, int causal, int q_off, void* stream_) {
+  return pt_attn_bwd_split_reach(q, k, v, out, dout, lse, row_lo, dq, dk, dv, delta, lse2, part, B, Sq, Sk, Hq, Hkv, dqk, dvd, ldq, ldk, ldv, ldo,
+                                 lddo, scale, causal, q_off, Sk, stream_);
 }

@@ -53,7 +53,7 @@ using F = float;
   X(pt_qk_norm_rope_bwd, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, L, L, I, P)                               \
   X(pt_attn_fwd, P, P, P, P, P, P, P, I, I, I, I, I, I, I, L, L, L, L, F, I, I, P)                                       \
   X(pt_attn_bwd, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, L, L, L, L, L, F, I, I, P)               \
-  X(pt_attn_bwd_split, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, L, L, L, L, L, F, I, I, P)            \
+  X(pt_attn_bwd_split_reach, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, L, L, L, L, L, F, I, I, I, P)   \
   X(pt_router_topk_fwd, P, I, P, P, P, I, I, I, I, I, F, P)                                                              \
   X(pt_router_given_fwd, P, I, P, P, P, I, I, I, I, F, P)                                                                \
   X(pt_router_topk_bwd, P, P, P, P, P, P, I, I, I, I, I, I, F, P)                                                        \
@@ -438,7 +438,7 @@ struct Grads {
 };
 
 Grads attention_backward(const Tensor& grad, const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& out_, const Tensor& lse_, double scale,
-                         bool causal, int64_t q_off, const Tensor& row_lo) {
+                         bool causal, int64_t q_off, const Tensor& row_lo, int64_t reach) {
   const Tensor q = as_token_major(q_), k = as_token_major(k_), v = as_token_major(v_), out = as_token_major(out_), lse = lse_.contiguous();
   // Unlike q, k and v the gradient comes to no tensor map that refuses a misaligned base or pitch
   Tensor d = as_token_major(grad);
@@ -467,9 +467,9 @@ Grads attention_backward(const Tensor& grad, const Tensor& q_, const Tensor& k_,
   float* delta = stats.data_ptr<float>();
   Tensor part;
   if (Hq != Hkv) part = empty({B * Sk * Hq * std::max(D, Dv)}, q, at::kFloat);
-  check(api.pt_attn_bwd_split(ptr(q), ptr(k), ptr(v), ptr(out), ptr(d), ptr(lse), ptr(row_lo), ptr(dq), ptr(dk), ptr(dv), delta, delta + ns + 128,
-                              ptr(part), B, Sq, Sk, Hq, Hkv, D, Dv, q.stride(1), k.stride(1), v.stride(1), out.stride(1), d.stride(1), sc, causal,
-                              q_off, current_stream()),
+  check(api.pt_attn_bwd_split_reach(ptr(q), ptr(k), ptr(v), ptr(out), ptr(d), ptr(lse), ptr(row_lo), ptr(dq), ptr(dk), ptr(dv), delta,
+                                    delta + ns + 128, ptr(part), B, Sq, Sk, Hq, Hkv, D, Dv, q.stride(1), k.stride(1), v.stride(1), out.stride(1),
+                                    d.stride(1), sc, causal, q_off, reach, current_stream()),
         "pt_attn_bwd_split", part.defined() ? 6 : 4);
   return {dq, dk, dv, stats.narrow(0, 0, ns).view({B, Hq, Sp}).narrow(2, 0, Sq)};
 }
@@ -478,7 +478,7 @@ struct AttentionBackward : Node {
   SavedVariable q, k, v, sinks, row_lo, out, lse;
   double scale = 0;
   bool causal = false;
-  int64_t q_off = 0;
+  int64_t q_off = 0, reach = 0;
 
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
@@ -486,7 +486,7 @@ struct AttentionBackward : Node {
     const Tensor qv = q.unpack(), kv = k.unpack(), vv = v.unpack(), sv = sinks.unpack(), rv = row_lo.unpack();
     const Tensor ov = out.unpack(shared_from_this()), lv = lse.unpack();
     Below guard;
-    Grads g = attention_backward(grads[0], qv, kv, vv, ov, lv, scale, causal, q_off, rv);
+    Grads g = attention_backward(grads[0], qv, kv, vv, ov, lv, scale, causal, q_off, rv, reach);
     Tensor ds;
     if (sv.defined())  // of the lse-normalised weight of the sink column, -exp(sink - lse) * delta, over batch and rows
       ds = ((sv.to(at::kFloat).view({1, -1, 1}) - lv).exp() * g.delta).sum(at::IntArrayRef{0, 2}).neg().to(sv.scalar_type());
@@ -498,9 +498,9 @@ struct AttentionBackward : Node {
   }
 };
 
-// out [B, Sq, Hq, Dv] bf16, lse [B, Hq, Sq] fp32 (not differentiable)
+// out [B, Sq, Hq, Dv] bf16, lse [B, Hq, Sq] fp32 (not differentiable); reach: about how many keys a query sees
 py::tuple attention(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& sinks_, const OptTensor& row_lo_, double scale, bool causal,
-                    int64_t q_off) {
+                    int64_t q_off, int64_t reach) {
   const Tensor sinks = opt(sinks_), row_lo = opt(row_lo_);
   refuse_transforms({q, k, v, sinks});
   check_operands(q, {k, v, sinks, row_lo});
@@ -526,7 +526,7 @@ py::tuple attention(const Tensor& q, const Tensor& k, const Tensor& v, const Opt
     node->row_lo = SavedVariable(row_lo, false);
     node->out = SavedVariable(out, true);
     node->lse = SavedVariable(lse, false);
-    node->scale = scale; node->causal = causal; node->q_off = q_off;
+    node->scale = scale; node->causal = causal; node->q_off = q_off; node->reach = reach;
   }
   return py::make_tuple(out, lse);
 }

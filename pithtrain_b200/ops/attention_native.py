@@ -176,7 +176,10 @@ def attention(q, k, v, causal, scale, window_left, sinks, cu_seqlens, return_lse
     row_lo = row_lower_bounds(B, Sq, q_off, window_left, cu_seqlens, q.device)
     from .. import _native
 
-    out, lse = _native.host().attention(q, k, v, sinks, row_lo, sc, bool(causal), int(q_off))
+    reach = Sk if cu_seqlens is None else B * Sq // max(1, cu_seqlens.numel() - 1)  # about how many keys a query sees
+    if window_left is not None and window_left >= 0:
+        reach = min(reach, int(window_left) + 1)
+    out, lse = _native.host().attention(q, k, v, sinks, row_lo, sc, bool(causal), int(q_off), min(int(reach), 2 ** 31 - 1))
     return (out, lse) if return_lse else out
 
 

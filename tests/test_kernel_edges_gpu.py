@@ -76,6 +76,24 @@ def test_attention_backward_split(Dqk, Dv, Hq, Hkv, B, Sq, Sk, causal, window, d
     assert _rel(got[3], want[3]) < 1e-5
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,S,Hq,Hkv,docs,window", [(1, 130, 148, 37, 1, None), (1, 130, 149, 149, 1, None), (5, 67, 64, 8, 1, None), (1, 130, 75, 25, 13, None),
+                                                    (1, 259, 50, 10, 1, 40), (1, 3, 300, 60, 1, None), (2, 1025, 33, 11, 1, None), (2, 770, 43, 43, 1, None)])
+def test_attention_backward_split_alone_and_paired(D, B, S, Hq, Hkv, docs, window):
+    """On both sides of the lines between one CTA an SM and two (148 SMs: 148, 296, 592 CTAs), by the number of CTAs and of keys a query sees."""
+    torch.manual_seed(S + Hq)
+    q, k, v = (torch.randn(B, S, h, D, device="cuda").bfloat16().requires_grad_() for h in (Hq, Hkv, Hkv))
+    cu = None if docs == 1 else torch.linspace(0, S, docs + 1).int().cuda()
+    out, lse = N.attention(q, k, v, True, None, window, None, cu, return_lse=True)
+    do = torch.randn_like(out)
+    got = torch.autograd.grad(out, (q, k, v), do)
+    row_lo = N.row_lower_bounds(B, S, 0, window, cu, q.device)
+    with torch.no_grad():
+        for a, b in zip(got, _backward64(do, q, k, v, out, lse, D ** -0.5, True, 0, row_lo)):
+            assert _rel(a, b) <= BF16_NORM
+    _native.check_status()
+
+
 @pytest.mark.parametrize("Dqk,Dv,Hq,Hkv", [(64, 64, 2, 1), (128, 128, 2, 1), (192, 128, 1, 1), (256, 256, 1, 1)])
 @pytest.mark.parametrize("Sq,docs", [(2113, 1), (2113, 40), (4201, 300), (2305, 2304)])
 def test_attention_backward_split_finds_its_tiles(Dqk, Dv, Hq, Hkv, Sq, docs):

@@ -93,8 +93,8 @@ def test_host_operators_refuse_operands_elsewhere():
         lambda: h.qk_norm_rope(_fake(8, 192), cpu(64), cpu(64), _fake(8, 64), _fake(8, 64), None, 1, 1, 64, 1e-6, 8, False),
         lambda: h.qk_norm_rope(_fake(8, 192), None, None, cpu(8, 64), cpu(8, 64), None, 1, 1, 64, 1e-6, 8, False),
         lambda: h.qk_norm_rope(_fake(8, 192), None, None, _fake(8, 64), _fake(8, 64), torch.zeros(8, dtype=torch.int32), 1, 1, 64, 1e-6, 8, False),
-        lambda: h.attention(_fake(1, 8, 1, 64), cpu(1, 8, 1, 64), _fake(1, 8, 1, 64), None, None, 1.0, True, 0),
-        lambda: h.attention(_fake(1, 8, 1, 64), _fake(1, 8, 1, 64), _fake(1, 8, 1, 64), None, torch.zeros(8, dtype=torch.int32), 1.0, True, 0),
+        lambda: h.attention(_fake(1, 8, 1, 64), cpu(1, 8, 1, 64), _fake(1, 8, 1, 64), None, None, 1.0, True, 0, 8),
+        lambda: h.attention(_fake(1, 8, 1, 64), _fake(1, 8, 1, 64), _fake(1, 8, 1, 64), None, torch.zeros(8, dtype=torch.int32), 1.0, True, 0, 8),
         lambda: h.router(x, ids, 2, 0, True, 1.0),
         lambda: h.moe_experts(x, _fake(8, 2), _fake(8, 2, dtype=torch.int32), w1.new_zeros(w1.shape, device="cpu"), w2, 16, 96, False, 1.0, 0.0, None),
         lambda: h.moe_experts(x, _fake(8, 2), _fake(8, 2, dtype=torch.int32), w1, w2.new_zeros(w2.shape, device="cpu"), 16, 96, False, 1.0, 0.0, None),
