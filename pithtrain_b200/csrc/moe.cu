@@ -333,7 +333,36 @@ embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const long long* __re
 
 // ----------------------------------------------------------------------------------------------
 // combine: out[t] = (res ? res[t] : 0) + sum_{j<k, row>=0} (w ? w[t,j] : 1) * y[row_of_slot[t*k+j]]
-// fp32 accumulation in slot order. Bound by the bytes of the rows, if enough of them are on their way: a row is contiguous, so
+// fp32 accumulation in slot order, in one of two kernels (pt_combine says when).
+// ----------------------------------------------------------------------------------------------
+// A warp a token, one row after the other: for many tokens of few or short rows.
+__global__ void __launch_bounds__(256)
+combine_warp_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_slot, const float* __restrict__ w,
+                    const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ out, const int* __restrict__ n_ptr, int n_max,
+                    int k, int H) {
+  const int n = n_ptr ? min(*n_ptr, n_max) : n_max;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int t = blockIdx.x * warps + (threadIdx.x >> 5); t < n; t += gridDim.x * warps) {
+    for (int c0 = lane * 8; c0 < H; c0 += 256) {
+      float acc[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+      if (res) load8(res + (size_t)t * H + c0, acc);
+      for (int j = 0; j < k; ++j) {
+        const int r = row_of_slot[(size_t)t * k + j];
+        if (r < 0) continue;
+        const float f = w ? w[(size_t)t * k + j] : 1.f;
+        float v[8];
+        load8(y + (size_t)r * H + c0, v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += f * v[e];
+      }
+      store8(out + (size_t)t * H + c0, acc);
+    }
+  }
+}
+
+// The ring. Bound by the bytes of the rows, if enough of them are on their way: a row is contiguous, so
 // one warp of the block fetches rows by bulk copies into a ring in shared memory, four rows of a token to a stage, a lane to a
 // row; the other warps add them up, a thread 8 columns wide. Rows in flight then cost shared memory and no registers. A block
 // has a run of tokens that follow one another, so that a load of 32 indices is several tokens' worth and is asked for one load
@@ -957,6 +986,30 @@ PT_API int pt_combine(const void* y, const int* row_of_slot, const float* w, con
   cudaStream_t st = (cudaStream_t)stream_;
   if (n_max <= 0) return 0;
   if (H % 8 != 0) return -1;
+  // Many tokens of few or short rows have more row loads than the ring's copies are worth: a warp a token asks for its row with all
+  // lanes, and there are warps enough. Measured, cold cache, us, ring / warp a token:
+  //   columns x k    1536 tokens   2560        4096        6144        12288       32768
+  //   512 x 1         9 / 8        10 / 8      10 / 8      12 / 8      16 / 11     31 / 17
+  //   2048 x 1       12 / 12       14 / 12     18 / 13     24 / 14     39 / 23     92 / 51
+  //   256 x 2         8 / 8        10 / 8      10 / 8      12 / 8      14 / 10     25 / 16
+  //   2048 x 2       12 / 18       14 / 18     19 / 18     25 / 21     43 / 35    100 / 80
+  //   4096 x 2       14 / 26       18 / 27     25 / 29     33 / 33     57 / 63    139 / 150
+  //   1536 x 3       12 / 19       14 / 19     18 / 21     23 / 21     37 / 35     82 / 80
+  //   512 x 4         9 / 12       10 / 12     12 / 12     14 / 12     21 / 18     39 / 38
+  //   1024 x 4       10 / 16       12 / 17     14 / 18     18 / 18     29 / 31     64 / 70
+  //   256 x 8        10 / 12       12 / 12     12 / 12     14 / 12     23 / 18     41 / 37
+  //   512 x 8        11 / 16       12 / 16     14 / 16     18 / 18     27 / 29     59 / 65
+  //   256 x 16       12 / 16       15 / 16     16 / 16     20 / 18     33 / 29     68 / 62
+  const long long cols = (long long)k * H;
+  const bool short_rows = (k <= 3 && cols <= 1024 && n_max >= 1536) ||
+                          (k == 1   ? n_max >= 2560
+                           : k == 2 ? n_max > 3072 && (cols <= 4608 || H > CB_COLS)
+                                    : n_max > 4096 && (cols <= (k == 3 ? 4608 : 3072) || H <= 256));
+  if (short_rows) {
+    combine_warp_kernel<<<grid_for(n_max, 8, 16), 256, 0, st>>>((const __nv_bfloat16*)y, row_of_slot, w, (const __nv_bfloat16*)res, (__nv_bfloat16*)out,
+                                                                n_ptr, n_max, k, H);
+    return (int)cudaGetLastError();
+  }
   const int pieces = H / 8, W = (pieces + (pieces + 511) / 512 - 1) / ((pieces + 511) / 512) * 8, slices = (H + W - 1) / W;
   const int adders = (W / 8 + 31) / 32;
   // Some sixteen adding warps an SM, in two to sixteen blocks, share 200 KB of rings: 3 to 8 stages each. Rows wider than the 2048
@@ -968,7 +1021,7 @@ PT_API int pt_combine(const void* y, const int* row_of_slot, const float* w, con
   //   2048 x 4           9 -> 8     16 -> 12  25 -> 16  33 -> 21  34 -> 25  59 -> 38   66 -> 51
   //   2880 x 4          10 -> 8     21 -> 14  33 -> 20  45 -> 25  47 -> 30  84 -> 49   90 -> 70
   //    512 x 8          11 -> 8     12 -> 10  17 -> 13  18 -> 15  19 -> 16  33 -> 23   37 -> 31
-  const int blocks = adders > 8 ? 2 : 16 / adders;
+  const int blocks = adders > 8 ? 2 : (16 + adders / 2) / adders;
   const int stage_bytes = CB_ROWS * W * 2, room = 200 * 1024 / blocks / stage_bytes, stages = room < CB_STAGES ? room : CB_STAGES;
   static bool configured = false;
   if (!configured) {

@@ -501,6 +501,13 @@ def test_combine_rows_runs_and_slices(n, H, k):
     assert (got[::5] == 0).all()
 
 
+@pytest.mark.parametrize("n,H,k", [(1535, 8, 3), (1536, 8, 3), (1536, 344, 3), (2559, 2056, 1), (2560, 2056, 1), (3072, 2304, 2), (3073, 2304, 2), (3073, 2312, 2),
+                                   (3073, 4104, 2), (4096, 768, 4), (4097, 768, 4), (4097, 1536, 3), (4097, 72, 40), (4097, 264, 12), (20001, 264, 1)])
+def test_combine_rows_of_either_kernel(n, H, k):
+    """On both sides of the lines between the ring and a warp a token."""
+    test_combine_rows_runs_and_slices(n, H, k)
+
+
 @pytest.mark.parametrize("pair", [False, True])
 @pytest.mark.parametrize("sizes,N,K", [([16], 8, 8), ([0, 16, 80], 136, 40), ([48, 0, 0, 64], 264, 296), ([32] * 40, 392, 776)])
 def test_grouped_weight_gradient_into_fp32(sizes, N, K, pair):
