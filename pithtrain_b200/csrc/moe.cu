@@ -307,26 +307,48 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict_
 }
 
 // ----------------------------------------------------------------------------------------------
-// embedding gradient: grad[ids[r]] += dy[r], fp32 from bf16. Bound by the rows of dy once and the touched rows of grad twice; a warp
-// walks a row, 8 columns a lane in two four-wide reductions, which the L2 performs, so that equal ids need no order. An id outside
-// the table is recorded and skipped.
+// embedding gradient: grad[ids[r]] += dy[r], fp32 from bf16. Bound by the rows of dy once and the touched rows of grad twice. A warp
+// has 256 columns of EB_ROWS rows that follow one another, 8 columns a lane in two four-wide reductions, which the L2 performs, so
+// that equal ids need no order; those of neighbours (padding) are added up first, since reductions of one address wait for one
+// another. An id outside the table is recorded and skipped.
 // ----------------------------------------------------------------------------------------------
+constexpr int EB_ROWS = 8;
+
 __global__ void __launch_bounds__(256)
 embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const long long* __restrict__ ids, float* __restrict__ grad, int n, int H,
                      long long V, int* __restrict__ err) {
-  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  for (int r = blockIdx.x * warps + (threadIdx.x >> 5); r < n; r += gridDim.x * warps) {
-    const long long id = ids[r];
-    if (id < 0 || id >= V) {
-      if (lane == 0) atomicCAS(err, 0, PT_ERR_BOUNDS);
-      continue;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5, slices = (H + 255) / 256;
+  const long long items = (long long)((n + EB_ROWS - 1) / EB_ROWS) * slices;
+  for (long long item = (long long)blockIdx.x * warps + (threadIdx.x >> 5); item < items; item += (long long)gridDim.x * warps) {
+    const int r0 = (int)(item / slices) * EB_ROWS, c = (int)(item % slices) * 256 + lane * 8;
+    long long mine = lane < EB_ROWS && r0 + lane < n ? ids[r0 + lane] : -1;
+    if (mine < 0 || mine >= V) {
+      if (lane < EB_ROWS && r0 + lane < n) atomicCAS(err, 0, PT_ERR_BOUNDS);
+      mine = -1;
     }
-    for (int c = lane * 8; c < H; c += 256) {
-      float v[8];
-      load8(dy + (size_t)r * H + c, v);
-      float* g = grad + (size_t)id * H + c;
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g + 4), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+    uint4 row[EB_ROWS];
+#pragma unroll
+    for (int i = 0; i < EB_ROWS; ++i)
+      if (r0 + i < n && c < H) row[i] = *reinterpret_cast<const uint4*>(dy + (size_t)(r0 + i) * H + c);
+    float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    long long id = __shfl_sync(0xffffffffu, mine, 0);
+#pragma unroll
+    for (int i = 0; i < EB_ROWS; ++i) {
+      const long long next = i + 1 < EB_ROWS ? __shfl_sync(0xffffffffu, mine, (i + 1) % EB_ROWS) : -1;
+      if (id >= 0 && c < H) {
+        float v[8];
+        load8(reinterpret_cast<const __nv_bfloat16*>(&row[i]), v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sum[e] += v[e];
+        if (next != id) {
+          float* g = grad + (size_t)id * H + c;
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g), "f"(sum[0]), "f"(sum[1]), "f"(sum[2]), "f"(sum[3]) : "memory");
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g + 4), "f"(sum[4]), "f"(sum[5]), "f"(sum[6]), "f"(sum[7]) : "memory");
+#pragma unroll
+          for (int e = 0; e < 8; ++e) sum[e] = 0.f;
+        }
+      }
+      id = next;
     }
   }
 }
@@ -973,11 +995,14 @@ PT_API int pt_gather_rows(const void* src, const int* idx, int div, void* dst, c
   return (int)cudaGetLastError();
 }
 
-// Into a table of 9496 x 2048: 4096 rows 77 -> 20 us, 256 rows 15 -> 9 us, against a conversion of dy and an indexed addition of one element a thread.
+// Cold cache, us, 2048 columns into 32000 rows: a conversion of dy and an indexed addition of one element a thread -> here (one row a
+// warp, without adding up neighbours -> here): 4096 random ids 77 -> 21 (21), 256: 15 -> 8; 4096 times one id 77 -> 18 (150), 16384: 309
+// -> 51 (533); 700 of every 1024 rows one id, 16384 rows 312 -> 53 (192). What is left to the L2's queue: two ids at random,
+// 16384 rows of 64 columns 48 -> 53 (90).
 PT_API int pt_embedding_bwd(const void* dy, const long long* ids, float* grad, int n, int H, long long V, void* stream_) {
   if (n <= 0 || H <= 0) return 0;
   if (H % 8 != 0) return -1;
-  embedding_bwd_kernel<<<grid_for(n, 8, 8), 256, 0, (cudaStream_t)stream_>>>((const __nv_bfloat16*)dy, ids, grad, n, H, V, device_status_word());
+  embedding_bwd_kernel<<<grid_for((long long)((n + EB_ROWS - 1) / EB_ROWS) * ((H + 255) / 256), 8, 8), 256, 0, (cudaStream_t)stream_>>>((const __nv_bfloat16*)dy, ids, grad, n, H, V, device_status_word());
   return (int)cudaGetLastError();
 }
 

@@ -1330,6 +1330,25 @@ def test_embedding_gradient(n, V, H):
     _native.check_status()
 
 
+@pytest.mark.parametrize("n,H", [(1, 8), (7, 264), (8, 256), (9, 64), (203, 520), (4099, 2048)])
+def test_embedding_gradient_of_equal_neighbours(n, H):
+    """Runs of one id within and across a warp's eight rows, ids outside the table among them (recorded, skipped, and no end of a run),
+    a last warp of fewer rows."""
+    torch.manual_seed(n)
+    V = 5
+    ids = torch.randint(0, V, (n,), device="cuda").repeat_interleave(torch.randint(1, 14, (n,), device="cuda"))[:n].contiguous()
+    if n > 8:
+        ids[torch.rand(n, device="cuda") < 0.1] = V  # outside
+    dy, start = torch.randn(n, H, device="cuda").bfloat16(), torch.randn(V, H, device="cuda")
+    grad = start.clone()
+    _native.check(_native.lib().pt_embedding_bwd(dy.data_ptr(), ids.data_ptr(), grad.data_ptr(), n, H, V, _native.stream_ptr()), "pt_embedding_bwd")
+    assert bool(_native.fetch_status()) == bool((ids == V).any())
+    want, size, inside = start.double(), start.double().abs(), ids < V
+    want.index_add_(0, ids[inside], dy[inside].double())
+    size.index_add_(0, ids[inside], dy[inside].double().abs())
+    assert ((grad.double() - want).abs() <= 2.0 ** -24 * (n + 1) * size).all()  # n fp32 additions at most, in any order
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 5120, 2048), (3, 136, 72), (64, 128, 64), (64, 2048, 4096), (64, 9496, 520), (65, 264, 1032), (127, 2048, 512), (128, 648, 4096),
                                    (129, 128, 2048), (200, 2048, 4096), (300, 376, 1024), (1000, 128, 2048), (64, 20000, 128)])
 def test_dense_few_rows(M, N, K):
