@@ -561,14 +561,28 @@ extern "C" int pt_gemm_bf16(const void* A, const void* B, void* D, int mode, int
                             const int* offs, int num_groups, int b_group_rows, long long d_group_stride, int out_fp32, int accumulate,
                             int use_tma_store, int epi, int bn, int max_ctas, const int* a_idx, int a_idx_div, long long a_idx_len, void* stream_);
 
+// Pairs cut the rows of D into 256, the single-CTA kernel of csrc/gemm.cu into 128: just past a whole number of pair tiles it can need
+// a wave less, which counts while the waves are few. Cold cache, us, pair / single, waves: input gradients: 1025 rows of [2048, 4096]
+// 31 / 23 (2 / 1), 3329: 54 / 51 (4 / 3), 4609: 68 / 66 (5 / 4), 6913: 90 / 93 (7 / 6); 4609 rows of [10944, 2048] 182 / 148 (3 / 2);
+// fp32 weight gradients of 4096 rows: [1032, 4096] 55 / 38 (2 / 1), [4616, 4096] 133 / 127 (5 / 4), [2056, 10944] 162 / 162 (6 / 5).
+namespace {
+bool fewer_waves_alone(long long rows, long long cols) {
+  using namespace pt;
+  const long long n_tiles = (cols + T2_BN - 1) / T2_BN, sms = sm_count(), slots = sms / 2 > 0 ? sms / 2 : 1;
+  const long long pairs = ((rows + 2 * T2_BM - 1) / (2 * T2_BM) * n_tiles + slots - 1) / slots;
+  const long long alone = ((rows + T2_BM - 1) / T2_BM * n_tiles + sms - 1) / sms;
+  return alone < pairs && pairs <= 5;
+}
+}  // namespace
+
 // dy [M, N], w [N, K] -> out [M, K] bf16, reduction over N (input gradient of a dense layer). K a multiple of 8.
-// Reductions below 512 take the single-CTA kernel: the launch of the pair costs what its tiles save (64 and 128 columns 9 us for
+// Reductions below 512 and products of fewer waves there take the single-CTA kernel: the launch of the pair costs what its tiles save (64 and 128 columns 9 us for
 // 11, from 512 on even or behind: csrc/gemm.cu 40, here 35 at 512 rows of [5120, 2048]).
 PT_API int pt_dense_nn(const void* dy, const void* w, void* out, int M, int K, int N, long long lda, long long ldb, long long ldd,
                        void* stream_) {
   using namespace pt;
   if (M <= 0 || N <= 0 || K <= 0 || K % 8 != 0) return -2;
-  if (N < 512)
+  if (N < 512 || fewer_waves_alone(M, K))
     return pt_gemm_bf16(dy, w, out, 0, M, K, N, 0, 1, M, N, lda, N, K, ldb, M, ldd, nullptr, 0, 0, 0, 0, 0, 1, 2, 0, 0, nullptr, 1, 0, stream_);
   Gemm2Args a = t2_args(M, K, N, 1);
   return t2_launch<false, true, T2_STORE>({dy, M, N, lda, lda * M}, {w, N, K, ldb, ldb * N}, {out, M, K, ldd, ldd * M}, a,
@@ -576,14 +590,15 @@ PT_API int pt_dense_nn(const void* dy, const void* w, void* out, int M, int K, i
 }
 
 // dy [M, N], x [M, K] -> D [N, K] += dy^T x in fp32 or bf16 (weight gradient of a dense layer). N and K multiples of 8.
-// fp32_sums: the error of an fp32 product, at about half the rate. Other reductions below 1024 rows take the single-CTA kernel
+// fp32_sums: the error of an fp32 product, at about half the rate. Other reductions below 1024 rows, and products of fewer waves
+// there, take the single-CTA kernel
 // ([5120, 2048] into fp32, single / pair: 64 rows 24 / 28 us, 512 rows 31 / 32, 2048 rows 57 / 51). Launches that add to the same
 // elements are ordered by the caller, as for pt_gemm_bf16.
 PT_API int pt_dense_tn(const void* dy, const void* x, void* D, int out_fp32, int fp32_sums, int N, int K, int M, long long lda,
                        long long ldb, long long ldd, void* stream_) {
   using namespace pt;
   if (M <= 0 || N <= 0 || K <= 0 || N % 8 != 0 || K % 8 != 0) return -2;
-  if (!fp32_sums && M < 1024)
+  if (!fp32_sums && (M < 1024 || fewer_waves_alone(N, K)))
     return pt_gemm_bf16(dy, x, D, 0, N, K, M, 1, 1, M, N, lda, M, K, ldb, N, ldd, nullptr, 0, 0, 0, out_fp32, 1, 1, 2, 0, 0, nullptr, 1, 0,
                         stream_);
   Gemm2Args a = t2_args(N, K, M, 1);

@@ -1369,6 +1369,26 @@ def test_dense_few_rows(M, N, K):
     _native.check_status()
 
 
+@pytest.mark.parametrize("M,N,K", [(1024, 512, 4096), (1025, 512, 4096), (1152, 520, 4104), (1281, 512, 4096), (300, 584, 10944), (4616, 1032, 264)])
+def test_dense_gradients_of_fewer_waves(M, N, K):
+    """Just past a whole wave of 256-row tiles and beyond what 128-row tiles save: input gradients [M, K], weight gradients [M, K] of
+    1024 rows and more."""
+    from pithtrain_b200.ops import gemm as G
+
+    torch.manual_seed(M)
+    m = (M + 7) // 8 * 8  # rows of a weight: a multiple of 8
+    for R in (N, 1024 + N):
+        dy, w = torch.randn(M, R, device="cuda").bfloat16(), torch.randn(R, K, device="cuda").bfloat16()
+        want, size = dy.double() @ w.double(), dy.double().abs() @ w.double().abs()
+        slack = 2.0 ** -22 * (R // 16 + 9) * size  # the tensor core cuts sums off at 24 bits or so, R / 16 times at most
+        assert ((G.gemm_nn(dy, w).double() - want).abs() <= BF16_MAX * want.abs() + slack).all()
+        dyt = torch.zeros(R, m, device="cuda").bfloat16()
+        dyt[:, :M] = dy.t()
+        grad = G.gemm_tn(dyt, w, out=torch.zeros(m, K, device="cuda"), accumulate=True)
+        assert ((grad[:M].double() - want).abs() <= slack).all() and not grad[M:].any()
+    _native.check_status()
+
+
 @pytest.mark.parametrize("extra", [False, True])
 @pytest.mark.parametrize("n,H", [(1, 8), (591, 2048), (592, 2056), (593, 4096), (1185, 520), (1777, 6152), (3, 8192)])
 def test_rmsnorm_backward_rows(n, H, extra):
