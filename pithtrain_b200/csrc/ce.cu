@@ -153,14 +153,15 @@ PT_API int pt_cross_entropy(void* logits, const long long* labels, float* loss, 
   // Cold cache, us, before (1024 threads and two reads for every row) -> now, and one read and one write at 6.5 TB/s. 4096 rows:
   // 1000 columns 37 -> 12 (3), 4096: 44 -> 18 (10), 8192: 53 -> 31 (21), 9496: 61 -> 42 (24), 12288: 63 -> 45 (31), 15520: 74 -> 59 (39).
   // 2048 rows: 20000 columns 46 -> 37 (25), 32000: 60 -> 51 (40), 50304: 87 -> 86 (63), 151936: 265 -> 252 (192); the last four read
-  // their rows twice, up to 32768 columns by 512 threads (by 1024: 47 and 57 us).
+  // their rows twice, up to 32768 columns by 512 threads (by 1024: 47 and 57 us) where there are more rows than SMs.
   const int nvec = V / 8;
   if (nvec <= 128 * 2) return launch(cross_entropy_kernel<128, 2>, 128);
   if (nvec <= 128 * 4) return launch(cross_entropy_kernel<128, 4>, 128);
   if (nvec <= 256 * 4) return launch(cross_entropy_kernel<256, 4>, 256);
   if (nvec <= 512 * 3) return launch(cross_entropy_kernel<512, 3>, 512);
   if (nvec <= 512 * 4) return launch(cross_entropy_kernel<512, 4>, 512);
-  if (nvec <= 4096) return launch(cross_entropy_kernel<512, 0>, 512);
+  // A row alone on its SM wants all the loads it can have on their way: 32000 columns, 1 to 148 rows, 512 / 1024 threads 12.3 / 10.2.
+  if (nvec <= 4096 && n > sm_count()) return launch(cross_entropy_kernel<512, 0>, 512);
   return launch(cross_entropy_kernel<1024, 0>, 1024);
 }
 
