@@ -544,13 +544,8 @@ int attn_fwd_launch_t(const void* q, const void* k, const void* v, const AttnArg
   if (encode_tmap_2d(&tmQ, q, TM_BF16, rows, (uint64_t)a.Hq * DQK, ldq, 128, 64, TM_SW_128)) return -3;
   if (encode_tmap_2d(&tmK, k, TM_BF16, kv_rows, (uint64_t)a.Hkv * DQK, ldk, 128, 64, TM_SW_128)) return -3;
   if (encode_tmap_2d(&tmV, v, TM_BF16, kv_rows, (uint64_t)a.Hkv * DV, ldv, 128, 64, TM_SW_128)) return -3;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel<DQK, DV, NQ, KST>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) !=
-        cudaSuccess)
-      return -4;
-    configured = true;
-  }
+  static SmemLimit smem;
+  if (smem.set(attn_fwd_kernel<DQK, DV, NQ, KST>, Cfg::SMEM) != cudaSuccess) return -4;
   const int nQ = (a.Sq + 127) / 128;
   dim3 grid(a.Hq * a.B, (nQ + NQ - 1) / NQ);
   attn_fwd_kernel<DQK, DV, NQ, KST><<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(tmQ, tmK, tmV, a);

@@ -595,11 +595,8 @@ int attn_bwd_launch_t(const void* q, const void* k, const void* v, const void* o
   if (encode_tmap_2d(&tmDQ, dq_acc, TM_F32, rows, (uint64_t)a.Hq * D, (uint64_t)a.Hq * D, 32, 32, TM_SW_128)) return -3;
   if (encode_tmap_2d(&tmDK, dk_acc, TM_F32, kv_rows, (uint64_t)a.Hkv * D, (uint64_t)a.Hkv * D, 32, 32, TM_SW_128)) return -3;
   if (encode_tmap_2d(&tmDV, dv_acc, TM_F32, kv_rows, (uint64_t)a.Hkv * D, (uint64_t)a.Hkv * D, 32, 32, TM_SW_128)) return -3;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attn_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess) return -4;
-    configured = true;
-  }
+  static SmemLimit smem;
+  if (smem.set(attn_bwd_kernel<D>, Cfg::SMEM) != cudaSuccess) return -4;
   {
     constexpr int TPR = D / 8;
     const long long threads = (long long)a.B * a.Sq * a.Hq * TPR;

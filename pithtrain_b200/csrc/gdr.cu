@@ -292,12 +292,12 @@ PT_API int pt_gdr_state_fwd(const float* w, const float* u, const float* qg, con
   dim3 grid(BH, dv / GD_VS);
   const int smem = (dk * GD_VS + GD_C * dk + GD_C * GD_VS) * (int)sizeof(float);
   if (dk == 128) {
-    static bool cfg = false;
-    if (!cfg) { if (cudaFuncSetAttribute(gdr_state_fwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4; cfg = true; }
+    static SmemLimit limit;
+    if (limit.set(gdr_state_fwd_kernel<128>, smem) != cudaSuccess) return -4;
     gdr_state_fwd_kernel<128><<<grid, GD_THREADS, smem, st>>>(p);
   } else {
-    static bool cfg = false;
-    if (!cfg) { if (cudaFuncSetAttribute(gdr_state_fwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4; cfg = true; }
+    static SmemLimit limit;
+    if (limit.set(gdr_state_fwd_kernel<64>, smem) != cudaSuccess) return -4;
     gdr_state_fwd_kernel<64><<<grid, GD_THREADS, smem, st>>>(p);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
@@ -314,12 +314,12 @@ PT_API int pt_gdr_state_bwd(const float* w, const float* qg, const float* kd, co
   dim3 grid(BH, dv / GD_VS);
   const int smem = (2 * dk * GD_VS + GD_C * dk + 2 * GD_C * GD_VS) * (int)sizeof(float);
   if (dk == 128) {
-    static bool cfg = false;
-    if (!cfg) { if (cudaFuncSetAttribute(gdr_state_bwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4; cfg = true; }
+    static SmemLimit limit;
+    if (limit.set(gdr_state_bwd_kernel<128>, smem) != cudaSuccess) return -4;
     gdr_state_bwd_kernel<128><<<grid, GD_THREADS, smem, st>>>(p);
   } else {
-    static bool cfg = false;
-    if (!cfg) { if (cudaFuncSetAttribute(gdr_state_bwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4; cfg = true; }
+    static SmemLimit limit;
+    if (limit.set(gdr_state_bwd_kernel<64>, smem) != cudaSuccess) return -4;
     gdr_state_bwd_kernel<64><<<grid, GD_THREADS, smem, st>>>(p);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;

@@ -664,12 +664,8 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMa
                 const CUtensorMap* tmB2 = nullptr) {
   auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, A_GATHER, DEEP_EPI>;
   constexpr int smem = gemm_smem_bytes<BN, DEEP_EPI>();
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const cudaError_t e = limit.set(kern, smem)) return (int)e;
   kern<<<grid, 192, smem, stream>>>(tmA, tmB, tmD, tmA2 ? *tmA2 : tmA, tmB2 ? *tmB2 : tmB, args);
   return (int)cudaGetLastError();
 }

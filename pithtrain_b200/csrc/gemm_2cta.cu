@@ -521,11 +521,8 @@ int t2_launch(const T2Mat& A, const T2Mat& B, const T2Mat& D, Gemm2Args& a, cuda
   a.err = device_status_word();
   auto kern = gemm2cta_kernel<A_MN, B_MN, EPI, EW>;
   constexpr int smem = t2_smem_bytes<EPI, EW>();
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (limit.set(kern, smem) != cudaSuccess) return -4;
   const long long m_tiles = (a.M + 2 * T2_BM - 1) / (2 * T2_BM), n_tiles = (a.N + T2_BN - 1) / T2_BN;
   const long long tiles = a.batch * (EPI == T2_FUSED && a.sym ? m_tiles * (m_tiles + 1) / 2 : m_tiles * n_tiles);
   if (tiles > 0x3fffffffLL) return -2;

@@ -336,12 +336,8 @@ PT_API int pt_gemm_fp8(const void* A, const void* B, void* D, int mode, int M, i
     if (tiles < grid) grid = (int)tiles;
   }
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const cudaError_t e = limit.set(gemm_fp8_kernel, SMEM_BYTES)) return (int)e;
   gemm_fp8_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(tmA, tmB, tmD, args);
   return (int)cudaGetLastError();
 }

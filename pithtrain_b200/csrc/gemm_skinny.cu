@@ -159,11 +159,8 @@ static int skinny_launch(const void* x, const void* w, SkinnyArgs a, long long l
   CUtensorMap tmW, tmX;
   if (encode_tmap_2d(&tmW, w, TM_BF16, a.N, a.K, ldb, SK_BW, SK_BK, TM_SW_128)) return -3;
   if (encode_tmap_2d(&tmX, x, TM_BF16, a.M, a.K, lda, TN, SK_BK, TM_SW_128)) return -3;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_skinny_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM) != cudaSuccess) return -4;
-    configured = true;
-  }
+  static SmemLimit smem;
+  if (smem.set(gemm_skinny_kernel<TN>, SK_SMEM) != cudaSuccess) return -4;
   const int n_tiles = (a.N + SK_BW - 1) / SK_BW, m_tiles = (a.M + TN - 1) / TN, num_kb = (a.K + SK_BK - 1) / SK_BK;
   // As many CTAs as are resident at once (two an SM, a few left over where clusters do not fit), two k-blocks or more for each.
   int split = (int)(sm_count() * 2LL * 7 / 8 / ((long long)n_tiles * m_tiles));

@@ -7,6 +7,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #define PT_API extern "C" __attribute__((visibility("default")))
 
 namespace pt {
@@ -15,6 +17,24 @@ namespace pt {
 int* device_status_word();
 // Number of SMs of the current device (cached).
 int sm_count();
+
+// A kernel's dynamic shared memory beyond 48 KB has to be asked for on each device; a static SmemLimit beside the launch remembers where.
+class SmemLimit {
+ public:
+  template <class Kernel>
+  cudaError_t set(Kernel* kernel, int bytes) {
+    int dev = 0;
+    if (const cudaError_t e = cudaGetDevice(&dev)) return e;
+    const uint64_t bit = uint64_t(1) << (dev & 63);
+    if (dev < 64 && (done_.load(std::memory_order_relaxed) & bit)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done_.fetch_or(bit, std::memory_order_relaxed);
+    return e;
+  }
+
+ private:
+  std::atomic<uint64_t> done_{0};
+};
 
 enum TmDtype { TM_BF16 = 0, TM_F32 = 1, TM_U8 = 2, TM_F16 = 3, TM_I32 = 4 };
 enum TmSwizzle { TM_SW_NONE = 0, TM_SW_32 = 1, TM_SW_64 = 2, TM_SW_128 = 3 };

@@ -911,12 +911,8 @@ PT_API int pt_route_sort(const int* eids, const int* n_ptr, int n_max, int E, in
   if (E <= 0 || n_max < 0 || align <= 0 || r_cap < 0) return -1;
   if (E <= RS_MAX_E) {
     const int smem = (RS_WARPS + 2) * E * (int)sizeof(int);
-    static bool configured = false;
-    if (!configured) {
-      const cudaError_t e = cudaFuncSetAttribute(route_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (RS_WARPS + 2) * RS_MAX_E * (int)sizeof(int));
-      if (e != cudaSuccess) return (int)e;
-      configured = true;
-    }
+    static SmemLimit limit;
+    if (const cudaError_t e = limit.set(route_sort_kernel, (RS_WARPS + 2) * RS_MAX_E * (int)sizeof(int))) return (int)e;
     route_sort_kernel<<<RS_CTAS, RS_WARPS * 32, smem, st>>>(eids, n_ptr, n_max, E, align, offs, row_of_slot, slot_of_row, r_cap, device_status_word());
     return (int)cudaGetLastError();
   }
@@ -1048,12 +1044,8 @@ PT_API int pt_combine(const void* y, const int* row_of_slot, const float* w, con
   //    512 x 8          11 -> 8     12 -> 10  17 -> 13  18 -> 15  19 -> 16  33 -> 23   37 -> 31
   const int blocks = adders > 8 ? 2 : (16 + adders / 2) / adders;
   const int stage_bytes = CB_ROWS * W * 2, room = 200 * 1024 / blocks / stage_bytes, stages = room < CB_STAGES ? room : CB_STAGES;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const cudaError_t e = limit.set(combine_kernel, 100 * 1024)) return (int)e;
   combine_kernel<<<grid_for((long long)n_max * slices, 1, blocks), adders * 32 + 32, stages * stage_bytes, st>>>(
       (const __nv_bfloat16*)y, row_of_slot, w, (const __nv_bfloat16*)res, (__nv_bfloat16*)out, n_ptr, n_max, k, H, slices, W, stages,
       device_status_word());

@@ -123,3 +123,39 @@ def test_host_operators_refuse_widths_of_zero():
             h.linear(x, _fake(64, 0), None, None, None)
         with pytest.raises(RuntimeError, match="no elements"):
             h.rmsnorm(x, _fake(0), 1e-6, None, False)
+
+
+def test_shared_memory_is_asked_for_on_each_device(tmp_path):
+    """A kernel of one translation unit on three devices, against a runtime that only counts; a refusal is passed on and tried again."""
+    import shutil
+    import subprocess
+    from pathlib import Path
+
+    import pithtrain_b200
+
+    if shutil.which("g++") is None or not Path("/usr/local/cuda/include/cuda_runtime.h").exists():
+        pytest.skip("no compiler or no CUDA headers")
+    csrc = Path(pithtrain_b200.__file__).parent / "csrc"
+    assert not any("static bool" in line and "false" in line for f in csrc.glob("*.cu") for line in f.read_text().splitlines())
+    (tmp_path / "t.cpp").write_text("""
+#include "host_common.h"
+static int device = 0, asked = 0;
+static cudaError_t answer = cudaSuccess;
+extern "C" cudaError_t cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
+extern "C" cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { ++asked; return answer; }
+void kernel(int) {}
+int main() {
+  static pt::SmemLimit limit;
+  for (int round = 0; round < 2; ++round)
+    for (device = 0; device < 3; ++device)
+      if (limit.set(kernel, 1 << 16) != cudaSuccess) return 1;
+  if (asked != 3) return 2;
+  static pt::SmemLimit other;
+  answer = cudaErrorInvalidValue;
+  if (other.set(kernel, 1 << 16) != cudaErrorInvalidValue) return 3;
+  answer = cudaSuccess;
+  return other.set(kernel, 1 << 16) == cudaSuccess && asked == 5 ? 0 : 4;
+}
+""")
+    subprocess.run(["g++", "-std=c++17", f"-I{csrc}", "-I/usr/local/cuda/include", str(tmp_path / "t.cpp"), "-o", str(tmp_path / "t")], check=True)
+    assert subprocess.run([str(tmp_path / "t")]).returncode == 0
