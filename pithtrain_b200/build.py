@@ -4,12 +4,14 @@ Every ``csrc/*.cu`` file is compiled to an object with
 ``-gencode arch=compute_100a,code=sm_100a -lineinfo`` and linked into
 ``pithtrain_b200/_lib/libpithb200.so``, which :mod:`pithtrain_b200._native` loads with ctypes. ``csrc/host_ops.cpp`` (the host side
 of the operators that run in every layer, with torch's headers) becomes ``_lib/pith_host_ops.so``.
-Objects are rebuilt only when their source (or a header) is newer.
+Objects are rebuilt only when their source (or a header) is newer; the host library also when its compiler command or torch, to
+whose C++ ABI it is bound, is another one (``_lib/pith_host_ops.txt`` says of which it is).
 """
 
 from __future__ import annotations
 
 import os
+import shutil
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -40,6 +42,11 @@ def _nvcc() -> str:
     return cand if os.path.exists(cand) else "nvcc"
 
 
+def _cuda_include() -> Path:
+    """Headers of the toolkit that nvcc belongs to."""
+    return Path(shutil.which(_nvcc()) or "/usr/local/cuda/bin/nvcc").resolve().parent.parent / "include"
+
+
 def _newest_header_mtime() -> float:
     return max((p.stat().st_mtime for p in list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))), default=0.0)
 
@@ -56,9 +63,21 @@ def host_ops_command(out: Path) -> list:
 
     # nvcc's host compiler, not $CXX: one that links its own libstdc++ in cannot share exceptions and streams with torch's
     return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=pith_host_ops",
-            *(f"-I{p}" for p in cpp_extension.include_paths()), "-I/usr/local/cuda/include", f"-I{sysconfig.get_paths()['include']}",
+            *(f"-I{p}" for p in cpp_extension.include_paths()), f"-I{_cuda_include()}", f"-I{sysconfig.get_paths()['include']}",
             str(CSRC / "host_ops.cpp"), "-o", str(out), f"-L{cpp_extension.library_paths()[0]}",
             "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python"]
+
+
+def _host_ops_stamp(cmd: list) -> str:
+    import torch
+
+    return f"torch {torch.__version__}\n{' '.join(cmd)}\n"
+
+
+def host_ops_stale(out: Path, src: Path, cmd: list) -> bool:
+    stamp = out.with_suffix(".txt")
+    return (not out.exists() or out.stat().st_mtime < src.stat().st_mtime
+            or not stamp.exists() or stamp.read_text() != _host_ops_stamp(cmd))
 
 
 def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False, bounds_check: bool = False) -> Path:
@@ -80,8 +99,9 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False, 
             jobs.append((src, cmd))
 
     host_out, host_src = LIBDIR / "pith_host_ops.so", CSRC / "host_ops.cpp"
-    if force or not host_out.exists() or host_out.stat().st_mtime < host_src.stat().st_mtime:
-        jobs.append((host_src, host_ops_command(host_out)))
+    host_cmd = host_ops_command(host_out)
+    if force or host_ops_stale(host_out, host_src, host_cmd):
+        jobs.append((host_src, host_cmd))
 
     def run(job):
         src, cmd = job
@@ -94,7 +114,9 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False, 
                 if verbose or ptxas_info or res.returncode != 0:
                     sys.stderr.write(f"[build] {src.name}\n{res.stdout}{res.stderr}\n")
                 if res.returncode != 0:
-                    raise RuntimeError(f"nvcc failed for {src}")
+                    raise RuntimeError(f"compiler failed for {src}")
+                if src == host_src:
+                    host_out.with_suffix(".txt").write_text(_host_ops_stamp(host_cmd))
     out = LIBDIR / "libpithb200_checked.so" if bounds_check else lib_path()
     objs = [str(objdir / (s.stem + ".o")) for s in sources]
     need_link = any(src.suffix == ".cu" for src, _ in jobs) or not out.exists()

@@ -481,6 +481,27 @@ def test_gated_delta_rule_chunked_equals_the_recurrence(S, chunk):
         assert torch.allclose(a, b, atol=5e-4, rtol=1e-3), float((a - b).abs().max())
 
 
+def test_host_library_is_rebuilt_for_another_torch_or_command(tmp_path, monkeypatch):
+    import os
+
+    import torch
+
+    from pithtrain_b200 import build
+
+    src, out = tmp_path / "host_ops.cpp", tmp_path / "pith_host_ops.so"
+    src.write_text("")
+    cmd = build.host_ops_command(out)
+    assert any(a.startswith("-I") and os.path.exists(os.path.join(a[2:], "cuda_runtime.h")) for a in cmd)
+    assert build.host_ops_stale(out, src, cmd)
+    out.write_text("")
+    assert build.host_ops_stale(out, src, cmd)  # of an unknown command
+    out.with_suffix(".txt").write_text(build._host_ops_stamp(cmd))
+    assert not build.host_ops_stale(out, src, cmd)
+    assert build.host_ops_stale(out, src, [*cmd, "-g"])
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    assert build.host_ops_stale(out, src, cmd)
+
+
 def test_new_entry_points_validate_their_arguments_on_the_host():
     """Shape errors are refused with -2 before any CUDA call; valid shapes get as far as the tensor-map encoder, which
     has no driver here and reports -3 — neither path launches or crashes without a GPU."""
