@@ -184,6 +184,7 @@ SIGS = {
     "pt_packed_positions": "PIPLP",
     "pt_row_lower_bounds": "PIPIIIIP",
     "pt_attn_bwd_split": "PPPPPPPPPPPPP" + "IIIIIII" + "LLLLL" + "F" + "II" + "P",
+    "pt_attn_bwd_split_reach": "PPPPPPPPPPPPP" + "IIIIIII" + "LLLLL" + "F" + "III" + "P",
     "pt_attn_bwd": "PPPPPPPPPPPPPPP" + "IIIIII" + "LLLLL" + "F" + "II" + "P",
     "pt_gemm2cta_nt": "PPPIIILLLP",
     "pt_dense_nn": "PPPIIILLLP",
