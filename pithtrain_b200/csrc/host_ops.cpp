@@ -3,8 +3,8 @@
 //
 // These run once or more per layer and micro-batch. From Python an operator spent 5 to 8 us in its launches and 15 to 30 us around
 // them (argument checks, views, autograd.Function, ctypes): without gradients an RMSNorm took 19 us and takes 7, a linear layer 24
-// and 8. Two micro-batches of 512 tokens through four narrow layers (forward and backward, 441 launches) 13.7 -> 7.2 ms, the 64-token
-// forward of two Qwen3 layers 2.87 -> 1.49 ms, of which the device works 1.36.
+// and 8. Two micro-batches of 512 tokens through four narrow layers (forward and backward, some 400 launches) 13.7 -> 7.2 ms, the
+// 64-token forward of two Qwen3 layers 2.87 -> 1.45 ms, of which the device works 1.17.
 //
 // The kernels stay in libpithb200.so; their entry points are looked up by name (bind) in the library that Python has loaded. What
 // a user can replace or observe is asked from Python when it is needed: the gradient buffer of a parameter (main_grad, else .grad)

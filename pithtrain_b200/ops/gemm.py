@@ -23,7 +23,8 @@ from .. import _native
 
 DENSE, MGROUP, KGROUP = 0, 1, 2
 
-# Module-level switches used by tests and tuning runs.
+# Module-level switches used by tests and tuning runs. They reach what goes through :func:`_launch`: grouped products, and dense ones
+# that are not on the 2-CTA kernel (USE_2CTA below). The C++ operators (csrc/host_ops.cpp) do not read them.
 USE_TMA_STORE = True
 FORCE_BN = 0
 # accumulate epilogue: 0 = staged coalesced read-modify-write, 1 = per-thread rows, 2 = TMA reduce-add
@@ -59,9 +60,10 @@ def _chk2d(t: torch.Tensor, name: str):
     assert t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0, f"{name} must be 16-byte aligned"
 
 
-# Dense products run on the 2-CTA kernel of csrc/gemm_2cta.cu (few rows: csrc/gemm_skinny.cu), whose CTA pair shares each B tile: at 4096 rows and the models'
-# projection shapes 7 to 16 % faster than the single-CTA family in all three forms (us, single / pair: [5120, 2048] 77 / 66 NT,
-# 75 / 67 NN, 91 / 82 TN into fp32; [10944, 2048] 146 / 122, 144 / 126, 151 / 134).
+# Dense products run on the 2-CTA kernel of csrc/gemm_2cta.cu, whose CTA pair shares each B tile (few rows: csrc/gemm_skinny.cu, so that
+# the order of a row's fp32 sums depends on the number of rows): at 4096 rows and the models' projection shapes 7 to 16 % faster
+# than the single-CTA family in all three forms (us, single / pair: [5120, 2048] 77 / 66 NT, 75 / 67 NN, 91 / 82 TN into fp32;
+# [10944, 2048] 146 / 122, 144 / 126, 151 / 134). Gradients that need fewer waves there keep the single-CTA family.
 USE_2CTA = True
 
 

@@ -23,7 +23,7 @@ def _rand(*shape):
 @pytest.mark.parametrize("M,N,K", [(128, 128, 64), (256, 256, 128), (384, 512, 192), (1000, 776, 328),
                                    (4096, 2048, 2048), (130, 136, 72)])
 def test_dense_nt(M, N, K, tma_store):
-    G.USE_TMA_STORE = tma_store
+    G.USE_TMA_STORE, G.USE_2CTA = tma_store, tma_store  # without it: the single-CTA kernel, the one that has the choice
     torch.manual_seed(0)
     x, w = _rand(M, K), _rand(N, K)
     out = G.gemm_nt(x, w)
@@ -31,19 +31,19 @@ def test_dense_nt(M, N, K, tma_store):
     ref = x.float() @ w.float().t()
     assert calc_diff(out.float(), ref) < 1e-4
     assert torch.allclose(out.float(), ref, atol=0.25, rtol=2e-2)
-    G.USE_TMA_STORE = True
+    G.USE_TMA_STORE = G.USE_2CTA = True
 
 
 @pytest.mark.parametrize("bn", [128, 256])
 def test_dense_bn(bn):
-    G.FORCE_BN = bn
+    G.FORCE_BN, G.USE_2CTA = bn, False  # the single-CTA kernel, which has two widths
     try:
         x, w = _rand(512, 256), _rand(512, 256)
         out = G.gemm_nt(x, w)
         _native.check_status()
         assert calc_diff(out.float(), x.float() @ w.float().t()) < 1e-4
     finally:
-        G.FORCE_BN = 0
+        G.FORCE_BN, G.USE_2CTA = 0, True
 
 
 @pytest.mark.parametrize("M,N,K", [(256, 256, 128), (1000, 776, 328), (4096, 4096, 2048)])
@@ -56,9 +56,9 @@ def test_dense_nn(M, N, K):
 
 @pytest.fixture(params=[0, 1, 2])
 def acc_epilogue(request):
-    G.ACC_EPILOGUE = request.param
+    G.ACC_EPILOGUE, G.USE_2CTA = request.param, False  # the single-CTA kernel, whose epilogues these are
     yield request.param
-    G.ACC_EPILOGUE = 2
+    G.ACC_EPILOGUE, G.USE_2CTA = 2, True
 
 
 @pytest.mark.parametrize("M,N,K", [(256, 256, 128), (1000, 776, 328), (4096, 512, 2048)])
@@ -75,6 +75,18 @@ def test_dense_tn(M, N, K, acc_epilogue):
     accb = ref.to(torch.bfloat16)
     G.gemm_tn(dy, x, out=accb, accumulate=True)
     assert calc_diff(accb.float(), 2 * ref) < 1e-4
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 128), (1000, 776, 328), (1024, 776, 328), (4096, 512, 2048)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_dense_tn_by_rows(M, N, K, dtype):
+    """Accumulation as ``gemm_tn`` runs it by default: reductions below 1024 rows on the single-CTA kernel, from there on CTA pairs."""
+    dy, x = _rand(M, N), _rand(M, K)
+    ref = dy.float().t() @ x.float()
+    acc = ref.to(dtype).clone()
+    G.gemm_tn(dy, x, out=acc, accumulate=True)
+    _native.check_status()
+    assert calc_diff(acc.float(), 2 * ref) < (1e-5 if dtype == torch.float32 else 1e-4)
 
 
 def _offsets(sizes):
