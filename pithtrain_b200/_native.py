@@ -63,7 +63,8 @@ _HOST_PATH = _LIB_PATH.with_name("pith_host_ops.so")
 
 
 @lru_cache(maxsize=1)
-def _host_module():
+def host():
+    """The operators whose host side is C++ (``csrc/host_ops.cpp``), bound to the kernels of :func:`lib`."""
     lib()
     if not _HOST_PATH.exists():
         raise NativeLibraryMissing(f"{_HOST_PATH} not found: run `python -m pithtrain_b200.build` (or __graft_entry__.build())")
@@ -98,15 +99,9 @@ class _TracedStep(torch.autograd.Function):
         return None, *(next(got) if grad else None for grad in ctx.needs_input_grad[1:])
 
 
-class _TracedHost:
-    def __getattr__(self, name):
-        op = getattr(_host_module(), name)
-        return lambda *args: _TracedStep.apply(op, *args)
-
-
-def host():
-    """The operators whose host side is C++ (``csrc/host_ops.cpp``), bound to the kernels of :func:`lib`."""
-    return _host_module() if torch._C._get_tracing_state() is None else _TracedHost()
+def _traced(name: str, *args):
+    """What a host operator calls in its place while a trace is recorded."""
+    return _TracedStep.apply(getattr(host(), name), *args)
 
 
 SIGS = {
@@ -274,12 +269,12 @@ class _Module(types.ModuleType):
 
     @property
     def LAUNCHES(self) -> int:
-        return _launches + (_host_module().launches() if _host_module.cache_info().currsize else 0)
+        return _launches + (host().launches() if host.cache_info().currsize else 0)
 
     @LAUNCHES.setter
     def LAUNCHES(self, value: int) -> None:
         global _launches
-        _launches = value - (_host_module().launches() if _host_module.cache_info().currsize else 0)
+        _launches = value - (host().launches() if host.cache_info().currsize else 0)
 
 
 sys.modules[__name__].__class__ = _Module

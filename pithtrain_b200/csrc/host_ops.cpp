@@ -17,9 +17,9 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
-#include <algorithm>
 #include <atomic>
 
 namespace {
@@ -91,19 +91,24 @@ P ptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
 // helpers
 // ------------------------------------------------------------------------------------------------
 // A custom operator without a vmap or jvp rule refuses transformed and dual inputs, as autograd.Function does.
-void refuse_transforms(std::initializer_list<Tensor> inputs) {
+void refuse_transforms(std::initializer_list<const Tensor*> inputs) {
   TORCH_CHECK(!c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode),
               "this operator does not support functorch transforms (vmap, grad, jvp, jacrev, ...)");
-  for (const Tensor& t : inputs)
-    TORCH_CHECK_NOT_IMPLEMENTED(!t.defined() || !t._fw_grad(0).defined(), "forward-mode differentiation is not implemented for this operator");
+  for (const Tensor* t : inputs)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(0).defined(), "forward-mode differentiation is not implemented for this operator");
 }
 // The kernels take raw pointers. Operands on the host or on different devices are refused, and those without memory of their own
 // (fake tensors, subclasses that wrap others).
-void check_operands(const Tensor& x, std::initializer_list<Tensor> others) {
+void check_operands(const Tensor& x, std::initializer_list<const Tensor*> others) {
   TORCH_CHECK(x.is_cuda(), "the first operand must be on a CUDA device, is on ", x.device());
-  for (const Tensor& t : others) TORCH_CHECK(!t.defined() || t.device() == x.device(), "operands on ", x.device(), " and ", t.device());
-  const auto has_memory = [](const Tensor& t) { return !t.defined() || t.numel() == 0 || t.const_data_ptr() != nullptr; };
-  TORCH_CHECK(has_memory(x) && std::all_of(others.begin(), others.end(), has_memory), "an operand has no memory");
+  const auto has_memory = [](const Tensor& t) { return t.const_data_ptr() != nullptr || t.numel() == 0; };
+  bool memory = has_memory(x);
+  for (const Tensor* t : others) {
+    if (!t->defined()) continue;
+    TORCH_CHECK(t->device() == x.device(), "operands on ", x.device(), " and ", t->device());
+    memory = memory && has_memory(*t);
+  }
+  TORCH_CHECK(memory, "an operand has no memory");
 }
 Tensor opt(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 Tensor empty(at::IntArrayRef sizes, const Tensor& like, at::ScalarType type) { return at::empty(sizes, like.options().dtype(type)); }
@@ -180,6 +185,18 @@ void accumulate_colsum_pair(const Tensor& p0, const Tensor& p1, const Tensor& pa
         "pt_colsum_accumulate_pair");
 }
 
+// While a torch.jit.trace is recorded, an operator hands itself to Python, which makes one step of the trace of it.
+thread_local bool in_traced_step = false;
+template <class R, class... A>
+R traced(const char* name, const A&... args) {
+  struct Step {
+    Step() { in_traced_step = true; }
+    ~Step() { in_traced_step = false; }
+  } step;
+  return python("pithtrain_b200._native", "_traced")(name, args...).template cast<R>();
+}
+bool tracing() { return torch::jit::tracer::isTracing() && !in_traced_step; }
+
 template <class N, class... T>
 std::shared_ptr<N> make_node(const T&... inputs) {
   if (!torch::autograd::compute_requires_grad(inputs...)) return nullptr;
@@ -224,9 +241,10 @@ struct RmsNormBackward : Node {
 };
 
 py::object rmsnorm(const Tensor& x, const Tensor& w, double eps, const OptTensor& residual_, bool zero_centered) {
+  if (tracing()) return traced<py::object>("rmsnorm", x, w, eps, residual_, zero_centered);
   const Tensor residual = opt(residual_);
-  refuse_transforms({x, w, residual});
-  check_operands(x, {w, residual});
+  refuse_transforms({&x, &w, &residual});
+  check_operands(x, {&w, &residual});
   TORCH_CHECK(x.size(-1) > 0, "rmsnorm: rows of no elements");
   auto node = make_node<RmsNormBackward>(x, w, residual);
   Tensor xc, h, y, rstd;
@@ -297,9 +315,10 @@ struct LinearBackward : Node {
 
 // x [..., K], w [N, K]; the weight gradient goes where grad_getter() says, the bias gradient to bias_param.
 Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, const py::object& grad_getter, const py::object& bias_param) {
+  if (tracing()) return traced<Tensor>("linear", x, w, bias_, grad_getter, bias_param);
   const Tensor bias = opt(bias_);
-  refuse_transforms({x, w, bias});
-  check_operands(x, {w, bias});
+  refuse_transforms({&x, &w, &bias});
+  check_operands(x, {&w, &bias});
   auto node = make_node<LinearBackward>(x, w, bias);
   Tensor xc, y;
   {
@@ -330,7 +349,7 @@ Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, const py
 void wgrad_into(const Tensor& dy, const Tensor& x, const Tensor& target, bool fp32_sums) {
   check_rows(dy, "dy");
   check_rows(x, "x");
-  check_operands(dy, {x, target});
+  check_operands(dy, {&x, &target});
   check(api.pt_dense_tn(ptr(dy), ptr(x), target.data_ptr(), target.scalar_type() == at::kFloat, fp32_sums, dy.size(1), x.size(1), dy.size(0),
                         dy.stride(0), x.stride(0), target.stride(0), current_stream()),
         "pt_dense_tn");
@@ -376,9 +395,11 @@ struct QkNormRopeBackward : Node {
 
 py::tuple qk_norm_rope(const Tensor& qkv_, const OptTensor& q_w_, const OptTensor& k_w_, const Tensor& cos_, const Tensor& sin_,
                        const OptTensor& positions, int64_t Hq, int64_t Hkv, int64_t D, double eps, int64_t S, bool zero_centered) {
+  if (tracing()) return traced<py::tuple>("qk_norm_rope", qkv_, q_w_, k_w_, cos_, sin_, positions, Hq, Hkv, D, eps, S, zero_centered);
   const Tensor q_w = opt(q_w_), k_w = opt(k_w_);
-  refuse_transforms({qkv_, q_w, k_w});
-  check_operands(qkv_, {q_w, k_w, cos_, sin_, opt(positions)});
+  refuse_transforms({&qkv_, &q_w, &k_w});
+  const Tensor positions_ = opt(positions);
+  check_operands(qkv_, {&q_w, &k_w, &cos_, &sin_, &positions_});
   auto node = make_node<QkNormRopeBackward>(qkv_, q_w, k_w);
   Tensor qkv = qkv_, cos, sin, q, k, v, rq, rk, pos;
   {
@@ -466,7 +487,7 @@ Grads attention_backward(const Tensor& grad, const Tensor& q_, const Tensor& k_,
   Tensor stats = empty({2 * (ns + 128)}, q, at::kFloat);  // read in whole 64-row tiles: padded
   float* delta = stats.data_ptr<float>();
   Tensor part;
-  if (Hq != Hkv) part = empty({B * Sk * Hq * std::max(D, Dv)}, q, at::kFloat);
+  if (Hq != Hkv) part = empty({B * Sk * Hq * (D > Dv ? D : Dv)}, q, at::kFloat);
   check(api.pt_attn_bwd_split_reach(ptr(q), ptr(k), ptr(v), ptr(out), ptr(d), ptr(lse), ptr(row_lo), ptr(dq), ptr(dk), ptr(dv), delta,
                                     delta + ns + 128, ptr(part), B, Sq, Sk, Hq, Hkv, D, Dv, q.stride(1), k.stride(1), v.stride(1), out.stride(1),
                                     d.stride(1), sc, causal, q_off, reach, current_stream()),
@@ -501,9 +522,10 @@ struct AttentionBackward : Node {
 // out [B, Sq, Hq, Dv] bf16, lse [B, Hq, Sq] fp32 (not differentiable); reach: about how many keys a query sees
 py::tuple attention(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& sinks_, const OptTensor& row_lo_, double scale, bool causal,
                     int64_t q_off, int64_t reach) {
+  if (tracing()) return traced<py::tuple>("attention", q, k, v, sinks_, row_lo_, scale, causal, q_off, reach);
   const Tensor sinks = opt(sinks_), row_lo = opt(row_lo_);
-  refuse_transforms({q, k, v, sinks});
-  check_operands(q, {k, v, sinks, row_lo});
+  refuse_transforms({&q, &k, &v, &sinks});
+  check_operands(q, {&k, &v, &sinks, &row_lo});
   auto node = make_node<AttentionBackward>(q, k, v, sinks);
   Tensor out, lse;
   {
@@ -567,8 +589,10 @@ struct RouterBackward : Node {
 
 // (weights [n, k] fp32, picks [n, k] int32, probabilities [n, E] fp32 or None); given: the picks, else they are the top k
 py::tuple router(const Tensor& logits, const OptTensor& given, int64_t k, int64_t mode, bool renorm, double scale) {
-  refuse_transforms({logits});
-  check_operands(logits, {opt(given)});
+  if (tracing()) return traced<py::tuple>("router", logits, given, k, mode, renorm, scale);
+  refuse_transforms({&logits});
+  const Tensor picks = opt(given);
+  check_operands(logits, {&picks});
   auto node = make_node<RouterBackward>(logits);
   Tensor probs, idx, w;
   const int64_t n = logits.size(0), E = logits.size(1);
@@ -603,7 +627,8 @@ py::tuple router(const Tensor& logits, const OptTensor& given, int64_t k, int64_
 
 // The top k alone, [n, k] int32: what a replay of the routing is handed.
 Tensor router_picks(const Tensor& logits, int64_t k) {
-  refuse_transforms({logits});
+  if (tracing()) return traced<Tensor>("router_picks", logits, k);
+  refuse_transforms({&logits});
   check_operands(logits, {});
   Below guard;
   const Tensor lg = logits.contiguous();
@@ -692,7 +717,7 @@ void expert_wgrads(const Tensor& dyg, const Tensor& act, const Tensor& dgu, cons
     const int64_t R = dy.size(0), N = dy.size(1), K = a.size(1), E = g.size(0);
     TORCH_CHECK(g.dim() == 3 && g.size(1) == N && g.size(2) == K && g.is_contiguous(), "expert_wgrads: gradient buffer ", g.sizes());
     check_aligned(g, "the gradient buffer");
-    check_operands(dy, {g});
+    check_operands(dy, {&g});
     check(api.pt_gemm_bf16(ptr(dy), ptr(a), g.data_ptr(), 2, N, K, 0, 1, 1, R, N, dy.stride(0), R, K, a.stride(0), N, K, ptr(offs), E, 0, N * K,
                            g.scalar_type() == at::kFloat, 1, 1, 2, 0, 0, nullptr, 1, 0, current_stream()),
           "pt_gemm_bf16");
@@ -704,8 +729,9 @@ void expert_wgrads(const Tensor& dyg, const Tensor& act, const Tensor& dgu, cons
 // out[t] = sum_j w[t, j] * expert_{eids[t, j]}(x[t]); x [n, H], w and eids [n, k], w1 [E, 2I, H], w2 [E, H, I]
 Tensor moe_experts(const Tensor& x, const Tensor& w, const Tensor& eids, const Tensor& w1, const Tensor& w2, int64_t align, int64_t r_cap,
                    bool interleaved, double alpha, double limit, const py::object& queue_wgrad) {
-  refuse_transforms({x, w, w1, w2});
-  check_operands(x, {w, eids, w1, w2});
+  if (tracing()) return traced<Tensor>("moe_experts", x, w, eids, w1, w2, align, r_cap, interleaved, alpha, limit, queue_wgrad);
+  refuse_transforms({&x, &w, &w1, &w2});
+  check_operands(x, {&w, &eids, &w1, &w2});
   auto node = make_node<ExpertsBackward>(x, w);
   Tensor gu, out, offs, row_of_slot, slot_of_row;
   const int64_t n = eids.size(0), k = eids.size(1), E = w1.size(0), slots = n * k;
